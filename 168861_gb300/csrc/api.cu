@@ -151,13 +151,14 @@ HHKey hh_key(const nrt_problem &p, int32_t k) {
 
 }  // namespace
 
-int build_host_pack(const nrt_problem *probs, int32_t count, HostPack &hp) {
+int build_host_pack(const nrt_problem *probs, int32_t count, HostPack &hp, int align) {
   hp.ninst = count;
   hp.off.assign(count + 1, 0);
   hp.hh_off.assign(count + 1, 0);
   std::vector<int64_t> term_off(count + 1, 0);
   for (int32_t i = 0; i < count; i++) {
-    hp.off[i + 1] = hp.off[i] + probs[i].num_elem;
+    // every instance starts on a multiple of `align` elements, and ntot is one
+    hp.off[i + 1] = (hp.off[i] + probs[i].num_elem + align - 1) / align * align;
     hp.hh_off[i + 1] = hp.hh_off[i] + probs[i].num_hh;
     term_off[i + 1] = term_off[i] + probs[i].num_term;
   }
@@ -230,6 +231,13 @@ int build_host_pack(const nrt_problem *probs, int32_t count, HostPack &hp) {
       hp.Wfull[o + j] = p.W[j];
       hp.Kfull[o + j] = p.K[j];
       hp.gate[o + j] = hp.gate[N + o + j] = hp.gate[2 * N + o + j] = 0.0;
+    }
+    for (int64_t e = o + n; e < hp.off[i + 1]; e++) {  // padding: part of no tree
+      hp.topo[e] = Topo{(int32_t)e, (int32_t)e, (int32_t)e, F_TERM | ((uint32_t)i << INST_SHIFT)};
+      cls[e] = 0;
+      hp.cdt[e] = hp.gax[e] = hp.wdx[e] = hp.kdx[e] = hp.inp[e] = hp.V0[e] = hp.V1[e] = 0.0;
+      hp.c_m_dx[e] = hp.radx[e] = hp.Wfull[e] = hp.Kfull[e] = 0.0;
+      hp.gate[e] = hp.gate[N + e] = hp.gate[2 * N + e] = 0.0;
     }
     for (int32_t q = 0; q < p.num_term; q++) {
       const int32_t t = p.terminals[q];
@@ -372,7 +380,7 @@ int Engine::init(const nrt_problem *probs, int32_t count, const nrt_options *o) 
   if (opt.device >= 0) NRT_CUDA(cudaSetDevice(opt.device));
   NRT_CUDA(cudaGetDevice(&device));
   NRT_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-  TRY(build_host_pack(probs, count, host));
+  TRY(build_host_pack(probs, count, host, opt.mode == NRT_IMPLICIT_BE ? kRowAlign : 1));
   const int64_t N = host.ntot;
   const bool mixed = opt.precision == NRT_MIXED;
   // Sizes: V x2, topo, coefficient rows, gates, HH rows, instances, terminals, implicit.
@@ -860,7 +868,7 @@ int nrt_snapshot(nrt_solver *s, double *potential) {
     NRT_CUDA(cudaSetDevice(e.device));
     int rc = e.fixup();
     if (rc) return rc;
-    NRT_CUDA(cudaMemcpyAsync(potential, e.V[e.cur], sizeof(double) * e.host.ntot,
+    NRT_CUDA(cudaMemcpyAsync(potential, e.V[e.cur], sizeof(double) * e.host.num_elem[0],
                              cudaMemcpyDeviceToHost, e.stream));
     NRT_CUDA(cudaStreamSynchronize(e.stream));
     return nrt::implicit_check(e);
@@ -1064,8 +1072,13 @@ int nrt_batch_snapshot_all(nrt_batch *b, double *potential) {
     NRT_CUDA(cudaSetDevice(e.device));
     int rc = e.fixup();
     if (rc) return rc;
-    NRT_CUDA(cudaMemcpyAsync(potential, e.V[e.cur], sizeof(double) * e.host.ntot,
-                             cudaMemcpyDeviceToHost, e.stream));
+    const double *src = e.V[e.cur];
+    int64_t n = e.host.ntot;
+    if (e.opt.mode == NRT_IMPLICIT_BE) {  // without the padding between instances
+      rc = nrt::implicit_compact(e, src, n);
+      if (rc) return rc;
+    }
+    NRT_CUDA(cudaMemcpyAsync(potential, src, sizeof(double) * n, cudaMemcpyDeviceToHost, e.stream));
     NRT_CUDA(cudaStreamSynchronize(e.stream));
     return nrt::implicit_check(e);
   });

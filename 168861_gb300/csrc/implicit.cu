@@ -26,23 +26,23 @@
 // order (deterministic, identical in every CTA).  Initial guess: V^n extrapolated
 // linearly from V^{n-1}.  In mixed precision with the tree preconditioner a refinement
 // cycle is one preconditioned Richardson step, x += M^-1 r (see implicit_one_step), with
-// GMRES cycles taking over when a cycle lowers the true residual less than tenfold.
+// GMRES cycles taking over when a cycle lowers the true residual less than tenfold; that step
+// runs in fused passes over the rows (refine.cuh).
 //
-// Preconditioners: the exact tree factorisation (Hines order, see tree_factor), an exact
-// tridiagonal solve of every unbranched segment piece, Jacobi, or none.
+// Preconditioners: the exact tree factorisation (tree.cuh), an exact tridiagonal solve of
+// every unbranched segment piece, Jacobi, or none.
 //
-// Memory-level parallelism: every row loop keeps several rows per thread in flight and
-// issues all of a row's independent loads before it uses any: a compact per-row flag
+// Memory-level parallelism: the row loops keep several rows per thread in flight and
+// issue all of a row's independent loads before they use any: a compact per-row flag
 // byte replaces the topology record, the neighbours j-1 and j+1 are loaded speculatively
 // (the mother is j-1 except on the first row of a DL child), and only the rare rows with
 // a far neighbour make a second, dependent load.  The SpMV is fused with up to kG
 // Gram-Schmidt products; the update and the norm share a pass.
 //
 // Two launch shapes from one template:
-//  * kGrid  (one tree): a cooperative launch over the whole GPU; rows are split into
-//    contiguous per-CTA ranges aligned with segment pieces; grid-wide syncs separate the
-//    phases (two per Arnoldi step).
-//  * block  (batches): a persistent block-per-instance scheduler; each CTA takes the next
+//  * kGrid  (one tree): a cooperative launch over the whole GPU; rows and windows are split
+//    into contiguous per-CTA ranges; grid-wide syncs separate the phases.
+//  * kBlock (batches): a persistent block-per-instance scheduler; each CTA takes the next
 //    instance (largest first) from an atomic queue and runs all of its steps with
 //    __syncthreads only.
 #include <cooperative_groups.h>
@@ -52,11 +52,11 @@
 #include <memory>
 #include <vector>
 
+#include "cvt.cuh"
 #include "hh.cuh"
 #include "nrt_solver.h"
 #include "pdl.cuh"
 #include "record.cuh"
-#include "tma.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -66,7 +66,10 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxPiece = 256;                 // longest segment piece one sweep handles
 constexpr int kMaxDots = kMaxRestart + 1;
-constexpr int kTileBytes = 44 * 1024;          // shared-memory staging for the sweeps
+constexpr int kTileBytes = 44 * 1024;          // shared memory of the preconditioners
+constexpr int kWalkBytes = 96 * 1024;          // shared memory of the one-tree launch's walk
+constexpr int kRW = 4;                         // tree preconditioner: rows per thread of a window
+constexpr int kWin = kThreads * kRW;           // rows of a window
 constexpr int kU = 4;                          // rows per thread in flight: SpMV + products
 constexpr int kV = 4;                          // rows per thread in flight: streaming passes
 constexpr int kA = 1;                          // rows per thread in flight: assembly
@@ -119,31 +122,38 @@ struct ImView {
   const int2 *pieces;             // (first row, length) of every segment piece
   const int *tiles;               // piece index where each tile starts (sentinel at end)
   const int *cta_row;             // kGrid: per-CTA row range [cta_row[c], cta_row[c+1])
+  const int *cta_win;             // kGrid: per-CTA window range (tree preconditioner)
   const int *cta_tile;            // kGrid: per-CTA tile range
-  const int64_t *inst_row;        // per instance row range (ninst + 1)
+  const int64_t *inst_row;        // per instance first row (ninst + 1)
   const int *inst_tile;           // per instance tile range (ninst + 1)
   const int *order;               // batch: instance processing order
   int *queue;                     // batch: next index into order
   double *partials;               // kGrid: 2 x gridDim x kMaxDots
   InstStat *stats;
   int *err;                       // set when a bounded wait gives up (device fault report)
-  // exact tree preconditioner (NRT_PRECOND_TREE).  Segments in tile order; per-slot
-  // arrays in slot order (slots: the rows of a worker's segments, level by level, deepest
-  // level first; every tile starts on a multiple of 16 slots, padding slots have row -1).
-  void *cdiag;                    // T[ntot]: c_j = c_m dX / dT - W dX, written by the assembly
-  const int *seg_len, *seg_c1, *seg_c2, *seg_prow, *seg_soff;
-  const int *tile_seg;            // segments of tree tile q: [tile_seg[q], tile_seg[q+1])
-  const int *tile_slot;           // slots of tree tile q: [tile_slot[q], tile_slot[q+1])
-  const int *srow;                // row behind each slot (-1: padding)
-  const uint8_t *sflag;           // SL_* flags per slot
-  const int *lev_tile;            // tree tiles of level entry e: [lev_tile[e], lev_tile[e+1])
-  const int *work_lev;            // level entries of a worker (CTA or instance), deepest first
-  const void *sg;                 // T per slot: conductance to the mother (0 without a column)
-  void *sinv, *se, *sy;           // T per slot: 1 / pivot, g / pivot, eliminated right side
-  void *exp_d, *exp_b;            // T per segment: what it passes to its parent row
-  int tree_cap;                   // staging slots per tree tile (multiple of 16)
-  int local_top;                  // one tree: levels 0 .. local_top all belong to CTA 0, which
-                                  // passes between them with CTA barriers only (-1: none)
+  int64_t ld;                     // row-vector stride: ntot rounded up to kRW rows
+  const int *inst_n;              // rows of each instance (inst_row holds where they start)
+  const int64_t *inst_out;        // where each instance's rows go without the padding
+  // exact tree preconditioner (NRT_PRECOND_TREE, tree.cuh): windows, pieces and levels of
+  // each instance.  Piece ids are local to the instance, in level order (deepest first).
+  void *cdiag;                    // T[ld]: c_j = c_m dX / dT - W dX, written by the assembly
+  const uint8_t *pfl;             // [ld] row flags: R_IDENT .. R_FAR, P_FIRST, P_LAST
+  const uint16_t *wtp;            // [window][thread]: pieces that start in the window before it
+  const int *wbase;               // [window] ordinal (row order) of its first piece
+  const int *pmap;                // [piece ordinal] -> piece id
+  const int4 *plink;              // [piece id]: ids of its children at DR (or the next row) and
+                                  // DL and of its parent (-1: none); w: 1 for a one-row piece
+  const int *lev_off;             // per instance: the id one past each level's last piece
+  const int *inst_win, *inst_piece, *inst_lev;  // [instance + 1] offsets
+  int64_t npieces;                // pieces of all instances
+  void *pmob;                     // T[4] per piece: its map in the factorisation
+  void *pstat;                    // T[4] per piece: B, bL, inv_f beta_f, e_f of the factors
+  void *pval;                     // T[4] per piece, two buffers: A, aL, inv_f alpha_f of a solve
+  double *pxb;                    // double[2] per piece, two buffers: V of its first, last row
+  const double *pgf;              // per piece: FP64 conductance of its first row to the mother
+  void *tinv, *te, *tbeta, *talpha;  // T[ld]: 1 / pivot, g / pivot, beta, alpha
+  void *gwalk;                    // walk_bytes per piece: the walk's numbers beyond walk_cap
+  int walk_cap;                   // pieces whose walk fits a CTA's shared memory
 };
 
 template <typename T>
@@ -154,9 +164,8 @@ struct Work {
 struct Shared {
   double *H, *cs, *sn, *g, *s, *y, *red, *warp;
   void *coef;      // T[kMaxDots]: update / solution coefficients
-  int *flag;       // [0] convergence, [1] queue slot, [2] tile barrier phase
-  uint64_t *bar;   // mbarrier of the tile bulk copies
-  void *tile;      // staging area
+  int *flag;       // [0] convergence, [1] queue slot
+  void *tile;      // staging area (segment preconditioner) or the tree walk's numbers
 };
 
 __host__ __device__ inline size_t shared_fixed_bytes(int m) {
@@ -182,9 +191,32 @@ __device__ Shared carve(double *base, int m) {
   S.warp = S.red + kMaxDots;
   S.coef = (void *)(S.warp + kWarps * kMaxDots);
   S.flag = (int *)((double *)S.coef + kMaxDots);
-  S.bar = (uint64_t *)(S.flag + 4);
   S.tile = (void *)((char *)base + ((shared_fixed_bytes(m) + 127) & ~(size_t)127));
   return S;
+}
+
+// ---------------------------------------------------------------- groups
+//
+// The CTAs that step one instance: the CTA itself (kBlock), or the whole cooperative launch
+// (kGrid).
+enum : int { kBlock = 0, kGrid = 1 };
+
+template <int kMode>
+__device__ __forceinline__ int group_rank() {
+  return kMode == kGrid ? (int)blockIdx.x : 0;
+}
+template <int kMode>
+__device__ __forceinline__ int group_size() {
+  return kMode == kGrid ? (int)gridDim.x : 1;
+}
+template <int kMode>
+__device__ __forceinline__ void group_sync() {
+  if (kMode == kGrid) {
+    __threadfence();
+    cg::this_grid().sync();
+  } else {
+    __syncthreads();
+  }
 }
 
 // ---------------------------------------------------------------- reductions
@@ -212,20 +244,20 @@ __device__ __forceinline__ void block_reduce(const T (&acc)[kN], int k, double *
   __syncthreads();
 }
 
-// Grid-wide completion: per-CTA sums -> global partials -> grid sync -> every CTA sums
-// all CTAs' partials in the same order.
-__device__ void grid_finish(cg::grid_group &grid, int k, double *cta_sums, double *partials,
-                            int &parity) {
-  double *buf = partials + (size_t)parity * gridDim.x * kMaxDots;
+// Completion over the CTAs of a group: per-CTA sums -> global partials -> group sync ->
+// every CTA sums all CTAs' partials in the same order.
+template <int kMode>
+__device__ void group_finish(int k, double *cta_sums, double *partials, int &parity) {
+  const int size = group_size<kMode>(), rank = group_rank<kMode>();
+  double *buf = partials + (size_t)kMaxDots * (2 * (blockIdx.x - rank) + parity * size);
   parity ^= 1;
-  if (threadIdx.x < k) buf[(size_t)blockIdx.x * kMaxDots + threadIdx.x] = cta_sums[threadIdx.x];
+  if (threadIdx.x < k) buf[(size_t)rank * kMaxDots + threadIdx.x] = cta_sums[threadIdx.x];
   __syncthreads();
-  __threadfence();
-  grid.sync();
+  group_sync<kMode>();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int i = w; i < k; i += kWarps) {
     double v = 0;
-    for (int c = lane; c < (int)gridDim.x; c += 32) v += buf[(size_t)c * kMaxDots + i];
+    for (int c = lane; c < size; c += 32) v += buf[(size_t)c * kMaxDots + i];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane == 0) cta_sums[i] = v;
   }
@@ -233,22 +265,11 @@ __device__ void grid_finish(cg::grid_group &grid, int k, double *cta_sums, doubl
 }
 
 // Sums k accumulators over the group into S.red[off .. off + k).
-template <bool kGrid, typename T, int kN>
-__device__ __forceinline__ void group_reduce(cg::grid_group &grid, const T (&acc)[kN], int k,
-                                             Shared &S, double *partials, int &parity,
-                                             int off = 0) {
+template <int kMode, typename T, int kN>
+__device__ __forceinline__ void group_reduce(const T (&acc)[kN], int k, Shared &S,
+                                             double *partials, int &parity, int off = 0) {
   block_reduce(acc, k, S.warp, S.red + off);
-  if (kGrid) grid_finish(grid, k, S.red + off, partials, parity);
-}
-
-template <bool kGrid>
-__device__ __forceinline__ void group_sync(cg::grid_group &grid) {
-  if (kGrid) {
-    __threadfence();
-    grid.sync();
-  } else {
-    __syncthreads();
-  }
+  if (kMode != kBlock) group_finish<kMode>(k, S.red + off, partials, parity);
 }
 
 // ---------------------------------------------------------------- row kernels
@@ -360,455 +381,40 @@ __device__ __forceinline__ void apply_rows_c(const PackView &pv, const ImView &i
 
 // ---------------------------------------------------------------- kernel context
 
-template <typename T, bool kGrid>
+template <typename T, int kMode>
 struct Ctx {
   // device-memory copies of the launch's views: phases read the fields they need
   const PackView *pv;
   const ImView *iv;
   Work<T> w;
-  int64_t r0, r1;   // rows of this CTA (kGrid) or instance (batch)
+  int64_t r0, r1;   // rows of this CTA in the row passes
   int t0, t1;       // segment-preconditioner tiles
-  int l0, l1;       // tree-preconditioner level entries (deepest first)
+  // tree preconditioner: this CTA's windows, the instance's first window and row, the end of
+  // its rows (a multiple of kRW after its first), its pieces and level entries
+  int w0, w1, iw0;
+  int64_t wrow0, wend;
+  int ip0, np, l0, l1;
+  int rank;         // this CTA in its group
 };
 
-template <bool kGrid>
-__device__ __forceinline__ void level_sync(cg::grid_group &grid) {
-  if (kGrid) {
-    __threadfence();
-    grid.sync();
-  }
+// A sync of the group where one CTA's rows reach another's (nothing to do in one CTA).
+template <int kMode>
+__device__ __forceinline__ void level_sync() {
+  if (kMode != kBlock) group_sync<kMode>();
 }
 
-// ---------------------------------------------------------------- tree preconditioner
-//
-// Exact factorisation of the tree matrix in Hines order (leaves to root), written for
-// the input conductance eta of the subtree below each row: with d_k = g_k + eta_k (g_k
-// the conductance to the mother, 0 on a row without that column),
-//
-//   eta_k = c_k + sum over children ch of g_ch eta_ch / (g_ch + eta_ch),
-//
-// which is d_k = D_k - sum g_ch^2 / d_ch rewritten without the cancellation between D_k
-// and the children's terms (every term is positive), so the pivots keep full relative
-// precision in FP32.  Per slot it stores inv_k = 1 / d_k and e_k = g_k / d_k; a segment
-// passes e_first * eta_first (= g eta / (g + eta)) to its parent row.  Solve: elimination
-// y_k = v_k + e_{k+1} y_{k+1} leaves to root, then x_k = inv_k y_k + e_k x_mother root to
-// leaves.
-//
-// Work order: the segments of one level at a time (deepest first for the factorisation
-// and the elimination), tile by tile through shared memory.  Inside a tile the
-// recurrences along the segments run as segmented parallel scans over all the tile's
-// slots, so a long unbranched cable costs a few scan rounds, not one thread walking it:
-// the elimination and the substitution are first-order affine recurrences (maps
-// y -> A + M y compose associatively), and the pivot recurrence is a Moebius map of eta,
-// i.e. a product of 2x2 matrices acting on (p, q) with eta = p / q, normalised by powers
-// of two as it goes.
-
-enum : uint8_t { SL_FIRST = 1, SL_LAST = 2, SL_PAD = 4 };  // slot flags (ImView::sflag)
-
-// bulk (TMA) copies, mbarriers and the bounded wait: tma.cuh
-
-// Shared-memory tile of the tree preconditioner: three T rows, the slot flags and the
-// slot rows, `cap` slots each.
-template <typename T>
-struct TreeTile {
-  T *a, *b, *d;
-  uint8_t *f;
-  int *r;
-};
-
-template <typename T>
-__device__ __forceinline__ TreeTile<T> tree_tile(const Shared &S, int cap) {
-  TreeTile<T> t;
-  t.a = (T *)S.tile;
-  t.b = t.a + cap;
-  t.d = t.b + cap;
-  t.r = (int *)(t.d + cap);
-  t.f = (uint8_t *)(t.r + cap);
-  return t;
+// The initial guess of a step: V^n extrapolated from V^{n-1} (which Vout holds until the
+// first solution update writes it).
+__device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, int64_t j) {
+  return 2.0 * Vin[j] - Vout[j];
 }
 
-// Bulk-copies slots [s0, s0 + cnt) of the slot rows, the slot flags and up to three T
-// arrays (null sources are skipped) into the tile, then waits for them.  s0 is a multiple
-// of 16 slots and the slot arrays are padded, so every copy starts 16-byte aligned and
-// its size rounded up to 16 bytes stays inside the arrays and the tile.
-// Tile q_next (-1: none) is the one this CTA stages after this one: its arrays are
-// prefetched into L2 while this tile is worked on.
-template <typename T>
-__device__ __forceinline__ void tile_bulk_load(const ImView &iv, const Shared &S,
-                                               const TreeTile<T> &t, int s0, int cnt,
-                                               const T *x0, T *d0, const T *x1, T *d1,
-                                               const T *x2, T *d2, int q_next = -1) {
-  const uint32_t nt = ((uint32_t)cnt * sizeof(T) + 15u) & ~15u;
-  const uint32_t nr = ((uint32_t)cnt * 4u + 15u) & ~15u;
-  const uint32_t nf = ((uint32_t)cnt + 15u) & ~15u;
-  if (threadIdx.x == 0) {
-    fence_proxy_async();
-    const uint32_t total = nr + nf + (x0 ? nt : 0) + (x1 ? nt : 0) + (x2 ? nt : 0);
-    mbar_expect_tx(S.bar, total);
-    bulk_load(t.r, iv.srow + s0, nr, S.bar);
-    bulk_load(t.f, iv.sflag + s0, nf, S.bar);
-    if (x0) bulk_load(d0, x0 + s0, nt, S.bar);
-    if (x1) bulk_load(d1, x1 + s0, nt, S.bar);
-    if (x2) bulk_load(d2, x2 + s0, nt, S.bar);
-    if (q_next >= 0) {
-      const int s1 = iv.tile_slot[q_next], c1 = iv.tile_slot[q_next + 1] - s1;
-      const uint32_t mt = ((uint32_t)c1 * sizeof(T) + 15u) & ~15u;
-      prefetch_l2(iv.srow + s1, ((uint32_t)c1 * 4u + 15u) & ~15u);
-      prefetch_l2(iv.sflag + s1, ((uint32_t)c1 + 15u) & ~15u);
-      if (x0) prefetch_l2(x0 + s1, mt);
-      if (x1) prefetch_l2(x1 + s1, mt);
-      if (x2) prefetch_l2(x2 + s1, mt);
-    }
-  }
-  const uint32_t ph = (uint32_t)S.flag[2];
-  mbar_wait(S.bar, ph, iv.err);
-  __syncthreads();
-  if (threadIdx.x == 0) S.flag[2] = (int)(ph ^ 1u);
-}
+}  // namespace nrt
 
-// dst[k] = src[row of slot k] for the slots of the tile (0 for padding slots).
-template <typename T>
-__device__ __forceinline__ void tile_gather(T *dst, const int *rows, const T *src, int cnt) {
-  for (int k = threadIdx.x; k < cnt; k += 8 * blockDim.x) {
-    T v[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int kk = k + u * blockDim.x;
-      const int r = kk < cnt ? rows[kk] : -1;
-      v[u] = r >= 0 ? src[r] : (T)0;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int kk = k + u * blockDim.x;
-      if (kk < cnt) dst[kk] = v[u];
-    }
-  }
-}
+#include "tree.cuh"
+#include "refine.cuh"
 
-// dst[s0 + k] = src[k] for the tile's slots.
-template <typename T>
-__device__ __forceinline__ void store_contig(T *dst, const T *src, int s0, int count) {
-  for (int k = threadIdx.x; k < count; k += blockDim.x) dst[s0 + k] = src[k];
-}
-
-// dst[row of slot k] = src[k] for the real slots of the tile.
-template <typename T>
-__device__ __forceinline__ void tile_scatter(T *dst, const int *rows, const T *src, int cnt) {
-  for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
-    const int r = rows[k];
-    if (r >= 0) dst[r] = src[k];
-  }
-}
-
-// The contiguous run of slots thread t owns in a tile scan.  The run length is odd, so
-// the threads of a warp touch distinct shared-memory banks.
-__device__ __forceinline__ void scan_run(int cnt, int &k0, int &k1) {
-  const int R = ((cnt + (int)blockDim.x - 1) / (int)blockDim.x) | 1;
-  k0 = min(cnt, (int)threadIdx.x * R);
-  k1 = min(cnt, k0 + R);
-}
-
-// Segmented first-order recurrence over a tile's slots, in place in a[]:
-//   kDesc:  y_k = a_k + m_k y_{k+1}, k = cnt-1 .. 0 (nothing enters the top)
-//   !kDesc: y_k = a_k + m_k y_{k-1}, k = 0 .. cnt-1
-// with m_k = link(k) (0 where a segment starts in scan order).  Each thread composes the
-// maps of its run, a warp shuffle scan and one pass over the warps give every run its
-// entering value, and the run is then evaluated.  scratch: 3 * warps T values.
-// Links of the two solve recurrences: elimination (descending) uses e_{k+1} unless slot k
-// ends its segment; substitution (ascending) uses e_k unless slot k starts one.
-template <typename T, bool kDesc>
-struct SlotLink {
-  const T *e;
-  const uint8_t *f;
-  __device__ __forceinline__ T operator()(int k) const {
-    if (kDesc) return (f[k] & SL_LAST) ? (T)0 : e[k + 1];
-    return (f[k] & SL_FIRST) ? (T)0 : e[k];
-  }
-};
-
-template <typename T, bool kDesc>
-__device__ __noinline__ void tile_affine_scan(T *a, int cnt, SlotLink<T, kDesc> link, T *scratch) {
-  int k0, k1;
-  scan_run(cnt, k0, k1);
-  T A = 0, M = 1;  // the run's map y_in -> A + M y_in
-  if (kDesc) {
-    for (int k = k1 - 1; k >= k0; k--) {
-      const T m = link(k);
-      A = a[k] + m * A;
-      M = m * M;
-    }
-  } else {
-    for (int k = k0; k < k1; k++) {
-      const T m = link(k);
-      A = a[k] + m * A;
-      M = m * M;
-    }
-  }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int sl = kDesc ? 31 - lane : lane;  // position in scan order inside the warp
-  T iA = A, iM = M;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int src = (kDesc ? lane + off : lane - off) & 31;
-    const T pA = __shfl_sync(0xffffffffu, iA, src), pM = __shfl_sync(0xffffffffu, iM, src);
-    if (sl >= off) {  // (this part) after (the earlier part)
-      iA = iA + iM * pA;
-      iM = iM * pM;
-    }
-  }
-  const int prv = (kDesc ? lane + 1 : lane - 1) & 31;
-  T eA = __shfl_sync(0xffffffffu, iA, prv), eM = __shfl_sync(0xffffffffu, iM, prv);
-  if (sl == 0) {
-    eA = 0;
-    eM = 1;
-  }
-  if (sl == 31) {
-    scratch[2 * w] = iA;
-    scratch[2 * w + 1] = iM;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    T y = 0;
-    for (int q = 0; q < nw; q++) {
-      const int ww = kDesc ? nw - 1 - q : q;
-      scratch[2 * nw + ww] = y;
-      y = scratch[2 * ww] + scratch[2 * ww + 1] * y;
-    }
-  }
-  __syncthreads();
-  T y = eA + eM * scratch[2 * nw + w];
-  if (kDesc) {
-    for (int k = k1 - 1; k >= k0; k--) {
-      y = a[k] + link(k) * y;
-      a[k] = y;
-    }
-  } else {
-    for (int k = k0; k < k1; k++) {
-      y = a[k] + link(k) * y;
-      a[k] = y;
-    }
-  }
-  __syncthreads();
-}
-
-// 2x2 matrices and vectors of the pivot recurrence, scaled by powers of two.
-template <typename T>
-struct Mob {
-  T a, b, c, d;  // [[a, b], [c, d]]
-};
-
-template <typename T>
-__device__ __forceinline__ T pow2_scale_of(T m) {
-  int e;
-  frexp(m, &e);
-  return ldexp((T)1, -e);
-}
-
-template <typename T>
-__device__ __forceinline__ Mob<T> mob_mul(const Mob<T> &x, const Mob<T> &y) {  // x * y
-  Mob<T> r{x.a * y.a + x.b * y.c, x.a * y.b + x.b * y.d, x.c * y.a + x.d * y.c,
-           x.c * y.b + x.d * y.d};
-  const T m = fmax(fmax(r.a, r.b), fmax(r.c, r.d));  // entries are non-negative
-  if (m > (T)0) {
-    const T s = pow2_scale_of(m);
-    r.a *= s;
-    r.b *= s;
-    r.c *= s;
-    r.d *= s;
-  }
-  return r;
-}
-
-// Per-slot map of the pivot recurrence.  The vector entering slot k is (a, b) with
-// a / b = g_{k+1} eta_{k+1} / (g_{k+1} + eta_{k+1}) when slot k+1 continues the segment;
-// the slot forms (p, q) = (a + c b, b) (or (c b, b) at a segment's last slot, where c
-// already holds the children's terms), eta_k = p / q, and passes (g p, p + g q) on.
-template <typename T>
-__device__ __forceinline__ Mob<T> slot_map(T c, T g, uint8_t f) {
-  if (f & SL_PAD) return Mob<T>{1, 0, 0, 1};
-  if (f & SL_LAST) return Mob<T>{0, g * c, 0, c + g};
-  return Mob<T>{g, g * c, 1, c + g};
-}
-
-// One tile of the factorisation: sc = c (in) -> 1/pivot, sg = g -> e = g / pivot,
-// sh -> e * eta; scratch: 12 * warps T values.
-template <typename T>
-__device__ __noinline__ void tile_factor_scan(T *sc, T *sg, T *sh, const uint8_t *sf, int cnt,
-                                              T *scratch) {
-  int k0, k1;
-  scan_run(cnt, k0, k1);
-  Mob<T> P{1, 0, 0, 1};  // the run's map, scan order = descending slots
-  for (int k = k1 - 1; k >= k0; k--) P = mob_mul(slot_map(sc[k], sg[k], sf[k]), P);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int sl = 31 - lane;
-  Mob<T> I = P;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int src = (lane + off) & 31;
-    Mob<T> Q{__shfl_sync(0xffffffffu, I.a, src), __shfl_sync(0xffffffffu, I.b, src),
-             __shfl_sync(0xffffffffu, I.c, src), __shfl_sync(0xffffffffu, I.d, src)};
-    if (sl >= off) I = mob_mul(I, Q);
-  }
-  const int prv = (lane + 1) & 31;
-  Mob<T> E{__shfl_sync(0xffffffffu, I.a, prv), __shfl_sync(0xffffffffu, I.b, prv),
-           __shfl_sync(0xffffffffu, I.c, prv), __shfl_sync(0xffffffffu, I.d, prv)};
-  if (sl == 0) E = Mob<T>{1, 0, 0, 1};
-  if (sl == 31) {
-    scratch[4 * w] = I.a;
-    scratch[4 * w + 1] = I.b;
-    scratch[4 * w + 2] = I.c;
-    scratch[4 * w + 3] = I.d;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {  // vector entering each warp; (0, 1) enters the tile's top slot
-    T va = 0, vb = 1;
-    for (int q = nw - 1; q >= 0; q--) {
-      scratch[4 * nw + 2 * q] = va;
-      scratch[4 * nw + 2 * q + 1] = vb;
-      const T na = scratch[4 * q] * va + scratch[4 * q + 1] * vb;
-      const T nb = scratch[4 * q + 2] * va + scratch[4 * q + 3] * vb;
-      const T s = pow2_scale_of(fmax(na, nb));
-      va = na * s;
-      vb = nb * s;
-    }
-  }
-  __syncthreads();
-  T va = scratch[4 * nw + 2 * w], vb = scratch[4 * nw + 2 * w + 1];
-  {
-    const T na = E.a * va + E.b * vb, nb = E.c * va + E.d * vb;
-    const T s = pow2_scale_of(fmax(na, nb));
-    va = na * s;
-    vb = nb * s;
-  }
-  for (int k = k1 - 1; k >= k0; k--) {
-    const uint8_t f = sf[k];
-    const T c = sc[k], g = sg[k];
-    if (f & SL_PAD) {
-      sc[k] = 0;
-      sg[k] = 0;
-      sh[k] = 0;
-      continue;
-    }
-    const T p = (f & SL_LAST) ? c * vb : va + c * vb;
-    const T eta = p / vb;
-    const T inv = (T)1 / (g + eta);
-    const T e = g * inv;
-    sc[k] = inv;
-    sg[k] = e;
-    sh[k] = e * eta;
-    const T na = g * p, nb = p + g * vb;
-    const T s = pow2_scale_of(fmax(na, nb));
-    va = na * s;
-    vb = nb * s;
-  }
-  __syncthreads();
-}
-
-template <typename T, bool kGrid>
-__device__ __noinline__ void tree_factor(Ctx<T, kGrid> c) {
-  const ImView &iv = *c.iv;
-  cg::grid_group grid = cg::this_grid();
-  Shared S = carve(dyn_smem(), iv.m);
-  const TreeTile<T> t = tree_tile<T>(S, iv.tree_cap);
-  T *scratch = (T *)S.warp;
-  T *exp_d = (T *)iv.exp_d;
-  for (int e = c.l0; e < c.l1; e++) {
-    for (int q = iv.lev_tile[e]; q < iv.lev_tile[e + 1]; q++) {
-      const int s0 = iv.tile_slot[q], cnt = iv.tile_slot[q + 1] - s0;
-      const int qn = q + 1 < iv.lev_tile[c.l1] ? q + 1 : -1;
-      tile_bulk_load<T>(iv, S, t, s0, cnt, (const T *)iv.sg, t.b, nullptr, nullptr, nullptr,
-                        nullptr, qn);
-      tile_gather(t.a, t.r, (const T *)iv.cdiag, cnt);  // c of every slot's row
-      __syncthreads();
-      for (int s = iv.tile_seg[q] + threadIdx.x; s < iv.tile_seg[q + 1]; s += blockDim.x) {
-        const int last = iv.seg_soff[s] + iv.seg_len[s] - 1;
-        const int c1 = iv.seg_c1[s], c2 = iv.seg_c2[s];
-        T add = 0;
-        if (c1 >= 0) add += exp_d[c1];
-        if (c2 >= 0) add += exp_d[c2];
-        t.a[last] += add;
-      }
-      __syncthreads();
-      tile_factor_scan(t.a, t.b, t.d, t.f, cnt, scratch);
-      for (int s = iv.tile_seg[q] + threadIdx.x; s < iv.tile_seg[q + 1]; s += blockDim.x)
-        exp_d[s] = t.d[iv.seg_soff[s]];  // 0 when the first row has no mother column
-      store_contig((T *)iv.sinv, t.a, s0, cnt);
-      store_contig((T *)iv.se, t.b, s0, cnt);
-      fence_proxy_async();  // the solves read sinv / se back with bulk copies
-      __syncthreads();
-    }
-    // entry e is level c.l1 - 1 - e; the next (shallower) one is CTA 0's alone when this
-    // one is (every CTA evaluates the same test, so all take the same grid syncs)
-    if (c.l1 - 1 - e > iv.local_top) level_sync<kGrid>(grid);
-  }
-}
-
-// z = A^-1 v (up to rounding) with the factors of tree_factor.
-template <typename T, bool kGrid>
-__device__ __noinline__ void tree_apply(Ctx<T, kGrid> c, const T *v, T *z) {
-  const ImView &iv = *c.iv;
-  cg::grid_group grid = cg::this_grid();
-  Shared S = carve(dyn_smem(), iv.m);
-  const TreeTile<T> t = tree_tile<T>(S, iv.tree_cap);
-  T *scratch = (T *)S.warp;
-  T *exp_b = (T *)iv.exp_b;
-  // elimination, deepest level first: y_k = v_k + e_{k+1} y_{k+1} inside a segment
-  for (int e = c.l0; e < c.l1; e++) {
-    for (int q = iv.lev_tile[e]; q < iv.lev_tile[e + 1]; q++) {
-      const int s0 = iv.tile_slot[q], cnt = iv.tile_slot[q + 1] - s0;
-      const int qn = q + 1 < iv.lev_tile[c.l1] ? q + 1 : -1;
-      tile_bulk_load<T>(iv, S, t, s0, cnt, (const T *)iv.se, t.b, nullptr, nullptr, nullptr,
-                        nullptr, qn);
-      tile_gather(t.a, t.r, v, cnt);
-      __syncthreads();
-      for (int s = iv.tile_seg[q] + threadIdx.x; s < iv.tile_seg[q + 1]; s += blockDim.x) {
-        const int last = iv.seg_soff[s] + iv.seg_len[s] - 1;
-        const int c1 = iv.seg_c1[s], c2 = iv.seg_c2[s];
-        T add = 0;
-        if (c1 >= 0) add += exp_b[c1];
-        if (c2 >= 0) add += exp_b[c2];
-        t.a[last] += add;
-      }
-      __syncthreads();
-      tile_affine_scan<T, true>(t.a, cnt, SlotLink<T, true>{t.b, t.f}, scratch);
-      for (int s = iv.tile_seg[q] + threadIdx.x; s < iv.tile_seg[q + 1]; s += blockDim.x) {
-        const int o = iv.seg_soff[s];
-        exp_b[s] = t.b[o] * t.a[o];
-      }
-      store_contig((T *)iv.sy, t.a, s0, cnt);
-      fence_proxy_async();  // the substitution reads sy back with bulk copies
-      __syncthreads();
-    }
-    // as in tree_factor; after level 0 the substitution starts at level 0, in CTA 0
-    if (c.l1 - 1 - e > iv.local_top) level_sync<kGrid>(grid);
-  }
-  // substitution, root level first: x_k = inv_k y_k + e_k x_{k-1} (x_mother on a first row)
-  for (int e = c.l1 - 1; e >= c.l0; e--) {
-    for (int q = iv.lev_tile[e]; q < iv.lev_tile[e + 1]; q++) {
-      const int s0 = iv.tile_slot[q], cnt = iv.tile_slot[q + 1] - s0;
-      // next: the following tile of this level, else the first tile of the level above
-      const int qn = q + 1 < iv.lev_tile[e + 1] ? q + 1
-                                                : (e > c.l0 ? iv.lev_tile[e - 1] : -1);
-      tile_bulk_load<T>(iv, S, t, s0, cnt, (const T *)iv.sy, t.a, (const T *)iv.se, t.b,
-                        (const T *)iv.sinv, t.d, qn);
-      for (int k = threadIdx.x; k < cnt; k += blockDim.x) t.a[k] *= t.d[k];
-      __syncthreads();
-      for (int s = iv.tile_seg[q] + threadIdx.x; s < iv.tile_seg[q + 1]; s += blockDim.x) {
-        const int pr = iv.seg_prow[s];
-        if (pr >= 0) {
-          const int o = iv.seg_soff[s];
-          t.a[o] += t.b[o] * z[pr];
-        }
-      }
-      __syncthreads();
-      tile_affine_scan<T, false>(t.a, cnt, SlotLink<T, false>{t.b, t.f}, scratch);
-      tile_scatter(z, t.r, t.a, cnt);
-      __syncthreads();
-    }
-    // the next (deeper) level is CTA 0's alone when it is within the top levels
-    if (c.l1 - 1 - e >= iv.local_top) level_sync<kGrid>(grid);
-  }
-}
+namespace nrt {
 
 // ---------------------------------------------------------------- segment preconditioner
 
@@ -822,8 +428,8 @@ __device__ __forceinline__ void tile_rows(const ImView &iv, int q, int64_t &a, i
 
 // Thomas factorisation of every piece (once per step): pd = 1/pivot, pc = c'.
 // Staged through shared memory tile by tile; one thread per piece.
-template <typename T, bool kGrid>
-__device__ __noinline__ void factor_pieces(Ctx<T, kGrid> c) {
+template <typename T, int kMode>
+__device__ __noinline__ void factor_pieces(Ctx<T, kMode> c) {
   Shared S = carve(dyn_smem(), c.iv->m);
   T *sd = (T *)S.tile;                          // diag, then pivots^-1
   T *sg = sd + c.iv->tile_rows;                  // conductance to the mother
@@ -858,14 +464,15 @@ __device__ __noinline__ void factor_pieces(Ctx<T, kGrid> c) {
   }
 }
 
-// z = M^-1 v over this CTA's rows (identity rows: v and z are 0).
-template <typename T, bool kGrid>
-__device__ __noinline__ void apply_precond(Ctx<T, kGrid> c, const T *v, T *z) {
-  cg::grid_group grid = cg::this_grid();
+// z = M^-1 v over this CTA's rows (identity rows: v and z are 0).  eliminated: the tree
+// factorisation has eliminated v already.
+template <typename T, int kMode>
+__device__ __noinline__ void apply_precond(Ctx<T, kMode> c, const T *v, T *z,
+                                           bool eliminated = false) {
   Shared S = carve(dyn_smem(), c.iv->m);
   if (c.iv->precond == NRT_PRECOND_TREE) {
-    level_sync<kGrid>(grid);  // v of every row visible (tree tiles span other CTAs' rows)
-    tree_apply(c, v, z);
+    group_sync<kMode>();  // v of every row visible (windows hold other threads' and CTAs' rows)
+    tree_apply(c, v, z, eliminated);
   } else if (c.iv->precond == NRT_PRECOND_SEGMENT) {
     T *sv = (T *)S.tile;
     T *sd = sv + c.iv->tile_rows;
@@ -923,18 +530,12 @@ struct DotAcc {
   T v[kG];
 };
 
-// The initial guess of a step: V^n extrapolated from V^{n-1} (which Vout holds until the
-// first solution update writes it).
-__device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, int64_t j) {
-  return 2.0 * Vin[j] - Vout[j];
-}
-
 // Assembly: gates (from V^n), W, K, diagonal, c and right-hand side, fused with the first
 // true residual r = b - A x0 (into W_0).  Nothing writes V here, so the neighbours' x0 are
 // formed from V^n and V^{n-1} directly (a row's columns are never identity rows).  Returns
 // the thread's parts of ||b||^2 and ||r||^2.
-template <typename T, bool kGrid>
-__device__ __noinline__ double2 ph_assemble(Ctx<T, kGrid> c, const double *Vin,
+template <typename T, int kMode>
+__device__ __noinline__ double2 ph_assemble(Ctx<T, kMode> c, const double *Vin,
                                             const double *Vout, int active, int inst) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
@@ -1071,8 +672,8 @@ __device__ __noinline__ double2 ph_assemble(Ctx<T, kGrid> c, const double *Vin,
 }
 
 // Vout = x0 for the rows of this group (when a step ends before any solution update).
-template <typename T, bool kGrid>
-__device__ __noinline__ void ph_x0(Ctx<T, kGrid> c, const double *Vin, double *Vout) {
+template <typename T, int kMode>
+__device__ __noinline__ void ph_x0(Ctx<T, kMode> c, const double *Vin, double *Vout) {
   const uint8_t *rowf = c.iv->rowf;
   for (int64_t j = c.r0 + threadIdx.x; j < c.r1; j += blockDim.x)
     if (!(rowf[j] & R_IDENT)) Vout[j] = x0_of(Vin, Vout, j);
@@ -1084,8 +685,8 @@ __device__ __noinline__ void ph_x0(Ctx<T, kGrid> c, const double *Vin, double *V
 // an FP32 basis: it keeps the sum off the FP64 pipe, and the caller passes a power of two
 // near 1 / (the previous residual norm), which keeps the entries in FP32's range.  FP64
 // solves and BiCGSTAB (whose rho_0 is this norm squared) take the FP64 sum.
-template <typename T, bool kGrid>
-__device__ __noinline__ double ph_residual(Ctx<T, kGrid> c, const double *x, float scale) {
+template <typename T, int kMode>
+__device__ __noinline__ double ph_residual(Ctx<T, kMode> c, const double *x, float scale) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
   const int64_t stride = blockDim.x;
@@ -1116,14 +717,14 @@ __device__ __noinline__ double ph_residual(Ctx<T, kGrid> c, const double *x, flo
 }
 
 // y = s_j A Z_j, fused with the thread's parts of <y, W_i> for i < g1.
-template <typename T, bool kGrid>
-__device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kGrid> c, int j, T sj, int g1) {
+template <typename T, int kMode>
+__device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kMode> c, int j, T sj, int g1) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
-  const int64_t N = pv.ntot, stride = blockDim.x;
+  const int64_t ld = iv.ld, stride = blockDim.x;
   const T *CT = (const T *)iv.cdiag;
   const T *GT = sizeof(T) == 4 ? (const T *)(const void *)iv.gf : (const T *)(const void *)iv.g64;
-  const T *Zj = c.w.Z + (size_t)j * N;
+  const T *Zj = c.w.Z + (size_t)j * ld;
   DotAcc<T> acc;
 #pragma unroll
   for (int i = 0; i < kG; i++) acc.v[i] = 0;
@@ -1140,7 +741,7 @@ __device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kGrid> c, int j, T sj, int g1) 
 #pragma unroll
     for (int i = 0; i < kG; i++) {
       if (i < g1) {
-        const T *Wi = c.w.Wb + (size_t)i * N;
+        const T *Wi = c.w.Wb + (size_t)i * ld;
 #pragma unroll
         for (int u = 0; u < kU; u++) {
           const int64_t r = rb + u * stride;
@@ -1153,9 +754,9 @@ __device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kGrid> c, int j, T sj, int g1) 
 }
 
 // The thread's parts of <y, W_{i0+i}> for i < gk.
-template <typename T, bool kGrid>
-__device__ __noinline__ DotAcc<T> ph_products(Ctx<T, kGrid> c, int i0, int gk) {
-  const int64_t N = c.pv->ntot, stride = blockDim.x;
+template <typename T, int kMode>
+__device__ __noinline__ DotAcc<T> ph_products(Ctx<T, kMode> c, int i0, int gk) {
+  const int64_t ld = c.iv->ld, stride = blockDim.x;
   DotAcc<T> acc;
 #pragma unroll
   for (int i = 0; i < kG; i++) acc.v[i] = 0;
@@ -1169,7 +770,7 @@ __device__ __noinline__ DotAcc<T> ph_products(Ctx<T, kGrid> c, int i0, int gk) {
 #pragma unroll
     for (int i = 0; i < kG; i++) {
       if (i < gk) {
-        const T *Wi = c.w.Wb + (size_t)(i0 + i) * N;
+        const T *Wi = c.w.Wb + (size_t)(i0 + i) * ld;
 #pragma unroll
         for (int u = 0; u < kV; u++) {
           const int64_t r = rb + u * stride;
@@ -1182,10 +783,10 @@ __device__ __noinline__ DotAcc<T> ph_products(Ctx<T, kGrid> c, int i0, int gk) {
 }
 
 // W_{j+1} = y - sum_{i <= j} coef_i W_i; returns the thread's part of ||W_{j+1}||^2.
-template <typename T, bool kGrid>
-__device__ __noinline__ T ph_update(Ctx<T, kGrid> c, int j, const T *coef) {
-  const int64_t N = c.pv->ntot, stride = blockDim.x;
-  T *Wn = c.w.Wb + (size_t)(j + 1) * N;
+template <typename T, int kMode>
+__device__ __noinline__ T ph_update(Ctx<T, kMode> c, int j, const T *coef) {
+  const int64_t ld = c.iv->ld, stride = blockDim.x;
+  T *Wn = c.w.Wb + (size_t)(j + 1) * ld;
   T nacc = 0;
   for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
     T a[kV];
@@ -1197,7 +798,7 @@ __device__ __noinline__ T ph_update(Ctx<T, kGrid> c, int j, const T *coef) {
 #pragma unroll 1
     for (int i = 0; i <= j; i++) {
       const T ci = coef[i];
-      const T *Wi = c.w.Wb + (size_t)i * N;
+      const T *Wi = c.w.Wb + (size_t)i * ld;
       T w[kV];
 #pragma unroll
       for (int u = 0; u < kV; u++) {
@@ -1221,10 +822,10 @@ __device__ __noinline__ T ph_update(Ctx<T, kGrid> c, int j, const T *coef) {
 
 // V += sum_{i < k} coef_i Z_i (identity rows keep their value).  With Vin non-null this is
 // the step's first update and V starts from x0 = 2 Vin - V.
-template <typename T, bool kGrid>
-__device__ __noinline__ void ph_xupdate(Ctx<T, kGrid> c, int k, const T *coef, double *Vout,
+template <typename T, int kMode>
+__device__ __noinline__ void ph_xupdate(Ctx<T, kMode> c, int k, const T *coef, double *Vout,
                                         const double *Vin) {
-  const int64_t N = c.pv->ntot, stride = blockDim.x;
+  const int64_t ld = c.iv->ld, stride = blockDim.x;
   const uint8_t *rowf = c.iv->rowf;
   for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
     T a[kV];
@@ -1238,7 +839,7 @@ __device__ __noinline__ void ph_xupdate(Ctx<T, kGrid> c, int k, const T *coef, d
 #pragma unroll 1
     for (int i = 0; i < k; i++) {
       const T ci = coef[i];
-      const T *Zi = c.w.Z + (size_t)i * N;
+      const T *Zi = c.w.Z + (size_t)i * ld;
       T z[kV];
 #pragma unroll
       for (int u = 0; u < kV; u++) {
@@ -1259,41 +860,11 @@ __device__ __noinline__ void ph_xupdate(Ctx<T, kGrid> c, int k, const T *coef, d
   }
 }
 
-// A Richardson step's update V += Z_0 (identity rows keep their value), with every load of
-// a thread's kV rows issued before any use.  With Vin non-null this is the step's first
-// update and V starts from x0 = 2 Vin - V.  Equal bit for bit to ph_xupdate with k = 1 and
-// coefficient 1.
-template <typename T, bool kGrid>
-__device__ __noinline__ void ph_rich_update(Ctx<T, kGrid> c, double *Vout, const double *Vin) {
-  const int64_t stride = blockDim.x;
-  const uint8_t *rowf = c.iv->rowf;
-  const T *Z = c.w.Z;
-  for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
-    uint8_t fl[kV];
-    T z[kV];
-    double v[kV], w[kV];
-#pragma unroll
-    for (int u = 0; u < kV; u++) {
-      const int64_t r = rb + u * stride;
-      const bool ok = r < c.r1;
-      fl[u] = ok ? rowf[r] : (uint8_t)R_IDENT;
-      z[u] = ok ? Z[r] : (T)0;
-      v[u] = ok ? Vout[r] : 0.0;
-      w[u] = ok && Vin ? Vin[r] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < kV; u++) {
-      const int64_t r = rb + u * stride;
-      if (!(fl[u] & R_IDENT)) Vout[r] = (Vin ? 2.0 * w[u] - v[u] : v[u]) + (double)z[u];
-    }
-  }
-}
-
 // ---- BiCGSTAB (right-preconditioned, on the correction equation of one refinement cycle)
 
 // p = r + beta (p - omega v); beta == 0 gives p = r.
-template <typename T, bool kGrid>
-__device__ __noinline__ void ph_bicg_dir(Ctx<T, kGrid> c, const T *r, T *p, const T *v, T beta,
+template <typename T, int kMode>
+__device__ __noinline__ void ph_bicg_dir(Ctx<T, kMode> c, const T *r, T *p, const T *v, T beta,
                                          T omega) {
   const int64_t stride = blockDim.x;
   for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
@@ -1315,8 +886,8 @@ __device__ __noinline__ void ph_bicg_dir(Ctx<T, kGrid> c, const T *r, T *p, cons
 }
 
 // out = A x; returns the thread's parts of <out, d0> and <out, d1> (d1 may be null).
-template <typename T, bool kGrid>
-__device__ __noinline__ DotAcc<T> ph_matvec(Ctx<T, kGrid> c, const T *x, T *out, const T *d0,
+template <typename T, int kMode>
+__device__ __noinline__ DotAcc<T> ph_matvec(Ctx<T, kMode> c, const T *x, T *out, const T *d0,
                                             const T *d1) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
@@ -1348,8 +919,8 @@ __device__ __noinline__ DotAcc<T> ph_matvec(Ctx<T, kGrid> c, const T *x, T *out,
 }
 
 // s = r - alpha v; returns the thread's part of ||s||^2.
-template <typename T, bool kGrid>
-__device__ __noinline__ T ph_bicg_s(Ctx<T, kGrid> c, const T *r, const T *v, T alpha, T *s) {
+template <typename T, int kMode>
+__device__ __noinline__ T ph_bicg_s(Ctx<T, kMode> c, const T *r, const T *v, T alpha, T *s) {
   const int64_t stride = blockDim.x;
   T acc = 0;
   for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
@@ -1373,8 +944,8 @@ __device__ __noinline__ T ph_bicg_s(Ctx<T, kGrid> c, const T *r, const T *v, T a
 
 // V += alpha ph + omega sh (FP64 accumulation; identity rows keep their value) and
 // r = s - omega t; returns the thread's parts of ||r||^2 and <rh, r>.
-template <typename T, bool kGrid>
-__device__ __noinline__ DotAcc<T> ph_bicg_x(Ctx<T, kGrid> c, const T *ph, const T *sh,
+template <typename T, int kMode>
+__device__ __noinline__ DotAcc<T> ph_bicg_x(Ctx<T, kMode> c, const T *ph, const T *sh,
                                             const T *s, const T *t, T alpha, T omega, T *r,
                                             const T *rh, double *Vout) {
   const int64_t stride = blockDim.x;
@@ -1415,27 +986,26 @@ __device__ __noinline__ DotAcc<T> ph_bicg_x(Ctx<T, kGrid> c, const T *ph, const 
 // budget, so repeated breakdowns still end the step.
 // Not inlined, so that the GMRES path's register allocation does not carry it.
 // Returns {parity, iters}.
-template <typename T, bool kGrid>
-__device__ __noinline__ int2 bicgstab_cycle(Ctx<T, kGrid> c, int parity, double res,
+template <typename T, int kMode>
+__device__ __noinline__ int2 bicgstab_cycle(Ctx<T, kMode> c, int parity, double res,
                                             double cycle_target, int budget, int iters,
                                             double *Vout) {
   const ImView &iv = *c.iv;
-  cg::grid_group grid = cg::this_grid();
   Shared S = carve(dyn_smem(), iv.m);
-  const int64_t N = c.pv->ntot;
-  T *rh = c.w.Wb, *r1 = c.w.Wb + N, *p = c.w.Wb + 2 * N, *v = c.w.Wb + 3 * N;
-  T *ph = c.w.Z, *sh = c.w.Z + N, *s = c.w.Z + 2 * N, *t = c.w.Z + 3 * N;
+  const int64_t ld = iv.ld;
+  T *rh = c.w.Wb, *r1 = c.w.Wb + ld, *p = c.w.Wb + 2 * ld, *v = c.w.Wb + 3 * ld;
+  T *ph = c.w.Z, *sh = c.w.Z + ld, *s = c.w.Z + 2 * ld, *t = c.w.Z + 3 * ld;
   const T *r = rh;  // the first iteration reads r0 itself
   double rho = res * res, rho_prev = 1.0, alpha = 1.0, omega = 1.0;
   for (int it = 0; iters < budget; it++) {
     const double beta = it == 0 ? 0.0 : (rho / rho_prev) * (alpha / omega);
     ph_bicg_dir(c, r, p, v, (T)beta, (T)omega);
-    group_sync<kGrid>(grid);
+    group_sync<kMode>();
     apply_precond(c, p, ph);
-    group_sync<kGrid>(grid);
+    group_sync<kMode>();
     {
       DotAcc<T> acc = ph_matvec(c, ph, v, rh, (const T *)nullptr);
-      group_reduce<kGrid>(grid, acc.v, 1, S, iv.partials, parity);
+      group_reduce<kMode>(acc.v, 1, S, iv.partials, parity);
     }
     const double rv = S.red[0];
     if (rv == 0.0 || !(rv == rv) || !(rho == rho)) {  // breakdown: restart from r0
@@ -1445,25 +1015,25 @@ __device__ __noinline__ int2 bicgstab_cycle(Ctx<T, kGrid> c, int parity, double 
     alpha = rho / rv;
     {
       T acc[1] = {ph_bicg_s(c, r, v, (T)alpha, s)};
-      group_reduce<kGrid>(grid, acc, 1, S, iv.partials, parity);
+      group_reduce<kMode>(acc, 1, S, iv.partials, parity);
     }
     iters++;
     if (sqrt(S.red[0]) <= cycle_target) {  // x += alpha ph completes the cycle
       ph_bicg_x(c, ph, ph, s, s, (T)alpha, (T)0, r1, rh, Vout);
-      group_sync<kGrid>(grid);
+      group_sync<kMode>();
       break;
     }
     apply_precond(c, s, sh);
-    group_sync<kGrid>(grid);
+    group_sync<kMode>();
     {
       DotAcc<T> acc = ph_matvec(c, sh, t, s, t);
-      group_reduce<kGrid>(grid, acc.v, 2, S, iv.partials, parity);
+      group_reduce<kMode>(acc.v, 2, S, iv.partials, parity);
     }
     const double ts = S.red[0], tt = S.red[1];
     omega = tt > 0.0 ? ts / tt : 0.0;
     {
       DotAcc<T> acc = ph_bicg_x(c, ph, sh, s, t, (T)alpha, (T)omega, r1, rh, Vout);
-      group_reduce<kGrid>(grid, acc.v, 2, S, iv.partials, parity);
+      group_reduce<kMode>(acc.v, 2, S, iv.partials, parity);
     }
     r = r1;
     const double rn = sqrt(S.red[0]);
@@ -1471,42 +1041,59 @@ __device__ __noinline__ int2 bicgstab_cycle(Ctx<T, kGrid> c, int parity, double 
     rho = S.red[1];
     if (rn <= cycle_target || omega == 0.0 || rho == 0.0) break;
   }
-  group_sync<kGrid>(grid);  // V complete before the next true residual
+  group_sync<kMode>();  // V complete before the next true residual
   return make_int2(parity, iters);
 }
 
 // One backward-Euler step of one group (CTA or grid) for instance `inst`.
-template <typename T, bool kGrid>
-__device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_group &grid,
-                                                  Shared &S, int &parity, const double *Vin,
+template <typename T, int kMode>
+__device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, int &parity, const double *Vin,
                                                   double *Vout, bool active, int64_t inst_n,
                                                   int inst) {
   const ImView &iv = *c.iv;
   const int m = iv.m;
   T *coef = (T *)S.coef;
   // ---- assembly, fused with the first true residual (W_0); V still holds V^{n-1}
-  const double2 br = ph_assemble(c, Vin, Vout, active ? 1 : 0, inst);
-  __syncthreads();
+  const bool tree = iv.precond == NRT_PRECOND_TREE;
+  const bool fused = sizeof(T) == 4 && iv.rich != 0;  // by windows, with the pieces' matrices
+  double2 br;
+  if constexpr (sizeof(T) == 4) {
+    if (!fused)
+      br = ph_assemble(c, Vin, Vout, active ? 1 : 0, inst);
+    else if (iv.scheme == NRT_CRANK_NICOLSON)
+      br = refine_assemble<kMode, true>(c, Vin, Vout, active ? 1 : 0, inst);
+    else
+      br = refine_assemble<kMode, false>(c, Vin, Vout, active ? 1 : 0, inst);
+  } else {
+    br = ph_assemble(c, Vin, Vout, active ? 1 : 0, inst);
+  }
   if (iv.precond == NRT_PRECOND_SEGMENT) {
+    __syncthreads();
     factor_pieces(c);
-  } else if (iv.precond == NRT_PRECOND_TREE) {
-    level_sync<kGrid>(grid);  // c of every row visible before the elimination
-    tree_factor(c);
+  } else if (tree && !fused) {
+    group_sync<kMode>();  // c of every row visible before the factorisation
+    tree_maps(c);
+    __syncthreads();
   }
   double target = iv.tol, res0 = 0;
   {
     double acc[2] = {br.x, br.y};
-    group_reduce<kGrid>(grid, acc, 2, S, iv.partials, parity);  // also publishes W_0
+    group_reduce<kMode>(acc, 2, S, iv.partials, parity);  // also publishes W_0, the matrices
     if (iv.tol_mode == NRT_TOL_REL) target = iv.tol * sqrt(S.red[0]);
     res0 = sqrt(S.red[1]);
-    if (!kGrid) __syncthreads();
+    if (kMode == kBlock) __syncthreads();
   }
+  if (tree) tree_factor(c, c.w.Wb, fused ? Vin : (const double *)nullptr, Vout);
   const int budget = iv.max_iter > 0 ? iv.max_iter : (iv.max_iter < 0 ? 0 : (int)inst_n);
   const double inner_rel = iv.inner_rel;
   int iters = 0, n_res = 0, n_app = 0, n_xup = 0, n_basis = 0, n_rich = 0;
   double res = 0, prev_res = 0;
   bool converged = false;
   bool x0_pending = true;  // V holds V^{n-1} until the first solution update
+  bool rich_done = false;  // the last cycle's update has left the true residual in res
+  bool w0_valid = true;    // W_0 holds the residual
+  int pb = 0;              // the buffer of the pieces' values that the next walk reads
+  bool eliminated = tree;  // the right-hand side W_0 has been eliminated
   // Mixed precision with the tree preconditioner: M is the FP32 factorisation of A itself,
   // so GMRES's one Arnoldi step per cycle takes x += y M^-1 r with y within rounding of 1.
   // A Richardson step takes x += M^-1 r without the SpMV, the products and the basis
@@ -1517,15 +1104,16 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
     // ---- cycle start: true residual r = b - A x in FP64, W_0 = r, Z_0 = M^-1 r
     if (cycle == 0) {
       res = res0;
-    } else {
+    } else if (!rich_done) {
       // res > 0 here (a zero residual has converged); the scale stays a normal FP32 number
       const bool f32 = sizeof(T) == 4 && iv.krylov == NRT_GMRES;
       const int e = f32 ? max(-126, min(126, ilogb(res))) : 0;
       double acc[1] = {ph_residual(c, Vout, f32 ? exp2f((float)-e) : 0.0f)};
-      group_reduce<kGrid>(grid, acc, 1, S, iv.partials, parity);
+      group_reduce<kMode>(acc, 1, S, iv.partials, parity);
       res = sqrt(S.red[0]) * exp2((double)e);
       n_res++;
     }
+    rich_done = false;
     if (res <= target) {
       converged = true;
       break;
@@ -1536,7 +1124,7 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
       if (x0_pending) {
         ph_x0(c, Vin, Vout);
         x0_pending = false;
-        group_sync<kGrid>(grid);
+        group_sync<kMode>();
       }
       const int2 pi = bicgstab_cycle(c, parity, res, fmax(target, inner_rel * res), budget,
                                      iters, Vout);
@@ -1544,18 +1132,45 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
       iters = pi.y;
       continue;
     }
-    apply_precond(c, c.w.Wb, c.w.Z);
-    n_app++;
-    group_sync<kGrid>(grid);  // Z_0 of every row visible before the SpMV
-    if (rich) {  // x += M^-1 r
-      ph_rich_update(c, Vout, x0_pending ? Vin : (const double *)nullptr);
-      group_sync<kGrid>(grid);
-      n_xup++;
-      n_rich++;
-      x0_pending = false;
-      prev_res = res;
-      continue;
+    if constexpr (sizeof(T) == 4) {
+      if (rich) {  // x += M^-1 r and the residual of the new x
+        if (!eliminated) tree_eliminate(c, c.w.Wb, pb, Vout);
+        group_sync<kMode>();  // every window's elimination visible to the walk
+        if (walks(c, iv)) refine_walk(c, pb);
+        if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
+        const double *from = x0_pending ? Vin : (const double *)nullptr;
+        const int e = max(-126, min(126, ilogb(res)));
+        const float scale = exp2f((float)-e);
+        // The first cycle's residual is eliminated at once: it is rarely the last.
+        double acc[1];
+        if (cycle == 0) {
+          pb ^= 1;
+          acc[0] = (double)refine_update<kMode, true>(c, from, Vout, scale, pb);
+        } else {
+          acc[0] = (double)refine_update<kMode, false>(c, from, Vout, scale, pb);
+        }
+        eliminated = cycle == 0;
+        group_reduce<kMode>(acc, 1, S, iv.partials, parity);  // V and W_0 complete
+        prev_res = res;
+        res = sqrt(S.red[0]) * exp2((double)e);
+        w0_valid = cycle != 0;
+        rich_done = true;
+        x0_pending = false;
+        n_app++;
+        n_xup++;
+        n_rich++;
+        n_res++;
+        continue;
+      }
     }
+    if (!w0_valid) {  // after the first refinement cycle W_0 is not stored
+      (void)ph_residual(c, Vout, 1.0f);
+      w0_valid = true;
+    }
+    apply_precond(c, c.w.Wb, c.w.Z, eliminated && cycle == 0);
+    n_app++;
+    eliminated = false;
+    group_sync<kMode>();  // Z_0 of every row visible before the SpMV
     if (threadIdx.x == 0) {
       S.g[0] = res;
       for (int i = 1; i <= m; i++) S.g[i] = 0;
@@ -1569,12 +1184,12 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
       const int g1 = min(j + 1, kG);
       {
         DotAcc<T> acc = ph_spmv(c, j, (T)S.s[j], g1);
-        group_reduce<kGrid>(grid, acc.v, g1, S, iv.partials, parity);
+        group_reduce<kMode>(acc.v, g1, S, iv.partials, parity);
       }
       for (int i0 = kG; i0 <= j; i0 += kG) {  // remaining products, kG at a time
         const int gk = min(j + 1 - i0, kG);
         DotAcc<T> acc = ph_products(c, i0, gk);
-        group_reduce<kGrid>(grid, acc.v, gk, S, iv.partials, parity, i0);
+        group_reduce<kMode>(acc.v, gk, S, iv.partials, parity, i0);
       }
       if (threadIdx.x <= j) {
         const double h = S.s[threadIdx.x] * S.red[threadIdx.x];
@@ -1584,7 +1199,7 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
       __syncthreads();
       // w = y - sum_i h_ij s_i W_i -> W_{j+1}; ||w||^2
       T nacc[1] = {ph_update(c, j, coef)};
-      group_reduce<kGrid>(grid, nacc, 1, S, iv.partials, parity);  // publishes W_{j+1}
+      group_reduce<kMode>(nacc, 1, S, iv.partials, parity);  // publishes W_{j+1}
       if (threadIdx.x == 0) {
         const double hn = sqrt(S.red[0]);
         S.s[j + 1] = hn > 0 ? 1.0 / hn : 0.0;
@@ -1608,9 +1223,9 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
       n_basis += j + 1;
       if (S.flag[0] || iters + n_rich >= budget || k >= m) break;
       // Z_{j+1} = M^-1 W_{j+1}, only when another Arnoldi step will use it
-      apply_precond(c, c.w.Wb + (size_t)(j + 1) * c.pv->ntot, c.w.Z + (size_t)(j + 1) * c.pv->ntot);
+      apply_precond(c, c.w.Wb + (size_t)(j + 1) * iv.ld, c.w.Z + (size_t)(j + 1) * iv.ld);
       n_app++;
-      group_sync<kGrid>(grid);  // Z_{j+1} of every row visible before the next SpMV
+      group_sync<kMode>();  // Z_{j+1} of every row visible before the next SpMV
     }
     // ---- x += sum_i y_i s_i Z_i
     if (threadIdx.x == 0) {
@@ -1623,12 +1238,12 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
     }
     __syncthreads();
     ph_xupdate(c, k, coef, Vout, x0_pending ? Vin : (const double *)nullptr);
-    group_sync<kGrid>(grid);
+    group_sync<kMode>();
     n_xup++;
     x0_pending = false;
   }
   if (x0_pending) ph_x0(c, Vin, Vout);  // converged (or out of budget) at x0 itself
-  if (threadIdx.x == 0 && (!kGrid || blockIdx.x == 0)) {
+  if (threadIdx.x == 0 && c.rank == 0) {
     InstStat &st = iv.stats[inst];
     st.iters += iters;
     st.last_iters = iters;
@@ -1640,7 +1255,7 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kGrid> &c, cg::grid_gro
     st.basis += n_basis;
     st.rich += n_rich;
   }
-  group_sync<kGrid>(grid);  // V^{n+1} complete before the next step reads it
+  group_sync<kMode>();  // V^{n+1} complete before the next step reads it
 }
 
 // Recording at the probes of instance `inst` after the step at loop index i (V is that
@@ -1653,21 +1268,23 @@ __device__ __noinline__ void ph_record(const RecView *rp, int inst, int64_t i, c
   for (int p = a + threadIdx.x; p < b; p += blockDim.x) record_probe(r, p, i, V[r.src[p]], dT);
 }
 
-template <typename T, bool kGrid>
-__global__ void __launch_bounds__(kThreads, 4) implicit_steps(const PackView *pvp, const ImView *ivp,
+// Resident CTAs per SM that the registers allow.  FP32: 3 (80 registers; the 2048-tree batch
+// took 51.1 ms per 8 steps at 4, whose 64 registers spill in the fused passes, 41.7 at 3 and
+// 48.9 at 2).  FP64: 2 (128 registers): its FP64 pipe is full with 16 warps.
+template <typename T>
+constexpr int ctas_per_sm() {
+  return sizeof(T) == 4 ? 3 : 2;
+}
+
+template <typename T, int kMode>
+__global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(const PackView *pvp, const ImView *ivp,
                                                            int nsteps, int force, double *V0,
                                                            double *V1, int cur,
                                                            const RecView *rec) {
   const ImView &iv = *ivp;
   Shared S = carve(dyn_smem(), iv.m);
-  cg::grid_group grid = cg::this_grid();
   int parity = 0;
-  if (threadIdx.x == 0) {
-    mbar_init(S.bar, 1);
-    S.flag[2] = 0;
-  }
-  __syncthreads();
-  Ctx<T, kGrid> c;
+  Ctx<T, kMode> c;
   c.pv = pvp;
   c.iv = ivp;
   c.w.Wb = (T *)iv.Wb;
@@ -1675,79 +1292,74 @@ __global__ void __launch_bounds__(kThreads, 4) implicit_steps(const PackView *pv
   c.w.y = (T *)iv.yv;
   c.w.pd = (T *)iv.pcd;
   c.w.pc = (T *)iv.pcc;
-  if (kGrid) {
-    c.r0 = iv.cta_row[blockIdx.x];
-    c.r1 = iv.cta_row[blockIdx.x + 1];
-    c.t0 = iv.cta_tile[blockIdx.x];
-    c.t1 = iv.cta_tile[blockIdx.x + 1];
-    c.l0 = iv.work_lev ? iv.work_lev[blockIdx.x] : 0;
-    c.l1 = iv.work_lev ? iv.work_lev[blockIdx.x + 1] : 0;
-    const InstDev in = pvp->inst[0];
-    const int64_t inst_n = iv.inst_row[1] - iv.inst_row[0];
-    int s = 0;
-    for (; s < nsteps; s++) {
-      const int64_t i = in.base + s;
-      if (i >= in.iend) break;
-      const bool active = force >= 0 ? force != 0
-                                     : (i >= in.ion && i <= in.ioff);
-      implicit_one_step<T, kGrid>(c, grid, S, parity, ((cur + s) & 1) ? V1 : V0,
-                                  ((cur + s + 1) & 1) ? V1 : V0, active, inst_n, 0);
-      if (rec && blockIdx.x == 0) ph_record(rec, 0, i, ((cur + s + 1) & 1) ? V1 : V0, in.dT);
-    }
-    if ((nsteps - s) & 1) {  // the run ended inside the launch: each CTA moves its rows
-      double *dst = ((cur + nsteps) & 1) ? V1 : V0;
-      const double *src = ((cur + s) & 1) ? V1 : V0;
-      for (int64_t j = c.r0 + threadIdx.x; j < c.r1; j += blockDim.x) dst[j] = src[j];
-    }
-  } else {
-    for (;;) {
+  c.rank = group_rank<kMode>();
+  for (;;) {
+    int inst = 0;
+    if (kMode == kBlock) {
       if (threadIdx.x == 0) S.flag[1] = atomicAdd(iv.queue, 1);
       __syncthreads();
       const int q = S.flag[1];
       __syncthreads();
       if (q >= iv.ninst) break;
-      const int inst = iv.order[q];
-      c.r0 = iv.inst_row[inst];
-      c.r1 = iv.inst_row[inst + 1];
+      inst = iv.order[q];
+    }
+    const int n = iv.inst_n[inst];
+    c.r0 = iv.inst_row[inst];
+    c.r1 = c.r0 + n;
+    const bool tree = iv.precond == NRT_PRECOND_TREE;
+    c.wrow0 = c.r0;
+    c.wend = c.r0 + ((n + kRW - 1) & ~(kRW - 1));
+    c.iw0 = tree ? iv.inst_win[inst] : 0;
+    c.w0 = c.iw0;
+    c.w1 = tree ? iv.inst_win[inst + 1] : 0;
+    c.ip0 = tree ? iv.inst_piece[inst] : 0;
+    c.np = tree ? iv.inst_piece[inst + 1] - c.ip0 : 0;
+    c.l0 = tree ? iv.inst_lev[inst] : 0;
+    c.l1 = tree ? iv.inst_lev[inst + 1] : 0;
+    if (kMode == kGrid) {
+      c.r0 = iv.cta_row[blockIdx.x];
+      c.r1 = iv.cta_row[blockIdx.x + 1];
+      c.t0 = iv.cta_tile[blockIdx.x];
+      c.t1 = iv.cta_tile[blockIdx.x + 1];
+      if (tree) {
+        c.w0 = iv.cta_win[blockIdx.x];
+        c.w1 = iv.cta_win[blockIdx.x + 1];
+      }
+    } else {
       c.t0 = iv.inst_tile[inst];
       c.t1 = iv.inst_tile[inst + 1];
-      c.l0 = iv.work_lev ? iv.work_lev[inst] : 0;
-      c.l1 = iv.work_lev ? iv.work_lev[inst + 1] : 0;
-      const InstDev in = pvp->inst[inst];
-      int s = 0;
-      for (; s < nsteps; s++) {
-        const int64_t i = in.base + s;
-        if (i >= in.iend) break;
-        const bool active = force >= 0 ? force != 0
-                                       : (i >= in.ion && i <= in.ioff);
-        implicit_one_step<T, kGrid>(c, grid, S, parity, ((cur + s) & 1) ? V1 : V0,
-                                    ((cur + s + 1) & 1) ? V1 : V0, active, c.r1 - c.r0, inst);
-        if (rec) ph_record(rec, inst, i, ((cur + s + 1) & 1) ? V1 : V0, in.dT);
-      }
-      if ((nsteps - s) & 1) {  // finished early: put its latest V where the others' is
-        double *dst = ((cur + nsteps) & 1) ? V1 : V0;
-        const double *src = ((cur + s) & 1) ? V1 : V0;
-        for (int64_t j = c.r0 + threadIdx.x; j < c.r1; j += blockDim.x) dst[j] = src[j];
-      }
-      __syncthreads();
     }
+    const InstDev in = pvp->inst[inst];
+    int s = 0;
+    for (; s < nsteps; s++) {
+      const int64_t i = in.base + s;
+      if (i >= in.iend) break;
+      const bool active = force >= 0 ? force != 0 : (i >= in.ion && i <= in.ioff);
+      implicit_one_step<T, kMode>(c, S, parity, ((cur + s) & 1) ? V1 : V0,
+                                  ((cur + s + 1) & 1) ? V1 : V0, active, n, inst);
+      if (rec && c.rank == 0) ph_record(rec, inst, i, ((cur + s + 1) & 1) ? V1 : V0, in.dT);
+    }
+    if ((nsteps - s) & 1) {  // the run ended inside the launch: its latest V goes where the
+      double *dst = ((cur + nsteps) & 1) ? V1 : V0;  // others' is, each CTA moving its rows
+      const double *src = ((cur + s) & 1) ? V1 : V0;
+      for (int64_t j = c.r0 + threadIdx.x; j < c.r1; j += blockDim.x) dst[j] = src[j];
+    }
+    if (kMode == kGrid) break;
+    __syncthreads();
   }
 }
 
 // ---------------------------------------------------------------- host side
 
-// Schedule of the exact tree preconditioner.  Segments are maximal runs of physical rows
-// each linked to the previous row (mother == j - 1), broken after every branch point and
-// at `cap` rows; a segment's parent row (the mother of its first row) is then always the
-// last row of its parent segment.  Level = number of segments above.  Each worker (one
-// CTA of the cooperative launch, or one instance of a batch) gets, per level (deepest
-// first), tiles of whole segments whose slots fit the shared-memory staging area; every
-// tile starts on a multiple of 16 slots (padding slots in between have row -1).
-struct TreeSchedule {  // sized without a fill: every entry is written by the builders
-  hvec<int> seg_len, seg_c1, seg_c2, seg_prow, seg_soff;  // tile order
-  hvec<int> tile_seg, tile_slot, slot_row, lev_tile, work_lev;
-  hvec<uint8_t> slot_flag;
-  int local_top = -1;  // ImView::local_top
+// Windows, pieces and levels of the exact tree preconditioner (tree.cuh), per instance and
+// then concatenated.
+struct TreePlan {  // sized without a fill: every entry is written by the builder
+  hvec<uint8_t> pfl;
+  hvec<uint16_t> wtp;
+  hvec<int> wbase, pmap, lev_off, inst_win, inst_piece, inst_lev;
+  hvec<int4> plink;
+  hvec<double> pgf;
+  int max_pieces = 0;
 };
 
 struct ImplicitState {
@@ -1756,20 +1368,23 @@ struct ImplicitState {
   ImView *d_iv = nullptr;
   hvec<uint8_t> rowf;  // sized without a fill: implicit_plan writes every row
   hvec<int2> pieces;
-  std::vector<int> tiles, cta_row, cta_tile, inst_tile, order;
+  std::vector<int> tiles, cta_row, cta_tile, cta_win, inst_tile, order, inst_n;
   std::vector<int64_t> inst_row;
-  TreeSchedule tree;
+  TreePlan tree;
   int grid_blocks = 0;
   bool grid_mode = false;
   int tile_rows = 0;
   size_t smem = 0;
 };
 
-static size_t smem_bytes(int m) { return ((shared_fixed_bytes(m) + 127) & ~(size_t)127) + kTileBytes; }
+static size_t smem_bytes(int m, size_t tile) {
+  return ((shared_fixed_bytes(m) + 127) & ~(size_t)127) + tile;
+}
 
+// Takes room for max(count, room) entries and uploads count of them (src may be null).
 template <typename X>
-static int up(Arena &a, X *&dst, const X *src, size_t count, cudaStream_t st) {
-  dst = (X *)a.take(sizeof(X) * (count ? count : 1));
+static int up(Arena &a, X *&dst, const X *src, size_t count, cudaStream_t st, size_t room = 1) {
+  dst = (X *)a.take(sizeof(X) * std::max(count, room));
   if (!dst) {
     set_error("arena exhausted");
     return NRT_ENOMEM;
@@ -1784,263 +1399,116 @@ static int up(Arena &a, X *&dst, const X *src, size_t count, cudaStream_t st) {
     if (_rc != NRT_OK) return _rc;  \
   } while (0)
 
-static void build_tree_schedule(const HostPack &host, int cap, bool grid_mode, int ctas,
-                                TreeSchedule &T) {
-  struct Seg {
-    int start, len, prow, parent, level, c1, c2;
-  };
-  std::vector<Seg> segs;
-  std::vector<int> seg_of(host.ntot, -1);
-  std::vector<int> inst_seg(host.ninst + 1, 0);
-  for (int32_t i = 0; i < host.ninst; i++) {
-    const int64_t o = host.off[i], n = host.num_elem[i];
-    int cur = -1;
-    for (int64_t jl = 0; jl < n; jl++) {
-      const int64_t j = o + jl;
-      const Topo &t = host.topo[j];
-      if (t.flags & F_IDENT) {
-        cur = -1;
-        continue;
-      }
-      const bool linked = cur >= 0 && (t.flags & F_UP) && t.mother == j - 1 &&
-                          !(host.topo[j - 1].flags & F_BRANCH) && segs[cur].len < cap;
-      if (linked) {
-        segs[cur].len++;
-      } else {
-        Seg s;
-        s.start = (int)j;
-        s.len = 1;
-        s.prow = (t.flags & F_UP) ? t.mother : -1;
-        s.parent = s.prow >= 0 ? seg_of[s.prow] : -1;
-        s.level = s.parent >= 0 ? segs[s.parent].level + 1 : 0;
-        s.c1 = s.c2 = -1;
-        segs.push_back(s);
-        cur = (int)segs.size() - 1;
-        if (s.parent >= 0) {
-          Seg &p = segs[s.parent];
-          (p.c1 < 0 ? p.c1 : p.c2) = cur;
-        }
-      }
-      seg_of[j] = cur;
-    }
-    inst_seg[i + 1] = (int)segs.size();
-  }
-  // Workers: instances (batch) or CTAs (one tree; each level's segments dealt out to the
-  // CTAs by rows).  Every worker of a cooperative launch sees the same number of levels.
-  const int nwork = grid_mode ? ctas : host.ninst;
-  int max_level = 0;
-  for (const Seg &s : segs) max_level = std::max(max_level, s.level);
-  std::vector<std::vector<std::vector<int>>> lists(nwork);  // [worker][level] -> segments
-  if (grid_mode) {
-    std::vector<std::vector<int>> by_level(max_level + 1);
-    for (int s = 0; s < (int)segs.size(); s++) by_level[segs[s].level].push_back(s);
-    for (int w = 0; w < nwork; w++) lists[w].resize(max_level + 1);
-    std::vector<int64_t> level_rows(max_level + 1, 0);
-    for (int L = 0; L <= max_level; L++)
-      for (int s : by_level[L]) level_rows[L] += segs[s].len;
-    // The top levels, while together they fit one tile, all go to CTA 0: a grid-wide sync
-    // between two of them would wait on CTAs that have nothing to do there.
-    int64_t top_rows = 0;
-    T.local_top = -1;
-    for (int L = 0; L <= max_level && top_rows + level_rows[L] <= cap; L++) {
-      top_rows += level_rows[L];
-      T.local_top = L;
-    }
-    for (int L = 0; L <= max_level; L++) {
-      int64_t acc = 0;
-      for (int s : by_level[L]) {
-        const int w = L <= T.local_top ? 0
-                                       : (int)std::min<int64_t>(nwork - 1, acc * nwork /
-                                                                std::max<int64_t>(level_rows[L], 1));
-        lists[w][L].push_back(s);
-        acc += segs[s].len;
-      }
-    }
-  } else {
-    for (int32_t i = 0; i < host.ninst; i++) {
-      int ml = 0;
-      for (int s = inst_seg[i]; s < inst_seg[i + 1]; s++) ml = std::max(ml, segs[s].level);
-      lists[i].resize(ml + 1);
-      for (int s = inst_seg[i]; s < inst_seg[i + 1]; s++) lists[i][segs[s].level].push_back(s);
-    }
-  }
-  // Emit in (worker, level deepest first, tile) order; renumber segments accordingly.
-  std::vector<int> newid(segs.size(), -1);
-  std::vector<int> order;
-  auto pad = [&]() {
-    T.slot_row.push_back(-1);
-    T.slot_flag.push_back(SL_PAD | SL_FIRST | SL_LAST);
-  };
-  auto new_tile = [&]() {
-    while (T.slot_row.size() & 15) pad();
-    T.tile_seg.push_back((int)order.size());
-    T.tile_slot.push_back((int)T.slot_row.size());
-  };
-  T.work_lev.assign(nwork + 1, 0);
-  for (int w = 0; w < nwork; w++) {
-    T.work_lev[w] = (int)T.lev_tile.size();
-    for (int L = (int)lists[w].size() - 1; L >= 0; L--) {
-      T.lev_tile.push_back((int)T.tile_seg.size());
-      int used = cap;  // forces a new tile for the first segment
-      for (int s : lists[w][L]) {
-        if (used + segs[s].len > cap) {
-          new_tile();
-          used = 0;
-        }
-        newid[s] = (int)order.size();
-        order.push_back(s);
-        T.seg_soff.push_back(used);
-        for (int k = 0; k < segs[s].len; k++) {
-          T.slot_row.push_back(segs[s].start + k);
-          T.slot_flag.push_back((k == 0 ? SL_FIRST : 0) | (k == segs[s].len - 1 ? SL_LAST : 0));
-        }
-        used += segs[s].len;
-      }
-    }
-  }
-  T.work_lev[nwork] = (int)T.lev_tile.size();
-  T.lev_tile.push_back((int)T.tile_seg.size());
-  new_tile();  // sentinel: end of the last tile
-  for (int k = 0; k < 16; k++) pad();  // bulk copies round their size up to 16 bytes
-  for (int s : order) {
-    const Seg &g = segs[s];
-    T.seg_len.push_back(g.len);
-    T.seg_prow.push_back(g.prow);
-    T.seg_c1.push_back(g.c1 >= 0 ? newid[g.c1] : -1);
-    T.seg_c2.push_back(g.c2 >= 0 ? newid[g.c2] : -1);
-  }
-}
-
-// The same schedule for a batch (one worker per instance), built per instance on all host
-// cores and concatenated: every instance's slots are padded to a multiple of 16, which is
-// where the sequential builder's next tile would start, so the result is the same.
-struct InstSchedule {
-  std::vector<int> seg_len, seg_c1, seg_c2, seg_prow, seg_soff, tile_seg, tile_slot, slot_row,
-      lev_tile;
-  std::vector<uint8_t> slot_flag;
+// One instance's pieces: runs of rows linked to the row before them (mother == j - 1),
+// broken after branch points, at identity rows and at window edges.  A piece's parent row
+// (the mother of its first row) is always the last row of another piece.  Level = number of
+// pieces above it; ids count the pieces level by level, deepest level first.
+struct InstPieces {
+  std::vector<int> wbase, pmap, lev_off;
+  std::vector<int4> plink;
+  std::vector<double> pgf;
 };
 
-static void instance_schedule(const HostPack &host, int cap, int32_t i, InstSchedule &L) {
-  struct Seg {
-    int start, len, prow, parent, level, c1, c2;
+static void instance_pieces(const HostPack &host, const uint8_t *rowf, int32_t i, uint8_t *pfl,
+                            uint16_t *wtp, InstPieces &L) {
+  struct Piece {
+    int parent, level, c1, c2;
+    int64_t row;
+    int len;
   };
   const int64_t o = host.off[i], n = host.num_elem[i];
-  std::vector<Seg> segs;
-  std::vector<int> seg_of(n, -1);
-  int cur = -1;
-  for (int64_t jl = 0; jl < n; jl++) {
-    const int64_t j = o + jl;
-    const Topo &t = host.topo[j];
-    if (t.flags & F_IDENT) {
+  const int64_t n4 = (n + kRW - 1) & ~(int64_t)(kRW - 1), nw = (n + kWin - 1) / kWin;
+  constexpr uint8_t keep = R_IDENT | R_UP | R_DOWNR | R_DOWNL | R_FAR;
+  std::vector<Piece> pc;
+  std::vector<int> piece_of(n, -1);
+  L.wbase.resize(nw);
+  int cur = -1, max_level = -1;
+  for (int64_t j = 0; j < nw * kWin; j++) {
+    if (j % kWin == 0) L.wbase[j / kWin] = (int)pc.size();
+    if (j % kRW == 0)
+      wtp[(j / kWin) * kThreads + (j % kWin) / kRW] = (uint16_t)(pc.size() - L.wbase[j / kWin]);
+    if (j >= n) {
+      if (j < n4) pfl[j] = P_IDENT;
+      continue;
+    }
+    const uint8_t f = rowf[j] & keep;
+    pfl[j] = f;
+    if (f & R_IDENT) {
       cur = -1;
       continue;
     }
-    const bool linked = cur >= 0 && (t.flags & F_UP) && t.mother == j - 1 &&
-                        !(host.topo[j - 1].flags & F_BRANCH) && segs[cur].len < cap;
-    if (linked) {
-      segs[cur].len++;
-    } else {
-      Seg s;
-      s.start = (int)j;
-      s.len = 1;
-      s.prow = (t.flags & F_UP) ? t.mother : -1;
-      s.parent = s.prow >= 0 ? seg_of[s.prow - o] : -1;
-      s.level = s.parent >= 0 ? segs[s.parent].level + 1 : 0;
-      s.c1 = s.c2 = -1;
-      segs.push_back(s);
-      cur = (int)segs.size() - 1;
-      if (s.parent >= 0) {
-        Seg &p = segs[s.parent];
-        (p.c1 < 0 ? p.c1 : p.c2) = cur;
+    const bool linked = cur >= 0 && j % kWin != 0 && (f & R_UP) && !(f & R_FAR) &&
+                        !(host.topo[o + j - 1].flags & F_BRANCH);
+    if (!linked) {
+      const int64_t m = (f & R_UP) ? host.topo[o + j].mother - o : -1;
+      Piece p{m >= 0 ? piece_of[m] : -1, 0, -1, -1, o + j, 0};
+      if (p.parent >= 0) {
+        p.level = pc[p.parent].level + 1;
+        Piece &q = pc[p.parent];
+        (q.c1 < 0 ? q.c1 : q.c2) = (int)pc.size();
       }
+      max_level = std::max(max_level, p.level);
+      pc.push_back(p);
+      cur = (int)pc.size() - 1;
+      pfl[j] |= P_FIRST;
     }
-    seg_of[jl] = cur;
+    piece_of[j] = cur;
+    pc[cur].len++;
+    // the piece ends here unless the next row continues it
+    const bool more = j + 1 < n && (j + 1) % kWin != 0 && !(rowf[j + 1] & R_IDENT) &&
+                      (rowf[j + 1] & R_UP) && !(rowf[j + 1] & R_FAR) &&
+                      !(host.topo[o + j].flags & F_BRANCH);
+    if (!more) pfl[j] |= P_LAST;
   }
-  int ml = 0;
-  for (const Seg &s : segs) ml = std::max(ml, s.level);
-  std::vector<std::vector<int>> lists(segs.empty() ? 0 : ml + 1);
-  for (int s = 0; s < (int)segs.size(); s++) lists[segs[s].level].push_back(s);
-  std::vector<int> newid(segs.size(), -1), order;
-  auto pad = [&]() {
-    L.slot_row.push_back(-1);
-    L.slot_flag.push_back(SL_PAD | SL_FIRST | SL_LAST);
-  };
-  for (int lv = (int)lists.size() - 1; lv >= 0; lv--) {
-    L.lev_tile.push_back((int)L.tile_seg.size());
-    int used = cap;
-    for (int s : lists[lv]) {
-      if (used + segs[s].len > cap) {
-        while (L.slot_row.size() & 15) pad();
-        L.tile_seg.push_back((int)order.size());
-        L.tile_slot.push_back((int)L.slot_row.size());
-        used = 0;
-      }
-      newid[s] = (int)order.size();
-      order.push_back(s);
-      L.seg_soff.push_back(used);
-      for (int q = 0; q < segs[s].len; q++) {
-        L.slot_row.push_back(segs[s].start + q);
-        L.slot_flag.push_back((q == 0 ? SL_FIRST : 0) | (q == segs[s].len - 1 ? SL_LAST : 0));
-      }
-      used += segs[s].len;
-    }
-  }
-  while (L.slot_row.size() & 15) pad();
-  for (int s : order) {
-    const Seg &g = segs[s];
-    L.seg_len.push_back(g.len);
-    L.seg_prow.push_back(g.prow);
-    L.seg_c1.push_back(g.c1 >= 0 ? newid[g.c1] : -1);
-    L.seg_c2.push_back(g.c2 >= 0 ? newid[g.c2] : -1);
+  const int np = (int)pc.size(), nl = max_level + 1;
+  std::vector<int> at(nl + 1, 0);
+  for (const Piece &p : pc) at[max_level - p.level + 1]++;  // deepest level first
+  for (int e = 0; e < nl; e++) at[e + 1] += at[e];
+  L.lev_off.assign(at.begin() + 1, at.end());
+  L.pmap.resize(np);
+  L.plink.resize(np);
+  for (int q = 0; q < np; q++) L.pmap[q] = at[max_level - pc[q].level]++;
+  auto id = [&](int q) { return q >= 0 ? L.pmap[q] : -1; };
+  L.pgf.resize(np);
+  for (int q = 0; q < np; q++) {
+    L.plink[L.pmap[q]] = make_int4(id(pc[q].c1), id(pc[q].c2), id(pc[q].parent), pc[q].len == 1);
+    L.pgf[L.pmap[q]] = host.gax[pc[q].row];
   }
 }
 
-static void build_tree_schedule_batch(const HostPack &host, int cap, TreeSchedule &T) {
+static void build_tree_plan(const HostPack &host, const uint8_t *rowf, int64_t ld, TreePlan &T) {
   const int32_t ni = host.ninst;
-  std::vector<InstSchedule> loc(ni);
-  parallel_for(ni, [&](int64_t i) { instance_schedule(host, cap, (int32_t)i, loc[i]); });
-  // bases: segments, slots, tiles, level entries
-  std::vector<size_t> sb(ni + 1, 0), lb(ni + 1, 0), tb(ni + 1, 0), eb(ni + 1, 0);
-  for (int32_t i = 0; i < ni; i++) {
-    sb[i + 1] = sb[i] + loc[i].seg_len.size();
-    lb[i + 1] = lb[i] + loc[i].slot_row.size();
-    tb[i + 1] = tb[i] + loc[i].tile_seg.size();
-    eb[i + 1] = eb[i] + loc[i].lev_tile.size();
-  }
-  T.seg_len.resize(sb[ni]); T.seg_c1.resize(sb[ni]); T.seg_c2.resize(sb[ni]);
-  T.seg_prow.resize(sb[ni]); T.seg_soff.resize(sb[ni]);
-  T.slot_row.resize(lb[ni]); T.slot_flag.resize(lb[ni]);
-  T.tile_seg.resize(tb[ni]); T.tile_slot.resize(tb[ni]);
-  T.lev_tile.resize(eb[ni]);
-  T.work_lev.assign(ni + 1, 0);
+  std::vector<InstPieces> loc(ni);
+  T.inst_win.resize(ni + 1);
+  T.inst_piece.resize(ni + 1);
+  T.inst_lev.resize(ni + 1);
+  T.inst_win[0] = T.inst_piece[0] = T.inst_lev[0] = 0;
+  for (int32_t i = 0; i < ni; i++)
+    T.inst_win[i + 1] = T.inst_win[i] + (host.num_elem[i] + kWin - 1) / kWin;
+  T.pfl.resize(ld);
+  T.wtp.resize((size_t)T.inst_win[ni] * kThreads);
   parallel_for(ni, [&](int64_t i) {
-    const InstSchedule &L = loc[i];
-    const int s0 = (int)sb[i], l0 = (int)lb[i], t0 = (int)tb[i];
-    for (size_t q = 0; q < L.seg_len.size(); q++) {
-      T.seg_len[s0 + q] = L.seg_len[q];
-      T.seg_prow[s0 + q] = L.seg_prow[q];
-      T.seg_soff[s0 + q] = L.seg_soff[q];
-      T.seg_c1[s0 + q] = L.seg_c1[q] >= 0 ? L.seg_c1[q] + s0 : -1;
-      T.seg_c2[s0 + q] = L.seg_c2[q] >= 0 ? L.seg_c2[q] + s0 : -1;
-    }
-    std::copy(L.slot_row.begin(), L.slot_row.end(), T.slot_row.begin() + l0);
-    std::copy(L.slot_flag.begin(), L.slot_flag.end(), T.slot_flag.begin() + l0);
-    for (size_t q = 0; q < L.tile_seg.size(); q++) {
-      T.tile_seg[t0 + q] = L.tile_seg[q] + s0;
-      T.tile_slot[t0 + q] = L.tile_slot[q] + l0;
-    }
-    for (size_t q = 0; q < L.lev_tile.size(); q++) T.lev_tile[eb[i] + q] = L.lev_tile[q] + t0;
-    T.work_lev[i] = (int)eb[i];
+    instance_pieces(host, rowf + host.off[i], (int32_t)i, T.pfl.data() + host.off[i],
+                    T.wtp.data() + (size_t)T.inst_win[i] * kThreads, loc[i]);
   });
-  T.work_lev[ni] = (int)T.lev_tile.size();
-  T.lev_tile.push_back((int)T.tile_seg.size());
-  // sentinel tile (the slot count is already a multiple of 16), then the copy overrun pad
-  T.tile_seg.push_back((int)T.seg_len.size());
-  T.tile_slot.push_back((int)T.slot_row.size());
-  for (int q = 0; q < 16; q++) {
-    T.slot_row.push_back(-1);
-    T.slot_flag.push_back(SL_PAD | SL_FIRST | SL_LAST);
+  for (int32_t i = 0; i < ni; i++) {
+    T.inst_piece[i + 1] = T.inst_piece[i] + (int)loc[i].pmap.size();
+    T.inst_lev[i + 1] = T.inst_lev[i] + (int)loc[i].lev_off.size();
+    T.max_pieces = std::max(T.max_pieces, (int)loc[i].pmap.size());
   }
+  T.wbase.resize(T.inst_win[ni]);
+  T.pmap.resize(T.inst_piece[ni]);
+  T.plink.resize(T.inst_piece[ni]);
+  T.pgf.resize(T.inst_piece[ni]);
+  T.lev_off.resize(T.inst_lev[ni]);
+  parallel_for(ni, [&](int64_t i) {
+    const InstPieces &L = loc[i];
+    std::copy(L.wbase.begin(), L.wbase.end(), T.wbase.begin() + T.inst_win[i]);
+    std::copy(L.pmap.begin(), L.pmap.end(), T.pmap.begin() + T.inst_piece[i]);
+    std::copy(L.plink.begin(), L.plink.end(), T.plink.begin() + T.inst_piece[i]);
+    std::copy(L.pgf.begin(), L.pgf.end(), T.pgf.begin() + T.inst_piece[i]);
+    std::copy(L.lev_off.begin(), L.lev_off.end(), T.lev_off.begin() + T.inst_lev[i]);
+  });
 }
 
 // Groups pieces [pa, pb) into tiles whose row span fits the shared-memory staging area.
@@ -2068,6 +1536,7 @@ int Engine::implicit_plan(size_t &bytes) {
   // Row structure (flags) per element.  The validator guaranteed the reference
   // numbering: mother < j, DR == j + 1 off terminals, terminals follow their mother.
   S.rowf.resize(N);
+  static_assert(kRowAlign == kRW, "instances start on whole row groups");
   parallel_for(ni, [&](int64_t i) {
     const int64_t o = host.off[i], n = host.num_elem[i];
     for (int64_t jl = 0; jl < n; jl++) {
@@ -2097,12 +1566,15 @@ int Engine::implicit_plan(size_t &bytes) {
       }
       S.rowf[j] = rf;
     }
+    for (int64_t j = o + n; j < host.off[i + 1]; j++) S.rowf[j] = R_IDENT;  // padding
   });
-  // Segment pieces: maximal runs of consecutive physical rows linked to their
-  // predecessor (mother == j - 1 with a mother column), cut at kMaxPiece rows.
   S.inst_row.assign(host.off.begin(), host.off.end());
+  S.inst_n.assign(host.num_elem.begin(), host.num_elem.end());
+  // Segment pieces (segment preconditioner): maximal runs of consecutive physical rows
+  // linked to their predecessor (mother == j - 1 with a mother column), cut at kMaxPiece rows.
+  const bool tree = opt.precond == NRT_PRECOND_TREE, segs = opt.precond == NRT_PRECOND_SEGMENT;
   std::vector<int> inst_piece(ni + 1, 0);
-  {
+  if (segs) {
     std::vector<std::vector<int2>> ip(ni);  // per instance, then concatenated in order
     parallel_for(ni, [&](int64_t i) {
       const int64_t o = host.off[i], n = host.num_elem[i];
@@ -2128,106 +1600,130 @@ int Engine::implicit_plan(size_t &bytes) {
     });
   }
   const int np = (int)S.pieces.size();
-  const size_t tb = opt.precision == NRT_MIXED ? 4 : 8;
+  const bool mixed = opt.precision == NRT_MIXED;
+  const size_t tb = mixed ? 4 : 8;
+  const int64_t ld = (N + kRW - 1) & ~(int64_t)(kRW - 1);
   S.tile_rows = (int)(kTileBytes / (4 * tb));
+  if (tree) build_tree_plan(host, S.rowf.data(), ld, S.tree);
   int dev_sms = 0;
   NRT_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
-  S.smem = smem_bytes(opt.restart);
-  const bool mixed = opt.precision == NRT_MIXED;
   S.grid_mode = ni == 1 && opt.schedule == 0;
+  const void *kern = mixed ? (S.grid_mode ? (const void *)implicit_steps<float, kGrid>
+                                          : (const void *)implicit_steps<float, kBlock>)
+                           : (S.grid_mode ? (const void *)implicit_steps<double, kGrid>
+                                          : (const void *)implicit_steps<double, kBlock>);
+  // shared memory: the segment preconditioner's staging, or the tree walk's numbers of
+  // every piece -- up to kTileBytes, which keeps four CTAs on an SM, or in the one-tree launch
+  // (at most two per SM) up to kWalkBytes; larger walks run in device memory
+  size_t tile = 0;
+  if (segs) tile = kTileBytes;
+  if (tree) {
+    const size_t cap = S.grid_mode ? kWalkBytes : kTileBytes;
+    S.iv.walk_cap = (int)std::min<size_t>(cap / walk_bytes(tb), (size_t)S.tree.max_pieces);
+    tile = (size_t)S.iv.walk_cap * walk_bytes(tb);
+  }
+  S.smem = smem_bytes(opt.restart, tile);
+  // The limit is the function's, not the handle's: all that a CTA can have, so that handles
+  // of any size launch in any order.
+  int smem_limit = 0;
+  cudaFuncAttributes fa;
+  NRT_CUDA(cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  NRT_CUDA(cudaFuncGetAttributes(&fa, kern));
+  smem_limit -= (int)fa.sharedSizeBytes;
+  NRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit));
+  int per_sm = 0;
+  NRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, S.smem));
+  if (per_sm < 1) {
+    set_error("implicit kernel does not fit on an SM");
+    return NRT_EDEVICE;
+  }
   if (S.grid_mode) {
-    // One tree: cooperative grid, row ranges aligned with pieces.
-    int per_sm = 0;
-    auto kern = mixed ? implicit_steps<float, true> : implicit_steps<double, true>;
-    NRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem));
-    NRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, S.smem));
-    if (per_sm < 1) {
-      set_error("implicit kernel does not fit on an SM");
-      return NRT_EDEVICE;
-    }
-    const int64_t want = (N + 4 * kThreads - 1) / (4 * kThreads);
+    // One tree: a cooperative grid.  Segment preconditioner: row ranges aligned with its
+    // pieces.  Otherwise the row passes and the windows are each split evenly: the rows over
+    // as many CTAs as leave each kRowsPerCta (FP64: an SM evaluates one HH row in about 60
+    // cycles of its FP64 pipe, so small trees gain from every SM), the windows over the same
+    // CTAs as far as they go.
+    const int64_t rows_per_cta = segs ? 4 * kThreads : (mixed ? 256 : 64);
+    const int64_t want = (N + rows_per_cta - 1) / rows_per_cta;
     int G = (int)std::min<int64_t>((int64_t)dev_sms * std::min(per_sm, 2), std::max<int64_t>(1, want));
     G = std::max(1, std::min(G, 4096));
-    std::vector<int> cta_piece(G + 1, np);
     S.cta_row.assign(G + 1, (int)N);
-    int q = 0;
-    for (int c = 0; c < G; c++) {
-      const int64_t goal = (N * (int64_t)c) / G;
-      while (q < np && S.pieces[q].x + S.pieces[q].y <= goal) q++;
-      cta_piece[c] = std::min(q, np);
-      S.cta_row[c] = c == 0 ? 0 : (q < np ? S.pieces[q].x : (int)N);
-    }
-    S.cta_row[0] = 0;
-    cta_piece[0] = 0;
-    for (int c = 1; c <= G; c++) {
-      S.cta_row[c] = std::max(S.cta_row[c], S.cta_row[c - 1]);
-      cta_piece[c] = std::max(cta_piece[c], cta_piece[c - 1]);
-    }
-    S.cta_row[G] = (int)N;
-    cta_piece[G] = np;
     S.cta_tile.assign(G + 1, 0);
-    for (int c = 0; c < G; c++) {
-      S.cta_tile[c] = (int)S.tiles.size();
-      make_tiles(S.pieces, cta_piece[c], cta_piece[c + 1], S.tile_rows, S.tiles);
+    S.cta_win.assign(G + 1, 0);
+    if (segs) {
+      std::vector<int> cta_piece(G + 1, np);
+      int q = 0;
+      for (int c = 0; c < G; c++) {
+        const int64_t goal = (N * (int64_t)c) / G;
+        while (q < np && S.pieces[q].x + S.pieces[q].y <= goal) q++;
+        cta_piece[c] = std::min(q, np);
+        S.cta_row[c] = c == 0 ? 0 : (q < np ? S.pieces[q].x : (int)N);
+      }
+      S.cta_row[0] = 0;
+      cta_piece[0] = 0;
+      for (int c = 1; c <= G; c++) {
+        S.cta_row[c] = std::max(S.cta_row[c], S.cta_row[c - 1]);
+        cta_piece[c] = std::max(cta_piece[c], cta_piece[c - 1]);
+      }
+      S.cta_row[G] = (int)N;
+      cta_piece[G] = np;
+      for (int c = 0; c < G; c++) {
+        S.cta_tile[c] = (int)S.tiles.size();
+        make_tiles(S.pieces, cta_piece[c], cta_piece[c + 1], S.tile_rows, S.tiles);
+      }
+      S.cta_tile[G] = (int)S.tiles.size();
+    } else {
+      const int64_t nw = tree ? S.tree.inst_win[1] : 0;
+      for (int c = 0; c <= G; c++) {
+        S.cta_row[c] = (int)(N * (int64_t)c / G);
+        S.cta_win[c] = (int)(nw * c / G);
+      }
     }
-    S.cta_tile[G] = (int)S.tiles.size();
     S.grid_blocks = G;
   } else {
     S.order.resize(ni);
     for (int32_t i = 0; i < ni; i++) S.order[i] = i;
     std::stable_sort(S.order.begin(), S.order.end(),
                      [&](int a, int b) { return host.num_elem[a] > host.num_elem[b]; });
-    int per_sm = 0;
-    auto kern = mixed ? implicit_steps<float, false> : implicit_steps<double, false>;
-    NRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem));
-    NRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, S.smem));
     // persistent CTAs: as many per SM as fit, or at most tile_ctas_per_sm (a tuned shape;
     // each instance is one CTA's from start to end, so results do not depend on it)
     if (opt.tile_ctas_per_sm > 0) per_sm = std::min(per_sm, opt.tile_ctas_per_sm);
     S.grid_blocks = std::max(1, std::min<int>(dev_sms * std::max(per_sm, 1), ni));
     S.inst_tile.assign(ni + 1, 0);
-    for (int32_t i = 0; i < ni; i++) {
+    for (int32_t i = 0; segs && i < ni; i++) {
       S.inst_tile[i] = (int)S.tiles.size();
       make_tiles(S.pieces, inst_piece[i], inst_piece[i + 1], S.tile_rows, S.tiles);
     }
     S.inst_tile[ni] = (int)S.tiles.size();
   }
   S.tiles.push_back(np);  // sentinel: end piece of the last tile
-  const bool tree = opt.precond == NRT_PRECOND_TREE;
-  S.iv.local_top = -1;
-  if (tree) {
-    // staging slots: three T rows, the slot row and the slot flag per slot
-    S.iv.tree_cap = (int)(kTileBytes / (3 * tb + 5)) & ~15;
-    if (S.grid_mode)
-      build_tree_schedule(host, S.iv.tree_cap, true, S.grid_blocks, S.tree);
-    else
-      build_tree_schedule_batch(host, S.iv.tree_cap, S.tree);
-    S.iv.local_top = S.tree.local_top;
-  }
   // device bytes, in the order implicit_init takes them
   const int m = opt.restart;
   size_t b = 0;
-  b += al256(N);                                            // rowf
-  b += 5 * al256(8 * N);                                    // cmdt, g64, wdx64, kdx64, inp64
-  b += 2 * al256(8 * N);                                    // diag, rhs
-  b += al256(4 * N) + al256(tb * N);                        // gf, cdiag
-  b += 2 * al256(tb * N * (m + 1)) + 3 * al256(tb * N);     // Wb, Z, y, pd, pc
+  b += al256(ld);                                           // rowf
+  b += 5 * al256(8 * ld);                                   // cmdt, g64, wdx64, kdx64, inp64
+  b += 2 * al256(8 * ld);                                   // diag, rhs
+  b += al256(4 * ld) + al256(tb * ld);                      // gf, cdiag
+  b += 2 * al256(tb * ld * (m + 1)) + al256(tb * ld);       // Wb, Z, y
+  if (segs) b += 2 * al256(tb * ld);                        // pd, pc
   b += al256(sizeof(int2) * std::max<size_t>(1, S.pieces.size()));
   b += al256(4 * S.tiles.size());
   if (S.grid_mode)
-    b += al256(4 * S.cta_row.size()) + al256(4 * S.cta_tile.size());
+    b += al256(4 * S.cta_row.size()) + al256(4 * S.cta_tile.size()) + al256(4 * S.cta_win.size());
   else
     b += al256(4 * S.inst_tile.size()) + al256(4 * S.order.size());
-  b += al256(8 * S.inst_row.size()) + 2 * al256(4) + al256(sizeof(double) * 2 * 4096 * kMaxDots);
+  b += 2 * al256(8 * S.inst_row.size()) + al256(4 * S.inst_n.size());
+  b += 2 * al256(4) + al256(sizeof(double) * 2 * 4096 * kMaxDots);
   b += al256(sizeof(InstStat) * ni) + al256(sizeof(PackView)) + al256(sizeof(ImView));
   if (tree) {
-    const TreeSchedule &T = S.tree;
-    const size_t ns = T.slot_row.size(), nseg = std::max<size_t>(1, T.seg_len.size());
-    b += 5 * al256(4 * nseg);                               // seg_len, c1, c2, prow, soff
-    b += al256(4 * T.tile_seg.size()) + al256(4 * T.tile_slot.size()) + al256(4 * ns) + al256(ns);
-    b += al256(4 * T.lev_tile.size()) + al256(4 * T.work_lev.size());
-    b += 4 * al256(tb * ns);                                // sg, sinv, se, sy
-    b += 2 * al256(tb * nseg);                              // exp_d, exp_b
+    const TreePlan &T = S.tree;
+    const size_t npc = std::max<size_t>(1, T.pmap.size());
+    b += al256(ld) + al256(2 * T.wtp.size()) + al256(4 * T.wbase.size());
+    b += al256(4 * npc) + al256(16 * npc) + al256(4 * std::max<size_t>(1, T.lev_off.size()));
+    b += 3 * al256(4 * (size_t)(ni + 1));                   // inst_win, inst_piece, inst_lev
+    b += 2 * al256(4 * tb * npc) + al256(8 * tb * npc) + al256(walk_bytes(tb) * npc);  // pmob, pstat, pval, gwalk
+    b += al256(8 * npc) + al256(32 * npc);                  // pgf, pxb
+    b += 4 * al256(tb * ld);                                // tinv, te, tbeta, talpha
   }
   bytes = b + 4096;
   return NRT_OK;
@@ -2243,7 +1739,10 @@ int Engine::implicit_init() {
                            cudaMemcpyHostToDevice, stream));
   cudaStream_t st = stream;
   ImView &iv = S.iv;
+  const int64_t ld = (N + kRW - 1) & ~(int64_t)(kRW - 1);
+  const bool tree = opt.precond == NRT_PRECOND_TREE, segs = opt.precond == NRT_PRECOND_SEGMENT;
   iv.ntot = N;
+  iv.ld = ld;
   iv.m = opt.restart;
   iv.precond = opt.precond;
   iv.krylov = opt.krylov;
@@ -2257,7 +1756,7 @@ int Engine::implicit_init() {
   iv.ninst = ni;
   iv.tile_rows = S.tile_rows;
   uint8_t *pr;
-  TRYI(up(arena, pr, S.rowf.data(), N, st)); iv.rowf = pr;
+  TRYI(up(arena, pr, S.rowf.data(), N, st, ld)); iv.rowf = pr;
   // c_m dX / dT and the FP32 conductances are staged (filled in parallel, no zero fill
   // first); the other FP64 rows go up straight from the host pack
   std::unique_ptr<double[]> cmdt_b(new double[N]);
@@ -2271,33 +1770,33 @@ int Engine::implicit_init() {
     }
   });
   double *p;
-  TRYI(up(arena, p, cmdt, N, st)); iv.cmdt = p;
-  TRYI(up(arena, p, host.gax.data(), N, st)); iv.g64 = p;
-  TRYI(up(arena, p, host.wdx.data(), N, st)); iv.wdx64 = p;
-  TRYI(up(arena, p, host.kdx.data(), N, st)); iv.kdx64 = p;
-  TRYI(up(arena, p, host.inp.data(), N, st)); iv.inp64 = p;
-  TRYI(up(arena, iv.diag, (const double *)nullptr, N, st));
-  TRYI(up(arena, iv.rhs, (const double *)nullptr, N, st));
+  TRYI(up(arena, p, cmdt, N, st, ld)); iv.cmdt = p;
+  TRYI(up(arena, p, host.gax.data(), N, st, ld)); iv.g64 = p;
+  TRYI(up(arena, p, host.wdx.data(), N, st, ld)); iv.wdx64 = p;
+  TRYI(up(arena, p, host.kdx.data(), N, st, ld)); iv.kdx64 = p;
+  TRYI(up(arena, p, host.inp.data(), N, st, ld)); iv.inp64 = p;
+  TRYI(up(arena, iv.diag, (const double *)nullptr, ld, st));
+  TRYI(up(arena, iv.rhs, (const double *)nullptr, ld, st));
   float *pf;
-  TRYI(up(arena, pf, gf, N, st)); iv.gf = pf;
-  iv.cdiag = arena.take(tb * N);
+  TRYI(up(arena, pf, gf, N, st, ld)); iv.gf = pf;
+  iv.cdiag = arena.take(tb * ld);
   if (!iv.cdiag) {
     set_error("arena exhausted");
     return NRT_ENOMEM;
   }
   const int m = opt.restart;
-  iv.Wb = arena.take(tb * N * (m + 1));
-  iv.Z = arena.take(tb * N * (m + 1));
-  iv.yv = arena.take(tb * N);
-  iv.pcd = arena.take(tb * N);
-  iv.pcc = arena.take(tb * N);
-  if (!iv.Wb || !iv.Z || !iv.yv || !iv.pcd || !iv.pcc) {
+  iv.Wb = arena.take(tb * ld * (m + 1));
+  iv.Z = arena.take(tb * ld * (m + 1));
+  iv.yv = arena.take(tb * ld);
+  iv.pcd = segs ? arena.take(tb * ld) : nullptr;
+  iv.pcc = segs ? arena.take(tb * ld) : nullptr;
+  if (!iv.Wb || !iv.Z || !iv.yv || (segs && (!iv.pcd || !iv.pcc))) {
     set_error("arena exhausted (Krylov workspace)");
     return NRT_ENOMEM;
   }
-  NRT_CUDA(cudaMemsetAsync(iv.Wb, 0, tb * N * (m + 1), st));
-  NRT_CUDA(cudaMemsetAsync(iv.Z, 0, tb * N * (m + 1), st));
-  NRT_CUDA(cudaMemsetAsync(iv.yv, 0, tb * N, st));
+  NRT_CUDA(cudaMemsetAsync(iv.Wb, 0, tb * ld * (m + 1), st));
+  NRT_CUDA(cudaMemsetAsync(iv.Z, 0, tb * ld * (m + 1), st));
+  NRT_CUDA(cudaMemsetAsync(iv.yv, 0, tb * ld, st));
   int2 *pc;
   TRYI(up(arena, pc, S.pieces.data(), S.pieces.size(), st)); iv.pieces = pc;
   int *pi;
@@ -2305,62 +1804,55 @@ int Engine::implicit_init() {
   if (S.grid_mode) {
     TRYI(up(arena, pi, S.cta_row.data(), S.cta_row.size(), st)); iv.cta_row = pi;
     TRYI(up(arena, pi, S.cta_tile.data(), S.cta_tile.size(), st)); iv.cta_tile = pi;
+    TRYI(up(arena, pi, S.cta_win.data(), S.cta_win.size(), st)); iv.cta_win = pi;
   } else {
     TRYI(up(arena, pi, S.inst_tile.data(), S.inst_tile.size(), st)); iv.inst_tile = pi;
     TRYI(up(arena, pi, S.order.data(), S.order.size(), st)); iv.order = pi;
   }
   int64_t *pl;
   TRYI(up(arena, pl, S.inst_row.data(), S.inst_row.size(), st)); iv.inst_row = pl;
+  TRYI(up(arena, pi, S.inst_n.data(), S.inst_n.size(), st)); iv.inst_n = pi;
+  std::vector<int64_t> out(ni + 1, 0);
+  for (int32_t i = 0; i < ni; i++) out[i + 1] = out[i] + host.num_elem[i];
+  TRYI(up(arena, pl, out.data(), out.size(), st)); iv.inst_out = pl;
   TRYI(up(arena, iv.queue, (const int *)nullptr, 1, st));
   TRYI(up(arena, iv.err, (const int *)nullptr, 1, st));
   NRT_CUDA(cudaMemsetAsync(iv.err, 0, sizeof(int), st));
   TRYI(up(arena, iv.partials, (const double *)nullptr, (size_t)2 * 4096 * kMaxDots, st));
   std::vector<InstStat> zero(ni, InstStat{0, 0, 0, 0.0, 0, 0, 0, 0, 0});
   TRYI(up(arena, iv.stats, zero.data(), ni, st));
-  iv.work_lev = nullptr;
-  std::vector<char> sgbuf;
-  if (opt.precond == NRT_PRECOND_TREE) {
-    const TreeSchedule &T = S.tree;
-    const size_t ns = T.slot_row.size(), nseg = std::max<size_t>(1, T.seg_len.size());
-    TRYI(up(arena, pi, T.seg_len.data(), T.seg_len.size(), st)); iv.seg_len = pi;
-    TRYI(up(arena, pi, T.seg_c1.data(), T.seg_c1.size(), st)); iv.seg_c1 = pi;
-    TRYI(up(arena, pi, T.seg_c2.data(), T.seg_c2.size(), st)); iv.seg_c2 = pi;
-    TRYI(up(arena, pi, T.seg_prow.data(), T.seg_prow.size(), st)); iv.seg_prow = pi;
-    TRYI(up(arena, pi, T.seg_soff.data(), T.seg_soff.size(), st)); iv.seg_soff = pi;
-    TRYI(up(arena, pi, T.tile_seg.data(), T.tile_seg.size(), st)); iv.tile_seg = pi;
-    TRYI(up(arena, pi, T.tile_slot.data(), T.tile_slot.size(), st)); iv.tile_slot = pi;
-    TRYI(up(arena, pi, T.slot_row.data(), ns, st)); iv.srow = pi;
-    uint8_t *pf8;
-    TRYI(up(arena, pf8, T.slot_flag.data(), ns, st)); iv.sflag = pf8;
-    TRYI(up(arena, pi, T.lev_tile.data(), T.lev_tile.size(), st)); iv.lev_tile = pi;
-    TRYI(up(arena, pi, T.work_lev.data(), T.work_lev.size(), st)); iv.work_lev = pi;
-    // static per-slot conductance to the mother (0 on a row without that column)
-    sgbuf.resize(tb * ns);
-    parallel_ranges((int64_t)ns, [&](int64_t a, int64_t b) {
-      for (int64_t k = a; k < b; k++) {
-        const int r = T.slot_row[k];
-        const double g = (r >= 0 && (host.topo[r].flags & F_UP)) ? host.gax[r] : 0.0;
-        if (mixed)
-          ((float *)sgbuf.data())[k] = (float)g;
-        else
-          ((double *)sgbuf.data())[k] = g;
-      }
-    });
-    void *sgd = arena.take(tb * ns);
-    iv.sinv = arena.take(tb * ns);
-    iv.se = arena.take(tb * ns);
-    iv.sy = arena.take(tb * ns);
-    iv.exp_d = arena.take(tb * nseg);
-    iv.exp_b = arena.take(tb * nseg);
-    if (!iv.cdiag || !sgd || !iv.sinv || !iv.se || !iv.sy || !iv.exp_d || !iv.exp_b) {
+  if (tree) {
+    const TreePlan &T = S.tree;
+    const size_t npc = std::max<size_t>(1, T.pmap.size());
+    uint8_t *p8;
+    uint16_t *p16;
+    int4 *p4;
+    TRYI(up(arena, p8, T.pfl.data(), T.pfl.size(), st)); iv.pfl = p8;
+    TRYI(up(arena, p16, T.wtp.data(), T.wtp.size(), st)); iv.wtp = p16;
+    TRYI(up(arena, pi, T.wbase.data(), T.wbase.size(), st)); iv.wbase = pi;
+    TRYI(up(arena, pi, T.pmap.data(), T.pmap.size(), st)); iv.pmap = pi;
+    TRYI(up(arena, p4, T.plink.data(), T.plink.size(), st)); iv.plink = p4;
+    TRYI(up(arena, pi, T.lev_off.data(), T.lev_off.size(), st)); iv.lev_off = pi;
+    TRYI(up(arena, pi, T.inst_win.data(), T.inst_win.size(), st)); iv.inst_win = pi;
+    TRYI(up(arena, pi, T.inst_piece.data(), T.inst_piece.size(), st)); iv.inst_piece = pi;
+    TRYI(up(arena, pi, T.inst_lev.data(), T.inst_lev.size(), st)); iv.inst_lev = pi;
+    iv.pmob = arena.take(4 * tb * npc);
+    double *pd;
+    TRYI(up(arena, pd, T.pgf.data(), T.pgf.size(), st)); iv.pgf = pd;
+    iv.npieces = (int64_t)T.pmap.size();
+    iv.pstat = arena.take(4 * tb * npc);
+    iv.pval = arena.take(8 * tb * npc);
+    iv.pxb = (double *)arena.take(32 * npc);
+    iv.gwalk = arena.take(walk_bytes(tb) * npc);
+    iv.tinv = arena.take(tb * ld);
+    iv.te = arena.take(tb * ld);
+    iv.tbeta = arena.take(tb * ld);
+    iv.talpha = arena.take(tb * ld);
+    if (!iv.pmob || !iv.pstat || !iv.pval || !iv.pxb || !iv.gwalk || !iv.tinv || !iv.te || !iv.tbeta ||
+        !iv.talpha) {
       set_error("arena exhausted (tree preconditioner)");
       return NRT_ENOMEM;
     }
-    NRT_CUDA(cudaMemcpyAsync(sgd, sgbuf.data(), tb * ns, cudaMemcpyHostToDevice, st));
-    iv.sg = sgd;
-    NRT_CUDA(cudaMemsetAsync(iv.sinv, 0, tb * ns, st));
-    NRT_CUDA(cudaMemsetAsync(iv.se, 0, tb * ns, st));
-    NRT_CUDA(cudaMemsetAsync(iv.sy, 0, tb * ns, st));
   }
   S.d_pv = (PackView *)arena.take(sizeof(PackView));
   S.d_iv = (ImView *)arena.take(sizeof(ImView));
@@ -2387,10 +1879,10 @@ static int implicit_launch(Engine &e, int nsteps, int force) {
   void *args[] = {&pv, &iv, &nsteps, &force, &V0, &V1, &cur, &rec};
   const bool mixed = e.opt.precision == NRT_MIXED;
   if (S.grid_mode) {
-    const void *k = mixed ? (const void *)implicit_steps<float, true> : (const void *)implicit_steps<double, true>;
+    const void *k = mixed ? (const void *)implicit_steps<float, kGrid> : (const void *)implicit_steps<double, kGrid>;
     NRT_CUDA(cudaLaunchCooperativeKernel(k, dim3(S.grid_blocks), dim3(kThreads), args, S.smem, e.stream));
   } else {
-    const void *k = mixed ? (const void *)implicit_steps<float, false> : (const void *)implicit_steps<double, false>;
+    const void *k = mixed ? (const void *)implicit_steps<float, kBlock> : (const void *)implicit_steps<double, kBlock>;
     NRT_CUDA(cudaLaunchKernel(k, dim3(S.grid_blocks), dim3(kThreads), args, S.smem, e.stream));
   }
   count_launch_on(e.stream);
@@ -2465,6 +1957,32 @@ int implicit_check(Engine &e) {
                      : "explicit step: a bounded wait for its tile copies expired");
     return NRT_EDEVICE;
   }
+  return NRT_OK;
+}
+
+__global__ void compact_rows(const double *__restrict__ V, double *__restrict__ out,
+                             const int64_t *__restrict__ from, const int *__restrict__ n,
+                             const int64_t *__restrict__ to) {
+  const int i = blockIdx.x;
+  const double *src = V + from[i];
+  double *dst = out + to[i];
+  for (int j = threadIdx.x; j < n[i]; j += blockDim.x) dst[j] = src[j];
+}
+
+// The Krylov workspace, dead between steps, takes the packed copy: Wb holds m + 1 >= 2 rows
+// of at least 4 bytes each.
+int implicit_compact(Engine &e, const double *&src, int64_t &n) {
+  const int32_t ni = e.host.ninst;
+  int64_t total = 0;
+  for (int32_t i = 0; i < ni; i++) total += e.host.num_elem[i];
+  n = total;
+  if (total == e.host.ntot) return NRT_OK;  // no padding
+  ImplicitState &S = *e.im;
+  double *out = (double *)S.iv.Wb;
+  compact_rows<<<ni, 256, 0, e.stream>>>(src, out, S.iv.inst_row, S.iv.inst_n, S.iv.inst_out);
+  count_launch_on(e.stream);
+  NRT_CUDA(cudaGetLastError());
+  src = out;
   return NRT_OK;
 }
 
@@ -2544,7 +2062,8 @@ int export_system(Engine &e, int input_active, int32_t *row_ptr, int32_t *col, d
   NRT_CUDA(cudaMemcpyAsync(S.iv.stats, &stat0, sizeof(InstStat), cudaMemcpyHostToDevice, e.stream));
   NRT_CUDA(cudaStreamSynchronize(e.stream));
   int32_t nnz = 0;
-  for (int64_t j = 0; j < N; j++) {
+  const int64_t n = e.host.num_elem[0];  // without the padding
+  for (int64_t j = 0; j < n; j++) {
     const Topo &t = e.host.topo[j];
     row_ptr[j] = nnz;
     if (t.flags & F_IDENT) {
@@ -2560,7 +2079,7 @@ int export_system(Engine &e, int input_active, int32_t *row_ptr, int32_t *col, d
     if (t.flags & F_DOWNL) { col[nnz] = t.dl; val[nnz++] = -g[t.dl]; }
     rhs[j] = rh[j];
   }
-  row_ptr[N] = nnz;
+  row_ptr[n] = nnz;
   *nnz_out = nnz;
   return NRT_OK;
 }

@@ -224,7 +224,11 @@ struct HostPack {
   bool invariant = true;            // initial V already has terminals equal to their sources
 };
 
-int build_host_pack(const nrt_problem *probs, int32_t count, HostPack &hp);
+// Instances of an implicit batch start on multiples of this many elements (16-byte loads of
+// FP32 rows).
+constexpr int kRowAlign = 4;
+
+int build_host_pack(const nrt_problem *probs, int32_t count, HostPack &hp, int align);
 
 // One column of the FP32 parameter table (three vector loads).
 struct HHParams32 {

@@ -89,6 +89,8 @@ int export_system(Engine &e, int input_active, int32_t *row_ptr, int32_t *col, d
                   double *rhs, int32_t *nnz_out);
 int64_t nonconverged_total(Engine &e);
 int implicit_check(Engine &e);
+// src / n: the potential of all instances back to back (compacted on the device if needed)
+int implicit_compact(Engine &e, const double *&src, int64_t &n);
 int instance_stats(Engine &e, int64_t *iters, int32_t *last_iters, int32_t *nonconv,
                    double *last_res);
 int pass_counts(Engine &e, int64_t *residuals, int64_t *applies, int64_t *xupdates,

@@ -6,6 +6,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "math64.cuh"
+
 namespace nrt {
 
 struct GateStep64 {
@@ -22,20 +24,20 @@ struct GateStep64 {
 //   beta_h  = 1 / (e^(3 - 0.1 v_Na) + 1)
 //   alpha_n = (0.1 - 0.01 v_K) / (e^xn - 1),  xn = 1 - 0.1 v_K
 //   beta_n  = 0.125 e^(-v_K/80)
-// (a product is divided by 1.0, which is exact; the selects keep e^x = inf from meeting a 0).
-// The a - b c terms are explicit fused multiply-adds, so that a constant q and a q chosen
-// per lane round them alike (left to contraction, a shared 0.1 v_Na product could be
-// rounded on its own in one and fused in the other).
+// (the factors 4 and 0.125 go into the exponential's scale, which is exact; the selects keep
+// e^x = inf from meeting a 0).  The a - b c terms are explicit fused multiply-adds, so that a
+// constant q and a q chosen per lane round them alike (left to contraction, a shared 0.1 v_Na
+// product could be rounded on its own in one and fused in the other).
 __device__ __forceinline__ double hh_rate64(int q, double vna, double vk) {
   const double xm = fma(-0.1, vna, 2.5);
   const double xn = fma(-0.1, vk, 1.0);
   const double x = q == 0 ? xm : q == 1 ? vna * (-1.0 / 18.0) : q == 2 ? vna * (-1.0 / 20.0)
                  : q == 3 ? fma(-0.1, vna, 3.0) : q == 4 ? xn : vk * (-1.0 / 80.0);
-  const double e = exp(x);
-  const double c = q == 1 ? 4.0 : q == 2 ? 0.07 : 0.125;
-  const double num = q == 0 ? xm : q == 3 ? 1.0 : q == 4 ? fma(-0.01, vk, 0.1) : c * e;
-  const double den = (q == 0 || q == 4) ? e - 1.0 : q == 3 ? e + 1.0 : 1.0;
-  return num / den;
+  const double e = exp64(x, q == 1 ? 2 : q == 5 ? -3 : 0);
+  if (q == 1 || q == 5) return e;
+  if (q == 2) return 0.07 * e;
+  const double num = q == 0 ? xm : q == 3 ? 1.0 : fma(-0.01, vk, 0.1);
+  return div64(num, q == 3 ? e + 1.0 : e - 1.0);
 }
 
 // The forward-Euler gate step and W, K from the six rates.  The fused multiply-adds are

@@ -153,6 +153,9 @@ struct Mob {
   T a, b, c, d;  // [[a, b], [c, d]]
 };
 
+__device__ __forceinline__ float quot(float a, float b) { return a / b; }
+__device__ __forceinline__ double quot(double a, double b) { return div64(a, b); }
+
 // A power of two near 1 / m for a positive normal m.
 __device__ __forceinline__ float pow2_near_inv(float m) {
   const int e = (__float_as_int(m) >> 23) & 255;
@@ -477,8 +480,8 @@ __device__ __noinline__ void tree_pivots(Ctx<T, kMode> c, const T *v, const doub
       ee[u] = 0;
       if (r.is(u, P_IDENT)) continue;
       const T p = (r.is(u, P_LAST)) ? cc[u] * vb : va + cc[u] * vb;
-      const T eta = p / vb;
-      inv[u] = (T)1 / (g[u] + eta);
+      const T eta = quot(p, vb);
+      inv[u] = quot((T)1, g[u] + eta);
       ee[u] = g[u] * inv[u];
       const T na = g[u] * p, nb = p + g[u] * vb;
       const T s = pow2_near_inv(max_of(na, nb));
@@ -554,7 +557,7 @@ __device__ __noinline__ void walk_factor(Ctx<T, kMode> c) {
   const Walk<T> k = walk_of(c, iv, S);
   const Mob<T> *mob = (const Mob<T> *)iv.pmob + c.ip0;
   walk_up<T, kMode, Mob<T>>(c, iv, k, [&](int q) { return mob[q]; },
-                            [](const Mob<T> &m, T s) { return (m.a * s + m.b) / (m.c * s + m.d); });
+                            [](const Mob<T> &m, T s) { return quot(m.a * s + m.b, m.c * s + m.d); });
 }
 
 // The factorisation once every piece's matrix is known (tree_maps, or the windowed assembly)

@@ -496,17 +496,173 @@ int Engine::init(const nrt_problem *probs, int32_t count, const nrt_options *o) 
   NRT_CUDA(cudaStreamSynchronize(st));
   hostf.clear();
   hostf.shrink_to_fit();
+  if (mixed && explicit_rows) TRY(block_init());
   return NRT_OK;
+}
+
+// The plan of several explicit steps per launch, its device copy and the second gate buffer.
+// Without the memory for them (or with a tree that does not tile) the time loop takes one
+// launch per step, as it does when the options name a shape of the per-step kernels other
+// than the staged tiles.
+int Engine::block_init() {
+  if (!host.fusable || opt.tiled == 0 || opt.step_threads > 0 || opt.step_launch != 0) return NRT_OK;
+  BlockPlan plan;
+  if (!choose_block_plan(host, pv, plan)) return NRT_OK;
+  const size_t bt = al(sizeof(BlockTile) * plan.tile.size()), bh = al(sizeof(int4) * plan.halo.size() + 16),
+               bx = al(sizeof(ushort4) * plan.spec.size() + 16), bg = al(12 * (size_t)host.ntot);
+  if (cudaMalloc(&block_mem, bt + bh + bx + bg) != cudaSuccess) {
+    cudaGetLastError();
+    block_mem = nullptr;
+    return NRT_OK;
+  }
+  char *m = (char *)block_mem;
+  NRT_CUDA(cudaMemcpyAsync(m, plan.tile.data(), sizeof(BlockTile) * plan.tile.size(),
+                           cudaMemcpyHostToDevice, stream));
+  NRT_CUDA(cudaMemcpyAsync(m + bt, plan.halo.data(), sizeof(int4) * plan.halo.size(),
+                           cudaMemcpyHostToDevice, stream));
+  NRT_CUDA(cudaMemcpyAsync(m + bt + bh, plan.spec.data(), sizeof(ushort4) * plan.spec.size(),
+                           cudaMemcpyHostToDevice, stream));
+  gate2[0] = pv.gatef;
+  gate2[1] = (float *)(m + bt + bh + bx);
+  // entries of passive elements are never written: the same in both
+  NRT_CUDA(cudaMemcpyAsync(gate2[1], gate2[0], 12 * (size_t)host.ntot, cudaMemcpyDeviceToDevice,
+                           stream));
+  NRT_CUDA(cudaStreamSynchronize(stream));
+  bv.tile = (const BlockTile *)m;
+  bv.halo = (const int4 *)(m + bt);
+  bv.spec = (const ushort4 *)(m + bt + bh);
+  bv.depth = plan.depth;
+  bv.cap = plan.cap;
+  bv.ntiles = (int)plan.tile.size();
+  btile.swap(plan.tile);
+  return NRT_OK;
+}
+
+// The probes of each tile (src: the element each recording slot reads).
+int Engine::block_probes(const std::vector<int64_t> *src) {
+  if (bv.ntiles == 0) return NRT_OK;
+  NRT_CUDA(cudaStreamSynchronize(stream));
+  if (probe_mem) cudaFree(probe_mem);
+  probe_mem = nullptr;
+  bv.probe = nullptr;
+  bv.max_probes = 0;
+  for (BlockTile &t : btile) t.p0 = t.p1 = 0;
+  std::vector<int2> list;
+  if (src && !src->empty()) {
+    std::vector<std::pair<int, int>> at;  // (tile, slot)
+    for (size_t s = 0; s < src->size(); s++) {
+      const int64_t j = (*src)[s];
+      const auto it = std::upper_bound(btile.begin(), btile.end(), j,
+                                       [](int64_t x, const BlockTile &t) { return x < t.s; });
+      at.emplace_back((int)(it - btile.begin()) - 1, (int)s);
+    }
+    std::stable_sort(at.begin(), at.end(), [](const std::pair<int, int> &a, const std::pair<int, int> &b) {
+      return a.first < b.first;
+    });
+    for (size_t q = 0; q < at.size(); q++) {
+      BlockTile &t = btile[at[q].first];
+      if (t.p1 == t.p0) t.p0 = t.p1 = (int32_t)q;
+      t.p1 = (int32_t)q + 1;
+      bv.max_probes = std::max(bv.max_probes, t.p1 - t.p0);
+      list.push_back(make_int2((int)((*src)[at[q].second] - t.s), at[q].second));
+    }
+    NRT_CUDA(cudaMalloc(&probe_mem, sizeof(int2) * list.size()));
+    NRT_CUDA(cudaMemcpyAsync(probe_mem, list.data(), sizeof(int2) * list.size(),
+                             cudaMemcpyHostToDevice, stream));
+    bv.probe = (const int2 *)probe_mem;
+  }
+  NRT_CUDA(cudaMemcpyAsync((void *)bv.tile, btile.data(), sizeof(BlockTile) * btile.size(),
+                           cudaMemcpyHostToDevice, stream));
+  NRT_CUDA(cudaStreamSynchronize(stream));  // the host list goes out of scope
+  return NRT_OK;
+}
+
+int Engine::block_steps(int k0, int nk) {
+  const RecView none_r{};
+  const StrainView none_s{};
+  const StrainView *sv = strain_view(*this);
+  while (nk > 0) {
+    const int n = std::min(nk, bv.depth);
+    TRY(launch_explicit_block(pv, bv, k0, n, V[cur], V[cur ^ 1], Vf[cur ^ 1], gate2[gcur],
+                              gate2[gcur ^ 1], rec ? rec_view_host() : none_r, sv ? *sv : none_s,
+                              stream));
+    cur ^= 1;
+    gcur ^= 1;
+    pv.gatef = gate2[gcur];
+    k0 += n;
+    nk -= n;
+  }
+  return NRT_OK;
+}
+
+// Steps in launches of up to bv.depth: chunks of kChunk steps, captured as a graph, and at the
+// end the last step alone in the per-step kernel, which leaves the step before it in the other
+// potential buffer (nrt_get_state's V_other) as a run of single steps does.
+int Engine::block_advance(int64_t left) {
+  static_assert(kChunk % 32 == 0, "an even number of launches per chunk at every depth");
+  while (left > kChunk) {
+    if (opt.use_graphs) {
+      cudaGraphExec_t &ex = block_exec[cur][gcur];
+      if (!ex) {
+        cudaGraph_t g;
+        NRT_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        int rc = strain ? launch_strain_derive(*this, kChunk, stream) : NRT_OK;
+        if (rc == NRT_OK) rc = block_steps(0, kChunk);  // cur and gcur return
+        if (rc == NRT_OK) rc = launch_advance_base(pv.inst, pv.ninst, kChunk, stream);
+        const cudaError_t e = cudaStreamEndCapture(stream, &g);
+        if (rc != NRT_OK) return rc;
+        NRT_CUDA(e);
+        size_t nodes = 0;  // every node is a kernel of this library
+        if (cudaGraphGetNodes(g, nullptr, &nodes) == cudaSuccess) block_nodes = (int64_t)nodes;
+        const cudaError_t e2 = cudaGraphInstantiate(&ex, g, 0);
+        cudaGraphDestroy(g);
+        NRT_CUDA(e2);
+      }
+      NRT_CUDA(cudaGraphLaunch(ex, stream));
+      count_launches(block_nodes);
+    } else {
+      if (strain) TRY(launch_strain_derive(*this, kChunk, stream));
+      TRY(block_steps(0, kChunk));
+      TRY(launch_advance_base(pv.inst, pv.ninst, kChunk, stream));
+    }
+    steps_done += kChunk;
+    left -= kChunk;
+  }
+  if (left <= 0) return NRT_OK;
+  const int n = (int)left, last = n - 1;
+  if (strain) TRY(launch_strain_derive(*this, n, stream));
+  TRY(block_steps(0, last));
+  if (strain) TRY(launch_strain_apply(*this, last, stream));
+  TRY(launch_explicit_step(pv, opt.precision, false, last, -1, V[cur], V[cur ^ 1], Vf[cur],
+                           Vf[cur ^ 1], stream));
+  cur ^= 1;
+  if (rec) TRY(launch_record_step(rec_view_host(), pv.inst, last, V[cur], stream));
+  TRY(launch_advance_base(pv.inst, pv.ninst, n, stream));
+  steps_done += n;
+  terminals_dirty = true;
+  return NRT_OK;
+}
+
+void Engine::drop_graphs() {
+  for (int q = 0; q < 2; q++) {
+    if (graph_exec[q]) cudaGraphExecDestroy(graph_exec[q]);
+    graph_exec[q] = nullptr;
+    for (int g = 0; g < 2; g++) {
+      if (block_exec[q][g]) cudaGraphExecDestroy(block_exec[q][g]);
+      block_exec[q][g] = nullptr;
+    }
+  }
 }
 
 Engine::~Engine() {
   if (device >= 0) cudaSetDevice(device);
-  for (int q = 0; q < 2; q++)
-    if (graph_exec[q]) cudaGraphExecDestroy(graph_exec[q]);
+  drop_graphs();
   if (stream) cudaStreamSynchronize(stream);
   implicit_release();
   record_release();
   strain_release();
+  if (block_mem) cudaFree(block_mem);
+  if (probe_mem) cudaFree(probe_mem);
   for (void *p : extra_mem) cudaFree(p);
   arena.release();
   if (stream) cudaStreamDestroy(stream);
@@ -630,6 +786,18 @@ bool Engine::chunk_kernel() const {
   return !strain || strain_tabled(*this);
 }
 
+// Whether `left` steps run several per launch.  Not the shortest calls (the last step is a
+// launch of its own anyway), and not up to two chunks of a pack of fewer than kBlockMinElems
+// elements: there the documented form, a launch per step, stays (callers can count on the launch
+// counter, and the whole call saves less than half a millisecond).
+bool Engine::use_blocks(int64_t left) const {
+  constexpr int64_t kBlockMinElems = 8192;
+  // (a tile's probes hold 8 bytes per step each in shared memory)
+  return left > 2 && bv.ntiles > 0 && (!strain || strain_tabled(*this)) &&
+         8 * (int64_t)bv.max_probes * bv.depth <= 24 * 1024 &&
+         (host.ntot >= kBlockMinElems || left > 2 * kChunk);
+}
+
 // Runs `steps` loop iterations from every instance's current base (device-side loop
 // indices): chunks of up to kChunk steps per launch when asked for, otherwise a captured
 // graph of kChunk steps where possible.
@@ -661,6 +829,7 @@ int Engine::advance(int64_t steps) {
     }
     return NRT_OK;
   }
+  if (use_blocks(left)) return block_advance(left);
   const bool graphs = opt.use_graphs != 0 && opt.mode == NRT_EXPLICIT && host.fusable;
   if (graphs && left >= kChunk) {
     if (!graph_exec[cur]) {

@@ -72,13 +72,27 @@ __device__ __forceinline__ GateStep64 hh_step64(double v, double m0, double h0, 
                     h0, n0, dt_ms, gNa, gK, GL, ENa, EK, EL);
 }
 
+// e^x and a / b by the fast units in their flush-to-zero forms: the values of __expf and
+// __fdividef wherever neither the result nor b is subnormal (rates below 1e-38 per ms), without
+// the scaling code around them (3 instructions less each, of about 260 per compartment-step).
+__device__ __forceinline__ float fast_exp(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  return y;
+}
+__device__ __forceinline__ float fast_div(float a, float b) {
+  float y;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+
 // x / (e^x - 1), the shape of alpha_m and alpha_n, with its removable singularity at 0
 // handled by the series 1 / (1 + x/2 + x^2/6) for |x| < 1e-3.  Both branches use the fast
 // reciprocal (a relative error of a few 1e-7, far below the FP32 gates' own rounding).
 __device__ __forceinline__ float xexpm1_ratio(float x, float ex) {
   const float den = fabsf(x) < 1e-3f ? fmaf(x, fmaf(x, 1.0f / 6.0f, 0.5f), 1.0f) : ex - 1.0f;
   const float num = fabsf(x) < 1e-3f ? 1.0f : x;
-  return __fdividef(num, den);
+  return fast_div(num, den);
 }
 
 struct GateStep32 {
@@ -93,14 +107,14 @@ __device__ __forceinline__ GateStep32 hh_step32(float dv_na, float dv_k, float m
   const float vna = dv_na * 1000.0f;
   const float vk = dv_k * 1000.0f;
   const float xm = fmaf(-0.1f, vna, 2.5f);
-  const float exm = __expf(xm);
+  const float exm = fast_exp(xm);
   const float am = xexpm1_ratio(xm, exm);
-  const float bm = 4.0f * __expf(vna * (-1.0f / 18.0f));
-  const float ah = 0.07f * __expf(vna * (-1.0f / 20.0f));
-  const float bh = __fdividef(1.0f, fmaf(exm, 1.6487212707001282f, 1.0f));
+  const float bm = 4.0f * fast_exp(vna * (-1.0f / 18.0f));
+  const float ah = 0.07f * fast_exp(vna * (-1.0f / 20.0f));
+  const float bh = fast_div(1.0f, fmaf(exm, 1.6487212707001282f, 1.0f));
   const float xn = fmaf(-0.1f, vk, 1.0f);
-  const float an = 0.1f * xexpm1_ratio(xn, __expf(xn));
-  const float bn = 0.125f * __expf(vk * (-1.0f / 80.0f));
+  const float an = 0.1f * xexpm1_ratio(xn, fast_exp(xn));
+  const float bn = 0.125f * fast_exp(vk * (-1.0f / 80.0f));
   GateStep32 r;
   r.m = fmaf(dt_ms, am * (1.0f - m0) - bm * m0, m0);
   r.h = fmaf(dt_ms, ah * (1.0f - h0) - bh * h0, h0);

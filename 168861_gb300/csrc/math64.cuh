@@ -279,7 +279,7 @@ static __device__ const double2 kExp2Frac[512] = {
 
 // e^x 2^scale.
 __device__ __forceinline__ double exp64(double x, int scale = 0) {
-  if (fabsf(__int_as_float(__double2hiint(x))) <= __int_as_float(0x40859000)) {  // |x| < 690
+  if (fabsf(__int_as_float(__double2hiint(x))) <= __int_as_float(0x40860800)) {  // |x| <= 705
     const double t = fma(x, 0x1.71547652b82fep+9, 0x1.8p52);  // 512/ln2: k in the low word
     const int k = __double2loint(t);
     const double kd = t - 0x1.8p52;

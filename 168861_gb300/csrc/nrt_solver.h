@@ -1,6 +1,7 @@
 // The engine behind a solver handle or a batch: one device arena holding the packed
 // trees, the two potential buffers, and (implicit mode) the Krylov workspace.
 #pragma once
+#include "block.h"
 #include "nrt_internal.h"
 
 namespace nrt {
@@ -41,12 +42,26 @@ struct Engine {
   RecState *rec = nullptr;                // recording at probes, or null
   StrainState *strain = nullptr;          // time-varying strain of some elements, or null
   GridBar *gbar = nullptr;                // the explicit chunk kernel's barrier words
+  // several explicit steps per launch (mixed precision; block.cu), or bv.ntiles == 0
+  BlockView bv{};
+  std::vector<BlockTile> btile;           // host copy of the tiles
+  void *block_mem = nullptr, *probe_mem = nullptr;
+  float *gate2[2] = {nullptr, nullptr};   // the two gate buffers; pv.gatef is gate2[gcur]
+  int gcur = 0;
+  cudaGraphExec_t block_exec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // by cur, gcur
+  int64_t block_nodes = 0;                // kernels per replay
   std::vector<void *> extra_mem;          // device tables that replaced the arena's (freed last)
 
   int init(const nrt_problem *probs, int32_t count, const nrt_options *o);
   int step(int k, int force);
   int advance(int64_t steps);
   bool chunk_kernel() const;  // explicit time loops run a chunk of steps per launch
+  int block_init();
+  int block_probes(const std::vector<int64_t> *src);  // null: no recording
+  int block_steps(int k0, int nk);   // launches for nk steps from loop index base + k0
+  bool use_blocks(int64_t left) const;
+  int block_advance(int64_t left);
+  void drop_graphs();                // the time loop's captured graphs are stale
   int fixup();
   bool needs_general() const { return general_next || (!host.invariant && steps_done == 0); }
   int get_state(int32_t q, double *Vc, double *Vo, double *m, double *h, double *n);

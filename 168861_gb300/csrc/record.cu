@@ -97,12 +97,12 @@ int Engine::record_config(const nrt_record_config *c) {
   }
   // the graphs of the explicit time loop carry (or lack) the record launches: recapture
   NRT_CUDA(cudaStreamSynchronize(stream));
-  for (int q = 0; q < 2; q++)
-    if (graph_exec[q]) {
-      cudaGraphExecDestroy(graph_exec[q]);
-      graph_exec[q] = nullptr;
-    }
+  drop_graphs();
   record_release();
+  {
+    const int rc = block_probes(nullptr);
+    if (rc) return rc;
+  }
   if (P == 0) return NRT_OK;
 
   RecState *R = new (std::nothrow) RecState();
@@ -172,6 +172,7 @@ int Engine::record_config(const nrt_record_config *c) {
   v.spk = (double *)take(8 * (size_t)P * (size_t)std::max<int64_t>(ms, 1));
   // installed only once complete: a failed call leaves no recording behind
   int rc = upload_and_init(R, src, raw, sinst, p0);
+  if (rc == NRT_OK) rc = block_probes(&src);
   if (rc) {
     cudaStreamSynchronize(stream);
     delete R;

@@ -162,6 +162,7 @@ int launch_strain_apply(const Engine &e, int k, cudaStream_t st) {
 void Engine::strain_release() {
   delete strain;
   strain = nullptr;
+  bv.scls = nullptr;
 }
 
 int Engine::strain_config(const nrt_strain_config *c) {
@@ -196,11 +197,7 @@ int Engine::strain_config(const nrt_strain_config *c) {
     }
   }
   NRT_CUDA(cudaStreamSynchronize(stream));
-  for (int q = 0; q < 2; q++)  // the graphs of the time loop gain (or lose) a launch
-    if (graph_exec[q]) {
-      cudaGraphExecDestroy(graph_exec[q]);
-      graph_exec[q] = nullptr;
-    }
+  drop_graphs();  // the time loop gains (or loses) launches
   strain_release();
   if (n == 0) return NRT_OK;
   std::unique_ptr<StrainState> S(new (std::nothrow) StrainState());
@@ -308,9 +305,12 @@ int Engine::strain_config(const nrt_strain_config *c) {
   const bool alt = tabled && mixed;
   auto rnd = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t fold_bytes = alt ? 4 * rnd(4 * (size_t)N) + rnd(48 * (size_t)pv.hp_ld) : 0;
+  // several steps per launch: each element's class (block.cu)
+  const bool classes = tabled && bv.ntiles > 0;
   const size_t bytes = 8 * (size_t)n * 2 + 4 * (size_t)n + 4 * (size_t)ncls * 2 +
                        8 * c_spec.size() +
-                       (tabled ? tab_entries * (8 * kStrainOut + 4) : 0) + fold_bytes + 256 * 8;
+                       (tabled ? tab_entries * (8 * kStrainOut + 4) : 0) + fold_bytes + 256 * 8 +
+                       (classes ? rnd(4 * (size_t)N) : 0);
   if (cudaMalloc(&S->mem, bytes) != cudaSuccess) {
     cudaGetLastError();
     set_error("device allocation for the strain");
@@ -334,6 +334,13 @@ int Engine::strain_config(const nrt_strain_config *c) {
   v.alt_wdxf = alt ? (float *)take(4 * (size_t)N) : nullptr;
   v.alt_kdxf = alt ? (float *)take(4 * (size_t)N) : nullptr;
   v.alt_hpq = alt ? (float4 *)take(48 * (size_t)pv.hp_ld) : nullptr;
+  int32_t *d_scls = classes ? (int32_t *)take(4 * (size_t)N) : nullptr;
+  hvec<int32_t> scls(classes ? N : 0);
+  if (classes) {
+    std::fill(scls.begin(), scls.end(), 0);
+    for (int32_t r = 0; r < n; r++) scls[s_elem[r]] = s_cls[r] + 1;
+    NRT_CUDA(cudaMemcpyAsync(d_scls, scls.data(), 4 * (size_t)N, cudaMemcpyHostToDevice, stream));
+  }
   NRT_CUDA(cudaMemcpyAsync(d_elem, s_elem.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, stream));
   NRT_CUDA(cudaMemcpyAsync(d_col, s_col.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, stream));
   NRT_CUDA(cudaMemcpyAsync(d_cls, s_cls.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, stream));
@@ -367,6 +374,8 @@ int Engine::strain_config(const nrt_strain_config *c) {
     NRT_CUDA(cudaMemcpyAsync(v.alt_hpq, pv.hpq, 48 * (size_t)pv.hp_ld, d2d, stream));
   }
   NRT_CUDA(cudaStreamSynchronize(stream));
+  bv.scls = d_scls;
+  bv.rows = 4 * (size_t)bv.depth * ncls * kStrainOut <= 8 * 1024;
   strain = S.release();
   return NRT_OK;
 }

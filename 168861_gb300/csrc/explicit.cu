@@ -83,115 +83,13 @@ __device__ __forceinline__ void f64_element(const PackView &p, int k, int force,
     kdx = p.kdx[j];
   }
   const bool active = input_on(in, i, force);
-  // src/solverEx-cpu.cpp:141-152, same summation order
-  double acc = 0.0;
-  const bool skip_dl = !kGeneral && (tj.flags & F_DL_TERM);
-  const bool skip_dr = !kGeneral && (tj.flags & F_DR_TERM);
-  const bool skip_mo = !kGeneral && (tj.flags & F_MO_TERM);
-  if ((tj.flags & F_BRANCH) && !skip_dl) acc = (Vin[tj.dl] - v) * p.gax[tj.dl];
-  if (!skip_dr) acc = acc + (Vin[tj.dr] - v) * p.gax[tj.dr];
-  if (!skip_mo) acc = acc + (Vin[tj.mother] - v) * p.gax[j];
-  acc = acc + wdx * v;
-  acc = acc + kdx;
-  if (active && (tj.flags & F_INP)) acc = acc + p.inp[j];  // adding a zero input is exact
-  Vout[j] = v + p.cdt[j] * acc;
-}
-
-// The same element for explicit_step_f64_lanes, in two parts: every load, none of which waits
-// for another but the topology record and the instance, and the arithmetic.  (The one-thread
-// kernel keeps its loads next to their uses: with this form a 65,000-compartment tree took
-// 28.1 us per step instead of 19.7.)
-struct F64Elem {
-  Topo t;
-  InstDev in;
-  int64_t i;              // loop index
-  bool live, skip;        // the instance still runs; nothing to do (a passive sealed end)
-  bool has_dl, has_dr, has_mo, on;
-  double v, vdl, vdr, vmo, gdl, gdr, gmo, cdt, inp, wdx, kdx, m, h, n;
-  double lsna, lsk, rest, dtms, gna, gk, gl, ena, ek, el, dx;
-};
-
-template <bool kGeneral>
-__device__ __forceinline__ void f64_load(const PackView &p, int k, int force, int64_t j,
-                                         const Topo &t, const double *Vin, F64Elem &e) {
-  e.t = t;
-  e.in = p.inst[t.flags >> INST_SHIFT];
-  const bool term = (t.flags & F_TERM) != 0, hh = (t.flags & F_HH) != 0;
-  e.v = Vin[(kGeneral || !term) ? j : ghost_source(t, j)];
-  e.skip = term && !hh;
-  e.has_dl = (t.flags & F_BRANCH) && (kGeneral || !(t.flags & F_DL_TERM)) && !term;
-  e.has_dr = (kGeneral || !(t.flags & F_DR_TERM)) && !term;
-  e.has_mo = (kGeneral || !(t.flags & F_MO_TERM)) && !term;
-  if (e.has_dl) {
-    e.vdl = Vin[t.dl];
-    e.gdl = p.gax[t.dl];
-  }
-  if (e.has_dr) {
-    e.vdr = Vin[t.dr];
-    e.gdr = p.gax[t.dr];
-  }
-  if (e.has_mo) {
-    e.vmo = Vin[t.mother];
-    e.gmo = p.gax[j];
-  }
-  if (!term) e.cdt = p.cdt[j];
-  if (hh) {
-    const int64_t N = p.ntot, L = p.hp_ld;
-    const double *hp = p.hp + hp_col(p, j, t.flags >> INST_SHIFT);
-    e.m = p.gate[j];
-    e.h = p.gate[N + j];
-    e.n = p.gate[2 * N + j];
-    e.lsna = hp[HP_LSNA * L];
-    e.lsk = hp[HP_LSK * L];
-    e.rest = hp[HP_REST * L];
-    e.dtms = hp[HP_DTMS * L];
-    e.gna = hp[HP_GNA * L];
-    e.gk = hp[HP_GK * L];
-    e.gl = hp[HP_GL * L];
-    e.ena = hp[HP_ENA * L];
-    e.ek = hp[HP_EK * L];
-    e.el = hp[HP_EL * L];
-    e.dx = hp[HP_DX * L];
-  } else if (!term) {
-    e.wdx = p.wdx[j];
-    e.kdx = p.kdx[j];
-  }
-  e.i = e.in.base + k;
-  e.live = e.i < e.in.iend;
-  e.on = input_on(e.in, e.i, force) && (t.flags & F_INP);
-  if (e.on) e.inp = p.inp[j];
-}
-
-// rates: the element's six HH rates, evaluated by its lanes (hh_rate64).
-__device__ __forceinline__ void f64_finish(const PackView &p, int64_t j, const F64Elem &e,
-                                           const double *Vin, double *Vout,
-                                           const double *rates) {
-  if (!e.live) {  // this instance is done: carry V over to the other buffer
-    Vout[j] = Vin[j];
-    return;
-  }
-  if (e.skip) return;
-  const int64_t N = p.ntot;
-  double wdx = e.wdx, kdx = e.kdx;
-  if (e.t.flags & F_HH) {
-    GateStep64 g = hh_gates64(rates[0], rates[1], rates[2], rates[3], rates[4], rates[5], e.m, e.h,
-                              e.n, e.dtms, e.gna, e.gk, e.gl, e.ena, e.ek, e.el);
-    p.gate[j] = g.m;
-    p.gate[N + j] = g.h;
-    p.gate[2 * N + j] = g.n;
-    if (e.t.flags & F_TERM) return;  // ghost: only its gates move
-    wdx = g.W * e.dx;
-    kdx = g.K * e.dx;
-  }
-  // src/solverEx-cpu.cpp:141-152, same summation order
-  double acc = 0.0;
-  if (e.has_dl) acc = (e.vdl - e.v) * e.gdl;
-  if (e.has_dr) acc = acc + (e.vdr - e.v) * e.gdr;
-  if (e.has_mo) acc = acc + (e.vmo - e.v) * e.gmo;
-  acc = acc + wdx * e.v;
-  acc = acc + kdx;
-  if (e.on) acc = acc + e.inp;  // adding a zero input is exact
-  Vout[j] = e.v + e.cdt * acc;
+  const bool dl = (tj.flags & F_BRANCH) && (kGeneral || !(tj.flags & F_DL_TERM));
+  const bool dr = kGeneral || !(tj.flags & F_DR_TERM), mo = kGeneral || !(tj.flags & F_MO_TERM);
+  const bool on = active && (tj.flags & F_INP);
+  Vout[j] = f64_update(v, dl, dl ? Vin[tj.dl] - v : 0.0, dl ? p.gax[tj.dl] : 0.0, dr,
+                       dr ? Vin[tj.dr] - v : 0.0, dr ? p.gax[tj.dr] : 0.0, mo,
+                       mo ? Vin[tj.mother] - v : 0.0, p.gax[j], wdx, kdx, on, on ? p.inp[j] : 0.0,
+                       p.cdt[j]);
 }
 
 template <bool kGeneral>
@@ -205,13 +103,9 @@ __global__ void __launch_bounds__(256) explicit_step_f64(PackView p, int k, int 
   f64_element<kGeneral>(p, k, force, j, Vin, Vout);
 }
 
-// Small FP64 packs: eight lanes per element.  One warp's FP64 work per element is the
-// step's floor when each warp holds 32 elements (six exponentials and three divisions each
-// on a pipe at 1/70 of FP32), so lanes 0-5 of an element's group evaluate one rate each with
-// the same code (hh_rate64), lane 0 gathers them by shuffles and finishes the element as
-// explicit_step_f64 does.  Every lane of a warp takes part in the shuffles; lanes of elements
-// that are out of range, finished, passive or sealed-end ghosts evaluate rates of a placeholder
-// potential that nobody reads.  The same values as explicit_step_f64, bit for bit.
+// Small FP64 packs: eight lanes per element (hh_group_step), bit for bit what explicit_step_f64
+// gives.  Every lane of a warp takes part in the shuffles; lanes of elements that are out of
+// range, finished, passive or sealed-end ghosts work on placeholders that nobody reads.
 // The step is a chain of latencies: what never changes (the topology, and the exponential's
 // table into L1) is fetched before the wait for the previous launch, and everything else in
 // one round of loads after it.
@@ -221,36 +115,69 @@ template <bool kGeneral>
 __global__ void __launch_bounds__(128) explicit_step_f64_lanes(PackView p, int k, int force,
                                                                const double *__restrict__ Vin,
                                                                double *__restrict__ Vout) {
-  const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kRateLanes;
+  const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kRateLanes, N = p.ntot;
   const int q = (int)(threadIdx.x % kRateLanes);
   exp64_prefetch();
-  Topo t{0, 0, 0, 0};
-  if (j < p.ntot) t = p.topo[j];
+  const bool in_range = j < N;
+  Topo t{0, 0, 0, F_TERM};
+  if (in_range) t = p.topo[j];
+  const bool hh = (t.flags & F_HH) != 0, term = (t.flags & F_TERM) != 0;
+  const bool dl = (t.flags & F_BRANCH) && (kGeneral || !(t.flags & F_DL_TERM)) && !term;
+  const bool dr = (kGeneral || !(t.flags & F_DR_TERM)) && !term;
+  const bool mo = (kGeneral || !(t.flags & F_MO_TERM)) && !term;
+  HHGroup h{};
+  h.r = hh_lane(q < 6 ? q : 5);
   chain_acquire();  // the previous launch of the time loop has finished
   chain_release();
-  double vna = 0.0, vk = 0.0;
-  F64Elem e;
-  if (j < p.ntot) {
-    if (q == 0) {
-      f64_load<kGeneral>(p, k, force, j, t, Vin, e);
-      if (t.flags & F_HH) {
-        vna = ((e.v + e.lsna) - e.rest) * 1000.0;
-        vk = ((e.v + e.lsk) - e.rest) * 1000.0;
-      }
-    } else if (t.flags & F_HH) {  // the element's potential and shifts, as f64_load reads them
-      const double v = Vin[(kGeneral || !(t.flags & F_TERM)) ? j : ghost_source(t, j)];
+  double v = 0.0, vn = 0.0, gate = 0.0, vself = 0.0;
+  double gdl = 0, gdr = 0, gmo = 0, cdt = 0, wdx = 0, kdx = 0, inp = 0;
+  bool live = false, on = false;
+  if (in_range) {
+    const InstDev in = p.inst[t.flags >> INST_SHIFT];
+    vself = Vin[j];
+    v = (kGeneral || !term) ? vself : Vin[ghost_source(t, j)];
+    if (q == 1 && dr) vn = Vin[t.dr];
+    if (q == 3 && mo) vn = Vin[t.mother];
+    if (q == 5 && dl) vn = Vin[t.dl];
+    if (hh) {
       const int64_t L = p.hp_ld;
       const double *hp = p.hp + hp_col(p, j, t.flags >> INST_SHIFT);
-      vna = ((v + hp[HP_LSNA * L]) - hp[HP_REST * L]) * 1000.0;
-      vk = ((v + hp[HP_LSK * L]) - hp[HP_REST * L]) * 1000.0;
+      h.ls = hp[(q < 4 ? HP_LSNA : HP_LSK) * L];
+      h.rest = hp[HP_REST * L];
+      h.dt = hp[HP_DTMS * L];
+      h.g = hp[(q < 4 ? HP_GNA : HP_GK) * L];
+      h.GL = hp[HP_GL * L];
+      h.e = hp[(q < 4 ? HP_ENA : HP_EK) * L];
+      h.EL = hp[HP_EL * L];
+      h.dx = hp[HP_DX * L];
+      if (q == 0 || q == 2 || q == 4) gate = p.gate[(q >> 1) * N + j];
     }
+    if (q == 0 && !term) {
+      if (dl) gdl = p.gax[t.dl];
+      if (dr) gdr = p.gax[t.dr];
+      if (mo) gmo = p.gax[j];
+      cdt = p.cdt[j];
+      if (!hh) {
+        wdx = p.wdx[j];
+        kdx = p.kdx[j];
+      }
+    }
+    const int64_t i = in.base + k;
+    live = i < in.iend;
+    on = input_on(in, i, force) && (t.flags & F_INP);
+    if (q == 0 && on) inp = p.inp[j];
   }
-  const double r = hh_rate64(q < 6 ? q : 5, vna, vk);
-  double rates[6];
-  const int base = (int)(threadIdx.x & 31) & ~(kRateLanes - 1);
-#pragma unroll
-  for (int s = 0; s < 6; s++) rates[s] = __shfl_sync(0xffffffffu, r, base + s);
-  if (q == 0 && j < p.ntot) f64_finish(p, j, e, Vin, Vout, rates);
+  double kd, d[3];
+  const double wd = hh_group_step(q, h, v, vn, gate, kd, d);
+  if (!in_range) return;
+  if (!live) {  // this instance is done: carry V over to the other buffer
+    if (q == 0) Vout[j] = vself;
+    return;
+  }
+  if (hh && (q == 0 || q == 2 || q == 4)) p.gate[(q >> 1) * N + j] = gate;
+  if (q != 0 || term) return;  // a sealed end: only its gates move
+  Vout[j] = f64_update(v, dl, d[2], gdl, dr, d[0], gdr, mo, d[1], gmo, hh ? wd : wdx, hh ? kd : kdx,
+                       on, inp, cdt);
 }
 
 // Mixed precision (element j of step k; the body of explicit_step_mixed and of the chunk

@@ -496,20 +496,25 @@ int Engine::init(const nrt_problem *probs, int32_t count, const nrt_options *o) 
   NRT_CUDA(cudaStreamSynchronize(st));
   hostf.clear();
   hostf.shrink_to_fit();
-  if (mixed && explicit_rows) TRY(block_init());
   return NRT_OK;
 }
 
-// The plan of several explicit steps per launch, its device copy and the second gate buffer.
+// The plan of several explicit steps per launch, its device copy and the second gate buffer:
+// made when a time loop, a recording or a strain first needs it (the drop-in's update() and
+// calculate() never do).
 // Without the memory for them (or with a tree that does not tile) the time loop takes one
 // launch per step, as it does when the options name a shape of the per-step kernels other
 // than the staged tiles.
 int Engine::block_init() {
+  if (block_tried || opt.mode != NRT_EXPLICIT) return NRT_OK;
+  block_tried = true;
   if (!host.fusable || opt.tiled == 0 || opt.step_threads > 0 || opt.step_launch != 0) return NRT_OK;
   BlockPlan plan;
-  if (!choose_block_plan(host, pv, plan)) return NRT_OK;
+  const bool mixed = opt.precision == NRT_MIXED;
+  const size_t gate_bytes = (mixed ? 12 : 24) * (size_t)host.ntot;
+  if (!choose_block_plan(host, pv, mixed, plan)) return NRT_OK;
   const size_t bt = al(sizeof(BlockTile) * plan.tile.size()), bh = al(sizeof(int4) * plan.halo.size() + 16),
-               bx = al(sizeof(ushort4) * plan.spec.size() + 16), bg = al(12 * (size_t)host.ntot);
+               bx = al(sizeof(ushort4) * plan.spec.size() + 16), bg = al(gate_bytes);
   if (cudaMalloc(&block_mem, bt + bh + bx + bg) != cudaSuccess) {
     cudaGetLastError();
     block_mem = nullptr;
@@ -522,17 +527,17 @@ int Engine::block_init() {
                            cudaMemcpyHostToDevice, stream));
   NRT_CUDA(cudaMemcpyAsync(m + bt + bh, plan.spec.data(), sizeof(ushort4) * plan.spec.size(),
                            cudaMemcpyHostToDevice, stream));
-  gate2[0] = pv.gatef;
-  gate2[1] = (float *)(m + bt + bh + bx);
+  gate2[0] = mixed ? (void *)pv.gatef : (void *)pv.gate;
+  gate2[1] = (void *)(m + bt + bh + bx);
   // entries of passive elements are never written: the same in both
-  NRT_CUDA(cudaMemcpyAsync(gate2[1], gate2[0], 12 * (size_t)host.ntot, cudaMemcpyDeviceToDevice,
-                           stream));
+  NRT_CUDA(cudaMemcpyAsync(gate2[1], gate2[0], gate_bytes, cudaMemcpyDeviceToDevice, stream));
   NRT_CUDA(cudaStreamSynchronize(stream));
   bv.tile = (const BlockTile *)m;
   bv.halo = (const int4 *)(m + bt);
   bv.spec = (const ushort4 *)(m + bt + bh);
   bv.depth = plan.depth;
   bv.cap = plan.cap;
+  bv.lanes = plan.lanes;
   bv.ntiles = (int)plan.tile.size();
   btile.swap(plan.tile);
   return NRT_OK;
@@ -583,12 +588,15 @@ int Engine::block_steps(int k0, int nk) {
   const StrainView *sv = strain_view(*this);
   while (nk > 0) {
     const int n = std::min(nk, bv.depth);
-    TRY(launch_explicit_block(pv, bv, k0, n, V[cur], V[cur ^ 1], Vf[cur ^ 1], gate2[gcur],
+    TRY(launch_explicit_block(pv, bv, opt.precision, k0, n, V[cur], V[cur ^ 1], Vf[cur ^ 1], gate2[gcur],
                               gate2[gcur ^ 1], rec ? rec_view_host() : none_r, sv ? *sv : none_s,
                               stream));
     cur ^= 1;
     gcur ^= 1;
-    pv.gatef = gate2[gcur];
+    if (opt.precision == NRT_MIXED)
+      pv.gatef = (float *)gate2[gcur];
+    else
+      pv.gate = (double *)gate2[gcur];
     k0 += n;
     nk -= n;
   }
@@ -787,15 +795,16 @@ bool Engine::chunk_kernel() const {
 }
 
 // Whether `left` steps run several per launch.  Not the shortest calls (the last step is a
-// launch of its own anyway), and not up to two chunks of a pack of fewer than kBlockMinElems
+// launch of its own anyway), and in mixed precision not up to two chunks of a pack of fewer than kBlockMinElems
 // elements: there the documented form, a launch per step, stays (callers can count on the launch
 // counter, and the whole call saves less than half a millisecond).
 bool Engine::use_blocks(int64_t left) const {
   constexpr int64_t kBlockMinElems = 8192;
   // (a tile's probes hold 8 bytes per step each in shared memory)
-  return left > 2 && bv.ntiles > 0 && (!strain || strain_tabled(*this)) &&
+  const bool mixed = opt.precision == NRT_MIXED;
+  return left > 2 && bv.ntiles > 0 && (!strain || (mixed && strain_tabled(*this))) &&
          8 * (int64_t)bv.max_probes * bv.depth <= 24 * 1024 &&
-         (host.ntot >= kBlockMinElems || left > 2 * kChunk);
+         (!mixed || host.ntot >= kBlockMinElems || left > 2 * kChunk);
 }
 
 // Runs `steps` loop iterations from every instance's current base (device-side loop
@@ -804,6 +813,7 @@ bool Engine::use_blocks(int64_t left) const {
 int Engine::advance(int64_t steps) {
   if (opt.mode == NRT_IMPLICIT_BE) return implicit_advance(*this, steps);
   int64_t left = steps;
+  if (left > 2) TRY(block_init());
   while (left > 0 && needs_general()) {  // exact first step
     if (strain) TRY(launch_strain_update(*this, 0, stream));
     TRY(step(0, -1));

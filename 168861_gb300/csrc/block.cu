@@ -1,4 +1,4 @@
-// Several explicit steps per launch (mixed precision): tiles with halos.
+// Several explicit steps per launch: tiles with halos.
 //
 // A step of the per-step kernels moves every element's state through memory (about 64 B) and
 // ends with a launch boundary, and what it computes per element is small: a pack in L2 is bound
@@ -10,7 +10,8 @@
 // memory, one CTA barrier per step.  A tile's results depend on elements up to `depth` away:
 // its halo, whose elements it advances as well, each while its value still reaches an owned
 // element (distance <= steps left).  The arithmetic per element is explicit_step_mixed's,
-// operation for operation, so every result is the per-step kernels' bit for bit.
+// operation for operation, so every result is the per-step kernels' bit for bit.  FP64 packs
+// have a form of their own (explicit_block_f64).
 //
 // Ownership: state is read from one set of buffers and written to another (potential, shadow
 // and gates), because neighbouring tiles read an element's old state as their halo.
@@ -19,6 +20,7 @@
 // and after the range along the cable plus, per branch whose two sides fall into different
 // tiles, as many along it.  The plan is the host's (build_block_plan).
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include <vector>
 
@@ -73,6 +75,24 @@ __device__ __forceinline__ void record_trace(const RecView &r, int slot, int64_t
 
 __device__ __forceinline__ int clip_int(int64_t x) {
   return x > 1 << 30 ? 1 << 30 : (x < -(1 << 30) ? -(1 << 30) : (int)x);
+}
+
+// Every probe of a tile from the trace (complete: the last step ended with a barrier).
+__device__ __forceinline__ void record_tile(const PackView &p, const BlockView &bv,
+                                            const BlockTile &t, const RecView &r, int k0, int nk,
+                                            const double *trace, int np) {
+  for (int e = threadIdx.x; e < np; e += blockDim.x) {
+    const int2 x = bv.probe[t.p0 + e];
+    int c0 = e;  // the column of the element's first probe
+    for (int u = 0; u < e; u++)
+      if (bv.probe[t.p0 + u].x == x.x) {
+        c0 = u;
+        break;
+      }
+    const InstDev in = p.inst[r.inst[x.y]];
+    record_trace(r, x.y, in.base + k0, min(nk, clip_int(in.iend - in.base - k0)), trace + c0, np,
+                 in.dT);
+  }
 }
 
 // One thread per local element.  kDense (most elements are HH): the channel parameters stay in
@@ -253,20 +273,170 @@ __global__ void __launch_bounds__(kDense ? 512 : 256, kDense ? 2 : 6)
       gout[2 * N + j] = n;
     }
   }
-  if (kRec) {  // (the trace is complete: the last step ended with a barrier)
-    for (int e = l; e < np; e += blockDim.x) {
-      const int2 x = bv.probe[t.p0 + e];
-      int c0 = e;  // the column of the element's first probe
-      for (int u = 0; u < e; u++)
-        if (bv.probe[t.p0 + u].x == x.x) {
-          c0 = u;
-          break;
-        }
-      const InstDev in = p.inst[r.inst[x.y]];
-      record_trace(r, x.y, in.base + k0, min(nk, clip_int(in.iend - in.base - k0)), trace + c0, np,
-                   in.dT);
+  if (kRec) record_tile(p, bv, t, r, k0, nk, trace, np);
+}
+
+// The FP64 form (no strain).  kLanes = 8: eight lanes per local element (hh_group_step); 1: one
+// thread each.  What bounds it is the FP64 pipe: a warp's dependent operations take 64 cycles
+// each, about 39 in sequence per step on eight lanes and 115 on one, and independent warps of an
+// SM partition share it.  So a small axon spreads over all SMs, four warps each, 16 local
+// elements of which half are halo at 4 steps per launch.
+template <int kLanes, bool kRec>
+__global__ void __launch_bounds__(256, 2)
+    explicit_block_f64(PackView p, BlockView bv, int k0, int nk, const double *Vin, double *Vout,
+                       const double *gin, double *gout, RecView r) {
+  extern __shared__ __align__(16) unsigned char bsm[];
+  double *Vs = (double *)bsm;                    // [2][cap]
+  double *G = Vs + 2 * bv.cap;                   // [cap]
+  double *trace = G + bv.cap;                    // [nk][probes]
+  ushort4 *nb = (ushort4 *)(trace + bv.depth * bv.max_probes);
+  const BlockTile t = bv.tile[blockIdx.x];
+  const int l = threadIdx.x / kLanes, q = threadIdx.x % kLanes;
+  const int64_t N = p.ntot;
+  exp64_prefetch();
+  // ---- what the time loop never changes: before the wait for the previous launch
+  int dist = 1 << 20;
+  int64_t j = -1;
+  if (l < t.cnt) {
+    j = t.s + l;
+    dist = 0;
+    if (q == 0) nb[l] = make_ushort4(l > 0 ? l - 1 : l, l + 1 < t.cnt ? l + 1 : l, l, 0);
+  } else if (l < t.cnt + t.nh) {
+    const int4 h = bv.halo[t.h0 + l - t.cnt];
+    j = h.x;
+    dist = h.z >> 16;
+    if (q == 0) nb[l] = make_ushort4(h.y & 0xffff, (unsigned)h.y >> 16, h.z & 0xffff, 0);
+  }
+  uint32_t fl = F_TERM;
+  double g0 = 0;
+  if (j >= 0) {
+    fl = p.topo[j].flags;
+    g0 = p.gax[j];
+    if (q == 0) G[l] = g0;
+  }
+  const bool hh = (fl & F_HH) != 0, term = (fl & F_TERM) != 0;
+  const bool dl = (fl & F_BRANCH) && !(fl & F_DL_TERM), dr = !(fl & F_DR_TERM), mo = !(fl & F_MO_TERM);
+  __syncthreads();
+  for (int e = threadIdx.x; e < t.nx; e += blockDim.x) {  // owned elements with far neighbours
+    const ushort4 x = bv.spec[t.x0 + e];
+    nb[x.x] = make_ushort4(x.y, x.z, x.w, 0);
+  }
+  __syncthreads();
+  int lm = 0, lr = 0, ll = 0;
+  double gdr = 0, gdl = 0;
+  if (j >= 0) {
+    const ushort4 x = nb[l];
+    lm = x.x;
+    lr = x.y;
+    ll = x.z;
+    gdr = G[lr];
+    gdl = G[ll];
+  }
+  chain_acquire();  // the previous launch of the time loop has finished
+  chain_release();
+  // ---- state
+  double V = 0, gate = 0, h0 = 0, n0 = 0;  // kLanes = 8: gate is lane 0's m, 2's h, 4's n
+  double cdt = 0, wdx = 0, kdx = 0, inp = 0;
+  int left = 0, on0 = 1, on1 = 0;
+  HHGroup hg{};
+  double lsk = 0, gk = 0, ek = 0;  // kLanes = 1: the K side (hg holds the Na side)
+  if (kLanes == 8) hg.r = hh_lane(q < 6 ? q : 5);
+  if (j >= 0) {
+    V = Vin[j];
+    if (q == 0) Vs[l] = V;
+    const InstDev in = p.inst[fl >> INST_SHIFT];
+    const int64_t i0 = in.base + k0;
+    left = clip_int(in.iend - i0);
+    on0 = clip_int(in.ion - i0);
+    on1 = clip_int(in.ioff - i0);
+    cdt = p.cdt[j];
+    if (hh) {
+      const int64_t L = p.hp_ld;
+      const double *hp = p.hp + hp_col(p, j, fl >> INST_SHIFT);
+      const bool na = kLanes == 1 || q < 4;
+      hg.ls = hp[(na ? HP_LSNA : HP_LSK) * L];
+      hg.rest = hp[HP_REST * L];
+      hg.dt = hp[HP_DTMS * L];
+      hg.g = hp[(na ? HP_GNA : HP_GK) * L];
+      hg.GL = hp[HP_GL * L];
+      hg.e = hp[(na ? HP_ENA : HP_EK) * L];
+      hg.EL = hp[HP_EL * L];
+      hg.dx = hp[HP_DX * L];
+      if (kLanes == 1) {
+        lsk = hp[HP_LSK * L];
+        gk = hp[HP_GK * L];
+        ek = hp[HP_EK * L];
+        gate = gin[j];
+        h0 = gin[N + j];
+        n0 = gin[2 * N + j];
+      } else if (q == 0 || q == 2 || q == 4) {
+        gate = gin[(q >> 1) * N + j];
+      }
+    } else {
+      wdx = p.wdx[j];
+      kdx = p.kdx[j];
+    }
+    if (fl & F_INP) inp = p.inp[j];
+  }
+  const int np = kRec ? t.p1 - t.p0 : 0;
+  int col = -1;  // the trace column (see explicit_block_mixed)
+  for (int e = 0; e < np && col < 0; e++)
+    if (bv.probe[t.p0 + e].x == l) col = e;
+  __syncthreads();
+  // ---- steps
+  for (int k = 0; k < nk; k++) {
+    const double *Vk = Vs + (k & 1) * bv.cap;
+    const bool reach = dist < nk - k;  // the value after this step still reaches an owned element
+    const bool act = reach && k < left && !(term && !hh);
+    double dd[3] = {0, 0, 0}, wd = wdx, kd = kdx;
+    const double v = j >= 0 ? (term ? Vk[lm] : (kLanes == 1 ? V : Vk[l])) : 0.0;
+    if (kLanes == 8) {
+      const int at = q == 1 ? lr : q == 3 ? lm : q == 5 ? ll : l;
+      double g2 = gate, kg;
+      const double wg = hh_group_step(q, hg, v, j >= 0 ? Vk[at] : 0.0, g2, kg, dd);
+      if (hh) {
+        if (act) gate = g2;
+        wd = wg;
+        kd = kg;
+      }
+    } else if (act) {
+      dd[0] = Vk[lr] - v;
+      dd[1] = Vk[lm] - v;
+      dd[2] = Vk[ll] - v;
+      if (hh) {
+        const GateStep64 s = hh_step64(v, gate, h0, n0, hg.ls, lsk, hg.rest, hg.dt, hg.g, gk, hg.GL,
+                                       hg.e, ek, hg.EL);
+        gate = s.m;
+        h0 = s.h;
+        n0 = s.n;
+        wd = s.W * hg.dx;
+        kd = s.K * hg.dx;
+      }
+    }
+    if (q == 0 && reach) {
+      if (act && !term) {
+        const bool on = (fl & F_INP) && k >= on0 && k <= on1;
+        V = f64_update(v, dl, dd[2], gdl, dr, dd[0], gdr, mo, dd[1], g0, wd, kd, on, inp, cdt);
+      }
+      Vs[((k + 1) & 1) * bv.cap + l] = V;
+      if (kRec && col >= 0) trace[k * np + col] = V;
+    }
+    __syncthreads();
+  }
+  // ---- owned state out
+  if (dist == 0) {
+    if (q == 0 && (!term || left <= 0)) Vout[j] = V;
+    if (hh) {
+      if (kLanes == 1) {
+        gout[j] = gate;
+        gout[N + j] = h0;
+        gout[2 * N + j] = n0;
+      } else if (q == 0 || q == 2 || q == 4) {
+        gout[(q >> 1) * N + j] = gate;
+      }
     }
   }
+  if (kRec) record_tile(p, bv, t, r, k0, nk, trace, np);
 }
 
 size_t block_smem(const BlockView &bv, const StrainView &s) {
@@ -316,7 +486,41 @@ static double block_cost(const BlockPlan &P) {
   return 4.0 / P.depth + 1e-5 * local;
 }
 
-bool choose_block_plan(const HostPack &host, const PackView &pv, BlockPlan &plan) {
+// FP64 shapes, by estimated microseconds per step: a launch boundary of 3 us, 1.3 us per round of
+// 16 eight-lane elements on an SM and 3.8 us per round of 128 one-thread ones (39 and 115
+// operations of 64 cycles), against the per-step kernels' 3.3 us and the same rounds without
+// halos.  Above a million elements the launch boundary is nothing to the rounds.
+static bool choose_f64(const HostPack &host, const PackView &pv, BlockPlan &plan) {
+  const int64_t N = host.ntot, sms = pv.sms > 0 ? pv.sms : 1;
+  if (N > 1000000) return false;
+  auto rounds = [&](int64_t local, int lanes) {
+    const double per = lanes == 8 ? 16.0 : 128.0, x = (double)local / (double)sms / per;
+    return (lanes == 8 ? 1.3 : 3.8) * (x < 4 ? std::max(1.0, std::ceil(x - 0.05)) : x);
+  };
+  double best = 3.3 + std::min(rounds(N, 1), N <= 8192 ? rounds(N, 8) : 1e30);
+  bool found = false;
+  const struct { int lanes, depth, cap; } shapes[] = {{8, 4, 16}, {8, 4, 32}, {1, 8, 128}, {1, 4, 128}, {1, 4, 256}, {1, 2, 256}};
+  for (const auto &s : shapes) {
+    const int own = s.cap - 2 * s.depth;  // at best: a cable
+    const int64_t tiles = (N + own - 1) / own;
+    auto cost = [&](int64_t n_tiles) {
+      // whole tiles go to an SM, so the fullest SM holds ceil(tiles / SMs) of them
+      return 3.0 / s.depth + rounds((n_tiles + sms - 1) / sms * s.cap * sms, s.lanes);
+    };
+    if (cost(tiles) >= best) continue;
+    BlockPlan P;
+    if (!build_block_plan(host, s.depth, s.cap, P)) continue;
+    if (cost((int64_t)P.tile.size()) >= best) continue;
+    best = cost((int64_t)P.tile.size());
+    P.lanes = s.lanes;
+    plan = std::move(P);
+    found = true;
+  }
+  return found;
+}
+
+bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, BlockPlan &plan) {
+  if (!mixed) return choose_f64(host, pv, plan);
   int depth = 0, cap = 0;
   block_shape(pv, depth, cap);
   const int largest = pv.hh_dense ? 512 : 256;
@@ -348,7 +552,7 @@ static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan
   plan.cap = cap;
   // elements tiled by one host thread at a time
   const int64_t N = host.ntot,
-                chunk = std::min<int64_t>(1 << 16, std::max<int64_t>(8 * cap, N / 64));
+                chunk = std::min<int64_t>(1 << 16, std::max<int64_t>(1 << 14, N / 64));
   const int64_t nc = (N + chunk - 1) / chunk;
   std::vector<BlockPlan> part(nc);
   std::vector<char> ok(nc, 1);
@@ -383,7 +587,7 @@ static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan
       return h;
     };
     int64_t s = c * chunk;
-    int64_t want = cap - 2 * depth;
+    int64_t want = cap - 2 * depth;  // then what the last tile held and a little more
     while (s < end) {
       int64_t cnt = std::min(want, end - s);
       int64_t d[3];
@@ -457,6 +661,7 @@ static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan
       }
       P.tile.push_back(t);
       s += cnt;
+      want = std::min<int64_t>(cap - 2 * depth, cnt + std::max(depth, cap / 32));
     }
   });
   size_t nt = 0, nh = 0, nx = 0;
@@ -482,19 +687,28 @@ static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan
   return true;
 }
 
-int launch_explicit_block(const PackView &pv, const BlockView &bv, int k0, int nk,
-                          const double *Vin, double *Vout, float *Fout, const float *gin,
-                          float *gout, const RecView &r, const StrainView &s, cudaStream_t st) {
+int launch_explicit_block(const PackView &pv, const BlockView &bv, int precision, int k0, int nk,
+                          const double *Vin, double *Vout, float *Fout, const void *gin, void *gout,
+                          const RecView &r, const StrainView &s, cudaStream_t st) {
   if (nk < 1 || nk > bv.depth) return NRT_EINVAL;
+  const bool rec = r.nprobe > 0 && bv.max_probes > 0;
+  if (precision != NRT_MIXED) {
+    auto kern = bv.lanes == 8 ? (rec ? explicit_block_f64<8, true> : explicit_block_f64<8, false>)
+                              : (rec ? explicit_block_f64<1, true> : explicit_block_f64<1, false>);
+    const size_t smem = (size_t)bv.cap * (24 + 8) + 8 * (size_t)bv.depth * bv.max_probes;
+    NRT_CUDA(launch_chained(kern, bv.ntiles, bv.cap * bv.lanes, smem, st, pv, bv, k0, nk, Vin, Vout,
+                            (const double *)gin, (double *)gout, r));
+    return NRT_OK;
+  }
   const bool strain = s.n > 0;
-  auto pick = [&](auto rec) {
-    constexpr bool R = decltype(rec)::value;
+  auto pick = [&](auto with_rec) {
+    constexpr bool R = decltype(with_rec)::value;
     return pv.hh_dense ? (strain ? explicit_block_mixed<true, true, R> : explicit_block_mixed<true, false, R>)
                        : (strain ? explicit_block_mixed<false, true, R> : explicit_block_mixed<false, false, R>);
   };
-  auto kern = r.nprobe > 0 && bv.max_probes > 0 ? pick(std::true_type()) : pick(std::false_type());
-  NRT_CUDA(launch_chained(kern, bv.ntiles, bv.cap, block_smem(bv, s), st, pv, bv, k0, nk, Vin,
-                          Vout, Fout, gin, gout, r, s));
+  auto kern = rec ? pick(std::true_type()) : pick(std::false_type());
+  NRT_CUDA(launch_chained(kern, bv.ntiles, bv.cap, block_smem(bv, s), st, pv, bv, k0, nk, Vin, Vout,
+                          Fout, (const float *)gin, (float *)gout, r, s));
   return NRT_OK;
 }
 

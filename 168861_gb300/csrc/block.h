@@ -26,6 +26,7 @@ struct BlockView {
   int cap;               // local elements at most
   int rows;              // strain: the classes' rows of a launch are staged in shared memory
   int max_probes;        // probes of a tile at most
+  int lanes;             // FP64: threads per local element
 };
 
 // The plan on the host.
@@ -34,16 +35,18 @@ struct BlockPlan {
   std::vector<int4> halo;
   std::vector<ushort4> spec;
   int depth = 0, cap = 0;
+  int lanes = 1;
 };
 
 // The plan expected to be fastest; false when one launch per step is.
-bool choose_block_plan(const HostPack &host, const PackView &pv, BlockPlan &plan);
+bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, BlockPlan &plan);
 
 struct StrainView;
 // nk (<= depth) steps from loop index base + k0: V and its FP32 shadow from Vin to Vout / Fout,
 // gates from gin to gout.  r.nprobe > 0: the tiles' probes record after every step.  s.n > 0:
-// strained elements take row k0 + k of the chunk table at step k.
-int launch_explicit_block(const PackView &pv, const BlockView &bv, int k0, int nk,
-                          const double *Vin, double *Vout, float *Fout, const float *gin,
-                          float *gout, const RecView &r, const StrainView &s, cudaStream_t st);
+// strained elements take row k0 + k of the chunk table at step k (mixed
+// precision only).  Gates are FP32 or FP64 with the precision.
+int launch_explicit_block(const PackView &pv, const BlockView &bv, int precision, int k0, int nk,
+                          const double *Vin, double *Vout, float *Fout, const void *gin, void *gout,
+                          const RecView &r, const StrainView &s, cudaStream_t st);
 }  // namespace nrt

@@ -42,11 +42,12 @@ struct Engine {
   RecState *rec = nullptr;                // recording at probes, or null
   StrainState *strain = nullptr;          // time-varying strain of some elements, or null
   GridBar *gbar = nullptr;                // the explicit chunk kernel's barrier words
-  // several explicit steps per launch (mixed precision; block.cu), or bv.ntiles == 0
+  // several explicit steps per launch (block.cu), or bv.ntiles == 0
   BlockView bv{};
+  bool block_tried = false;               // block_init has run
   std::vector<BlockTile> btile;           // host copy of the tiles
   void *block_mem = nullptr, *probe_mem = nullptr;
-  float *gate2[2] = {nullptr, nullptr};   // the two gate buffers; pv.gatef is gate2[gcur]
+  void *gate2[2] = {nullptr, nullptr};    // the two gate buffers; the pack's is gate2[gcur]
   int gcur = 0;
   cudaGraphExec_t block_exec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // by cur, gcur
   int64_t block_nodes = 0;                // kernels per replay

@@ -100,7 +100,8 @@ int Engine::record_config(const nrt_record_config *c) {
   drop_graphs();
   record_release();
   {
-    const int rc = block_probes(nullptr);
+    int rc = P > 0 ? block_init() : NRT_OK;
+    if (rc == NRT_OK) rc = block_probes(nullptr);
     if (rc) return rc;
   }
   if (P == 0) return NRT_OK;

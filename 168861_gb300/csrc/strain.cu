@@ -200,6 +200,10 @@ int Engine::strain_config(const nrt_strain_config *c) {
   drop_graphs();  // the time loop gains (or loses) launches
   strain_release();
   if (n == 0) return NRT_OK;
+  {
+    const int rc = block_init();
+    if (rc) return rc;
+  }
   std::unique_ptr<StrainState> S(new (std::nothrow) StrainState());
   if (!S) {
     set_error("host allocation");

@@ -140,9 +140,8 @@ typedef struct nrt_options {
                                     solves each cycle to the outer tolerance and ignores it */
   int32_t step_launch;           /* explicit time loops (nrt_run, nrt_batch_advance, the
                                     server): 0 = automatic (default): one launch per step, or
-                                    in mixed precision several steps per launch on tiles with
-                                    halos (4 to 16, where tiled is set and step_threads is
-                                    not), chained and replayed from a captured graph; 1 = up to
+                                    several steps per launch on tiles with halos (2 to 16,
+                                    where tiled is set and step_threads is not), chained and replayed from a captured graph; 1 = up to
                                     64 steps per
                                     cooperative launch with a grid barrier between steps (on a
                                     GB300 a barrier across both dies costs about what a chained

@@ -1,5 +1,5 @@
-"""Several explicit steps per launch (csrc/block.cu): every result equals the per-step kernels'
-(tiled = 0, one thread per element) bit for bit -- potentials, gates, the other potential
+"""Several explicit steps per launch (csrc/block.cu), mixed precision and FP64: every result
+equals the per-step kernels' (tiled = 0) bit for bit -- potentials, gates, the other potential
 buffer, samples and spikes -- over the sizes and calls where the tiles can go wrong: packs of
 one tile and of many, trees whose branches are shorter than a halo, mostly passive trees, runs
 that end inside a launch, calls that are no multiple of a launch or of a captured chunk, probes
@@ -11,12 +11,17 @@ pytestmark = pytest.mark.gpu
 
 
 def trees(model, name):
+    if name.startswith("axon") and len(name) > 4:
+        n = int(name[4:])
+        return [model.straight_axon(n_comp=n, length=1e-5 * n, dtf=0.8)]
     if name == "axon":
         return [model.straight_axon(n_comp=9000, length=9e-2, dtf=0.8)]
     if name == "myelin":
         return [model.myelinated_axon(n_nodes=12)]
     if name == "twigs":  # branches of 2 to 4 compartments
         return [model.random_binary_tree(depth=11, seed=4, len_lo=2e-6, len_hi=4e-6)]
+    if name == "few":
+        return [model.random_tree(seed=90 + q, n_target=n) for q, n in enumerate((700, 401, 350))]
     if name == "tree":
         return [model.random_tree(seed=5, n_target=30011)]
     return [model.random_tree(seed=70 + q, n_target=n) for q, n in
@@ -35,8 +40,8 @@ def problems(pkg, specs):
     return out
 
 
-def run(pkg, specs, probs, calls, strain, **opts):
-    b = pkg.Batch(probs, precision="mixed", **opts)
+def run(pkg, specs, probs, calls, strain, precision, **opts):
+    b = pkg.Batch(probs, precision=precision, **opts)
     if strain:
         sp = specs[-1]
         b.set_strain(len(specs) - 1, sp, np.arange(sp.n // 3, sp.n // 3 + 900), 0.0, 0.2, 0.0,
@@ -65,8 +70,21 @@ def run(pkg, specs, probs, calls, strain, **opts):
 def test_blocks_equal_single_steps(gpu, pkg, model, name, strain, calls):
     specs = trees(model, name)
     probs = problems(pkg, specs)
-    (a, ra, va) = run(pkg, specs, probs, calls, strain)
-    (b, rb, vb) = run(pkg, specs, probs, calls, strain, tiled=False)
+    compare(pkg, specs, probs, calls, strain, "mixed")
+
+
+# one and two rounds of eight-lane elements, one-thread elements, several tiles per SM
+@pytest.mark.parametrize("name", ["axon300", "axon1000", "few", "axon3000", "axon9000", "twigs",
+                                  "tree", "batch"])
+@pytest.mark.parametrize("calls", [(3, 70), (64, 65)])
+def test_fp64_blocks_equal_single_steps(gpu, pkg, model, name, calls):
+    specs = trees(model, name)
+    compare(pkg, specs, problems(pkg, specs), calls, False, "fp64")
+
+
+def compare(pkg, specs, probs, calls, strain, precision):
+    (a, ra, va) = run(pkg, specs, probs, calls, strain, precision)
+    (b, rb, vb) = run(pkg, specs, probs, calls, strain, precision, tiled=False)
     for x, y in zip(a, b):
         for part in ("V", "V_other", "m", "h", "n"):
             np.testing.assert_array_equal(getattr(x, part), getattr(y, part), err_msg=part)

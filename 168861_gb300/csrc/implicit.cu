@@ -39,12 +39,14 @@
 // a far neighbour make a second, dependent load.  The SpMV is fused with up to kG
 // Gram-Schmidt products; the update and the norm share a pass.
 //
-// Two launch shapes from one template:
+// Three launch shapes from one template:
 //  * kGrid  (one tree): a cooperative launch over the whole GPU; rows and windows are split
 //    into contiguous per-CTA ranges; grid-wide syncs separate the phases.
 //  * kBlock (batches): a persistent block-per-instance scheduler; each CTA takes the next
 //    instance (largest first) from an atomic queue and runs all of its steps with
-//    __syncthreads only.
+//    __syncthreads only;
+//  * kCluster (batches too small to fill the GPU, and small single trees): a cluster of up to
+//    eight CTAs per instance, with the cluster's barrier between the phases.
 #include <cooperative_groups.h>
 #include <string.h>
 
@@ -66,8 +68,11 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxPiece = 256;                 // longest segment piece one sweep handles
 constexpr int kMaxDots = kMaxRestart + 1;
+constexpr int kSumChunks = 8;                  // row chunks of an instance's sums (rows_reduce)
 constexpr int kTileBytes = 44 * 1024;          // shared memory of the preconditioners
-constexpr int kWalkBytes = 96 * 1024;          // shared memory of the one-tree launch's walk
+constexpr int kWalkBytes = 190 * 1024;         // shared memory of the one-tree launch's walk
+constexpr int kClusterWalkBytes = 64 * 1024;   // and of a cluster's
+constexpr int kClusterWindows = 8;             // one tree of at most this many windows: a cluster
 constexpr int kRW = 4;                         // tree preconditioner: rows per thread of a window
 constexpr int kWin = kThreads * kRW;           // rows of a window
 constexpr int kU = 4;                          // rows per thread in flight: SpMV + products
@@ -162,7 +167,7 @@ struct Work {
 };
 
 struct Shared {
-  double *H, *cs, *sn, *g, *s, *y, *red, *warp;
+  double *H, *cs, *sn, *g, *s, *y, *red, *warp, *part;
   void *coef;      // T[kMaxDots]: update / solution coefficients
   int *flag;       // [0] convergence, [1] queue slot
   void *tile;      // staging area (segment preconditioner) or the tree walk's numbers
@@ -170,7 +175,7 @@ struct Shared {
 
 __host__ __device__ inline size_t shared_fixed_bytes(int m) {
   return sizeof(double) * ((size_t)(m + 1) * m + 2 * m + 2 * (m + 1) + m + kMaxDots +
-                           kWarps * kMaxDots + kMaxDots) + 32;
+                           (kWarps + kSumChunks) * kMaxDots + kMaxDots) + 32;
 }
 
 // The dynamic shared memory of the launch.
@@ -189,7 +194,8 @@ __device__ Shared carve(double *base, int m) {
   S.y = S.s + (m + 1);
   S.red = S.y + m;
   S.warp = S.red + kMaxDots;
-  S.coef = (void *)(S.warp + kWarps * kMaxDots);
+  S.part = S.warp + kWarps * kMaxDots;
+  S.coef = (void *)(S.part + kSumChunks * kMaxDots);
   S.flag = (int *)((double *)S.coef + kMaxDots);
   S.tile = (void *)((char *)base + ((shared_fixed_bytes(m) + 127) & ~(size_t)127));
   return S;
@@ -197,26 +203,52 @@ __device__ Shared carve(double *base, int m) {
 
 // ---------------------------------------------------------------- groups
 //
-// The CTAs that step one instance: the CTA itself (kBlock), or the whole cooperative launch
-// (kGrid).
-enum : int { kBlock = 0, kGrid = 1 };
+// The CTAs that step one instance: the CTA itself (kBlock), the whole cooperative launch
+// (kGrid), or a thread-block cluster (kCluster).
+enum : int { kBlock = 0, kGrid = 1, kCluster = 2 };
+
+__device__ __forceinline__ int cluster_rank() {
+  int r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ int cluster_size() {
+  int r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
 
 template <int kMode>
 __device__ __forceinline__ int group_rank() {
-  return kMode == kGrid ? (int)blockIdx.x : 0;
+  return kMode == kGrid ? (int)blockIdx.x : kMode == kCluster ? cluster_rank() : 0;
 }
 template <int kMode>
 __device__ __forceinline__ int group_size() {
-  return kMode == kGrid ? (int)gridDim.x : 1;
+  return kMode == kGrid ? (int)gridDim.x : kMode == kCluster ? cluster_size() : 1;
 }
 template <int kMode>
 __device__ __forceinline__ void group_sync() {
   if (kMode == kGrid) {
     __threadfence();
     cg::this_grid().sync();
+  } else if (kMode == kCluster) {
+    __threadfence();  // what other CTAs of the cluster read goes through device memory
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
+                     : "memory");
+    __threadfence();
   } else {
     __syncthreads();
   }
+}
+
+// Where a group's CTAs leave partial sums (slot: CTA, or chunk of rows): two buffers in turn.
+template <int kMode>
+__device__ __forceinline__ double *group_partials(double *partials, int parity) {
+  if (kMode == kCluster) {
+    const int cluster = (int)blockIdx.x / cluster_size();
+    return partials + (size_t)kMaxDots * kSumChunks * (2 * cluster + parity);
+  }
+  return partials + (size_t)kMaxDots * parity * group_size<kMode>();
 }
 
 // ---------------------------------------------------------------- reductions
@@ -249,7 +281,7 @@ __device__ __forceinline__ void block_reduce(const T (&acc)[kN], int k, double *
 template <int kMode>
 __device__ void group_finish(int k, double *cta_sums, double *partials, int &parity) {
   const int size = group_size<kMode>(), rank = group_rank<kMode>();
-  double *buf = partials + (size_t)kMaxDots * (2 * (blockIdx.x - rank) + parity * size);
+  double *buf = group_partials<kMode>(partials, parity);
   parity ^= 1;
   if (threadIdx.x < k) buf[(size_t)rank * kMaxDots + threadIdx.x] = cta_sums[threadIdx.x];
   __syncthreads();
@@ -389,12 +421,13 @@ struct Ctx {
   Work<T> w;
   int64_t r0, r1;   // rows of this CTA in the row passes
   int t0, t1;       // segment-preconditioner tiles
-  // tree preconditioner: this CTA's windows, the instance's first window and row, the end of
+  // tree preconditioner: this CTA's windows, the instance's first and past-the-last window, its first row, the end of
   // its rows (a multiple of kRW after its first), its pieces and level entries
-  int w0, w1, iw0;
+  int w0, w1, iw0, iw1;
   int64_t wrow0, wend;
   int ip0, np, l0, l1;
   int rank;         // this CTA in its group
+  int n, v0, v1;    // rows of the instance; this CTA's chunks of them (rows_reduce)
 };
 
 // A sync of the group where one CTA's rows reach another's (nothing to do in one CTA).
@@ -408,6 +441,44 @@ __device__ __forceinline__ void level_sync() {
 __device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, int64_t j) {
   return 2.0 * Vin[j] - Vout[j];
 }
+
+// Sums k accumulators of a row pass f(context) over the instance into S.red[off .. off + k).  In
+// a block or a cluster the rows are taken in kSumChunks chunks whose sums are added in order,
+// so that the result does not depend on how many CTAs share the instance.
+template <typename T, int kMode, typename F>
+__device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Shared &S,
+                                            double *partials, int &parity, int off, F f) {
+  if (kMode == kGrid) {
+    auto acc = f(c);
+    group_reduce<kMode>(acc.v, k, S, partials, parity, off);
+    return;
+  }
+  double *sum = S.part;
+  if (kMode == kCluster) {
+    sum = group_partials<kMode>(partials, parity);
+    parity ^= 1;
+  }
+  for (int v = c.v0; v < c.v1; v++) {
+    Ctx<T, kMode> d = c;
+    d.r0 = c.wrow0 + (int64_t)c.n * v / kSumChunks;
+    d.r1 = c.wrow0 + (int64_t)c.n * (v + 1) / kSumChunks;
+    auto acc = f(d);
+    block_reduce(acc.v, k, S.warp, S.red + off);
+    if (threadIdx.x < k) sum[v * kMaxDots + threadIdx.x] = S.red[off + threadIdx.x];
+  }
+  group_sync<kMode>();
+  if (threadIdx.x < k) {
+    double s = 0;
+    for (int v = 0; v < kSumChunks; v++) s += sum[v * kMaxDots + threadIdx.x];
+    S.red[off + threadIdx.x] = s;
+  }
+  __syncthreads();
+}
+
+template <typename X, int kN>
+struct Sums {
+  X v[kN];
+};
 
 }  // namespace nrt
 
@@ -1056,32 +1127,30 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
   // ---- assembly, fused with the first true residual (W_0); V still holds V^{n-1}
   const bool tree = iv.precond == NRT_PRECOND_TREE;
   const bool fused = sizeof(T) == 4 && iv.rich != 0;  // by windows, with the pieces' matrices
-  double2 br;
-  if constexpr (sizeof(T) == 4) {
-    if (!fused)
-      br = ph_assemble(c, Vin, Vout, active ? 1 : 0, inst);
-    else if (iv.scheme == NRT_CRANK_NICOLSON)
-      br = refine_assemble<kMode, true>(c, Vin, Vout, active ? 1 : 0, inst);
-    else
-      br = refine_assemble<kMode, false>(c, Vin, Vout, active ? 1 : 0, inst);
+  double target = iv.tol, res0 = 0;
+  auto assemble = [&](const Ctx<T, kMode> &d) {
+    const double2 br = ph_assemble(d, Vin, Vout, active ? 1 : 0, inst);
+    return Sums<double, 2>{{br.x, br.y}};
+  };
+  if (fused) {
+    if constexpr (sizeof(T) == 4) {
+      const double2 br = iv.scheme == NRT_CRANK_NICOLSON
+                             ? refine_assemble<kMode, true>(c, Vin, Vout, active ? 1 : 0, inst)
+                             : refine_assemble<kMode, false>(c, Vin, Vout, active ? 1 : 0, inst);
+      const double acc[2] = {br.x, br.y};
+      group_reduce<kMode>(acc, 2, S, iv.partials, parity);  // also publishes W_0, the matrices
+    }
   } else {
-    br = ph_assemble(c, Vin, Vout, active ? 1 : 0, inst);
+    rows_reduce(c, 2, S, iv.partials, parity, 0, assemble);  // also publishes W_0 and c
   }
+  if (iv.tol_mode == NRT_TOL_REL) target = iv.tol * sqrt(S.red[0]);
+  res0 = sqrt(S.red[1]);
+  __syncthreads();  // S.red is read before the next sum
   if (iv.precond == NRT_PRECOND_SEGMENT) {
-    __syncthreads();
     factor_pieces(c);
   } else if (tree && !fused) {
-    group_sync<kMode>();  // c of every row visible before the factorisation
     tree_maps(c);
-    __syncthreads();
-  }
-  double target = iv.tol, res0 = 0;
-  {
-    double acc[2] = {br.x, br.y};
-    group_reduce<kMode>(acc, 2, S, iv.partials, parity);  // also publishes W_0, the matrices
-    if (iv.tol_mode == NRT_TOL_REL) target = iv.tol * sqrt(S.red[0]);
-    res0 = sqrt(S.red[1]);
-    if (kMode == kBlock) __syncthreads();
+    group_sync<kMode>();
   }
   if (tree) tree_factor(c, c.w.Wb, fused ? Vin : (const double *)nullptr, Vout);
   const int budget = iv.max_iter > 0 ? iv.max_iter : (iv.max_iter < 0 ? 0 : (int)inst_n);
@@ -1108,8 +1177,10 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
       // res > 0 here (a zero residual has converged); the scale stays a normal FP32 number
       const bool f32 = sizeof(T) == 4 && iv.krylov == NRT_GMRES;
       const int e = f32 ? max(-126, min(126, ilogb(res))) : 0;
-      double acc[1] = {ph_residual(c, Vout, f32 ? exp2f((float)-e) : 0.0f)};
-      group_reduce<kMode>(acc, 1, S, iv.partials, parity);
+      const float scale = f32 ? exp2f((float)-e) : 0.0f;
+      rows_reduce(c, 1, S, iv.partials, parity, 0, [&](const Ctx<T, kMode> &d) {
+        return Sums<double, 1>{{ph_residual(d, Vout, scale)}};
+      });
       res = sqrt(S.red[0]) * exp2((double)e);
       n_res++;
     }
@@ -1183,13 +1254,13 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
       // y = s_j A Z_j fused with p_i = <y, W_i> for the first kG of i <= j
       const int g1 = min(j + 1, kG);
       {
-        DotAcc<T> acc = ph_spmv(c, j, (T)S.s[j], g1);
-        group_reduce<kMode>(acc.v, g1, S, iv.partials, parity);
+        rows_reduce(c, g1, S, iv.partials, parity, 0,
+                    [&](const Ctx<T, kMode> &d) { return ph_spmv(d, j, (T)S.s[j], g1); });
       }
       for (int i0 = kG; i0 <= j; i0 += kG) {  // remaining products, kG at a time
         const int gk = min(j + 1 - i0, kG);
-        DotAcc<T> acc = ph_products(c, i0, gk);
-        group_reduce<kMode>(acc.v, gk, S, iv.partials, parity, i0);
+        rows_reduce(c, gk, S, iv.partials, parity, i0,
+                    [&](const Ctx<T, kMode> &d) { return ph_products(d, i0, gk); });
       }
       if (threadIdx.x <= j) {
         const double h = S.s[threadIdx.x] * S.red[threadIdx.x];
@@ -1198,8 +1269,9 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
       }
       __syncthreads();
       // w = y - sum_i h_ij s_i W_i -> W_{j+1}; ||w||^2
-      T nacc[1] = {ph_update(c, j, coef)};
-      group_reduce<kMode>(nacc, 1, S, iv.partials, parity);  // publishes W_{j+1}
+      rows_reduce(c, 1, S, iv.partials, parity, 0, [&](const Ctx<T, kMode> &d) {
+        return Sums<T, 1>{{ph_update(d, j, coef)}};  // publishes W_{j+1}
+      });
       if (threadIdx.x == 0) {
         const double hn = sqrt(S.red[0]);
         S.s[j + 1] = hn > 0 ? 1.0 / hn : 0.0;
@@ -1293,25 +1365,33 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
   c.w.pd = (T *)iv.pcd;
   c.w.pc = (T *)iv.pcc;
   c.rank = group_rank<kMode>();
+  const int gsize = group_size<kMode>();
+  int q = kMode == kCluster ? (int)blockIdx.x / gsize : 0;
   for (;;) {
     int inst = 0;
     if (kMode == kBlock) {
       if (threadIdx.x == 0) S.flag[1] = atomicAdd(iv.queue, 1);
       __syncthreads();
-      const int q = S.flag[1];
+      q = S.flag[1];
       __syncthreads();
+    }
+    if (kMode != kGrid) {
       if (q >= iv.ninst) break;
       inst = iv.order[q];
     }
     const int n = iv.inst_n[inst];
-    c.r0 = iv.inst_row[inst];
-    c.r1 = c.r0 + n;
     const bool tree = iv.precond == NRT_PRECOND_TREE;
-    c.wrow0 = c.r0;
-    c.wend = c.r0 + ((n + kRW - 1) & ~(kRW - 1));
+    c.n = n;
+    c.v0 = kSumChunks * c.rank / gsize;
+    c.v1 = kSumChunks * (c.rank + 1) / gsize;
+    c.wrow0 = iv.inst_row[inst];
+    c.wend = c.wrow0 + ((n + kRW - 1) & ~(kRW - 1));
+    c.r0 = c.wrow0 + (int64_t)n * c.v0 / kSumChunks;
+    c.r1 = c.wrow0 + (int64_t)n * c.v1 / kSumChunks;
     c.iw0 = tree ? iv.inst_win[inst] : 0;
-    c.w0 = c.iw0;
-    c.w1 = tree ? iv.inst_win[inst + 1] : 0;
+    c.iw1 = tree ? iv.inst_win[inst + 1] : 0;
+    c.w0 = c.iw0 + (c.iw1 - c.iw0) * c.rank / gsize;
+    c.w1 = c.iw0 + (c.iw1 - c.iw0) * (c.rank + 1) / gsize;
     c.ip0 = tree ? iv.inst_piece[inst] : 0;
     c.np = tree ? iv.inst_piece[inst + 1] - c.ip0 : 0;
     c.l0 = tree ? iv.inst_lev[inst] : 0;
@@ -1329,6 +1409,7 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
       c.t0 = iv.inst_tile[inst];
       c.t1 = iv.inst_tile[inst + 1];
     }
+    if (tree) stage_links(c);
     const InstDev in = pvp->inst[inst];
     int s = 0;
     for (; s < nsteps; s++) {
@@ -1345,7 +1426,8 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
       for (int64_t j = c.r0 + threadIdx.x; j < c.r1; j += blockDim.x) dst[j] = src[j];
     }
     if (kMode == kGrid) break;
-    __syncthreads();
+    if (kMode == kCluster) q += (int)gridDim.x / gsize;
+    group_sync<kMode>();
   }
 }
 
@@ -1373,9 +1455,21 @@ struct ImplicitState {
   TreePlan tree;
   int grid_blocks = 0;
   bool grid_mode = false;
+  int cluster = 0;  // CTAs per cluster (0: not a cluster launch)
   int tile_rows = 0;
   size_t smem = 0;
+  const void *kern = nullptr;
 };
+
+static const void *implicit_kernel(bool mixed, int group) {
+  if (mixed)
+    return group == kGrid ? (const void *)implicit_steps<float, kGrid>
+           : group == kCluster ? (const void *)implicit_steps<float, kCluster>
+                               : (const void *)implicit_steps<float, kBlock>;
+  return group == kGrid ? (const void *)implicit_steps<double, kGrid>
+         : group == kCluster ? (const void *)implicit_steps<double, kCluster>
+                             : (const void *)implicit_steps<double, kBlock>;
+}
 
 static size_t smem_bytes(int m, size_t tile) {
   return ((shared_fixed_bytes(m) + 127) & ~(size_t)127) + tile;
@@ -1608,19 +1702,38 @@ int Engine::implicit_plan(size_t &bytes) {
   int dev_sms = 0;
   NRT_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
   S.grid_mode = ni == 1 && opt.schedule == 0;
-  const void *kern = mixed ? (S.grid_mode ? (const void *)implicit_steps<float, kGrid>
-                                          : (const void *)implicit_steps<float, kBlock>)
-                           : (S.grid_mode ? (const void *)implicit_steps<double, kGrid>
-                                          : (const void *)implicit_steps<double, kBlock>);
+  // Clusters (tree preconditioner with GMRES): an instance's rows and windows split over 2, 4 or
+  // 8 CTAs, as many as leave every cluster resident at once.  One CTA per instance leaves SMs
+  // idle as long as there are fewer instances than SMs, and a small single tree spends most of a
+  // cooperative launch's step in its grid-wide syncs (1.5 to 2 us each; a cluster's barrier
+  // takes about 0.4).
+  int64_t max_win = 0;
+  for (int32_t i = 0; tree && i < ni; i++)
+    max_win = std::max<int64_t>(max_win, S.tree.inst_win[i + 1] - S.tree.inst_win[i]);
+  S.cluster = 0;
+  if (tree && opt.krylov == NRT_GMRES && opt.schedule == 0 && opt.tile_ctas_per_sm == 0) {
+    if (ni == 1) {
+      if (max_win <= kClusterWindows) S.cluster = 8;
+    } else {
+      for (int cs = 2; cs <= 8; cs *= 2)
+        if ((int64_t)ni * cs <= (int64_t)dev_sms * (mixed ? 3 : 2)) S.cluster = cs;
+    }
+  }
+  if (S.cluster) S.grid_mode = false;
+  const int group = S.cluster ? kCluster : S.grid_mode ? kGrid : kBlock;
+  const void *kern = implicit_kernel(mixed, group);
+  S.kern = kern;
   // shared memory: the segment preconditioner's staging, or the tree walk's numbers of
-  // every piece -- up to kTileBytes, which keeps four CTAs on an SM, or in the one-tree launch
-  // (at most two per SM) up to kWalkBytes; larger walks run in device memory
+  // every piece -- up to kTileBytes, which keeps three CTAs on an SM, or in the one-tree launch,
+  // whose CTAs then have an SM each, up to kWalkBytes; larger walks run in device memory
   size_t tile = 0;
   if (segs) tile = kTileBytes;
   if (tree) {
-    const size_t cap = S.grid_mode ? kWalkBytes : kTileBytes;
-    S.iv.walk_cap = (int)std::min<size_t>(cap / walk_bytes(tb), (size_t)S.tree.max_pieces);
-    tile = (size_t)S.iv.walk_cap * walk_bytes(tb);
+    const bool grp = group != kBlock;
+    const size_t cap = S.grid_mode ? kWalkBytes : S.cluster ? kClusterWalkBytes : kTileBytes;
+    S.iv.walk_cap = (int)std::min<size_t>(std::min<size_t>(cap / walk_bytes(tb, grp), kNoPiece - 1),
+                                          (size_t)S.tree.max_pieces);
+    tile = (size_t)S.iv.walk_cap * walk_bytes(tb, grp);
   }
   S.smem = smem_bytes(opt.restart, tile);
   // The limit is the function's, not the handle's: all that a CTA can have, so that handles
@@ -1689,6 +1802,7 @@ int Engine::implicit_plan(size_t &bytes) {
     // each instance is one CTA's from start to end, so results do not depend on it)
     if (opt.tile_ctas_per_sm > 0) per_sm = std::min(per_sm, opt.tile_ctas_per_sm);
     S.grid_blocks = std::max(1, std::min<int>(dev_sms * std::max(per_sm, 1), ni));
+    if (S.cluster) S.grid_blocks = ni * S.cluster;
     S.inst_tile.assign(ni + 1, 0);
     for (int32_t i = 0; segs && i < ni; i++) {
       S.inst_tile[i] = (int)S.tiles.size();
@@ -1721,7 +1835,7 @@ int Engine::implicit_plan(size_t &bytes) {
     b += al256(ld) + al256(2 * T.wtp.size()) + al256(4 * T.wbase.size());
     b += al256(4 * npc) + al256(16 * npc) + al256(4 * std::max<size_t>(1, T.lev_off.size()));
     b += 3 * al256(4 * (size_t)(ni + 1));                   // inst_win, inst_piece, inst_lev
-    b += 2 * al256(4 * tb * npc) + al256(8 * tb * npc) + al256(walk_bytes(tb) * npc);  // pmob, pstat, pval, gwalk
+    b += 2 * al256(4 * tb * npc) + al256(8 * tb * npc) + al256(walk_bytes(tb, false) * npc);  // pmob, pstat, pval, gwalk
     b += al256(8 * npc) + al256(32 * npc);                  // pgf, pxb
     b += 4 * al256(tb * ld);                                // tinv, te, tbeta, talpha
   }
@@ -1843,7 +1957,7 @@ int Engine::implicit_init() {
     iv.pstat = arena.take(4 * tb * npc);
     iv.pval = arena.take(8 * tb * npc);
     iv.pxb = (double *)arena.take(32 * npc);
-    iv.gwalk = arena.take(walk_bytes(tb) * npc);
+    iv.gwalk = arena.take(walk_bytes(tb, false) * npc);
     iv.tinv = arena.take(tb * ld);
     iv.te = arena.take(tb * ld);
     iv.tbeta = arena.take(tb * ld);
@@ -1877,13 +1991,21 @@ static int implicit_launch(Engine &e, int nsteps, int force) {
   // the drop-in per-call loop (force >= 0) has no device loop index: it is not recorded
   const RecView *rec = force < 0 ? e.record_view() : nullptr;
   void *args[] = {&pv, &iv, &nsteps, &force, &V0, &V1, &cur, &rec};
-  const bool mixed = e.opt.precision == NRT_MIXED;
   if (S.grid_mode) {
-    const void *k = mixed ? (const void *)implicit_steps<float, kGrid> : (const void *)implicit_steps<double, kGrid>;
-    NRT_CUDA(cudaLaunchCooperativeKernel(k, dim3(S.grid_blocks), dim3(kThreads), args, S.smem, e.stream));
+    NRT_CUDA(cudaLaunchCooperativeKernel(S.kern, dim3(S.grid_blocks), dim3(kThreads), args, S.smem, e.stream));
   } else {
-    const void *k = mixed ? (const void *)implicit_steps<float, kBlock> : (const void *)implicit_steps<double, kBlock>;
-    NRT_CUDA(cudaLaunchKernel(k, dim3(S.grid_blocks), dim3(kThreads), args, S.smem, e.stream));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S.grid_blocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = S.smem;
+    cfg.stream = e.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)std::max(1, S.cluster);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = S.cluster ? 1 : 0;
+    NRT_CUDA(cudaLaunchKernelExC(&cfg, S.kern, args));
   }
   count_launch_on(e.stream);
   return NRT_OK;

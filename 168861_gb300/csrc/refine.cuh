@@ -177,12 +177,13 @@ __device__ __noinline__ double2 refine_assemble(Ctx<float, kMode> c, const doubl
 }
 
 struct RefineX {
-  WalkX<float> w;
-  double2 b;  // the potential of the piece's first and last row before the update
+  float4 s, v;  // pstat, pval
+  double2 b;    // the potential of the piece's first and last row before the update
 };
 
 // The walks of one refinement cycle, with the new potential of the pieces' first and last
-// rows.  pb: the buffer of the pieces' values.
+// rows (in a group: of this CTA's pieces and the ones next to them).  pb: the buffer of the
+// pieces' values.
 template <int kMode>
 __device__ __noinline__ void refine_walk(Ctx<float, kMode> c, int pb) {
   const ImView &iv = *c.iv;
@@ -192,22 +193,51 @@ __device__ __noinline__ void refine_walk(Ctx<float, kMode> c, int pb) {
   const float4 *pa = (const float4 *)iv.pval + (c.ip0 + (int64_t)pb * iv.npieces);
   const double2 *px = (const double2 *)iv.pxb + (c.ip0 + (int64_t)pb * iv.npieces);
   const int4 *lk = iv.plink + c.ip0;
+  auto up = [](const Mob<float> &x, float s) { return x.c + x.a * s; };
+  auto last = [](float B, float bL, float aL, float y, float zp) { return aL + bL * y + B * zp; };
+  auto put = [&](int q, const RefineX &x, float y, float zp, float zl, bool one) {
+    const float zf = x.v.z + x.s.z * y + x.s.w * zp;
+    const double xl = x.b.y + f2d(zl);
+    k.px[q] = make_double2(one ? xl : x.b.x + f2d(zf), xl);  // one row: first is last
+  };
   auto get = [&](int q) {
     const float4 a = ps[q], b = pa[q];
-    return WalkX<float>{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    return Mob<float>{a.x, a.y, b.x, b.y};
   };
-  walk_up<float, kMode, WalkX<float>>(
-      c, iv, k, get, [](const WalkX<float> &x, float s) { return x.A + x.B * s; });
-  auto getx = [&](int q) { return RefineX{get(q), px[q]}; };
-  walk_down<float, kMode, RefineX>(
-      c, iv, k, getx, [&](int q, const RefineX &x, float y, float zp) {
-        const float zl = x.w.aL + x.w.bL * y + x.w.B * zp;
-        const float zf = x.w.ifa + x.w.ifb * y + x.w.ef * zp;
-        const double xl = x.b.y + f2d(zl);
-        // one row: first and last are the same
-        k.px[q] = make_double2(lk[q].w ? xl : x.b.x + f2d(zf), xl);
-        return zl;
-      });
+  if (staged(c, iv)) {
+#pragma unroll 4
+    for (int q = threadIdx.x; q < c.np; q += kThreads) k.st[q] = get(q);
+    __syncthreads();
+    auto sget = [&](int q) { return k.st[q]; };
+    walk_up<float, kMode, Mob<float>>(c, iv, k, sget, up);
+    walk_down<float, kMode, Mob<float>>(c, iv, k, sget,
+                                        [&](int, const Mob<float> &x, float y, float zp) {
+                                          return last(x.a, x.b, x.d, y, zp);
+                                        });
+    auto one = [&](int q) {
+      if (q == kNoPiece) return;
+      put(q, RefineX{ps[q], pa[q], px[q]}, k.yin[q], k.zpar[q], k.val[q], k.link[q].w != 0);
+    };
+    const int a = c.w0 < c.w1 ? iv.wbase[c.w0] : 0;
+    const int b = c.w0 < c.w1 ? (c.w1 < c.iw1 ? iv.wbase[c.w1] : c.np) : 0;
+    for (int o = a + threadIdx.x; o < b; o += kThreads) {
+      const int q = iv.pmap[c.ip0 + o];
+      const ushort4 t = k.link[q];
+      one(q);
+      one(t.x);
+      one(t.y);
+      one(t.z);
+    }
+    __syncthreads();
+    return;
+  }
+  walk_up<float, kMode, Mob<float>>(c, iv, k, get, up);
+  auto getx = [&](int q) { return RefineX{ps[q], pa[q], px[q]}; };
+  walk_down<float, kMode, RefineX>(c, iv, k, getx, [&](int q, const RefineX &x, float y, float zp) {
+    const float zl = last(x.s.x, x.s.y, x.v.y, y, zp);
+    put(q, x, y, zp, zl, lk[q].w != 0);
+    return zl;
+  });
 }
 
 // x += z by substitution (x0 = 2 Vin - Vout when Vin is not null, else Vout), then the FP64

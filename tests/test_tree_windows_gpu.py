@@ -60,8 +60,9 @@ def test_one_tree(gpu, pkg, orc, model, name, scheme):
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_batch_of_all(gpu, pkg, orc, model, precision):
-    """The same trees in one batch (instances start on multiples of four rows)."""
-    specs = [tree(model, n) for n in TREES]
+    """The same trees in one batch (instances start on multiples of four rows), with trees of
+    more pieces than shared memory holds at several places in it."""
+    specs = [tree(model, n) for n in ["cable5", "twigs", "71x4117"] + TREES]
     probs = [pkg.ProblemArrays.from_spec(sp, pkg.derive(sp)) for sp in specs]
     steps = 12
     out = {}

@@ -1018,7 +1018,7 @@ int nrt_calculate(nrt_solver *s) {
     if (!s) return nrt::fail(NRT_EINVAL, "null solver");
     if (!s->have_update) return nrt::fail(NRT_ESTATE, "calculate() without a preceding update()");
     NRT_CUDA(cudaSetDevice(s->eng.device));
-    const int64_t before = s->eng.opt.mode == NRT_IMPLICIT_BE ? nrt::nonconverged_total(s->eng) : 0;
+    const int64_t before = s->eng.nonconv_seen;  // every step of the handle ends with a look
     int rc = s->eng.step(0, s->pending_input);
     s->have_update = false;
     if (rc == NRT_OK && s->eng.opt.mode == NRT_IMPLICIT_BE) {
@@ -1069,11 +1069,13 @@ int nrt_run(nrt_solver *s, int64_t i_begin, int64_t i_end, double init_time, dou
     e.host.inst[0] = in;
     NRT_CUDA(cudaMemcpyAsync(e.pv.inst, &e.host.inst[0], sizeof(in), cudaMemcpyHostToDevice, e.stream));
     const bool implicit = e.opt.mode == NRT_IMPLICIT_BE;
-    const int64_t before = implicit ? nrt::nonconverged_total(e) : 0;
+    const int64_t before = e.nonconv_seen;
     int rc = e.advance(i_end - i_begin);
     if (rc) return rc;
-    if (implicit && nrt::nonconverged_total(e) > before)
-      rc = nrt::fail(NRT_ENOCONV, "an implicit step hit its Krylov iteration budget");
+    if (implicit) {
+      const int64_t after = nrt::nonconverged_total(e);
+      if (after > before) rc = nrt::fail(NRT_ENOCONV, "an implicit step hit its Krylov iteration budget");
+    }
     // leave the drop-in path's device loop range open again
     e.host.inst[0].base = 0;
     e.host.inst[0].iend = INT64_MAX;

@@ -70,11 +70,13 @@ constexpr int kMaxPiece = 256;                 // longest segment piece one swee
 constexpr int kMaxDots = kMaxRestart + 1;
 constexpr int kSumChunks = 8;                  // row chunks of an instance's sums (rows_reduce)
 constexpr int kTileBytes = 44 * 1024;          // shared memory of the preconditioners
+constexpr int kLevels = 128;                   // level offsets kept in shared memory
+constexpr int kBlockWalkBytes = 24 * 1024;     // shared memory of a block's walk
 constexpr int kWalkBytes = 190 * 1024;         // shared memory of the one-tree launch's walk
 constexpr int kClusterWalkBytes = 64 * 1024;   // and of a cluster's
-constexpr int kClusterWindows = 8;             // one tree of at most this many windows: a cluster
+constexpr int kClusterRows = 8 * 1024;         // one tree of at most this many rows: a cluster
 constexpr int kRW = 4;                         // tree preconditioner: rows per thread of a window
-constexpr int kWin = kThreads * kRW;           // rows of a window
+constexpr int kMaxWin = kThreads * kRW;        // rows of a window at most
 constexpr int kU = 4;                          // rows per thread in flight: SpMV + products
 constexpr int kV = 4;                          // rows per thread in flight: streaming passes
 constexpr int kA = 1;                          // rows per thread in flight: assembly
@@ -102,6 +104,8 @@ struct InstStat {
   // vectors read by the Arnoldi steps (sum of j + 1), and Richardson refinement steps
   int64_t residuals, applies, xupdates, basis, rich;
 };
+
+constexpr size_t kErrBytes = 16;  // the error word's place before the statistics
 
 struct ImView {
   int64_t ntot;
@@ -142,8 +146,9 @@ struct ImView {
   // exact tree preconditioner (NRT_PRECOND_TREE, tree.cuh): windows, pieces and levels of
   // each instance.  Piece ids are local to the instance, in level order (deepest first).
   void *cdiag;                    // T[ld]: c_j = c_m dX / dT - W dX, written by the assembly
+  int win;                        // rows of a window (a multiple of kRW)
   const uint8_t *pfl;             // [ld] row flags: R_IDENT .. R_FAR, P_FIRST, P_LAST
-  const uint16_t *wtp;            // [window][thread]: pieces that start in the window before it
+  const uint16_t *wtp;            // [window][win / kRW]: pieces that start in the window before it
   const int *wbase;               // [window] ordinal (row order) of its first piece
   const int *pmap;                // [piece ordinal] -> piece id
   const int4 *plink;              // [piece id]: ids of its children at DR (or the next row) and
@@ -157,6 +162,7 @@ struct ImView {
   double *pxb;                    // double[2] per piece, two buffers: V of its first, last row
   const double *pgf;              // per piece: FP64 conductance of its first row to the mother
   void *tinv, *te, *tbeta, *talpha;  // T[ld]: 1 / pivot, g / pivot, beta, alpha
+  void *tent;                     // T[4] per thread of a window: the map of its piece's later rows
   void *gwalk;                    // walk_bytes per piece: the walk's numbers beyond walk_cap
   int walk_cap;                   // pieces whose walk fits a CTA's shared memory
 };
@@ -428,6 +434,7 @@ struct Ctx {
   int ip0, np, l0, l1;
   int rank;         // this CTA in its group
   int n, v0, v1;    // rows of the instance; this CTA's chunks of them (rows_reduce)
+  const int *lev;   // the instance's level offsets (in shared memory, when they fit)
 };
 
 // A sync of the group where one CTA's rows reach another's (nothing to do in one CTA).
@@ -442,14 +449,14 @@ __device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, i
   return 2.0 * Vin[j] - Vout[j];
 }
 
-// Sums k accumulators of a row pass f(context) over the instance into S.red[off .. off + k).  In
+// Sums k accumulators of a row pass f(first row, end) over the instance into S.red[off .. off + k).  In
 // a block or a cluster the rows are taken in kSumChunks chunks whose sums are added in order,
 // so that the result does not depend on how many CTAs share the instance.
 template <typename T, int kMode, typename F>
 __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Shared &S,
                                             double *partials, int &parity, int off, F f) {
   if (kMode == kGrid) {
-    auto acc = f(c);
+    auto acc = f(c.r0, c.r1);
     group_reduce<kMode>(acc.v, k, S, partials, parity, off);
     return;
   }
@@ -459,10 +466,7 @@ __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Share
     parity ^= 1;
   }
   for (int v = c.v0; v < c.v1; v++) {
-    Ctx<T, kMode> d = c;
-    d.r0 = c.wrow0 + (int64_t)c.n * v / kSumChunks;
-    d.r1 = c.wrow0 + (int64_t)c.n * (v + 1) / kSumChunks;
-    auto acc = f(d);
+    auto acc = f(c.wrow0 + (int64_t)c.n * v / kSumChunks, c.wrow0 + (int64_t)c.n * (v + 1) / kSumChunks);
     block_reduce(acc.v, k, S.warp, S.red + off);
     if (threadIdx.x < k) sum[v * kMaxDots + threadIdx.x] = S.red[off + threadIdx.x];
   }
@@ -500,7 +504,7 @@ __device__ __forceinline__ void tile_rows(const ImView &iv, int q, int64_t &a, i
 // Thomas factorisation of every piece (once per step): pd = 1/pivot, pc = c'.
 // Staged through shared memory tile by tile; one thread per piece.
 template <typename T, int kMode>
-__device__ __noinline__ void factor_pieces(Ctx<T, kMode> c) {
+__device__ __noinline__ void factor_pieces(const Ctx<T, kMode> &c) {
   Shared S = carve(dyn_smem(), c.iv->m);
   T *sd = (T *)S.tile;                          // diag, then pivots^-1
   T *sg = sd + c.iv->tile_rows;                  // conductance to the mother
@@ -538,7 +542,7 @@ __device__ __noinline__ void factor_pieces(Ctx<T, kMode> c) {
 // z = M^-1 v over this CTA's rows (identity rows: v and z are 0).  eliminated: the tree
 // factorisation has eliminated v already.
 template <typename T, int kMode>
-__device__ __noinline__ void apply_precond(Ctx<T, kMode> c, const T *v, T *z,
+__device__ __noinline__ void apply_precond(const Ctx<T, kMode> &c, const T *v, T *z,
                                            bool eliminated = false) {
   Shared S = carve(dyn_smem(), c.iv->m);
   if (c.iv->precond == NRT_PRECOND_TREE) {
@@ -606,7 +610,7 @@ struct DotAcc {
 // formed from V^n and V^{n-1} directly (a row's columns are never identity rows).  Returns
 // the thread's parts of ||b||^2 and ||r||^2.
 template <typename T, int kMode>
-__device__ __noinline__ double2 ph_assemble(Ctx<T, kMode> c, const double *Vin,
+__device__ __noinline__ double2 ph_assemble(const Ctx<T, kMode> &c, int64_t r0, int64_t r1, const double *Vin,
                                             const double *Vout, int active, int inst) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
@@ -620,7 +624,7 @@ __device__ __noinline__ double2 ph_assemble(Ctx<T, kMode> c, const double *Vin,
   // gates of this precision (the mixed path keeps them in FP32)
   T *gate = sizeof(T) == 4 ? (T *)(void *)pv.gatef : (T *)(void *)pv.gate;
   const bool cn = iv.scheme == NRT_CRANK_NICOLSON;
-  for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kA * stride) {
+  for (int64_t rb = r0 + threadIdx.x; rb < r1; rb += kA * stride) {
     uint8_t f[kA];
     double v[kA], vo[kA], cm[kA], gj[kA], gn[kA], inp[kA], xm[kA], xp[kA], vm[kA], vp[kA];
     int64_t hc[kA];
@@ -629,7 +633,7 @@ __device__ __noinline__ double2 ph_assemble(Ctx<T, kMode> c, const double *Vin,
 #pragma unroll
     for (int u = 0; u < kA; u++) {
       const int64_t r = rb + u * stride;
-      const bool ok = r < c.r1;
+      const bool ok = r < r1;
       const int64_t rp = r + 1 < N ? r + 1 : r, rm = r > 0 ? r - 1 : r;
       hc[u] = ok && pv.hp_cls ? (int64_t)pv.hp_cls[r] : (pv.hp_inst ? (int64_t)inst : r);
       const bool gl = ok && pv.hh_dense;
@@ -651,7 +655,7 @@ __device__ __noinline__ double2 ph_assemble(Ctx<T, kMode> c, const double *Vin,
 #pragma unroll
     for (int u = 0; u < kA; u++) {
       const int64_t r = rb + u * stride;
-      if (r >= c.r1) continue;
+      if (r >= r1) continue;
       double wdx, kdx;
       if (f[u] & R_HH) {
         const int64_t L = pv.hp_ld;
@@ -744,7 +748,7 @@ __device__ __noinline__ double2 ph_assemble(Ctx<T, kMode> c, const double *Vin,
 
 // Vout = x0 for the rows of this group (when a step ends before any solution update).
 template <typename T, int kMode>
-__device__ __noinline__ void ph_x0(Ctx<T, kMode> c, const double *Vin, double *Vout) {
+__device__ __noinline__ void ph_x0(const Ctx<T, kMode> &c, const double *Vin, double *Vout) {
   const uint8_t *rowf = c.iv->rowf;
   for (int64_t j = c.r0 + threadIdx.x; j < c.r1; j += blockDim.x)
     if (!(rowf[j] & R_IDENT)) Vout[j] = x0_of(Vin, Vout, j);
@@ -757,20 +761,20 @@ __device__ __noinline__ void ph_x0(Ctx<T, kMode> c, const double *Vin, double *V
 // near 1 / (the previous residual norm), which keeps the entries in FP32's range.  FP64
 // solves and BiCGSTAB (whose rho_0 is this norm squared) take the FP64 sum.
 template <typename T, int kMode>
-__device__ __noinline__ double ph_residual(Ctx<T, kMode> c, const double *x, float scale) {
+__device__ __noinline__ double ph_residual(const Ctx<T, kMode> &c, int64_t r0, int64_t r1, const double *x, float scale) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
   const int64_t stride = blockDim.x;
   float acc = 0;
   double acc64 = 0;
-  for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kR * stride) {
+  for (int64_t rb = r0 + threadIdx.x; rb < r1; rb += kR * stride) {
     double rr[kR];
     uint8_t fl[kR];
-    residual_rows<kR>(pv, iv, iv.rhs, iv.diag, iv.g64, x, rb, stride, c.r1, rr, fl);
+    residual_rows<kR>(pv, iv, iv.rhs, iv.diag, iv.g64, x, rb, stride, r1, rr, fl);
 #pragma unroll
     for (int u = 0; u < kR; u++) {
       const int64_t r = rb + u * stride;
-      if (r >= c.r1) continue;
+      if (r >= r1) continue;
       if (fl[u] & R_IDENT) {
         c.w.Wb[r] = 0;
         continue;
@@ -789,7 +793,7 @@ __device__ __noinline__ double ph_residual(Ctx<T, kMode> c, const double *x, flo
 
 // y = s_j A Z_j, fused with the thread's parts of <y, W_i> for i < g1.
 template <typename T, int kMode>
-__device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kMode> c, int j, T sj, int g1) {
+__device__ __noinline__ DotAcc<T> ph_spmv(const Ctx<T, kMode> &c, int64_t r0, int64_t r1, int j, T sj, int g1) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
   const int64_t ld = iv.ld, stride = blockDim.x;
@@ -799,15 +803,15 @@ __device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kMode> c, int j, T sj, int g1) 
   DotAcc<T> acc;
 #pragma unroll
   for (int i = 0; i < kG; i++) acc.v[i] = 0;
-  for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kU * stride) {
+  for (int64_t rb = r0 + threadIdx.x; rb < r1; rb += kU * stride) {
     T y[kU];
     uint8_t fl[kU];
-    apply_rows_c<kU>(pv, iv, CT, GT, Zj, rb, stride, c.r1, y, fl);
+    apply_rows_c<kU>(pv, iv, CT, GT, Zj, rb, stride, r1, y, fl);
 #pragma unroll
     for (int u = 0; u < kU; u++) {
       const int64_t r = rb + u * stride;
       y[u] *= sj;
-      if (r < c.r1) c.w.y[r] = y[u];
+      if (r < r1) c.w.y[r] = y[u];
     }
 #pragma unroll
     for (int i = 0; i < kG; i++) {
@@ -816,7 +820,7 @@ __device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kMode> c, int j, T sj, int g1) 
 #pragma unroll
         for (int u = 0; u < kU; u++) {
           const int64_t r = rb + u * stride;
-          if (r < c.r1) acc.v[i] += y[u] * Wi[r];
+          if (r < r1) acc.v[i] += y[u] * Wi[r];
         }
       }
     }
@@ -826,17 +830,17 @@ __device__ __noinline__ DotAcc<T> ph_spmv(Ctx<T, kMode> c, int j, T sj, int g1) 
 
 // The thread's parts of <y, W_{i0+i}> for i < gk.
 template <typename T, int kMode>
-__device__ __noinline__ DotAcc<T> ph_products(Ctx<T, kMode> c, int i0, int gk) {
+__device__ __noinline__ DotAcc<T> ph_products(const Ctx<T, kMode> &c, int64_t r0, int64_t r1, int i0, int gk) {
   const int64_t ld = c.iv->ld, stride = blockDim.x;
   DotAcc<T> acc;
 #pragma unroll
   for (int i = 0; i < kG; i++) acc.v[i] = 0;
-  for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
+  for (int64_t rb = r0 + threadIdx.x; rb < r1; rb += kV * stride) {
     T y[kV];
 #pragma unroll
     for (int u = 0; u < kV; u++) {
       const int64_t r = rb + u * stride;
-      y[u] = r < c.r1 ? c.w.y[r] : (T)0;
+      y[u] = r < r1 ? c.w.y[r] : (T)0;
     }
 #pragma unroll
     for (int i = 0; i < kG; i++) {
@@ -845,7 +849,7 @@ __device__ __noinline__ DotAcc<T> ph_products(Ctx<T, kMode> c, int i0, int gk) {
 #pragma unroll
         for (int u = 0; u < kV; u++) {
           const int64_t r = rb + u * stride;
-          if (r < c.r1) acc.v[i] += y[u] * Wi[r];
+          if (r < r1) acc.v[i] += y[u] * Wi[r];
         }
       }
     }
@@ -855,16 +859,16 @@ __device__ __noinline__ DotAcc<T> ph_products(Ctx<T, kMode> c, int i0, int gk) {
 
 // W_{j+1} = y - sum_{i <= j} coef_i W_i; returns the thread's part of ||W_{j+1}||^2.
 template <typename T, int kMode>
-__device__ __noinline__ T ph_update(Ctx<T, kMode> c, int j, const T *coef) {
+__device__ __noinline__ T ph_update(const Ctx<T, kMode> &c, int64_t r0, int64_t r1, int j, const T *coef) {
   const int64_t ld = c.iv->ld, stride = blockDim.x;
   T *Wn = c.w.Wb + (size_t)(j + 1) * ld;
   T nacc = 0;
-  for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
+  for (int64_t rb = r0 + threadIdx.x; rb < r1; rb += kV * stride) {
     T a[kV];
 #pragma unroll
     for (int u = 0; u < kV; u++) {
       const int64_t r = rb + u * stride;
-      a[u] = r < c.r1 ? c.w.y[r] : (T)0;
+      a[u] = r < r1 ? c.w.y[r] : (T)0;
     }
 #pragma unroll 1
     for (int i = 0; i <= j; i++) {
@@ -874,7 +878,7 @@ __device__ __noinline__ T ph_update(Ctx<T, kMode> c, int j, const T *coef) {
 #pragma unroll
       for (int u = 0; u < kV; u++) {
         const int64_t r = rb + u * stride;
-        w[u] = r < c.r1 ? Wi[r] : (T)0;
+        w[u] = r < r1 ? Wi[r] : (T)0;
       }
 #pragma unroll
       for (int u = 0; u < kV; u++) a[u] -= ci * w[u];
@@ -882,7 +886,7 @@ __device__ __noinline__ T ph_update(Ctx<T, kMode> c, int j, const T *coef) {
 #pragma unroll
     for (int u = 0; u < kV; u++) {
       const int64_t r = rb + u * stride;
-      if (r < c.r1) {
+      if (r < r1) {
         Wn[r] = a[u];
         nacc += a[u] * a[u];
       }
@@ -894,7 +898,7 @@ __device__ __noinline__ T ph_update(Ctx<T, kMode> c, int j, const T *coef) {
 // V += sum_{i < k} coef_i Z_i (identity rows keep their value).  With Vin non-null this is
 // the step's first update and V starts from x0 = 2 Vin - V.
 template <typename T, int kMode>
-__device__ __noinline__ void ph_xupdate(Ctx<T, kMode> c, int k, const T *coef, double *Vout,
+__device__ __noinline__ void ph_xupdate(const Ctx<T, kMode> &c, int k, const T *coef, double *Vout,
                                         const double *Vin) {
   const int64_t ld = c.iv->ld, stride = blockDim.x;
   const uint8_t *rowf = c.iv->rowf;
@@ -935,7 +939,7 @@ __device__ __noinline__ void ph_xupdate(Ctx<T, kMode> c, int k, const T *coef, d
 
 // p = r + beta (p - omega v); beta == 0 gives p = r.
 template <typename T, int kMode>
-__device__ __noinline__ void ph_bicg_dir(Ctx<T, kMode> c, const T *r, T *p, const T *v, T beta,
+__device__ __noinline__ void ph_bicg_dir(const Ctx<T, kMode> &c, const T *r, T *p, const T *v, T beta,
                                          T omega) {
   const int64_t stride = blockDim.x;
   for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
@@ -958,7 +962,7 @@ __device__ __noinline__ void ph_bicg_dir(Ctx<T, kMode> c, const T *r, T *p, cons
 
 // out = A x; returns the thread's parts of <out, d0> and <out, d1> (d1 may be null).
 template <typename T, int kMode>
-__device__ __noinline__ DotAcc<T> ph_matvec(Ctx<T, kMode> c, const T *x, T *out, const T *d0,
+__device__ __noinline__ DotAcc<T> ph_matvec(const Ctx<T, kMode> &c, const T *x, T *out, const T *d0,
                                             const T *d1) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
@@ -991,7 +995,7 @@ __device__ __noinline__ DotAcc<T> ph_matvec(Ctx<T, kMode> c, const T *x, T *out,
 
 // s = r - alpha v; returns the thread's part of ||s||^2.
 template <typename T, int kMode>
-__device__ __noinline__ T ph_bicg_s(Ctx<T, kMode> c, const T *r, const T *v, T alpha, T *s) {
+__device__ __noinline__ T ph_bicg_s(const Ctx<T, kMode> &c, const T *r, const T *v, T alpha, T *s) {
   const int64_t stride = blockDim.x;
   T acc = 0;
   for (int64_t rb = c.r0 + threadIdx.x; rb < c.r1; rb += kV * stride) {
@@ -1016,7 +1020,7 @@ __device__ __noinline__ T ph_bicg_s(Ctx<T, kMode> c, const T *r, const T *v, T a
 // V += alpha ph + omega sh (FP64 accumulation; identity rows keep their value) and
 // r = s - omega t; returns the thread's parts of ||r||^2 and <rh, r>.
 template <typename T, int kMode>
-__device__ __noinline__ DotAcc<T> ph_bicg_x(Ctx<T, kMode> c, const T *ph, const T *sh,
+__device__ __noinline__ DotAcc<T> ph_bicg_x(const Ctx<T, kMode> &c, const T *ph, const T *sh,
                                             const T *s, const T *t, T alpha, T omega, T *r,
                                             const T *rh, double *Vout) {
   const int64_t stride = blockDim.x;
@@ -1058,7 +1062,7 @@ __device__ __noinline__ DotAcc<T> ph_bicg_x(Ctx<T, kMode> c, const T *ph, const 
 // Not inlined, so that the GMRES path's register allocation does not carry it.
 // Returns {parity, iters}.
 template <typename T, int kMode>
-__device__ __noinline__ int2 bicgstab_cycle(Ctx<T, kMode> c, int parity, double res,
+__device__ __noinline__ int2 bicgstab_cycle(const Ctx<T, kMode> &c, int parity, double res,
                                             double cycle_target, int budget, int iters,
                                             double *Vout) {
   const ImView &iv = *c.iv;
@@ -1118,7 +1122,7 @@ __device__ __noinline__ int2 bicgstab_cycle(Ctx<T, kMode> c, int parity, double 
 
 // One backward-Euler step of one group (CTA or grid) for instance `inst`.
 template <typename T, int kMode>
-__device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, int &parity, const double *Vin,
+__device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared &S, int &parity, const double *Vin,
                                                   double *Vout, bool active, int64_t inst_n,
                                                   int inst) {
   const ImView &iv = *c.iv;
@@ -1128,8 +1132,8 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
   const bool tree = iv.precond == NRT_PRECOND_TREE;
   const bool fused = sizeof(T) == 4 && iv.rich != 0;  // by windows, with the pieces' matrices
   double target = iv.tol, res0 = 0;
-  auto assemble = [&](const Ctx<T, kMode> &d) {
-    const double2 br = ph_assemble(d, Vin, Vout, active ? 1 : 0, inst);
+  auto assemble = [&](int64_t r0, int64_t r1) {
+    const double2 br = ph_assemble(c, r0, r1, Vin, Vout, active ? 1 : 0, inst);
     return Sums<double, 2>{{br.x, br.y}};
   };
   if (fused) {
@@ -1178,8 +1182,8 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
       const bool f32 = sizeof(T) == 4 && iv.krylov == NRT_GMRES;
       const int e = f32 ? max(-126, min(126, ilogb(res))) : 0;
       const float scale = f32 ? exp2f((float)-e) : 0.0f;
-      rows_reduce(c, 1, S, iv.partials, parity, 0, [&](const Ctx<T, kMode> &d) {
-        return Sums<double, 1>{{ph_residual(d, Vout, scale)}};
+      rows_reduce(c, 1, S, iv.partials, parity, 0, [&](int64_t r0, int64_t r1) {
+        return Sums<double, 1>{{ph_residual(c, r0, r1, Vout, scale)}};
       });
       res = sqrt(S.red[0]) * exp2((double)e);
       n_res++;
@@ -1235,7 +1239,7 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
       }
     }
     if (!w0_valid) {  // after the first refinement cycle W_0 is not stored
-      (void)ph_residual(c, Vout, 1.0f);
+      (void)ph_residual(c, c.r0, c.r1, Vout, 1.0f);
       w0_valid = true;
     }
     apply_precond(c, c.w.Wb, c.w.Z, eliminated && cycle == 0);
@@ -1255,12 +1259,12 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
       const int g1 = min(j + 1, kG);
       {
         rows_reduce(c, g1, S, iv.partials, parity, 0,
-                    [&](const Ctx<T, kMode> &d) { return ph_spmv(d, j, (T)S.s[j], g1); });
+                    [&](int64_t r0, int64_t r1) { return ph_spmv(c, r0, r1, j, (T)S.s[j], g1); });
       }
       for (int i0 = kG; i0 <= j; i0 += kG) {  // remaining products, kG at a time
         const int gk = min(j + 1 - i0, kG);
         rows_reduce(c, gk, S, iv.partials, parity, i0,
-                    [&](const Ctx<T, kMode> &d) { return ph_products(d, i0, gk); });
+                    [&](int64_t r0, int64_t r1) { return ph_products(c, r0, r1, i0, gk); });
       }
       if (threadIdx.x <= j) {
         const double h = S.s[threadIdx.x] * S.red[threadIdx.x];
@@ -1269,8 +1273,8 @@ __device__ __forceinline__ void implicit_one_step(Ctx<T, kMode> &c, Shared &S, i
       }
       __syncthreads();
       // w = y - sum_i h_ij s_i W_i -> W_{j+1}; ||w||^2
-      rows_reduce(c, 1, S, iv.partials, parity, 0, [&](const Ctx<T, kMode> &d) {
-        return Sums<T, 1>{{ph_update(d, j, coef)}};  // publishes W_{j+1}
+      rows_reduce(c, 1, S, iv.partials, parity, 0, [&](int64_t r0, int64_t r1) {
+        return Sums<T, 1>{{ph_update(c, r0, r1, j, coef)}};  // publishes W_{j+1}
       });
       if (threadIdx.x == 0) {
         const double hn = sqrt(S.red[0]);
@@ -1353,18 +1357,33 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
                                                            int nsteps, int force, double *V0,
                                                            double *V1, int cur,
                                                            const RecView *rec) {
-  const ImView &iv = *ivp;
+  // The views and the context live in shared memory: the passes read their fields all the time,
+  // and from device memory (or the stack) those reads were evicted from L1 by the rows that
+  // stream through it.
+  __shared__ PackView s_pv;
+  __shared__ ImView s_iv;
+  __shared__ Ctx<T, kMode> c;
+  __shared__ int s_lev[kLevels];
+  static_assert(sizeof(PackView) % 4 == 0 && sizeof(ImView) % 4 == 0, "copied by words");
+  for (int u = threadIdx.x; u < (int)(sizeof(PackView) / 4); u += kThreads)
+    ((int *)&s_pv)[u] = ((const int *)pvp)[u];
+  for (int u = threadIdx.x; u < (int)(sizeof(ImView) / 4); u += kThreads)
+    ((int *)&s_iv)[u] = ((const int *)ivp)[u];
+  __syncthreads();
+  const ImView &iv = s_iv;
   Shared S = carve(dyn_smem(), iv.m);
   int parity = 0;
-  Ctx<T, kMode> c;
-  c.pv = pvp;
-  c.iv = ivp;
-  c.w.Wb = (T *)iv.Wb;
-  c.w.Z = (T *)iv.Z;
-  c.w.y = (T *)iv.yv;
-  c.w.pd = (T *)iv.pcd;
-  c.w.pc = (T *)iv.pcc;
-  c.rank = group_rank<kMode>();
+  if (threadIdx.x == 0) {
+    c.pv = &s_pv;
+    c.iv = &s_iv;
+    c.w.Wb = (T *)iv.Wb;
+    c.w.Z = (T *)iv.Z;
+    c.w.y = (T *)iv.yv;
+    c.w.pd = (T *)iv.pcd;
+    c.w.pc = (T *)iv.pcc;
+    c.rank = group_rank<kMode>();
+  }
+  __syncthreads();
   const int gsize = group_size<kMode>();
   int q = kMode == kCluster ? (int)blockIdx.x / gsize : 0;
   for (;;) {
@@ -1381,36 +1400,44 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
     }
     const int n = iv.inst_n[inst];
     const bool tree = iv.precond == NRT_PRECOND_TREE;
-    c.n = n;
-    c.v0 = kSumChunks * c.rank / gsize;
-    c.v1 = kSumChunks * (c.rank + 1) / gsize;
-    c.wrow0 = iv.inst_row[inst];
-    c.wend = c.wrow0 + ((n + kRW - 1) & ~(kRW - 1));
-    c.r0 = c.wrow0 + (int64_t)n * c.v0 / kSumChunks;
-    c.r1 = c.wrow0 + (int64_t)n * c.v1 / kSumChunks;
-    c.iw0 = tree ? iv.inst_win[inst] : 0;
-    c.iw1 = tree ? iv.inst_win[inst + 1] : 0;
-    c.w0 = c.iw0 + (c.iw1 - c.iw0) * c.rank / gsize;
-    c.w1 = c.iw0 + (c.iw1 - c.iw0) * (c.rank + 1) / gsize;
-    c.ip0 = tree ? iv.inst_piece[inst] : 0;
-    c.np = tree ? iv.inst_piece[inst + 1] - c.ip0 : 0;
-    c.l0 = tree ? iv.inst_lev[inst] : 0;
-    c.l1 = tree ? iv.inst_lev[inst + 1] : 0;
-    if (kMode == kGrid) {
-      c.r0 = iv.cta_row[blockIdx.x];
-      c.r1 = iv.cta_row[blockIdx.x + 1];
-      c.t0 = iv.cta_tile[blockIdx.x];
-      c.t1 = iv.cta_tile[blockIdx.x + 1];
-      if (tree) {
-        c.w0 = iv.cta_win[blockIdx.x];
-        c.w1 = iv.cta_win[blockIdx.x + 1];
+    if (threadIdx.x == 0) {
+      c.n = n;
+      c.v0 = kSumChunks * c.rank / gsize;
+      c.v1 = kSumChunks * (c.rank + 1) / gsize;
+      c.wrow0 = iv.inst_row[inst];
+      c.wend = c.wrow0 + ((n + kRW - 1) & ~(kRW - 1));
+      c.r0 = c.wrow0 + (int64_t)n * c.v0 / kSumChunks;
+      c.r1 = c.wrow0 + (int64_t)n * c.v1 / kSumChunks;
+      c.iw0 = tree ? iv.inst_win[inst] : 0;
+      c.iw1 = tree ? iv.inst_win[inst + 1] : 0;
+      c.w0 = c.iw0 + (c.iw1 - c.iw0) * c.rank / gsize;
+      c.w1 = c.iw0 + (c.iw1 - c.iw0) * (c.rank + 1) / gsize;
+      c.ip0 = tree ? iv.inst_piece[inst] : 0;
+      c.np = tree ? iv.inst_piece[inst + 1] - c.ip0 : 0;
+      c.l0 = tree ? iv.inst_lev[inst] : 0;
+      c.l1 = tree ? iv.inst_lev[inst + 1] : 0;
+      if (kMode == kGrid) {
+        c.r0 = iv.cta_row[blockIdx.x];
+        c.r1 = iv.cta_row[blockIdx.x + 1];
+        c.t0 = iv.cta_tile[blockIdx.x];
+        c.t1 = iv.cta_tile[blockIdx.x + 1];
+        if (tree) {
+          c.w0 = iv.cta_win[blockIdx.x];
+          c.w1 = iv.cta_win[blockIdx.x + 1];
+        }
+      } else {
+        c.t0 = iv.inst_tile[inst];
+        c.t1 = iv.inst_tile[inst + 1];
       }
-    } else {
-      c.t0 = iv.inst_tile[inst];
-      c.t1 = iv.inst_tile[inst + 1];
     }
+    __syncthreads();
+    // a walk reads its level offsets level by level: from shared memory
+    const int nlev = c.l1 - c.l0;
+    for (int u = threadIdx.x; u < nlev && nlev <= kLevels; u += kThreads) s_lev[u] = iv.lev_off[c.l0 + u];
+    if (threadIdx.x == 0) c.lev = nlev <= kLevels ? s_lev : iv.lev_off + c.l0;
+    __syncthreads();
     if (tree) stage_links(c);
-    const InstDev in = pvp->inst[inst];
+    const InstDev in = s_pv.inst[inst];
     int s = 0;
     for (; s < nsteps; s++) {
       const int64_t i = in.base + s;
@@ -1456,6 +1483,7 @@ struct ImplicitState {
   int grid_blocks = 0;
   bool grid_mode = false;
   int cluster = 0;  // CTAs per cluster (0: not a cluster launch)
+  int win = 0;      // rows per window of the tree preconditioner
   int tile_rows = 0;
   size_t smem = 0;
   const void *kern = nullptr;
@@ -1503,24 +1531,24 @@ struct InstPieces {
   std::vector<double> pgf;
 };
 
-static void instance_pieces(const HostPack &host, const uint8_t *rowf, int32_t i, uint8_t *pfl,
-                            uint16_t *wtp, InstPieces &L) {
+static void instance_pieces(const HostPack &host, const uint8_t *rowf, int32_t i, int win,
+                            uint8_t *pfl, uint16_t *wtp, InstPieces &L) {
   struct Piece {
     int parent, level, c1, c2;
     int64_t row;
     int len;
   };
   const int64_t o = host.off[i], n = host.num_elem[i];
-  const int64_t n4 = (n + kRW - 1) & ~(int64_t)(kRW - 1), nw = (n + kWin - 1) / kWin;
+  const int64_t n4 = (n + kRW - 1) & ~(int64_t)(kRW - 1), nw = (n + win - 1) / win;
   constexpr uint8_t keep = R_IDENT | R_UP | R_DOWNR | R_DOWNL | R_FAR;
   std::vector<Piece> pc;
   std::vector<int> piece_of(n, -1);
   L.wbase.resize(nw);
   int cur = -1, max_level = -1;
-  for (int64_t j = 0; j < nw * kWin; j++) {
-    if (j % kWin == 0) L.wbase[j / kWin] = (int)pc.size();
+  for (int64_t j = 0; j < nw * win; j++) {
+    if (j % win == 0) L.wbase[j / win] = (int)pc.size();
     if (j % kRW == 0)
-      wtp[(j / kWin) * kThreads + (j % kWin) / kRW] = (uint16_t)(pc.size() - L.wbase[j / kWin]);
+      wtp[(j / win) * (win / kRW) + (j % win) / kRW] = (uint16_t)(pc.size() - L.wbase[j / win]);
     if (j >= n) {
       if (j < n4) pfl[j] = P_IDENT;
       continue;
@@ -1531,7 +1559,7 @@ static void instance_pieces(const HostPack &host, const uint8_t *rowf, int32_t i
       cur = -1;
       continue;
     }
-    const bool linked = cur >= 0 && j % kWin != 0 && (f & R_UP) && !(f & R_FAR) &&
+    const bool linked = cur >= 0 && j % win != 0 && (f & R_UP) && !(f & R_FAR) &&
                         !(host.topo[o + j - 1].flags & F_BRANCH);
     if (!linked) {
       const int64_t m = (f & R_UP) ? host.topo[o + j].mother - o : -1;
@@ -1549,7 +1577,7 @@ static void instance_pieces(const HostPack &host, const uint8_t *rowf, int32_t i
     piece_of[j] = cur;
     pc[cur].len++;
     // the piece ends here unless the next row continues it
-    const bool more = j + 1 < n && (j + 1) % kWin != 0 && !(rowf[j + 1] & R_IDENT) &&
+    const bool more = j + 1 < n && (j + 1) % win != 0 && !(rowf[j + 1] & R_IDENT) &&
                       (rowf[j + 1] & R_UP) && !(rowf[j + 1] & R_FAR) &&
                       !(host.topo[o + j].flags & F_BRANCH);
     if (!more) pfl[j] |= P_LAST;
@@ -1570,7 +1598,8 @@ static void instance_pieces(const HostPack &host, const uint8_t *rowf, int32_t i
   }
 }
 
-static void build_tree_plan(const HostPack &host, const uint8_t *rowf, int64_t ld, TreePlan &T) {
+static void build_tree_plan(const HostPack &host, const uint8_t *rowf, int64_t ld, int win,
+                            TreePlan &T) {
   const int32_t ni = host.ninst;
   std::vector<InstPieces> loc(ni);
   T.inst_win.resize(ni + 1);
@@ -1578,12 +1607,12 @@ static void build_tree_plan(const HostPack &host, const uint8_t *rowf, int64_t l
   T.inst_lev.resize(ni + 1);
   T.inst_win[0] = T.inst_piece[0] = T.inst_lev[0] = 0;
   for (int32_t i = 0; i < ni; i++)
-    T.inst_win[i + 1] = T.inst_win[i] + (host.num_elem[i] + kWin - 1) / kWin;
+    T.inst_win[i + 1] = T.inst_win[i] + (host.num_elem[i] + win - 1) / win;
   T.pfl.resize(ld);
-  T.wtp.resize((size_t)T.inst_win[ni] * kThreads);
+  T.wtp.resize((size_t)T.inst_win[ni] * (win / kRW));
   parallel_for(ni, [&](int64_t i) {
-    instance_pieces(host, rowf + host.off[i], (int32_t)i, T.pfl.data() + host.off[i],
-                    T.wtp.data() + (size_t)T.inst_win[i] * kThreads, loc[i]);
+    instance_pieces(host, rowf + host.off[i], (int32_t)i, win, T.pfl.data() + host.off[i],
+                    T.wtp.data() + (size_t)T.inst_win[i] * (win / kRW), loc[i]);
   });
   for (int32_t i = 0; i < ni; i++) {
     T.inst_piece[i + 1] = T.inst_piece[i] + (int)loc[i].pmap.size();
@@ -1698,7 +1727,6 @@ int Engine::implicit_plan(size_t &bytes) {
   const size_t tb = mixed ? 4 : 8;
   const int64_t ld = (N + kRW - 1) & ~(int64_t)(kRW - 1);
   S.tile_rows = (int)(kTileBytes / (4 * tb));
-  if (tree) build_tree_plan(host, S.rowf.data(), ld, S.tree);
   int dev_sms = 0;
   NRT_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
   S.grid_mode = ni == 1 && opt.schedule == 0;
@@ -1707,19 +1735,30 @@ int Engine::implicit_plan(size_t &bytes) {
   // idle as long as there are fewer instances than SMs, and a small single tree spends most of a
   // cooperative launch's step in its grid-wide syncs (1.5 to 2 us each; a cluster's barrier
   // takes about 0.4).
-  int64_t max_win = 0;
-  for (int32_t i = 0; tree && i < ni; i++)
-    max_win = std::max<int64_t>(max_win, S.tree.inst_win[i + 1] - S.tree.inst_win[i]);
+  int64_t max_n = 0;
+  for (int32_t i = 0; i < ni; i++) max_n = std::max<int64_t>(max_n, host.num_elem[i]);
   S.cluster = 0;
   if (tree && opt.krylov == NRT_GMRES && opt.schedule == 0 && opt.tile_ctas_per_sm == 0) {
     if (ni == 1) {
-      if (max_win <= kClusterWindows) S.cluster = 8;
+      if (max_n <= kClusterRows) S.cluster = 8;
     } else {
       for (int cs = 2; cs <= 8; cs *= 2)
         if ((int64_t)ni * cs <= (int64_t)dev_sms * (mixed ? 3 : 2)) S.cluster = cs;
     }
   }
   if (S.cluster) S.grid_mode = false;
+  if (tree) {
+    // Rows per window: 1024; in a single tree fewer (down to 128, one warp's) where its CTAs
+    // would otherwise not all have a window.  A window's FP64 arithmetic is bound by its SM's
+    // FP64 pipe, so a small tree's windows go to as many SMs as it has CTAs.  (The windows set
+    // the order of the scans' sums, so those of a batch do not depend on its size.)
+    S.win = kMaxWin;
+    if (ni == 1) {
+      const int64_t ctas = S.cluster ? S.cluster : S.grid_mode ? dev_sms : 1;
+      while (S.win > 128 && S.win * ctas >= 2 * max_n) S.win /= 2;
+    }
+    build_tree_plan(host, S.rowf.data(), ld, S.win, S.tree);
+  }
   const int group = S.cluster ? kCluster : S.grid_mode ? kGrid : kBlock;
   const void *kern = implicit_kernel(mixed, group);
   S.kern = kern;
@@ -1730,7 +1769,7 @@ int Engine::implicit_plan(size_t &bytes) {
   if (segs) tile = kTileBytes;
   if (tree) {
     const bool grp = group != kBlock;
-    const size_t cap = S.grid_mode ? kWalkBytes : S.cluster ? kClusterWalkBytes : kTileBytes;
+    const size_t cap = S.grid_mode ? kWalkBytes : S.cluster ? kClusterWalkBytes : kBlockWalkBytes;
     S.iv.walk_cap = (int)std::min<size_t>(std::min<size_t>(cap / walk_bytes(tb, grp), kNoPiece - 1),
                                           (size_t)S.tree.max_pieces);
     tile = (size_t)S.iv.walk_cap * walk_bytes(tb, grp);
@@ -1827,8 +1866,8 @@ int Engine::implicit_plan(size_t &bytes) {
   else
     b += al256(4 * S.inst_tile.size()) + al256(4 * S.order.size());
   b += 2 * al256(8 * S.inst_row.size()) + al256(4 * S.inst_n.size());
-  b += 2 * al256(4) + al256(sizeof(double) * 2 * 4096 * kMaxDots);
-  b += al256(sizeof(InstStat) * ni) + al256(sizeof(PackView)) + al256(sizeof(ImView));
+  b += al256(4) + al256(sizeof(double) * 2 * 4096 * kMaxDots);
+  b += al256(kErrBytes + sizeof(InstStat) * ni) + al256(sizeof(PackView)) + al256(sizeof(ImView));
   if (tree) {
     const TreePlan &T = S.tree;
     const size_t npc = std::max<size_t>(1, T.pmap.size());
@@ -1838,6 +1877,7 @@ int Engine::implicit_plan(size_t &bytes) {
     b += 2 * al256(4 * tb * npc) + al256(8 * tb * npc) + al256(walk_bytes(tb, false) * npc);  // pmob, pstat, pval, gwalk
     b += al256(8 * npc) + al256(32 * npc);                  // pgf, pxb
     b += 4 * al256(tb * ld);                                // tinv, te, tbeta, talpha
+    b += al256(4 * tb * T.wtp.size());                      // tent
   }
   bytes = b + 4096;
   return NRT_OK;
@@ -1857,6 +1897,7 @@ int Engine::implicit_init() {
   const bool tree = opt.precond == NRT_PRECOND_TREE, segs = opt.precond == NRT_PRECOND_SEGMENT;
   iv.ntot = N;
   iv.ld = ld;
+  iv.win = S.win;
   iv.m = opt.restart;
   iv.precond = opt.precond;
   iv.krylov = opt.krylov;
@@ -1930,11 +1971,16 @@ int Engine::implicit_init() {
   for (int32_t i = 0; i < ni; i++) out[i + 1] = out[i] + host.num_elem[i];
   TRYI(up(arena, pl, out.data(), out.size(), st)); iv.inst_out = pl;
   TRYI(up(arena, iv.queue, (const int *)nullptr, 1, st));
-  TRYI(up(arena, iv.err, (const int *)nullptr, 1, st));
-  NRT_CUDA(cudaMemsetAsync(iv.err, 0, sizeof(int), st));
   TRYI(up(arena, iv.partials, (const double *)nullptr, (size_t)2 * 4096 * kMaxDots, st));
-  std::vector<InstStat> zero(ni, InstStat{0, 0, 0, 0.0, 0, 0, 0, 0, 0});
-  TRYI(up(arena, iv.stats, zero.data(), ni, st));
+  // the error word and the statistics lie side by side: one copy reads both
+  char *es = (char *)arena.take(kErrBytes + sizeof(InstStat) * ni);
+  if (!es) {
+    set_error("arena exhausted (statistics)");
+    return NRT_ENOMEM;
+  }
+  NRT_CUDA(cudaMemsetAsync(es, 0, kErrBytes + sizeof(InstStat) * ni, st));
+  iv.err = (int *)es;
+  iv.stats = (InstStat *)(es + kErrBytes);
   if (tree) {
     const TreePlan &T = S.tree;
     const size_t npc = std::max<size_t>(1, T.pmap.size());
@@ -1962,8 +2008,9 @@ int Engine::implicit_init() {
     iv.te = arena.take(tb * ld);
     iv.tbeta = arena.take(tb * ld);
     iv.talpha = arena.take(tb * ld);
+    iv.tent = arena.take(4 * tb * T.wtp.size());
     if (!iv.pmob || !iv.pstat || !iv.pval || !iv.pxb || !iv.gwalk || !iv.tinv || !iv.te || !iv.tbeta ||
-        !iv.talpha) {
+        !iv.talpha || !iv.tent) {
       set_error("arena exhausted (tree preconditioner)");
       return NRT_ENOMEM;
     }
@@ -1983,7 +2030,7 @@ int Engine::implicit_init() {
 // Runs `nsteps` implicit steps for every instance (one launch).
 static int implicit_launch(Engine &e, int nsteps, int force) {
   ImplicitState &S = *e.im;
-  NRT_CUDA(cudaMemsetAsync(S.iv.queue, 0, sizeof(int), e.stream));
+  if (!S.grid_mode && !S.cluster) NRT_CUDA(cudaMemsetAsync(S.iv.queue, 0, sizeof(int), e.stream));
   const PackView *pv = S.d_pv;
   const ImView *iv = S.d_iv;
   double *V0 = e.V[0], *V1 = e.V[1];
@@ -2108,17 +2155,27 @@ int implicit_compact(Engine &e, const double *&src, int64_t &n) {
   return NRT_OK;
 }
 
-// Sum of non-converged steps over all instances (-1 on a device error).
+// Sum of non-converged steps over all instances (-1 on a device error); waits for the stream.
 int64_t nonconverged_total(Engine &e) {
   if (!e.im) return 0;
-  if (implicit_check(e) != NRT_OK) return -1;
-  std::vector<InstStat> s(e.host.ninst);
-  if (cudaMemcpyAsync(s.data(), e.im->iv.stats, sizeof(InstStat) * e.host.ninst,
-                      cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
+  const size_t bytes = kErrBytes + sizeof(InstStat) * e.host.ninst;
+  std::vector<int64_t> buf(bytes / 8);  // InstStat is made of 8-byte fields and pairs of 4
+  if (cudaMemcpyAsync(buf.data(), e.im->iv.err, bytes, cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
       cudaStreamSynchronize(e.stream) != cudaSuccess)
     return -1;
+  int err;
+  memcpy(&err, buf.data(), sizeof(err));
+  if (err) {
+    set_error("implicit kernel: a bounded wait expired");
+    return -1;
+  }
   int64_t t = 0;
-  for (const InstStat &x : s) t += x.nonconv;
+  for (int32_t i = 0; i < e.host.ninst; i++) {
+    InstStat x;
+    memcpy(&x, (const char *)buf.data() + kErrBytes + sizeof(InstStat) * i, sizeof(x));
+    t += x.nonconv;
+  }
+  e.nonconv_seen = t;
   return t;
 }
 

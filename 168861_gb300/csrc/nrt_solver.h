@@ -33,6 +33,7 @@ struct Engine {
   int cur = 0;
   int64_t *terms = nullptr;
   int64_t steps_done = 0;
+  int64_t nonconv_seen = 0;   // implicit: non-converged steps at the last look (nonconverged_total)
   bool terminals_dirty = false;
   bool general_next = false;  // explicit: the next step runs in the general form
   cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};  // one per starting buffer parity

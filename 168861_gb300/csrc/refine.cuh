@@ -36,7 +36,7 @@ __device__ __forceinline__ void window_ends(const double (&x)[kRW], double *ends
 
 // kCn: Crank-Nicolson.
 template <int kMode, bool kCn>
-__device__ __noinline__ double2 refine_assemble(Ctx<float, kMode> c, const double *Vin,
+__device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, const double *Vin,
                                                 const double *Vout, int active, int inst) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
@@ -51,126 +51,123 @@ __device__ __noinline__ double2 refine_assemble(Ctx<float, kMode> c, const doubl
     float *sc = (float *)S.warp + par * 5 * kWarps;
     par ^= 1;
     WinRows<float, kMode> r(c, iv, w);
-    const int64_t rb = r.rb;
-    float cc[kRW] = {}, gf[kRW] = {}, rr4[kRW] = {};
-    if (r.ok) {
-      double v[kRW], xv[kRW], cm[kRW], g[kRW];
-      ld_rows(Vin + rb, v);
-      ld_rows(Vout + rb, xv);
-      ld_rows(iv.cmdt + rb, cm);
-      ld_rows(iv.g64 + rb, g);
-      const int64_t rm = rb > 0 ? rb - 1 : 0, rp = rb + kRW < N ? rb + kRW : N - 1;
-      const double vmo = Vin[rm], vno = Vin[rp], omo = Vout[rm], ono = Vout[rp];
-      const double gnext = iv.g64[rp];
-      const uint32_t rf = *(const uint32_t *)(iv.rowf + rb);
-      float g0[kRW] = {}, g1[kRW] = {}, g2[kRW] = {};
+    float cc[kRW] = {}, gf[kRW] = {};
+    // two rows at a time: four would not fit the registers
+#pragma unroll
+    for (int u0 = 0; u0 < kRW; u0 += 2) {
+      if (!r.ok) continue;
+      asm volatile("" ::: "memory");  // the second pair's loads stay behind the first's work
+      const int64_t rb = r.rb + u0;
+      const double2 v2 = *(const double2 *)(Vin + rb), o2 = *(const double2 *)(Vout + rb);
+      const double2 cm2 = *(const double2 *)(iv.cmdt + rb), g2 = *(const double2 *)(iv.g64 + rb);
+      const float2 gf2 = *(const float2 *)(iv.gf + rb);
+      const int64_t rm = rb > 0 ? rb - 1 : 0, rp = rb + 2 < N ? rb + 2 : N - 1;
+      const double vb = Vin[rm], va = Vin[rp], ob = Vout[rm], oa = Vout[rp], ga = iv.g64[rp];
+      const uint32_t rf = *(const uint16_t *)(iv.rowf + rb);
+      float2 m2 = make_float2(0, 0), h2 = m2, n2 = m2;
       if (dense) {
-        ld_rows(gate + rb, g0);
-        ld_rows(gate + N + rb, g1);
-        ld_rows(gate + 2 * N + rb, g2);
+        m2 = *(const float2 *)(gate + rb);
+        h2 = *(const float2 *)(gate + N + rb);
+        n2 = *(const float2 *)(gate + 2 * N + rb);
       }
-      uint4 cls = make_uint4(0, 0, 0, 0);
-      if (pv.hp_cls) cls = *(const uint4 *)(pv.hp_cls + rb);
-      const double xm = 2.0 * vmo - omo, xp = 2.0 * vno - ono;
+      uint2 cls = make_uint2(0, 0);
+      if (pv.hp_cls) cls = *(const uint2 *)(pv.hp_cls + rb);
+      const double v[2] = {v2.x, v2.y}, cm[2] = {cm2.x, cm2.y}, g[3] = {g2.x, g2.y, ga};
+      // x0 of the rows before, of this pair and after it
+      const double x[4] = {2.0 * vb - ob, 2.0 * v2.x - o2.x, 2.0 * v2.y - o2.y, 2.0 * va - oa};
+      float gm[2] = {m2.x, m2.y}, gh[2] = {h2.x, h2.y}, gn[2] = {n2.x, n2.y}, rr[2];
+      double dg[2], rh[2];
 #pragma unroll
-      for (int u = 0; u < kRW; u++) xv[u] = 2.0 * v[u] - xv[u];  // x0
-      double dg[kRW], rh[kRW];
-#pragma unroll
-      for (int u = 0; u < kRW; u++) {
-        const int64_t row = rb + u;
-        const uint32_t f = (rf >> (8 * u)) & 0xffu;
-        dg[u] = rh[u] = 0.0;
-        float wdxf, kdxf;
-        double wdx, kdx;
-        if (!r.is(u, P_IDENT) || (f & R_HH)) {  // identity rows' gates move too
-          if (f & R_HH) {
-            if (!dense) {
-              g0[u] = gate[row];
-              g1[u] = gate[N + row];
-              g2[u] = gate[2 * N + row];
-            }
-            const uint32_t cl = u == 0 ? cls.x : u == 1 ? cls.y : u == 2 ? cls.z : cls.w;
-            const HHParams32 q =
-                hh_params32(pv.hpq, pv.hp_cls ? (int64_t)cl : (pv.hp_inst ? (int64_t)inst : row));
-            const float dv = d2f(v[u] - f2d(q.v[HP_REST]));
-            GateStep32 s = hh_step32(dv + q.v[HP_LSNA], dv + q.v[HP_LSK], g0[u], g1[u], g2[u],
-                                     q.v[HP_DTMS], q.v[HP_GNA], q.v[HP_GK], q.v[HP_GL],
-                                     q.v[HP_ENA], q.v[HP_EK], q.v[HP_EL]);
-            g0[u] = s.m;
-            g1[u] = s.h;
-            g2[u] = s.n;
-            if (!dense) {
-              gate[row] = s.m;
-              gate[N + row] = s.h;
-              gate[2 * N + row] = s.n;
-            }
-            wdxf = s.W * q.v[HP_DX];
-            kdxf = s.K * q.v[HP_DX];
-            wdx = f2d(wdxf);
-            kdx = f2d(kdxf);
-          } else {
-            wdx = iv.wdx64[row];
-            kdx = iv.kdx64[row];
+      for (int e = 0; e < 2; e++) {
+        const int u = u0 + e;
+        const int64_t row = rb + e;
+        const uint32_t f = (rf >> (8 * e)) & 0xffu;
+        const bool phys = !(f & R_IDENT);
+        double wdx = 0.0, kdx = 0.0;
+        if (f & R_HH) {  // identity rows' gates move too
+          if (!dense) {
+            gm[e] = gate[row];
+            gh[e] = gate[N + row];
+            gn[e] = gate[2 * N + row];
           }
+          const HHParams32 q = hh_params32(
+              pv.hpq, pv.hp_cls ? (int64_t)(e ? cls.y : cls.x) : (pv.hp_inst ? (int64_t)inst : row));
+          const float dv = d2f(v[e] - f2d(q.v[HP_REST]));
+          const GateStep32 s = hh_step32(dv + q.v[HP_LSNA], dv + q.v[HP_LSK], gm[e], gh[e], gn[e],
+                                         q.v[HP_DTMS], q.v[HP_GNA], q.v[HP_GK], q.v[HP_GL],
+                                         q.v[HP_ENA], q.v[HP_EK], q.v[HP_EL]);
+          gm[e] = s.m;
+          gh[e] = s.h;
+          gn[e] = s.n;
+          if (!dense) {
+            gate[row] = s.m;
+            gate[N + row] = s.h;
+            gate[2 * N + row] = s.n;
+          }
+          wdx = f2d(s.W * q.v[HP_DX]);
+          kdx = f2d(s.K * q.v[HP_DX]);
+        } else if (phys) {
+          wdx = iv.wdx64[row];
+          kdx = iv.kdx64[row];
         }
-        if (r.is(u, P_IDENT)) continue;
-        const double gn = u + 1 < kRW ? g[u + 1 < kRW ? u + 1 : 0] : gnext;
-        const double cj = (kCn ? 2.0 * cm[u] : cm[u]) - wdx;
-        double d = cj, gl = 0.0, xl = 0.0, xmo = u > 0 ? xv[u > 0 ? u - 1 : 0] : xm;
-        double vmother = u > 0 ? v[u > 0 ? u - 1 : 0] : vmo, vl = 0.0;
+        // rare rows: the mother is not the row before, or there is a DL child
+        double gl = 0.0, xl = 0.0, vl = 0.0, xmo = x[e], vmo = e ? v[0] : vb;
         if (f & (R_DOWNL | R_FAR)) {
           const Topo t = pv.topo[row];
           if (f & R_DOWNL) {
             gl = iv.g64[t.dl];
             xl = x0_of(Vin, Vout, t.dl);
             if (kCn) vl = Vin[t.dl];
-            d += gl;
           }
           if (f & R_FAR) {
             xmo = x0_of(Vin, Vout, t.mother);
-            vmother = Vin[t.mother];
+            if (kCn) vmo = Vin[t.mother];
           }
         }
-        if (f & R_DOWNR) d += gn;
-        if (f & R_UP) d += g[u];
-        dg[u] = d;
-        cc[u] = d2f(cj);
-        if (f & R_UP) gf[u] = d2f(g[u]);
-        const bool inj = active && (f & R_INP);
+        // the rest without branches but the rare ones: conductances of missing columns are 0
+        const double gup = (f & R_UP) ? g[e] : 0.0, gdn = (f & R_DOWNR) ? g[e + 1] : 0.0;
+        const double cj = (kCn ? 2.0 * cm[e] : cm[e]) - wdx;
+        double d = (cj + gdn) + gup;
+        if (f & R_DOWNL) d += gl;
         double b;
         if (!kCn) {
-          b = cm[u] * v[u] + kdx;
-          if (inj) b += iv.inp64[row];
+          b = cm[e] * v[e] + kdx;
+          if (active && (f & R_INP)) b += iv.inp64[row];
         } else {  // (2 c_m dX/dT + W dX) V^n - sum g (V^n - V^n_q) + 2 (K dX + I)
-          b = (2.0 * cm[u] + wdx) * v[u];
-          if (f & R_UP) b -= g[u] * (v[u] - vmother);
-          if (f & R_DOWNR) b -= gn * (v[u] - (u + 1 < kRW ? v[u + 1 < kRW ? u + 1 : 0] : vno));
-          if (f & R_DOWNL) b -= gl * (v[u] - vl);
+          b = (2.0 * cm[e] + wdx) * v[e];
+          b -= gup * (v[e] - vmo);
+          b -= gdn * (v[e] - (e ? va : v[1]));
+          if (f & R_DOWNL) b -= gl * (v[e] - vl);
           b += 2.0 * kdx;
-          if (inj) b += 2.0 * iv.inp64[row];
+          if (active && (f & R_INP)) b += 2.0 * iv.inp64[row];
         }
-        rh[u] = b;
+        double res = fma(-d, x[e + 1], b);
+        res = fma(gup, xmo, res);
+        res = fma(gdn, x[e + 2], res);
+        if (f & R_DOWNL) res = fma(gl, xl, res);
+        if (!phys) b = res = 0.0;
+        dg[e] = d;
+        rh[e] = b;
+        cc[u] = d2f(cj);
+        gf[u] = (f & R_UP) ? (e ? gf2.y : gf2.x) : 0.0f;
+        rr[e] = d2f(res);
         const float bf = d2f(b);
         bacc += bf * bf;
-        double rr = fma(-d, xv[u], b);
-        if (f & R_UP) rr = fma(g[u], xmo, rr);
-        if (f & R_DOWNR) rr = fma(gn, u + 1 < kRW ? xv[u + 1 < kRW ? u + 1 : 0] : xp, rr);
-        if (f & R_DOWNL) rr = fma(gl, xl, rr);
-        rr4[u] = d2f(rr);
-        racc += rr * rr;
+        racc += res * res;
       }
       if (dense) {
-        st_rows(gate + rb, g0);
-        st_rows(gate + N + rb, g1);
-        st_rows(gate + 2 * N + rb, g2);
+        *(float2 *)(gate + rb) = make_float2(gm[0], gm[1]);
+        *(float2 *)(gate + N + rb) = make_float2(gh[0], gh[1]);
+        *(float2 *)(gate + 2 * N + rb) = make_float2(gn[0], gn[1]);
       }
-      st_rows(iv.diag + rb, dg);
-      st_rows(iv.rhs + rb, rh);
-      st_rows((float *)iv.cdiag + rb, cc);
-      st_rows(c.w.Wb + rb, rr4);
+      *(double2 *)(iv.diag + rb) = make_double2(dg[0], dg[1]);
+      *(double2 *)(iv.rhs + rb) = make_double2(rh[0], rh[1]);
+      *(float2 *)((float *)iv.cdiag + rb) = make_float2(cc[u0], cc[u0 + 1]);
+      *(float2 *)(c.w.Wb + rb) = make_float2(rr[0], rr[1]);
     }
     r.ids(c, iv);
-    window_maps(r, cc, gf, (Mob<float> *)iv.pmob + c.ip0, sc);
+    window_maps(r, cc, gf, (Mob<float> *)iv.pmob + c.ip0,
+                (float *)iv.tent + 4 * thread_slot(iv, w), sc);
   }
   __syncthreads();  // its scans' scratch is free for the next reduction
   return make_double2((double)bacc, racc);
@@ -185,7 +182,7 @@ struct RefineX {
 // rows (in a group: of this CTA's pieces and the ones next to them).  pb: the buffer of the
 // pieces' values.
 template <int kMode>
-__device__ __noinline__ void refine_walk(Ctx<float, kMode> c, int pb) {
+__device__ __noinline__ void refine_walk(const Ctx<float, kMode> &c, int pb) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<float> k = walk_of(c, iv, S);
@@ -244,7 +241,7 @@ __device__ __noinline__ void refine_walk(Ctx<float, kMode> c, int pb) {
 // residual b - A x; returns the thread's part of ||scale r||^2 in FP32 (see ph_residual).
 // kElim: eliminates r into buffer pb of the pieces' values; else stores it (W_0).
 template <int kMode, bool kElim>
-__device__ __noinline__ float refine_update(Ctx<float, kMode> c, const double *Vin, double *Vout,
+__device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const double *Vin, double *Vout,
                                             float scale, int pb) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
@@ -289,7 +286,7 @@ __device__ __noinline__ float refine_update(Ctx<float, kMode> c, const double *V
         M *= ee[u];
       }
     }
-    affine_enter<float, 1, false>(A, M, scz, y);
+    affine_enter<float, 1, false>(A, M, scz, y, r.idle);
     float cur = y[0];
 #pragma unroll
     for (int u = 0; u < kRW; u++) {

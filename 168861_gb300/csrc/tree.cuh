@@ -13,9 +13,10 @@
 // children, leaves to root, then z_k = inv_k y_k + e_k z_mother, root to leaves.
 //
 // Work is split into *pieces*: runs of consecutive rows in which each row's mother is the row
-// before it, ended by branch points, sealed ends and window edges.  A window is kWin
-// consecutive rows of an instance, kRW consecutive rows per thread of a CTA; a piece lies in
-// one window.  Everything a piece passes to the rest of the tree is a map of one number in,
+// before it, ended by branch points, sealed ends and window edges.  A window is ImView::win
+// consecutive rows of an instance, kRW consecutive rows per thread of a CTA (at most 1024; fewer
+// where a small tree's rows are to be spread over more SMs, and then the CTA's last warps have
+// none); a piece lies in one window.  Everything a piece passes to the rest of the tree is a map of one number in,
 // one number out, whatever the rest of the tree holds:
 //   - factorisation: the conductance s that its children give its last row -> the
 //     conductance e_f eta_f its first row gives its mother, a Moebius map (2x2 matrix);
@@ -65,6 +66,11 @@ __device__ __forceinline__ void st_rows(T *p, const T (&o)[kRW]) {
   }
 }
 
+// This thread's place in the arrays of one entry per thread of a window.
+__device__ __forceinline__ int64_t thread_slot(const ImView &iv, int w) {
+  return (int64_t)w * (iv.win / kRW) + threadIdx.x;
+}
+
 // This thread's rows of window w: first row, whether they belong to the instance, flags
 // (rows that belong to no piece read as P_IDENT) and, after ids(), the id of each row's piece.
 // ids() waits for the window's tables and makes a dependent load, so callers issue the loads
@@ -72,15 +78,18 @@ __device__ __forceinline__ void st_rows(T *p, const T (&o)[kRW]) {
 template <typename T, int kMode>
 struct WinRows {
   int64_t rb;
-  bool ok;
+  bool ok, idle;  // idle: no thread of this warp has rows in a window
   uint32_t q;
   int ord;   // ordinal (in row order) of the piece of the row before this thread's first
   int pid[kRW];
   __device__ __forceinline__ WinRows(const Ctx<T, kMode> &c, const ImView &iv, int w) {
-    rb = c.wrow0 + (int64_t)(w - c.iw0) * kWin + threadIdx.x * kRW;
-    ok = rb < c.wend;
+    const int l = (int)threadIdx.x * kRW;
+    rb = c.wrow0 + (int64_t)(w - c.iw0) * iv.win + l;
+    ok = l < iv.win && rb < c.wend;
+    idle = ((int)threadIdx.x & ~31) * kRW >= iv.win;
     q = ok ? *(const uint32_t *)(iv.pfl + rb) : 0x01010101u * P_IDENT;
-    ord = iv.wbase[w] + (int)iv.wtp[(int64_t)w * kThreads + threadIdx.x] - 1;
+    ord = iv.wbase[w] - 1;
+    if (ok) ord += (int)iv.wtp[thread_slot(iv, w)];
   }
   __device__ __forceinline__ bool is(int u, uint32_t flag) const { return (q >> (8 * u)) & flag; }
   __device__ __forceinline__ void ids(const Ctx<T, kMode> &c, const ImView &iv) {
@@ -100,10 +109,22 @@ struct WinRows {
 // Value entering this thread's part of kN affine recurrences y <- A + M y that share M, in
 // ascending or (kDesc) descending thread order, with 0 entering the first thread.
 // sc: (kN + 1) * kWarps values.  One CTA barrier; a caller alternates between two scratch
-// areas, so that the next scan's writes never meet this one's reads.
+// areas, so that the next scan's writes never meet this one's reads.  idle: the warp has no rows
+// (its part is the identity and nobody reads its y).
 template <typename T, int kN, bool kDesc>
-__device__ __forceinline__ void affine_enter(const T (&A)[kN], T M, T *sc, T (&y)[kN]) {
+__device__ __forceinline__ void affine_enter(const T (&A)[kN], T M, T *sc, T (&y)[kN], bool idle) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (idle) {
+    if (lane == 0) {
+      sc[w] = 1;
+#pragma unroll
+      for (int q = 0; q < kN; q++) sc[(q + 1) * kWarps + w] = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kN; q++) y[q] = 0;
+    return;
+  }
   const int sl = kDesc ? 31 - lane : lane;  // position in scan order inside the warp
   T iA[kN], iM = M;
 #pragma unroll
@@ -260,7 +281,7 @@ __device__ __forceinline__ bool staged(const Ctx<T, kMode> &c, const ImView &iv)
 
 // The links of a group's instance, staged once per launch.
 template <typename T, int kMode>
-__device__ __noinline__ void stage_links(Ctx<T, kMode> c) {
+__device__ __noinline__ void stage_links(const Ctx<T, kMode> &c) {
   const ImView &iv = *c.iv;
   if (!staged(c, iv)) return;
   Shared S = carve(dyn_smem(), iv.m);
@@ -278,7 +299,7 @@ __device__ __noinline__ void stage_links(Ctx<T, kMode> c) {
 template <typename T, int kMode, typename X, typename Get, typename F>
 __device__ __forceinline__ void walk_up(const Ctx<T, kMode> &c, const ImView &iv, Walk<T> k,
                                         Get get, F f) {
-  const int *lo = iv.lev_off + c.l0;
+  const int *lo = c.lev;
   const int nl = c.l1 - c.l0;
   if (staged(c, iv)) {
     int qb = 0, qe = lo[0];
@@ -333,7 +354,7 @@ __device__ __forceinline__ void walk_up(const Ctx<T, kMode> &c, const ImView &iv
 template <typename T, int kMode, typename X, typename Get, typename F>
 __device__ __forceinline__ void walk_down(const Ctx<T, kMode> &c, const ImView &iv, Walk<T> k,
                                           Get get, F f) {
-  const int *lo = iv.lev_off + c.l0;
+  const int *lo = c.lev;
   const int nl = c.l1 - c.l0;
   int qe = nl > 0 ? lo[nl - 1] : 0, qb = nl > 1 ? lo[nl - 2] : 0;
   if (staged(c, iv)) {
@@ -386,13 +407,23 @@ __device__ __forceinline__ void walk_down(const Ctx<T, kMode> &c, const ImView &
 // ---- factorisation
 
 // The 2x2 matrices of the pieces of one window: cc, g the thread's rows (g changed to 0 on
-// rows without a mother column).  sc: 5 * kWarps values; one CTA barrier.
+// rows without a mother column).  ent: the thread's place for the map of the rows of its last
+// row's piece that later threads hold, which tree_pivots starts from.  sc: 5 * kWarps values; one
+// CTA barrier.
 template <typename T, int kMode>
 __device__ __forceinline__ void window_maps(const WinRows<T, kMode> &r, const T (&cc)[kRW],
-                                            T (&g)[kRW], Mob<T> *out, T *sc) {
+                                            T (&g)[kRW], Mob<T> *out, T *ent, T *sc) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  // rows in descending order; a piece's last row starts its matrix afresh
   const Mob<T> one{1, 0, 0, 1};
+  if (r.idle) {
+    if (lane == 0) {
+      sc[wp] = sc[3 * kWarps + wp] = 1;
+      sc[kWarps + wp] = sc[2 * kWarps + wp] = sc[4 * kWarps + wp] = 0;
+    }
+    __syncthreads();
+    return;
+  }
+  // rows in descending order; a piece's last row starts its matrix afresh
   Mob<T> P = one;
   bool R = false;
 #pragma unroll
@@ -438,6 +469,10 @@ __device__ __forceinline__ void window_maps(const WinRows<T, kMode> &r, const T 
       X = mob_mul(Mob<T>{sc[p], sc[kWarps + p], sc[2 * kWarps + p], sc[3 * kWarps + p]}, X);
     E = mob_mul(E, X);
   }
+  if (r.ok) {
+    const T e4[4] = {E.a, E.b, E.c, E.d};
+    st_rows(ent, e4);
+  }
   Mob<T> cur = E;
 #pragma unroll
   for (int u = kRW - 1; u >= 0; u--) {
@@ -449,7 +484,7 @@ __device__ __forceinline__ void window_maps(const WinRows<T, kMode> &r, const T 
 }
 
 template <typename T, int kMode>
-__device__ __noinline__ void tree_maps(Ctx<T, kMode> c) {
+__device__ __noinline__ void tree_maps(const Ctx<T, kMode> &c) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const T *C = (const T *)iv.cdiag;
@@ -465,7 +500,8 @@ __device__ __noinline__ void tree_maps(Ctx<T, kMode> c) {
       ld_rows(G + r.rb, g);
     }
     r.ids(c, iv);
-    window_maps(r, cc, g, (Mob<T> *)iv.pmob + c.ip0, sc);
+    window_maps(r, cc, g, (Mob<T> *)iv.pmob + c.ip0,
+                (T *)iv.tent + 4 * thread_slot(iv, w), sc);
   }
 }
 
@@ -475,7 +511,7 @@ __device__ __noinline__ void tree_maps(Ctx<T, kMode> c) {
 // potential x0 = 2 Vin - Vout of each piece's first and last row is exported too (for the
 // refinement's updates).
 template <typename T, int kMode>
-__device__ __noinline__ void tree_pivots(Ctx<T, kMode> c, const T *v, const double *Vin,
+__device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, const double *Vin,
                                          const double *Vout) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
@@ -484,58 +520,25 @@ __device__ __noinline__ void tree_pivots(Ctx<T, kMode> c, const T *v, const doub
   const T *G = sizeof(T) == 4 ? (const T *)(const void *)iv.gf : (const T *)(const void *)iv.g64;
   T *pstat = (T *)iv.pstat + 4 * (int64_t)c.ip0, *pval = (T *)iv.pval + 4 * (int64_t)c.ip0;
   double *pxb = (double *)iv.pxb + 2 * (int64_t)c.ip0;
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   for (int w = c.w0; w < c.w1; w++) {
-    T *sc0 = (T *)S.warp, *sc1 = sc0 + 4 * kWarps, *sc2 = sc1 + 3 * kWarps;
+    T *sc1 = (T *)S.warp, *sc2 = sc1 + 3 * kWarps;
     WinRows<T, kMode> r(c, iv, w);
-    T cc[kRW] = {}, g[kRW] = {}, al[kRW] = {};
+    T cc[kRW] = {}, g[kRW] = {}, al[kRW] = {}, en[4] = {1, 0, 0, 1};
     if (r.ok) {
+      ld_rows((const T *)iv.tent + 4 * thread_slot(iv, w), en);
       ld_rows(C + r.rb, cc);
       ld_rows(G + r.rb, g);
       ld_rows(v + r.rb, al);
     }
     r.ids(c, iv);
-    Mob<T> P{1, 0, 0, 1};
-#pragma unroll
-    for (int u = kRW - 1; u >= 0; u--) {
-      if (r.is(u, P_IDENT)) continue;
-      if (!(r.is(u, P_UP))) g[u] = 0;
-      if (r.is(u, P_LAST)) {
-        // the map that forgets what came before: (a, b) -> (s + c, 1) b, then the row's own
-        cc[u] += k.yin[r.pid[u]];
-        P = mob_scaled(Mob<T>{0, g[u] * cc[u], 0, cc[u] + g[u]});
-      } else {
-        P = mob_row(cc[u], g[u], P);
-      }
-    }
-    Mob<T> I = P;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const Mob<T> Q = mob_shfl_down(I, off);
-      if (31 - lane >= off) I = mob_mul(I, Q);
-    }
-    Mob<T> E = mob_shfl_down(I, 1);
-    if (lane == 31) E = Mob<T>{1, 0, 0, 1};
-    if (lane == 0) {
-      sc0[wp] = I.a;
-      sc0[kWarps + wp] = I.b;
-      sc0[2 * kWarps + wp] = I.c;
-      sc0[3 * kWarps + wp] = I.d;
-    }
-    __syncthreads();
-    T va = 0, vb = 1;  // the vector entering the warp, then the thread
-    for (int p = kWarps - 1; p > wp; p--) {
-      const T na = sc0[p] * va + sc0[kWarps + p] * vb;
-      const T nb = sc0[2 * kWarps + p] * va + sc0[3 * kWarps + p] * vb;
-      const T s = pow2_near_inv(max_of(na, nb));
-      va = na * s;
-      vb = nb * s;
-    }
-    {
-      const T na = E.a * va + E.b * vb, nb = E.c * va + E.d * vb;
-      const T s = pow2_near_inv(max_of(na, nb));
-      va = na * s;
-      vb = nb * s;
+    // the vector entering the thread's last row: its piece's (s, 1) through the later rows
+    T va = 0, vb = 1;
+    if (!r.idle) {
+      const T s = k.yin[r.pid[kRW - 1]];
+      const T na = en[0] * s + en[1], nb = en[2] * s + en[3];
+      const T f = pow2_near_inv(max_of(na, nb));
+      va = na * f;
+      vb = nb * f;
     }
     T inv[kRW], ee[kRW], beta[kRW];
     // what a row passes on: beta u <- e u with 1 entering each piece's last row, alpha
@@ -546,11 +549,16 @@ __device__ __noinline__ void tree_pivots(Ctx<T, kMode> c, const T *v, const doub
       inv[u] = 0;
       ee[u] = 0;
       if (r.is(u, P_IDENT)) continue;
-      const T p = (r.is(u, P_LAST)) ? cc[u] * vb : va + cc[u] * vb;
-      const T eta = quot(p, vb);
-      inv[u] = quot((T)1, g[u] + eta);
-      ee[u] = g[u] * inv[u];
+      if (!(r.is(u, P_UP))) g[u] = 0;
+      if (r.is(u, P_LAST)) {
+        va = k.yin[r.pid[u]];
+        vb = 1;
+      }
+      // eta = p / vb; the pivot g + eta = (p + g vb) / vb
+      const T p = va + cc[u] * vb;
       const T na = g[u] * p, nb = p + g[u] * vb;
+      inv[u] = quot(vb, nb);
+      ee[u] = g[u] * inv[u];
       const T s = pow2_near_inv(max_of(na, nb));
       va = na * s;
       vb = nb * s;
@@ -565,7 +573,7 @@ __device__ __noinline__ void tree_pivots(Ctx<T, kMode> c, const T *v, const doub
       }
     }
     T y[2];
-    affine_enter<T, 2, true>(A, M, sc1, y);
+    affine_enter<T, 2, true>(A, M, sc1, y, r.idle);
     T sb[2] = {0, 0}, sm = 1, cur = y[0], cua = y[1];
 #pragma unroll
     for (int u = kRW - 1; u >= 0; u--) {
@@ -595,7 +603,7 @@ __device__ __noinline__ void tree_pivots(Ctx<T, kMode> c, const T *v, const doub
       sb[0] += wb * beta[u];
       sb[1] += wb * al[u];
     }
-    affine_enter<T, 2, false>(sb, sm, sc2, y);
+    affine_enter<T, 2, false>(sb, sm, sc2, y, r.idle);
 #pragma unroll
     for (int u = 0; u < kRW; u++) {
       if (r.is(u, P_FIRST)) y[0] = y[1] = 0;
@@ -618,7 +626,7 @@ __device__ __noinline__ void tree_pivots(Ctx<T, kMode> c, const T *v, const doub
 }
 
 template <typename T, int kMode>
-__device__ __noinline__ void walk_factor(Ctx<T, kMode> c) {
+__device__ __noinline__ void walk_factor(const Ctx<T, kMode> &c) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<T> k = walk_of(c, iv, S);
@@ -637,7 +645,7 @@ __device__ __noinline__ void walk_factor(Ctx<T, kMode> c) {
 // The factorisation once every piece's matrix is known (tree_maps, or the windowed assembly)
 // and visible to the walk.
 template <typename T, int kMode>
-__device__ __noinline__ void tree_factor(Ctx<T, kMode> c, const T *v, const double *Vin,
+__device__ __noinline__ void tree_factor(const Ctx<T, kMode> &c, const T *v, const double *Vin,
                                          const double *Vout) {
   const ImView &iv = *c.iv;
   if (walks(c, iv)) walk_factor(c);
@@ -670,7 +678,7 @@ __device__ __forceinline__ void window_eliminate(const WinRows<T, kMode> &r, T (
       M *= ee[u];
     }
   }
-  affine_enter<T, 1, true>(A, M, sc0, y);
+  affine_enter<T, 1, true>(A, M, sc0, y, r.idle);
   T cur = y[0];
 #pragma unroll
   for (int u = kRW - 1; u >= 0; u--) {
@@ -688,7 +696,7 @@ __device__ __forceinline__ void window_eliminate(const WinRows<T, kMode> &r, T (
     if (r.is(u, P_FIRST)) sb[0] = sm = 0;
     sb[0] += inv[u] * be[u] * al[u];
   }
-  affine_enter<T, 1, false>(sb, sm, sc1, y);
+  affine_enter<T, 1, false>(sb, sm, sc1, y, r.idle);
 #pragma unroll
   for (int u = 0; u < kRW; u++) {
     if (r.is(u, P_FIRST)) y[0] = 0;
@@ -700,7 +708,7 @@ __device__ __forceinline__ void window_eliminate(const WinRows<T, kMode> &r, T (
 // alpha of every row and the pieces' values for the right-hand side v.  pb: the buffer of the
 // pieces' values; x (with Vin null) the potential whose first and last rows are exported.
 template <typename T, int kMode>
-__device__ __noinline__ void tree_eliminate(Ctx<T, kMode> c, const T *v, int pb, const double *x) {
+__device__ __noinline__ void tree_eliminate(const Ctx<T, kMode> &c, const T *v, int pb, const double *x) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   T *pval = (T *)iv.pval + 4 * ((int64_t)c.ip0 + (int64_t)pb * iv.npieces);
@@ -731,7 +739,7 @@ __device__ __noinline__ void tree_eliminate(Ctx<T, kMode> c, const T *v, int pb,
 // The solve's walks: a piece's numbers travel as Mob {B, bL, A, aL}.
 
 template <typename T, int kMode>
-__device__ __noinline__ void walk_solve(Ctx<T, kMode> c) {
+__device__ __noinline__ void walk_solve(const Ctx<T, kMode> &c) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<T> k = walk_of(c, iv, S);
@@ -754,7 +762,7 @@ __device__ __noinline__ void walk_solve(Ctx<T, kMode> c) {
 
 // Substitution: z of every row (identity rows 0).
 template <typename T, int kMode>
-__device__ __noinline__ void tree_substitute(Ctx<T, kMode> c, T *z) {
+__device__ __noinline__ void tree_substitute(const Ctx<T, kMode> &c, T *z) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<T> k = walk_of(c, iv, S);
@@ -785,7 +793,7 @@ __device__ __noinline__ void tree_substitute(Ctx<T, kMode> c, T *z) {
         M *= ee[u];
       }
     }
-    affine_enter<T, 1, false>(A, M, sc, y);
+    affine_enter<T, 1, false>(A, M, sc, y, r.idle);
     T cur = y[0];
 #pragma unroll
     for (int u = 0; u < kRW; u++) {
@@ -803,7 +811,7 @@ __device__ __noinline__ void tree_substitute(Ctx<T, kMode> c, T *z) {
 // z = A^-1 v (up to rounding) with the factors of tree_factor.  eliminated: v is the
 // right-hand side that tree_factor has eliminated.
 template <typename T, int kMode>
-__device__ __noinline__ void tree_apply(Ctx<T, kMode> c, const T *v, T *z, bool eliminated) {
+__device__ __noinline__ void tree_apply(const Ctx<T, kMode> &c, const T *v, T *z, bool eliminated) {
   const ImView &iv = *c.iv;
   if (!eliminated) tree_eliminate(c, v, 0, (const double *)nullptr);
   group_sync<kMode>();

@@ -1,9 +1,9 @@
 // Mixed-precision step with the tree preconditioner, by windows (included by implicit.cu).
 //
-// The step's passes over the rows are fused to four, each reading its rows in row order with
-// 16-byte loads, four rows per thread:
-//   - refine_assemble: gates, W, K, diagonal, right-hand side, the first residual, and the
-//     pieces' matrices of the factorisation;
+// The step's passes over the rows are fused to four:
+//   - refine_assemble: gates, W, K, diagonal, right-hand side, the first residual (a row per
+//     thread), and the pieces' matrices of the factorisation (four rows per thread, as in the
+//     passes below);
 //   - tree_pivots (tree.cuh): the factorisation and the elimination of that residual;
 //   - refine_update<true>: substitution, x += z, the FP64 residual of the new x, and its
 //     elimination, for the next refinement cycle;
@@ -34,7 +34,11 @@ __device__ __forceinline__ void window_ends(const double (&x)[kRW], double *ends
   if (lane == 31 && w + 1 < kWarps) xp = ends[kWarps + w + 1];
 }
 
-// kCn: Crank-Nicolson.
+// kCn: Crank-Nicolson.  The rows' part takes one row per thread, a warp 32 neighbours: with the
+// four rows per thread that the matrices' scan wants, its loads used half of each sector and its
+// numbers did not fit the registers (22 accesses of local memory per row and step, most of them
+// L2 round trips).  10k compartments x 2048: 39.2 -> 38.2 ms for 8 steps; one tree of 30k, whose
+// windows are smaller than a CTA's threads times four: 3.35 -> 3.13 ms for 32.
 template <int kMode, bool kCn>
 __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, const double *Vin,
                                                 const double *Vout, int active, int inst) {
@@ -44,126 +48,122 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
   const int64_t N = pv.ntot;
   float *gate = pv.gatef;
   const bool dense = pv.hh_dense != 0;
+  const int lane = threadIdx.x & 31;
   float bacc = 0;
   double racc = 0;
   int par = 0;
   for (int w = c.w0; w < c.w1; w++) {
     float *sc = (float *)S.warp + par * 5 * kWarps;
     par ^= 1;
+    const int64_t r0 = c.wrow0 + (int64_t)(w - c.iw0) * iv.win;
+    const int nr = (int)min((int64_t)iv.win, c.wend - r0);
+#pragma unroll 1
+    for (int l = threadIdx.x; l - lane < nr; l += kThreads) {
+      const int64_t row = min(r0 + l, N - 1);
+      const bool ok = l < nr;
+      const double v = Vin[row], o = Vout[row], cm = iv.cmdt[row], g = iv.g64[row];
+      const uint32_t f = ok ? iv.rowf[row] : R_IDENT;
+      float gm = 0, gh = 0, gn = 0;
+      if (dense || (f & R_HH)) {
+        gm = gate[row];
+        gh = gate[N + row];
+        gn = gate[2 * N + row];
+      }
+      // rows next to the warp's 32
+      double ev = 0, eo = 0, eg = 0;
+      if (lane == 0 || lane == 31) {
+        const int64_t q = lane == 0 ? max(row - 1, (int64_t)0) : min(row + 1, N - 1);
+        ev = Vin[q];
+        eo = Vout[q];
+        eg = iv.g64[q];
+      }
+      const double x = 2.0 * v - o, ex = 2.0 * ev - eo;
+      double xm = __shfl_up_sync(0xffffffffu, x, 1), xp = __shfl_down_sync(0xffffffffu, x, 1);
+      double gdn = __shfl_down_sync(0xffffffffu, g, 1), vm = 0, vp = 0;
+      if (kCn) {
+        vm = __shfl_up_sync(0xffffffffu, v, 1);
+        vp = __shfl_down_sync(0xffffffffu, v, 1);
+      }
+      if (lane == 0) {
+        xm = ex;
+        vm = ev;
+      }
+      if (lane == 31) {
+        xp = ex;
+        vp = ev;
+        gdn = eg;
+      }
+      if (!ok) continue;  // the loop's bound is the warp's
+      double wdx = 0.0, kdx = 0.0;
+      if (f & R_HH) {  // identity rows' gates move too
+        const HHParams32 q = hh_params32(
+            pv.hpq, pv.hp_cls ? (int64_t)pv.hp_cls[row] : (pv.hp_inst ? (int64_t)inst : row));
+        const float dv = d2f(v - f2d(q.v[HP_REST]));
+        const GateStep32 s = hh_step32(dv + q.v[HP_LSNA], dv + q.v[HP_LSK], gm, gh, gn, q.v[HP_DTMS],
+                                       q.v[HP_GNA], q.v[HP_GK], q.v[HP_GL], q.v[HP_ENA], q.v[HP_EK],
+                                       q.v[HP_EL]);
+        gate[row] = s.m;
+        gate[N + row] = s.h;
+        gate[2 * N + row] = s.n;
+        wdx = f2d(s.W * q.v[HP_DX]);
+        kdx = f2d(s.K * q.v[HP_DX]);
+      } else if (!(f & R_IDENT)) {
+        wdx = iv.wdx64[row];
+        kdx = iv.kdx64[row];
+      }
+      // columns that are not there: nothing of another tree's rows gets in
+      double gup = g;
+      if (!(f & R_UP)) gup = xm = vm = 0.0;
+      if (!(f & R_DOWNR)) gdn = xp = vp = 0.0;
+      // rare rows: the mother is not the row before, a DL child, an injected current
+      double gl = 0.0, xl = 0.0, vl = 0.0, in = 0.0;
+      const bool rare = f & (R_DOWNL | R_FAR | R_INP);
+      if (rare) {
+        const Topo t = pv.topo[row];
+        if (f & R_DOWNL) {
+          gl = iv.g64[t.dl];
+          xl = x0_of(Vin, Vout, t.dl);
+          if (kCn) vl = Vin[t.dl];
+        }
+        if (f & R_FAR) {
+          xm = x0_of(Vin, Vout, t.mother);
+          if (kCn) vm = Vin[t.mother];
+        }
+        if (active && (f & R_INP)) in = iv.inp64[row];
+      }
+      const double cj = (kCn ? 2.0 * cm : cm) - wdx;
+      double d = (cj + gdn) + gup, b;
+      if (!kCn) {
+        b = fma(cm, v, kdx);
+      } else {  // (2 c_m dX/dT + W dX) V^n - sum g (V^n - V^n_q) + 2 (K dX + I)
+        b = (2.0 * cm + wdx) * v;
+        b -= gup * (v - vm);
+        b -= gdn * (v - vp);
+        b += 2.0 * kdx;
+      }
+      if (rare) {
+        d += gl;
+        b += kCn ? 2.0 * in - gl * (v - vl) : in;
+      }
+      double res = fma(-d, x, b);
+      res = fma(gup, xm, res);
+      res = fma(gdn, xp, res);
+      if (rare) res = fma(gl, xl, res);
+      if (f & R_IDENT) b = res = 0.0;
+      iv.diag[row] = d;
+      iv.rhs[row] = b;
+      ((float *)iv.cdiag)[row] = d2f(cj);
+      c.w.Wb[row] = d2f(res);
+      const float bf = d2f(b);
+      bacc += bf * bf;
+      racc += res * res;
+    }
+    __syncthreads();  // the window's rows are there
     WinRows<float, kMode> r(c, iv, w);
     float cc[kRW] = {}, gf[kRW] = {};
-    // two rows at a time: four would not fit the registers
-#pragma unroll
-    for (int u0 = 0; u0 < kRW; u0 += 2) {
-      if (!r.ok) continue;
-      asm volatile("" ::: "memory");  // the second pair's loads stay behind the first's work
-      const int64_t rb = r.rb + u0;
-      const double2 v2 = *(const double2 *)(Vin + rb), o2 = *(const double2 *)(Vout + rb);
-      const double2 cm2 = *(const double2 *)(iv.cmdt + rb), g2 = *(const double2 *)(iv.g64 + rb);
-      const float2 gf2 = *(const float2 *)(iv.gf + rb);
-      const int64_t rm = rb > 0 ? rb - 1 : 0, rp = rb + 2 < N ? rb + 2 : N - 1;
-      const double vb = Vin[rm], va = Vin[rp], ob = Vout[rm], oa = Vout[rp], ga = iv.g64[rp];
-      const uint32_t rf = *(const uint16_t *)(iv.rowf + rb);
-      float2 m2 = make_float2(0, 0), h2 = m2, n2 = m2;
-      if (dense) {
-        m2 = *(const float2 *)(gate + rb);
-        h2 = *(const float2 *)(gate + N + rb);
-        n2 = *(const float2 *)(gate + 2 * N + rb);
-      }
-      uint2 cls = make_uint2(0, 0);
-      if (pv.hp_cls) cls = *(const uint2 *)(pv.hp_cls + rb);
-      const double v[2] = {v2.x, v2.y}, cm[2] = {cm2.x, cm2.y}, g[3] = {g2.x, g2.y, ga};
-      // x0 of the rows before, of this pair and after it
-      const double x[4] = {2.0 * vb - ob, 2.0 * v2.x - o2.x, 2.0 * v2.y - o2.y, 2.0 * va - oa};
-      float gm[2] = {m2.x, m2.y}, gh[2] = {h2.x, h2.y}, gn[2] = {n2.x, n2.y}, rr[2];
-      double dg[2], rh[2];
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int u = u0 + e;
-        const int64_t row = rb + e;
-        const uint32_t f = (rf >> (8 * e)) & 0xffu;
-        const bool phys = !(f & R_IDENT);
-        double wdx = 0.0, kdx = 0.0;
-        if (f & R_HH) {  // identity rows' gates move too
-          if (!dense) {
-            gm[e] = gate[row];
-            gh[e] = gate[N + row];
-            gn[e] = gate[2 * N + row];
-          }
-          const HHParams32 q = hh_params32(
-              pv.hpq, pv.hp_cls ? (int64_t)(e ? cls.y : cls.x) : (pv.hp_inst ? (int64_t)inst : row));
-          const float dv = d2f(v[e] - f2d(q.v[HP_REST]));
-          const GateStep32 s = hh_step32(dv + q.v[HP_LSNA], dv + q.v[HP_LSK], gm[e], gh[e], gn[e],
-                                         q.v[HP_DTMS], q.v[HP_GNA], q.v[HP_GK], q.v[HP_GL],
-                                         q.v[HP_ENA], q.v[HP_EK], q.v[HP_EL]);
-          gm[e] = s.m;
-          gh[e] = s.h;
-          gn[e] = s.n;
-          if (!dense) {
-            gate[row] = s.m;
-            gate[N + row] = s.h;
-            gate[2 * N + row] = s.n;
-          }
-          wdx = f2d(s.W * q.v[HP_DX]);
-          kdx = f2d(s.K * q.v[HP_DX]);
-        } else if (phys) {
-          wdx = iv.wdx64[row];
-          kdx = iv.kdx64[row];
-        }
-        // rare rows: the mother is not the row before, or there is a DL child
-        double gl = 0.0, xl = 0.0, vl = 0.0, xmo = x[e], vmo = e ? v[0] : vb;
-        if (f & (R_DOWNL | R_FAR)) {
-          const Topo t = pv.topo[row];
-          if (f & R_DOWNL) {
-            gl = iv.g64[t.dl];
-            xl = x0_of(Vin, Vout, t.dl);
-            if (kCn) vl = Vin[t.dl];
-          }
-          if (f & R_FAR) {
-            xmo = x0_of(Vin, Vout, t.mother);
-            if (kCn) vmo = Vin[t.mother];
-          }
-        }
-        // the rest without branches but the rare ones: conductances of missing columns are 0
-        const double gup = (f & R_UP) ? g[e] : 0.0, gdn = (f & R_DOWNR) ? g[e + 1] : 0.0;
-        const double cj = (kCn ? 2.0 * cm[e] : cm[e]) - wdx;
-        double d = (cj + gdn) + gup;
-        if (f & R_DOWNL) d += gl;
-        double b;
-        if (!kCn) {
-          b = cm[e] * v[e] + kdx;
-          if (active && (f & R_INP)) b += iv.inp64[row];
-        } else {  // (2 c_m dX/dT + W dX) V^n - sum g (V^n - V^n_q) + 2 (K dX + I)
-          b = (2.0 * cm[e] + wdx) * v[e];
-          b -= gup * (v[e] - vmo);
-          b -= gdn * (v[e] - (e ? va : v[1]));
-          if (f & R_DOWNL) b -= gl * (v[e] - vl);
-          b += 2.0 * kdx;
-          if (active && (f & R_INP)) b += 2.0 * iv.inp64[row];
-        }
-        double res = fma(-d, x[e + 1], b);
-        res = fma(gup, xmo, res);
-        res = fma(gdn, x[e + 2], res);
-        if (f & R_DOWNL) res = fma(gl, xl, res);
-        if (!phys) b = res = 0.0;
-        dg[e] = d;
-        rh[e] = b;
-        cc[u] = d2f(cj);
-        gf[u] = (f & R_UP) ? (e ? gf2.y : gf2.x) : 0.0f;
-        rr[e] = d2f(res);
-        const float bf = d2f(b);
-        bacc += bf * bf;
-        racc += res * res;
-      }
-      if (dense) {
-        *(float2 *)(gate + rb) = make_float2(gm[0], gm[1]);
-        *(float2 *)(gate + N + rb) = make_float2(gh[0], gh[1]);
-        *(float2 *)(gate + 2 * N + rb) = make_float2(gn[0], gn[1]);
-      }
-      *(double2 *)(iv.diag + rb) = make_double2(dg[0], dg[1]);
-      *(double2 *)(iv.rhs + rb) = make_double2(rh[0], rh[1]);
-      *(float2 *)((float *)iv.cdiag + rb) = make_float2(cc[u0], cc[u0 + 1]);
-      *(float2 *)(c.w.Wb + rb) = make_float2(rr[0], rr[1]);
+    if (r.ok) {
+      ld_rows((const float *)iv.cdiag + r.rb, cc);
+      ld_rows((const float *)iv.gf + r.rb, gf);
     }
     r.ids(c, iv);
     window_maps(r, cc, gf, (Mob<float> *)iv.pmob + c.ip0,

@@ -82,3 +82,24 @@ def test_batch_of_all(gpu, pkg, orc, model, precision):
         else:
             Vo, _, _, _ = orc.implicit_run(sp, orc.derive(sp), sp.dt_abs, 1, 1 + steps, linsolve=0)
             assert np.abs(out["auto"][q] - Vo).max() < 1e-9
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [40, WIN, 1500])
+def test_trees_next_to_one_that_overflowed(gpu, pkg, model, precision, n):
+    """Rows of different trees lie next to each other: a tree whose potential is not finite leaves
+    its neighbours' results as they are, bit for bit."""
+    sp = cable(model, n)
+    d = pkg.derive(sp)
+    opts = dict(mode=1, precision=precision, tol=1e-10, tol_mode="rel")
+    got = []
+    for bad in (False, True):
+        ends = pkg.ProblemArrays.from_spec(sp, d, V0=np.full(n, np.inf)) if bad else \
+            pkg.ProblemArrays.from_spec(sp, d)
+        b = pkg.Batch([ends, pkg.ProblemArrays.from_spec(sp, d), ends], **opts)
+        b.set_runs([(1, 13, sp.init_time, sp.end_input)] * 3)
+        b.advance(12)
+        got.append(b.snapshot(1))
+        b.close()
+    assert np.isfinite(got[0]).all()
+    np.testing.assert_array_equal(got[0], got[1])

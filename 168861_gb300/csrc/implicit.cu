@@ -1156,7 +1156,7 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
     tree_maps(c);
     group_sync<kMode>();
   }
-  if (tree) tree_factor(c, c.w.Wb, fused ? Vin : (const double *)nullptr, Vout);
+  if (tree) tree_factor(c, c.w.Wb, fused ? (const double *)c.w.Z : (const double *)nullptr);
   const int budget = iv.max_iter > 0 ? iv.max_iter : (iv.max_iter < 0 ? 0 : (int)inst_n);
   const double inner_rel = iv.inner_rel;
   int iters = 0, n_res = 0, n_app = 0, n_xup = 0, n_basis = 0, n_rich = 0;
@@ -1181,11 +1181,11 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
       // res > 0 here (a zero residual has converged); the scale stays a normal FP32 number
       const bool f32 = sizeof(T) == 4 && iv.krylov == NRT_GMRES;
       const int e = f32 ? max(-126, min(126, ilogb(res))) : 0;
-      const float scale = f32 ? exp2f((float)-e) : 0.0f;
+      const float scale = f32 ? pow2_of<float>(-e) : 0.0f;
       rows_reduce(c, 1, S, iv.partials, parity, 0, [&](int64_t r0, int64_t r1) {
         return Sums<double, 1>{{ph_residual(c, r0, r1, Vout, scale)}};
       });
-      res = sqrt(S.red[0]) * exp2((double)e);
+      res = sqrt(S.red[0]) * pow2_of<double>(e);
       n_res++;
     }
     rich_done = false;
@@ -1213,9 +1213,9 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
         group_sync<kMode>();  // every window's elimination visible to the walk
         if (walks(c, iv)) refine_walk(c, pb);
         if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
-        const double *from = x0_pending ? Vin : (const double *)nullptr;
+        const double *from = x0_pending ? (const double *)c.w.Z : Vout;
         const int e = max(-126, min(126, ilogb(res)));
-        const float scale = exp2f((float)-e);
+        const float scale = pow2_of<float>(-e);
         // The first cycle's residual is eliminated at once: it is rarely the last.
         double acc[1];
         if (cycle == 0) {
@@ -1227,7 +1227,7 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
         eliminated = cycle == 0;
         group_reduce<kMode>(acc, 1, S, iv.partials, parity);  // V and W_0 complete
         prev_res = res;
-        res = sqrt(S.red[0]) * exp2((double)e);
+        res = sqrt(S.red[0]) * pow2_of<double>(e);
         w0_valid = cycle != 0;
         rich_done = true;
         x0_pending = false;

@@ -39,6 +39,9 @@ __device__ __forceinline__ void window_ends(const double (&x)[kRW], double *ends
 // numbers did not fit the registers (22 accesses of local memory per row and step, most of them
 // L2 round trips).  10k compartments x 2048: 39.2 -> 38.2 ms for 8 steps; one tree of 30k, whose
 // windows are smaller than a CTA's threads times four: 3.35 -> 3.13 ms for 32.
+// What is left is bound by the FP64 pipe's latency and rate (16 cycles of an SM per warp's
+// operation), so rare rows share one x0 with the warp's ends, and x0 goes to Z for the passes that
+// would form it again (the pieces' ends, the first update): 3.13 -> 3.00 ms, 38.2 -> 37.8 ms.
 template <int kMode, bool kCn>
 __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, const double *Vin,
                                                 const double *Vout, int active, int inst) {
@@ -47,6 +50,7 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
   Shared S = carve(dyn_smem(), iv.m);
   const int64_t N = pv.ntot;
   float *gate = pv.gatef;
+  double *x0 = (double *)c.w.Z;
   const bool dense = pv.hh_dense != 0;
   const int lane = threadIdx.x & 31;
   float bacc = 0;
@@ -69,29 +73,12 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
         gh = gate[N + row];
         gn = gate[2 * N + row];
       }
-      // rows next to the warp's 32
-      double ev = 0, eo = 0, eg = 0;
-      if (lane == 0 || lane == 31) {
-        const int64_t q = lane == 0 ? max(row - 1, (int64_t)0) : min(row + 1, N - 1);
-        ev = Vin[q];
-        eo = Vout[q];
-        eg = iv.g64[q];
-      }
-      const double x = 2.0 * v - o, ex = 2.0 * ev - eo;
+      const double x = 2.0 * v - o;
       double xm = __shfl_up_sync(0xffffffffu, x, 1), xp = __shfl_down_sync(0xffffffffu, x, 1);
       double gdn = __shfl_down_sync(0xffffffffu, g, 1), vm = 0, vp = 0;
       if (kCn) {
         vm = __shfl_up_sync(0xffffffffu, v, 1);
         vp = __shfl_down_sync(0xffffffffu, v, 1);
-      }
-      if (lane == 0) {
-        xm = ex;
-        vm = ev;
-      }
-      if (lane == 31) {
-        xp = ex;
-        vp = ev;
-        gdn = eg;
       }
       if (!ok) continue;  // the loop's bound is the warp's
       double wdx = 0.0, kdx = 0.0;
@@ -111,26 +98,46 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
         wdx = iv.wdx64[row];
         kdx = iv.kdx64[row];
       }
+      // the neighbour that is not in the warp (the rows before and after it, a DL child, a far
+      // mother): one for nearly every row that has any, so one x0 for all of the warp
+      const bool dl = f & R_DOWNL, far = f & R_FAR, rare = dl || far;
+      double gl = 0.0, xl = 0.0, vl = 0.0;
+      if (rare || lane == 0 || lane == 31) {
+        int tm = 0, tl = 0;
+        if (rare) {
+          const Topo t = pv.topo[row];
+          tm = t.mother;
+          tl = t.dl;
+        }
+        const int64_t qm = far ? (int64_t)tm : max(row - 1, (int64_t)0), qp = min(row + 1, N - 1);
+        const int64_t q = dl ? (int64_t)tl : (far || lane == 0) ? qm : qp;
+        const double ev = Vin[q], ex = 2.0 * ev - Vout[q], eg = iv.g64[q];
+        if (dl) {
+          gl = eg;
+          xl = ex;
+          vl = ev;
+        } else if (far || lane == 0) {
+          xm = ex;
+          vm = ev;
+        } else {
+          xp = ex;
+          vp = ev;
+          gdn = eg;
+        }
+        if (dl && (far || lane == 0)) {
+          xm = x0_of(Vin, Vout, qm);
+          if (kCn) vm = Vin[qm];
+        }
+        if (rare && lane == 31) {
+          xp = x0_of(Vin, Vout, qp);
+          if (kCn) vp = Vin[qp];
+          gdn = iv.g64[qp];
+        }
+      }
       // columns that are not there: nothing of another tree's rows gets in
       double gup = g;
       if (!(f & R_UP)) gup = xm = vm = 0.0;
       if (!(f & R_DOWNR)) gdn = xp = vp = 0.0;
-      // rare rows: the mother is not the row before, a DL child, an injected current
-      double gl = 0.0, xl = 0.0, vl = 0.0, in = 0.0;
-      const bool rare = f & (R_DOWNL | R_FAR | R_INP);
-      if (rare) {
-        const Topo t = pv.topo[row];
-        if (f & R_DOWNL) {
-          gl = iv.g64[t.dl];
-          xl = x0_of(Vin, Vout, t.dl);
-          if (kCn) vl = Vin[t.dl];
-        }
-        if (f & R_FAR) {
-          xm = x0_of(Vin, Vout, t.mother);
-          if (kCn) vm = Vin[t.mother];
-        }
-        if (active && (f & R_INP)) in = iv.inp64[row];
-      }
       const double cj = (kCn ? 2.0 * cm : cm) - wdx;
       double d = (cj + gdn) + gup, b;
       if (!kCn) {
@@ -141,15 +148,17 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
         b -= gdn * (v - vp);
         b += 2.0 * kdx;
       }
-      if (rare) {
+      if (dl) {
         d += gl;
-        b += kCn ? 2.0 * in - gl * (v - vl) : in;
+        if (kCn) b -= gl * (v - vl);
       }
+      if (active && (f & R_INP)) b += kCn ? 2.0 * iv.inp64[row] : iv.inp64[row];
       double res = fma(-d, x, b);
       res = fma(gup, xm, res);
       res = fma(gdn, xp, res);
-      if (rare) res = fma(gl, xl, res);
+      if (dl) res = fma(gl, xl, res);
       if (f & R_IDENT) b = res = 0.0;
+      x0[row] = (f & R_IDENT) ? o : x;
       iv.diag[row] = d;
       iv.rhs[row] = b;
       ((float *)iv.cdiag)[row] = d2f(cj);
@@ -237,11 +246,11 @@ __device__ __noinline__ void refine_walk(const Ctx<float, kMode> &c, int pb) {
   });
 }
 
-// x += z by substitution (x0 = 2 Vin - Vout when Vin is not null, else Vout), then the FP64
+// x += z by substitution (x from Xin, to Vout), then the FP64
 // residual b - A x; returns the thread's part of ||scale r||^2 in FP32 (see ph_residual).
 // kElim: eliminates r into buffer pb of the pieces' values; else stores it (W_0).
 template <int kMode, bool kElim>
-__device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const double *Vin, double *Vout,
+__device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const double *Xin, double *Vout,
                                             float scale, int pb) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
@@ -261,14 +270,7 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const do
       ld_rows((const float *)iv.te + rb, ee);
       ld_rows((const float *)iv.tinv + rb, inv);
       ld_rows((const float *)iv.tbeta + rb, be);
-      ld_rows((const double *)Vout + rb, x);
-      if (Vin) {
-        double v[kRW];
-        ld_rows(Vin + rb, v);
-#pragma unroll
-        for (int u = 0; u < kRW; u++)
-          if (!r.is(u, P_IDENT)) x[u] = 2.0 * v[u] - x[u];
-      }
+      ld_rows(Xin + rb, x);
     }
     r.ids(c, iv);
     // substitution

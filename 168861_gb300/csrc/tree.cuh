@@ -177,6 +177,13 @@ struct Mob {
 __device__ __forceinline__ float quot(float a, float b) { return a / b; }
 __device__ __forceinline__ double quot(double a, double b) { return div64(a, b); }
 
+// 2^e, e in the exponent's normal range.
+template <typename T>
+__device__ __forceinline__ T pow2_of(int e) {
+  if constexpr (sizeof(T) == 4) return __int_as_float((e + 127) << 23);
+  else return __hiloint2double((e + 1023) << 20, 0);
+}
+
 // A power of two near 1 / m for a positive normal m.
 __device__ __forceinline__ float pow2_near_inv(float m) {
   const int e = (__float_as_int(m) >> 23) & 255;
@@ -507,12 +514,10 @@ __device__ __noinline__ void tree_maps(const Ctx<T, kMode> &c) {
 
 // Pivots from the children's conductances: inv, e, beta of every row, and per piece the
 // product B of its e and bL.  The rows of v, the first right-hand side, are eliminated in the
-// same pass (tree_eliminate, into buffer 0 of the pieces' values).  Vin / Vout: with Vin, the
-// potential x0 = 2 Vin - Vout of each piece's first and last row is exported too (for the
-// refinement's updates).
+// same pass (tree_eliminate, into buffer 0 of the pieces' values).  x0 (may be null): the potential
+// of which each piece's first and last row is exported too, for the refinement's updates.
 template <typename T, int kMode>
-__device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, const double *Vin,
-                                         const double *Vout) {
+__device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, const double *x0) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<T> k = walk_of(c, iv, S);
@@ -593,7 +598,7 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
         ps[3] = ee[u];
         pa[0] = cua;  // A
         pa[2] = inv[u] * al[u];
-        if (Vin) pxb[2 * (int64_t)r.pid[u]] = x0_of(Vin, Vout, r.rb + u);
+        if (x0) pxb[2 * (int64_t)r.pid[u]] = x0[r.rb + u];
       }
     }
 #pragma unroll
@@ -613,7 +618,7 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
       if (r.is(u, P_LAST)) {
         pstat[4 * (int64_t)r.pid[u] + 1] = y[0];  // bL
         pval[4 * (int64_t)r.pid[u] + 1] = y[1];   // aL
-        if (Vin) pxb[2 * (int64_t)r.pid[u] + 1] = x0_of(Vin, Vout, r.rb + u);
+        if (x0) pxb[2 * (int64_t)r.pid[u] + 1] = x0[r.rb + u];
       }
     }
     if (r.ok) {
@@ -645,12 +650,11 @@ __device__ __noinline__ void walk_factor(const Ctx<T, kMode> &c) {
 // The factorisation once every piece's matrix is known (tree_maps, or the windowed assembly)
 // and visible to the walk.
 template <typename T, int kMode>
-__device__ __noinline__ void tree_factor(const Ctx<T, kMode> &c, const T *v, const double *Vin,
-                                         const double *Vout) {
+__device__ __noinline__ void tree_factor(const Ctx<T, kMode> &c, const T *v, const double *x0) {
   const ImView &iv = *c.iv;
   if (walks(c, iv)) walk_factor(c);
   if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
-  tree_pivots(c, v, Vin, Vout);
+  tree_pivots(c, v, x0);
   __syncthreads();  // its scans' scratch is free for the next reduction
 }
 

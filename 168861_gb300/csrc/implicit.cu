@@ -68,7 +68,7 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxPiece = 256;                 // longest segment piece one sweep handles
 constexpr int kMaxDots = kMaxRestart + 1;
-constexpr int kSumChunks = 8;                  // row chunks of an instance's sums (rows_reduce)
+constexpr int kSumChunks = 8;                  // row chunks of an instance's sums at most (rows_reduce)
 constexpr int kTileBytes = 44 * 1024;          // shared memory of the preconditioners
 constexpr int kLevels = 128;                   // level offsets kept in shared memory
 constexpr int kBlockWalkBytes = 24 * 1024;     // shared memory of a block's walk
@@ -164,7 +164,9 @@ struct ImView {
   void *tinv, *te, *tbeta, *talpha;  // T[ld]: 1 / pivot, g / pivot, beta, alpha
   void *tent;                     // T[4] per thread of a window: the map of its piece's later rows
   void *gwalk;                    // walk_bytes per piece: the walk's numbers beyond walk_cap
+  int solo;                       // windows are a warp's (tree.cuh)
   int walk_cap;                   // pieces whose walk fits a CTA's shared memory
+  int stage_cap;                  // and those whose maps and links fit as well
 };
 
 template <typename T>
@@ -173,7 +175,7 @@ struct Work {
 };
 
 struct Shared {
-  double *H, *cs, *sn, *g, *s, *y, *red, *warp, *part;
+  double *H, *cs, *sn, *g, *s, *y, *red, *warp, *part, *wpart;
   void *coef;      // T[kMaxDots]: update / solution coefficients
   int *flag;       // [0] convergence, [1] queue slot
   void *tile;      // staging area (segment preconditioner) or the tree walk's numbers
@@ -181,7 +183,8 @@ struct Shared {
 
 __host__ __device__ inline size_t shared_fixed_bytes(int m) {
   return sizeof(double) * ((size_t)(m + 1) * m + 2 * m + 2 * (m + 1) + m + kMaxDots +
-                           (kWarps + kSumChunks) * kMaxDots + kMaxDots) + 32;
+                           (kWarps + kSumChunks) * kMaxDots + kSumChunks * kWarps * kG + kMaxDots) +
+         32;
 }
 
 // The dynamic shared memory of the launch.
@@ -201,7 +204,8 @@ __device__ Shared carve(double *base, int m) {
   S.red = S.y + m;
   S.warp = S.red + kMaxDots;
   S.part = S.warp + kWarps * kMaxDots;
-  S.coef = (void *)(S.part + kSumChunks * kMaxDots);
+  S.wpart = S.part + kSumChunks * kMaxDots;
+  S.coef = (void *)(S.wpart + kSumChunks * kWarps * kG);
   S.flag = (int *)((double *)S.coef + kMaxDots);
   S.tile = (void *)((char *)base + ((shared_fixed_bytes(m) + 127) & ~(size_t)127));
   return S;
@@ -433,7 +437,7 @@ struct Ctx {
   int64_t wrow0, wend;
   int ip0, np, l0, l1;
   int rank;         // this CTA in its group
-  int n, v0, v1;    // rows of the instance; this CTA's chunks of them (rows_reduce)
+  int n, chunks, v0, v1;  // rows of the instance; their chunks, this CTA's of them (rows_reduce)
   const int *lev;   // the instance's level offsets (in shared memory, when they fit)
 };
 
@@ -449,9 +453,13 @@ __device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, i
   return 2.0 * Vin[j] - Vout[j];
 }
 
-// Sums k accumulators of a row pass f(first row, end) over the instance into S.red[off .. off + k).  In
-// a block or a cluster the rows are taken in kSumChunks chunks whose sums are added in order,
-// so that the result does not depend on how many CTAs share the instance.
+// Sums k (<= kG) accumulators of a row pass f(first row, end) over the instance into S.red[off .. off + k).  In
+// a block or a cluster the rows are taken in up to kSumChunks chunks whose sums are added in
+// order, so that the result does not depend on how many CTAs share the instance.  A chunk has 128
+// rows or more: four warps keep an SM's FP64 pipe busy, and shorter ones, one after the other,
+// only add their latency (1000 cables of 60 compartments in FP64, 32 steps: 20.0 ms with 8 chunks
+// each, 6.4 with one).  The warps leave their sums of every chunk and meet once after the last
+// (400 trees of 3000: 27.0 -> 25.9 ms).
 template <typename T, int kMode, typename F>
 __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Shared &S,
                                             double *partials, int &parity, int off, F f) {
@@ -465,15 +473,32 @@ __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Share
     sum = group_partials<kMode>(partials, parity);
     parity ^= 1;
   }
-  for (int v = c.v0; v < c.v1; v++) {
-    auto acc = f(c.wrow0 + (int64_t)c.n * v / kSumChunks, c.wrow0 + (int64_t)c.n * (v + 1) / kSumChunks);
-    block_reduce(acc.v, k, S.warp, S.red + off);
-    if (threadIdx.x < k) sum[v * kMaxDots + threadIdx.x] = S.red[off + threadIdx.x];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int v = c.v0; v < c.v1; v++) {  // no barrier between the chunks
+    auto acc = f(c.wrow0 + (int64_t)c.n * v / c.chunks, c.wrow0 + (int64_t)c.n * (v + 1) / c.chunks);
+    double *to = S.wpart + ((v - c.v0) * kWarps + w) * kG;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(acc.v) / sizeof(acc.v[0])); i++) {
+      if (i < k) {
+        double x = (double)acc.v[i];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) to[i] = x;
+      }
+    }
+  }
+  __syncthreads();
+  // the warps' sums of a chunk: eight lanes each
+  const int count = (c.v1 - c.v0) * k;
+  for (int q0 = 4 * w; q0 < count; q0 += 4 * kWarps) {
+    const int q = q0 + (lane >> 3), v = q / k, i = q % k;
+    double x = q < count ? S.wpart[(v * kWarps + (lane & 7)) * kG + i] : 0.0;
+    for (int o = 4; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o, 8);
+    if (q < count && (lane & 7) == 0) sum[(c.v0 + v) * kMaxDots + i] = x;
   }
   group_sync<kMode>();
   if (threadIdx.x < k) {
     double s = 0;
-    for (int v = 0; v < kSumChunks; v++) s += sum[v * kMaxDots + threadIdx.x];
+    for (int v = 0; v < c.chunks; v++) s += sum[v * kMaxDots + threadIdx.x];
     S.red[off + threadIdx.x] = s;
   }
   __syncthreads();
@@ -1402,12 +1427,13 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
     const bool tree = iv.precond == NRT_PRECOND_TREE;
     if (threadIdx.x == 0) {
       c.n = n;
-      c.v0 = kSumChunks * c.rank / gsize;
-      c.v1 = kSumChunks * (c.rank + 1) / gsize;
+      c.chunks = min(kSumChunks, (n + 127) / 128);
+      c.v0 = c.chunks * c.rank / gsize;
+      c.v1 = c.chunks * (c.rank + 1) / gsize;
       c.wrow0 = iv.inst_row[inst];
       c.wend = c.wrow0 + ((n + kRW - 1) & ~(kRW - 1));
-      c.r0 = c.wrow0 + (int64_t)n * c.v0 / kSumChunks;
-      c.r1 = c.wrow0 + (int64_t)n * c.v1 / kSumChunks;
+      c.r0 = c.wrow0 + (int64_t)n * c.v0 / c.chunks;
+      c.r1 = c.wrow0 + (int64_t)n * c.v1 / c.chunks;
       c.iw0 = tree ? iv.inst_win[inst] : 0;
       c.iw1 = tree ? iv.inst_win[inst + 1] : 0;
       c.w0 = c.iw0 + (c.iw1 - c.iw0) * c.rank / gsize;
@@ -1748,11 +1774,16 @@ int Engine::implicit_plan(size_t &bytes) {
   }
   if (S.cluster) S.grid_mode = false;
   if (tree) {
-    // Rows per window: 1024; in a single tree fewer (down to 128, one warp's) where its CTAs
-    // would otherwise not all have a window.  A window's FP64 arithmetic is bound by its SM's
+    // Rows per window: 1024, a CTA's.  In an FP64 batch 128, a warp's: its passes lose their
+    // barriers, a cluster's CTAs share a tree evenly, and the longer chains of pieces cost less
+    // (48 trees of 10k, 8 steps: 2.50 -> 2.31 ms; 1000 of 300: 5.83 -> 5.18).  The mixed step
+    // does not gain: with its warps apart in its longer code 2048 trees of 10k took 43.0 ms
+    // instead of 37.8.  In a single tree fewer than 1024 (down to 128) where its CTAs
+    // would otherwise not all have a window: a window's FP64 arithmetic is bound by its SM's
     // FP64 pipe, so a small tree's windows go to as many SMs as it has CTAs.  (The windows set
     // the order of the scans' sums, so those of a batch do not depend on its size.)
-    S.win = kMaxWin;
+    S.iv.solo = ni > 1 && !mixed;
+    S.win = S.iv.solo ? 128 : kMaxWin;
     if (ni == 1) {
       const int64_t ctas = S.cluster ? S.cluster : S.grid_mode ? dev_sms : 1;
       while (S.win > 128 && S.win * ctas >= 2 * max_n) S.win /= 2;
@@ -1763,8 +1794,10 @@ int Engine::implicit_plan(size_t &bytes) {
   const void *kern = implicit_kernel(mixed, group);
   S.kern = kern;
   // shared memory: the segment preconditioner's staging, or the tree walk's numbers of
-  // every piece -- up to kTileBytes, which keeps three CTAs on an SM, or in the one-tree launch,
-  // whose CTAs then have an SM each, up to kWalkBytes; larger walks run in device memory
+  // every piece: up to kBlockWalkBytes, which keeps three CTAs on an SM, in a cluster
+  // kClusterWalkBytes, or in the one-tree launch, whose CTAs then have an SM each, up to
+  // kWalkBytes; larger walks run in device memory.  A block stages the maps and links too where
+  // they fit as well (1000 trees of 300 compartments, mixed, 32 steps: 6.03 -> 5.34 ms).
   size_t tile = 0;
   if (segs) tile = kTileBytes;
   if (tree) {
@@ -1772,7 +1805,8 @@ int Engine::implicit_plan(size_t &bytes) {
     const size_t cap = S.grid_mode ? kWalkBytes : S.cluster ? kClusterWalkBytes : kBlockWalkBytes;
     S.iv.walk_cap = (int)std::min<size_t>(std::min<size_t>(cap / walk_bytes(tb, grp), kNoPiece - 1),
                                           (size_t)S.tree.max_pieces);
-    tile = (size_t)S.iv.walk_cap * walk_bytes(tb, grp);
+    S.iv.stage_cap = grp ? S.iv.walk_cap : (int)std::min<size_t>(cap / walk_bytes(tb, true), S.tree.max_pieces);
+    tile = std::max(S.iv.walk_cap * walk_bytes(tb, grp), S.iv.stage_cap * walk_bytes(tb, true));
   }
   S.smem = smem_bytes(opt.restart, tile);
   // The limit is the function's, not the handle's: all that a CTA can have, so that handles

@@ -21,15 +21,16 @@
 namespace nrt {
 
 // x of the row before this thread's first and after its last, in the window.  ends: 2 * kWarps
-// doubles; one CTA barrier.
+// doubles; one CTA barrier unless solo.
 __device__ __forceinline__ void window_ends(const double (&x)[kRW], double *ends, double &xm,
-                                            double &xp) {
+                                            double &xp, bool solo) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  xm = __shfl_up_sync(0xffffffffu, x[kRW - 1], 1);
+  xp = __shfl_down_sync(0xffffffffu, x[0], 1);
+  if (solo) return;  // a piece never reaches over a window's ends
   if (lane == 31) ends[w] = x[kRW - 1];
   if (lane == 0) ends[kWarps + w] = x[0];
   __syncthreads();
-  xm = __shfl_up_sync(0xffffffffu, x[kRW - 1], 1);
-  xp = __shfl_down_sync(0xffffffffu, x[0], 1);
   if (lane == 0 && w > 0) xm = ends[w - 1];
   if (lane == 31 && w + 1 < kWarps) xp = ends[kWarps + w + 1];
 }
@@ -56,13 +57,13 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
   float bacc = 0;
   double racc = 0;
   int par = 0;
-  for (int w = c.w0; w < c.w1; w++) {
+  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
     float *sc = (float *)S.warp + par * 5 * kWarps;
     par ^= 1;
     const int64_t r0 = c.wrow0 + (int64_t)(w - c.iw0) * iv.win;
     const int nr = (int)min((int64_t)iv.win, c.wend - r0);
 #pragma unroll 1
-    for (int l = threadIdx.x; l - lane < nr; l += kThreads) {
+    for (int l = window_thread(iv); l - lane < nr; l += iv.solo ? 32 : kThreads) {
       const int64_t row = min(r0 + l, N - 1);
       const bool ok = l < nr;
       const double v = Vin[row], o = Vout[row], cm = iv.cmdt[row], g = iv.g64[row];
@@ -167,7 +168,8 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
       bacc += bf * bf;
       racc += res * res;
     }
-    __syncthreads();  // the window's rows are there
+    if (iv.solo) __syncwarp();  // the window's rows are there
+    else __syncthreads();
     WinRows<float, kMode> r(c, iv, w);
     float cc[kRW] = {}, gf[kRW] = {};
     if (r.ok) {
@@ -224,6 +226,11 @@ __device__ __noinline__ void refine_walk(const Ctx<float, kMode> &c, int pb) {
       if (q == kNoPiece) return;
       put(q, RefineX{ps[q], pa[q], px[q]}, k.yin[q], k.zpar[q], k.val[q], k.link[q].w != 0);
     };
+    if (kMode == kBlock) {
+      for (int q = threadIdx.x; q < c.np; q += kThreads) one(q);
+      __syncthreads();
+      return;
+    }
     const int a = c.w0 < c.w1 ? iv.wbase[c.w0] : 0;
     const int b = c.w0 < c.w1 ? (c.w1 < c.iw1 ? iv.wbase[c.w1] : c.np) : 0;
     for (int o = a + threadIdx.x; o < b; o += kThreads) {
@@ -260,7 +267,7 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const do
   float *pval = (float *)iv.pval + 4 * ((int64_t)c.ip0 + (int64_t)pb * iv.npieces);
   double *pxb = (double *)iv.pxb + 2 * ((int64_t)c.ip0 + (int64_t)pb * iv.npieces);
   float acc = 0;
-  for (int w = c.w0; w < c.w1; w++) {
+  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
     WinRows<float, kMode> r(c, iv, w);
     const int64_t rb = r.rb;
     float al[kRW] = {}, ee[kRW] = {}, inv[kRW] = {}, be[kRW] = {};
@@ -288,7 +295,7 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const do
         M *= ee[u];
       }
     }
-    affine_enter<float, 1, false>(A, M, scz, y, r.idle);
+    affine_enter<float, 1, false>(A, M, scz, y, r.idle, r.solo);
     float cur = y[0];
 #pragma unroll
     for (int u = 0; u < kRW; u++) {
@@ -301,7 +308,7 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const do
     }
     if (r.ok) st_rows(Vout + rb, x);
     double xm, xp;
-    window_ends(x, ends, xm, xp);
+    window_ends(x, ends, xm, xp, r.solo);
     // residual
     double rh[kRW] = {}, dg[kRW] = {}, g[kRW] = {}, gnext = 0;
     if (r.ok) {

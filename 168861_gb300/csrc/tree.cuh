@@ -66,9 +66,20 @@ __device__ __forceinline__ void st_rows(T *p, const T (&o)[kRW]) {
   }
 }
 
+// A window is the CTA's, or (iv.solo: windows of one warp's 128 rows) a warp's, which then takes
+// every kWarps-th of its CTA's and has no barrier with the others in a pass.
+__device__ __forceinline__ int window_thread(const ImView &iv) {
+  return iv.solo ? (int)threadIdx.x & 31 : (int)threadIdx.x;
+}
+template <typename T, int kMode>
+__device__ __forceinline__ int first_window(const Ctx<T, kMode> &c, const ImView &iv) {
+  return c.w0 + (iv.solo ? (int)threadIdx.x >> 5 : 0);
+}
+__device__ __forceinline__ int window_stride(const ImView &iv) { return iv.solo ? kWarps : 1; }
+
 // This thread's place in the arrays of one entry per thread of a window.
 __device__ __forceinline__ int64_t thread_slot(const ImView &iv, int w) {
-  return (int64_t)w * (iv.win / kRW) + threadIdx.x;
+  return (int64_t)w * (iv.win / kRW) + window_thread(iv);
 }
 
 // This thread's rows of window w: first row, whether they belong to the instance, flags
@@ -78,15 +89,16 @@ __device__ __forceinline__ int64_t thread_slot(const ImView &iv, int w) {
 template <typename T, int kMode>
 struct WinRows {
   int64_t rb;
-  bool ok, idle;  // idle: no thread of this warp has rows in a window
+  bool ok, solo, idle;  // idle: no thread of this warp has rows in a window
   uint32_t q;
   int ord;   // ordinal (in row order) of the piece of the row before this thread's first
   int pid[kRW];
   __device__ __forceinline__ WinRows(const Ctx<T, kMode> &c, const ImView &iv, int w) {
-    const int l = (int)threadIdx.x * kRW;
+    const int l = window_thread(iv) * kRW;
     rb = c.wrow0 + (int64_t)(w - c.iw0) * iv.win + l;
     ok = l < iv.win && rb < c.wend;
-    idle = ((int)threadIdx.x & ~31) * kRW >= iv.win;
+    solo = iv.solo;
+    idle = !solo && ((int)threadIdx.x & ~31) * kRW >= iv.win;
     q = ok ? *(const uint32_t *)(iv.pfl + rb) : 0x01010101u * P_IDENT;
     ord = iv.wbase[w] - 1;
     if (ok) ord += (int)iv.wtp[thread_slot(iv, w)];
@@ -110,9 +122,11 @@ struct WinRows {
 // ascending or (kDesc) descending thread order, with 0 entering the first thread.
 // sc: (kN + 1) * kWarps values.  One CTA barrier; a caller alternates between two scratch
 // areas, so that the next scan's writes never meet this one's reads.  idle: the warp has no rows
-// (its part is the identity and nobody reads its y).
+// (its part is the identity and nobody reads its y).  solo: the scan is the warp's, without the
+// barrier.
 template <typename T, int kN, bool kDesc>
-__device__ __forceinline__ void affine_enter(const T (&A)[kN], T M, T *sc, T (&y)[kN], bool idle) {
+__device__ __forceinline__ void affine_enter(const T (&A)[kN], T M, T *sc, T (&y)[kN], bool idle,
+                                             bool solo) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (idle) {
     if (lane == 0) {
@@ -145,6 +159,11 @@ __device__ __forceinline__ void affine_enter(const T (&A)[kN], T M, T *sc, T (&y
 #pragma unroll
   for (int q = 0; q < kN; q++)
     eA[q] = kDesc ? __shfl_down_sync(0xffffffffu, iA[q], 1) : __shfl_up_sync(0xffffffffu, iA[q], 1);
+  if (solo) {
+#pragma unroll
+    for (int q = 0; q < kN; q++) y[q] = sl == 0 ? (T)0 : eA[q];
+    return;
+  }
   if (sl == 31) {
     sc[w] = iM;
 #pragma unroll
@@ -199,14 +218,49 @@ __device__ __forceinline__ T max_of(T a, T b) {
   return a > b ? a : b;
 }
 
+// Scales the numbers by one power of two so that the largest lies in [1, 2) (FP32: [1, 4)).  In
+// FP64 on the exponents, in integers: a comparison or a product of doubles takes an SM's FP64 pipe
+// 16 cycles, and of a matrix product's 15 such operations 7 were its scaling (48 trees of 10k in
+// FP64, 8 steps: 2.31 -> 2.17 ms).  What would leave
+// the range is 0, as far below the largest as 2^-1022; a largest number that is no positive normal
+// one (0, infinite, NaN, or a negative entry among them) takes the general way.
+template <int kN>
+__device__ __forceinline__ void scale_to_one(float (&x)[kN]) {
+  float m = x[0];
+#pragma unroll
+  for (int i = 1; i < kN; i++) m = max_of(m, x[i]);
+  const float s = pow2_near_inv(m);
+#pragma unroll
+  for (int i = 0; i < kN; i++) x[i] *= s;
+}
+template <int kN>
+__device__ __forceinline__ void scale_to_one(double (&x)[kN]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < kN; i++) m = max(m, (uint32_t)__double2hiint(x[i]));
+  const uint32_t e = m >> 20;
+  if (e - 1u >= 2046u) {
+    double big = x[0];
+#pragma unroll
+    for (int i = 1; i < kN; i++) big = max_of(big, x[i]);
+    const double s = pow2_near_inv(big);
+#pragma unroll
+    for (int i = 0; i < kN; i++) x[i] *= s;
+    return;
+  }
+  const uint32_t low = (e > 1023u ? e - 1022u : 1u) << 20, d = (1023u - e) << 20;
+#pragma unroll
+  for (int i = 0; i < kN; i++) {
+    const uint32_t h = (uint32_t)__double2hiint(x[i]);
+    x[i] = h >= low ? __hiloint2double((int)(h + d), __double2loint(x[i])) : 0.0;
+  }
+}
+
 template <typename T>
-__device__ __forceinline__ Mob<T> mob_scaled(Mob<T> r) {
-  const T s = pow2_near_inv(max_of(max_of(r.a, r.b), max_of(r.c, r.d)));
-  r.a *= s;
-  r.b *= s;
-  r.c *= s;
-  r.d *= s;
-  return r;
+__device__ __forceinline__ Mob<T> mob_scaled(const Mob<T> &r) {
+  T x[4] = {r.a, r.b, r.c, r.d};
+  scale_to_one(x);
+  return Mob<T>{x[0], x[1], x[2], x[3]};
 }
 
 template <typename T>
@@ -232,9 +286,9 @@ __device__ __forceinline__ Mob<T> mob_shfl_down(const Mob<T> &m, int off) {
 // ---- the walk over the pieces (one CTA)
 
 // The numbers of the walk, one per piece of the instance (ids in level order, deepest first).
-// A CTA alone (kBlock) keeps the first four in shared memory (or in device memory when there are
-// too many pieces) and loads each level's maps and links one level ahead.  In a group every CTA
-// walks all pieces redundantly, with the maps and links staged in shared memory as well: the
+// A CTA alone (kBlock) with many pieces keeps the first four in shared memory (or in device memory
+// when there are too many) and loads each level's maps and links one level ahead.  In a group
+// every CTA walks all pieces redundantly, with the maps and links staged in shared memory as well: the
 // levels of a bushy tree hold a thousand pieces, and a walk that loads them level by level took
 // 10 to 17 us (2,937 pieces on 14 levels) where the staged one takes 3 to 4.
 template <typename T>
@@ -243,22 +297,22 @@ struct Walk {
   T *val;         // what the piece passes on: up (to its mother's piece), then z of its last row
   T *yin;         // what enters its last row (factorisation: the children's conductance)
   T *zpar;        // z of its first row's mother
-  Mob<T> *st;     // group, staged: its matrix, or B, bL, A, aL
-  ushort4 *link;  // group, staged: plink (65535: none)
+  Mob<T> *st;     // staged: its matrix, or B, bL, A, aL
+  ushort4 *link;  // staged: plink (65535: none)
 };
 
 constexpr int kNoPiece = 65535;
 
 // Bytes of the walk's numbers per piece.
-__host__ __device__ constexpr size_t walk_bytes(size_t tb, bool group) {
-  return 16 + 3 * tb + (group ? 4 * tb + 8 : 0);
+__host__ __device__ constexpr size_t walk_bytes(size_t tb, bool staged) {
+  return 16 + 3 * tb + (staged ? 4 * tb + 8 : 0);
 }
 
 template <typename T, int kMode>
 __device__ __forceinline__ Walk<T> walk_of(const Ctx<T, kMode> &c, const ImView &iv, const Shared &S) {
   Walk<T> k;
   if (c.np <= iv.walk_cap) {
-    const int ns = kMode != kBlock ? c.np : 0;
+    const int ns = c.np <= iv.stage_cap ? c.np : 0;
     k.px = (double2 *)S.tile;
     k.st = (Mob<T> *)(k.px + c.np);
     k.link = (ushort4 *)(k.st + ns);
@@ -280,13 +334,15 @@ template <typename T, int kMode>
 __device__ __forceinline__ bool walks(const Ctx<T, kMode> &c, const ImView &iv) {
   return kMode == kBlock || c.np <= iv.walk_cap || c.rank == 0;
 }
-// Whether the maps and links of this group's walk are staged.
+// Whether the maps and links of this walk are staged: in a group all that fit, in a block those
+// of few pieces (one warp's windows cut a long cable into a chain of them, and a level that waits
+// for device memory takes 1 us).
 template <typename T, int kMode>
 __device__ __forceinline__ bool staged(const Ctx<T, kMode> &c, const ImView &iv) {
-  return kMode != kBlock && c.np <= iv.walk_cap;
+  return c.np <= iv.stage_cap;
 }
 
-// The links of a group's instance, staged once per launch.
+// The links of the instance, staged once per launch.
 template <typename T, int kMode>
 __device__ __noinline__ void stage_links(const Ctx<T, kMode> &c) {
   const ImView &iv = *c.iv;
@@ -460,15 +516,17 @@ __device__ __forceinline__ void window_maps(const WinRows<T, kMode> &r, const T 
     E = one;
     ER = false;
   }
-  if (lane == 0) {
-    sc[wp] = I.a;
-    sc[kWarps + wp] = I.b;
-    sc[2 * kWarps + wp] = I.c;
-    sc[3 * kWarps + wp] = I.d;
-    sc[4 * kWarps + wp] = IR ? (T)1 : (T)0;
+  if (!r.solo) {
+    if (lane == 0) {
+      sc[wp] = I.a;
+      sc[kWarps + wp] = I.b;
+      sc[2 * kWarps + wp] = I.c;
+      sc[3 * kWarps + wp] = I.d;
+      sc[4 * kWarps + wp] = IR ? (T)1 : (T)0;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  if (!ER && !(r.is(kRW - 1, P_LAST))) {  // this thread continues an earlier warp's piece
+  if (!r.solo && !ER && !(r.is(kRW - 1, P_LAST))) {  // this thread continues an earlier warp's piece
     Mob<T> X = one;
     int p = wp + 1;
     while (p < kWarps && sc[4 * kWarps + p] == (T)0) p++;
@@ -497,7 +555,7 @@ __device__ __noinline__ void tree_maps(const Ctx<T, kMode> &c) {
   const T *C = (const T *)iv.cdiag;
   const T *G = sizeof(T) == 4 ? (const T *)(const void *)iv.gf : (const T *)(const void *)iv.g64;
   int par = 0;
-  for (int w = c.w0; w < c.w1; w++) {
+  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
     T *sc = (T *)S.warp + par * 5 * kWarps;
     par ^= 1;
     WinRows<T, kMode> r(c, iv, w);
@@ -525,7 +583,7 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
   const T *G = sizeof(T) == 4 ? (const T *)(const void *)iv.gf : (const T *)(const void *)iv.g64;
   T *pstat = (T *)iv.pstat + 4 * (int64_t)c.ip0, *pval = (T *)iv.pval + 4 * (int64_t)c.ip0;
   double *pxb = (double *)iv.pxb + 2 * (int64_t)c.ip0;
-  for (int w = c.w0; w < c.w1; w++) {
+  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
     T *sc1 = (T *)S.warp, *sc2 = sc1 + 3 * kWarps;
     WinRows<T, kMode> r(c, iv, w);
     T cc[kRW] = {}, g[kRW] = {}, al[kRW] = {}, en[4] = {1, 0, 0, 1};
@@ -541,9 +599,10 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
     if (!r.idle) {
       const T s = k.yin[r.pid[kRW - 1]];
       const T na = en[0] * s + en[1], nb = en[2] * s + en[3];
-      const T f = pow2_near_inv(max_of(na, nb));
-      va = na * f;
-      vb = nb * f;
+      T n2[2] = {na, nb};
+      scale_to_one(n2);
+      va = n2[0];
+      vb = n2[1];
     }
     T inv[kRW], ee[kRW], beta[kRW];
     // what a row passes on: beta u <- e u with 1 entering each piece's last row, alpha
@@ -564,9 +623,10 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
       const T na = g[u] * p, nb = p + g[u] * vb;
       inv[u] = quot(vb, nb);
       ee[u] = g[u] * inv[u];
-      const T s = pow2_near_inv(max_of(na, nb));
-      va = na * s;
-      vb = nb * s;
+      T n2[2] = {na, nb};
+      scale_to_one(n2);
+      va = n2[0];
+      vb = n2[1];
       if (r.is(u, P_LAST)) {
         A[0] = ee[u];
         A[1] = ee[u] * al[u];
@@ -578,7 +638,7 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
       }
     }
     T y[2];
-    affine_enter<T, 2, true>(A, M, sc1, y, r.idle);
+    affine_enter<T, 2, true>(A, M, sc1, y, r.idle, r.solo);
     T sb[2] = {0, 0}, sm = 1, cur = y[0], cua = y[1];
 #pragma unroll
     for (int u = kRW - 1; u >= 0; u--) {
@@ -608,7 +668,7 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
       sb[0] += wb * beta[u];
       sb[1] += wb * al[u];
     }
-    affine_enter<T, 2, false>(sb, sm, sc2, y, r.idle);
+    affine_enter<T, 2, false>(sb, sm, sc2, y, r.idle, r.solo);
 #pragma unroll
     for (int u = 0; u < kRW; u++) {
       if (r.is(u, P_FIRST)) y[0] = y[1] = 0;
@@ -682,7 +742,7 @@ __device__ __forceinline__ void window_eliminate(const WinRows<T, kMode> &r, T (
       M *= ee[u];
     }
   }
-  affine_enter<T, 1, true>(A, M, sc0, y, r.idle);
+  affine_enter<T, 1, true>(A, M, sc0, y, r.idle, r.solo);
   T cur = y[0];
 #pragma unroll
   for (int u = kRW - 1; u >= 0; u--) {
@@ -700,7 +760,7 @@ __device__ __forceinline__ void window_eliminate(const WinRows<T, kMode> &r, T (
     if (r.is(u, P_FIRST)) sb[0] = sm = 0;
     sb[0] += inv[u] * be[u] * al[u];
   }
-  affine_enter<T, 1, false>(sb, sm, sc1, y, r.idle);
+  affine_enter<T, 1, false>(sb, sm, sc1, y, r.idle, r.solo);
 #pragma unroll
   for (int u = 0; u < kRW; u++) {
     if (r.is(u, P_FIRST)) y[0] = 0;
@@ -718,7 +778,7 @@ __device__ __noinline__ void tree_eliminate(const Ctx<T, kMode> &c, const T *v, 
   T *pval = (T *)iv.pval + 4 * ((int64_t)c.ip0 + (int64_t)pb * iv.npieces);
   double *pxb = (double *)iv.pxb + 2 * ((int64_t)c.ip0 + (int64_t)pb * iv.npieces);
   T *sc0 = (T *)S.warp, *sc1 = sc0 + 2 * kWarps;
-  for (int w = c.w0; w < c.w1; w++) {
+  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
     WinRows<T, kMode> r(c, iv, w);
     T al[kRW] = {}, ee[kRW] = {}, inv[kRW] = {}, be[kRW] = {};
     if (r.ok) {
@@ -771,7 +831,7 @@ __device__ __noinline__ void tree_substitute(const Ctx<T, kMode> &c, T *z) {
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<T> k = walk_of(c, iv, S);
   int par = 0;
-  for (int w = c.w0; w < c.w1; w++) {
+  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
     T *sc = (T *)S.warp + par * 2 * kWarps;
     par ^= 1;
     WinRows<T, kMode> r(c, iv, w);
@@ -797,7 +857,7 @@ __device__ __noinline__ void tree_substitute(const Ctx<T, kMode> &c, T *z) {
         M *= ee[u];
       }
     }
-    affine_enter<T, 1, false>(A, M, sc, y, r.idle);
+    affine_enter<T, 1, false>(A, M, sc, y, r.idle, r.solo);
     T cur = y[0];
 #pragma unroll
     for (int u = 0; u < kRW; u++) {

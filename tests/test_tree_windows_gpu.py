@@ -58,11 +58,20 @@ def test_one_tree(gpu, pkg, orc, model, name, scheme):
     assert np.abs(a - b).max() < 1e-8
 
 
+# trees around a warp's window (128 rows) and the rows' chunks of 128, and trees whose pieces do
+# and do not all fit the staging of a block's walk
+SMALL = ["cable%d" % n for n in (4, 127, 128, 129, 130, 255, 257, 1151)] + \
+    ["5x%d" % n for n in (60, 130, 900, 1500, 2100, 2700, 3400)]
+
+
+@pytest.mark.parametrize("names,copies", [(["cable5", "twigs", "71x4117"] + TREES, 1), (SMALL, 1),
+                                          (SMALL, 24)], ids=["all", "small", "small360"])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-def test_batch_of_all(gpu, pkg, orc, model, precision):
+def test_batch_of_all(gpu, pkg, orc, model, precision, names, copies):
     """The same trees in one batch (instances start on multiples of four rows), with trees of
-    more pieces than shared memory holds at several places in it."""
-    specs = [tree(model, n) for n in ["cable5", "twigs", "71x4117"] + TREES]
+    more pieces than shared memory holds at several places in it.  Batches of few trees give each
+    a cluster, of many (copies) a CTA."""
+    specs = [tree(model, n) for n in names] * copies
     probs = [pkg.ProblemArrays.from_spec(sp, pkg.derive(sp)) for sp in specs]
     steps = 12
     out = {}
@@ -77,7 +86,9 @@ def test_batch_of_all(gpu, pkg, orc, model, precision):
         assert (b.instance_stats()["nonconverged"] == 0).all()
         b.close()
     for q, sp in enumerate(specs):
-        if precision == "mixed":
+        if q >= len(names):
+            np.testing.assert_array_equal(out["auto"][q], out["auto"][q - len(names)])
+        elif precision == "mixed":
             assert np.abs(out["auto"][q] - out["gmres"][q]).max() < 1e-8
         else:
             Vo, _, _, _ = orc.implicit_run(sp, orc.derive(sp), sp.dt_abs, 1, 1 + steps, linsolve=0)

@@ -1765,12 +1765,15 @@ int Engine::implicit_plan(size_t &bytes) {
   for (int32_t i = 0; i < ni; i++) max_n = std::max<int64_t>(max_n, host.num_elem[i]);
   S.cluster = 0;
   if (tree && opt.krylov == NRT_GMRES && opt.schedule == 0 && opt.tile_ctas_per_sm == 0) {
-    if (ni == 1) {
-      if (max_n <= kClusterRows) S.cluster = 8;
-    } else {
-      for (int cs = 2; cs <= 8; cs *= 2)
-        if ((int64_t)ni * cs <= (int64_t)dev_sms * (mixed ? 3 : 2)) S.cluster = cs;
-    }
+    // No more CTAs than gain by it, since their barriers cost more than a CTA's: FP64 one per
+    // chunk of 128 rows, mixed batches one per window, and a mixed single tree of one window stays
+    // with one CTA (32 steps: of 300 compartments 1.76 ms on 4 CTAs, 1.31 on one; of 1000 1.78 on
+    // 8, 1.65 on one; of 2000 1.75 on 8, 2.02 on 2; 48 of 300 2.21 ms on 8 CTAs each, 1.33 on one).
+    const int64_t part = mixed && (ni > 1 || max_n <= kMaxWin) ? kMaxWin : 128;
+    const int64_t parts = (max_n + part - 1) / part;
+    const int64_t room = ni > 1 ? (int64_t)dev_sms * (mixed ? 3 : 2) / ni : max_n <= kClusterRows ? 8 : 0;
+    for (int cs = 2; cs <= 8 && cs <= room && cs < 2 * parts; cs *= 2) S.cluster = cs;
+    if (room && parts == 1) S.grid_mode = false;
   }
   if (S.cluster) S.grid_mode = false;
   if (tree) {

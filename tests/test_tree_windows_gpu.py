@@ -31,7 +31,7 @@ def tree(model, name):
     return model.random_tree(seed=int(seed), n_target=int(n), dt=2.5e-5, tspan=1e-3)
 
 
-TREES = ["cable5", "cable%d" % (WIN - 1), "cable%d" % WIN, "cable%d" % (WIN + 1),
+TREES = ["cable5", "cable128", "cable129", "cable%d" % (WIN - 1), "cable%d" % WIN, "cable%d" % (WIN + 1),
          "cable%d" % (WIN + 2), "cable%d" % (5 * WIN + 3), "3x701", "8x2050", "11x6001", "twigs"]
 
 

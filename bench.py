@@ -41,11 +41,12 @@ METRIC = "compartment-steps/s"
 
 # DRAM bytes (read + write) per compartment-step of the dominant kernel, from ncu captures
 # above L2 (profiles/ gives the commands): the explicit step on 1024 trees (21.9M elements)
-# moved 1.394 GB per launch; the implicit launch on 608 trees of 10k elements (6.08M)
-# moved 3.720 GB over 3 steps.  The traffic of a full-size step is scaled from these by the
-# compartments it processes.
-TRAFFIC_PER_ELEMENT_STEP = {"batch-explicit-mixed": 1.394e9 / 21910344,
-                            "batch-implicit-mixed": 3.720006e9 / (3 * 6081291)}
+# moved 1.348 GB per launch of 8 steps; the implicit launch on 456 trees of 10k elements
+# (4.56M) moved 2.527 GB over 3 steps.  The traffic of a full-size step is scaled from these by
+# the compartments it processes.  The explicit step's is far below its algorithmic bytes, which
+# are those of one step at a time, so its roofline fraction can exceed 1.
+TRAFFIC_PER_ELEMENT_STEP = {"batch-explicit-mixed": 1.347680e9 / (8 * 21910344),
+                            "batch-implicit-mixed": 2.527273e9 / (3 * 4560926)}
 WORKLOADS = ("batch-implicit-mixed", "batch-explicit-mixed", "batch-explicit-fp64",
              "axon-explicit-fp64", "myelin-explicit-mixed", "serve")
 DEFAULT_WORKLOAD = "batch-implicit-mixed"
@@ -286,7 +287,9 @@ def algorithmic_bytes_implicit(probs, steps: int, iters, counts):
       FP64 SpMV of the residual that checks it (56 B).  It counts no preconditioner and no
       other refinement residual.
 
-    passes: what this kernel's passes must move per row, counted per pass:
+    passes: what the step's passes must move per row when each is a pass of its own (the kernel
+      fuses most of them and keeps rows in order, so it moves less; roofline.traffic has what
+      it moves), counted per pass:
       assembly (HH 85 / passive 77 B: rowf 1, V^n 8, V^n-1 8, c_m dX/dT 8, 1/(r_a dX) 8,
         class index 4, gates r/w 24 or W dX, K dX 16; writes diagonal 8, c 4, b 8, W_0 4),
       tree factorisation 21 (slot row 4, flag 1, conductance 4, c 4; 1/pivot 4, e 4),
@@ -468,7 +471,8 @@ def run_ours(args, rank: int, world: int, dist, wl: str, extras: bool = True, st
             "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
             "algorithmic_bytes_per_step": alg_all,
             "traffic_note": "DRAM bytes per step from an ncu capture above L2 (1024 trees "
-                            "explicit, 608 trees of 10k elements implicit), scaled by compartments"
+                            "explicit, 456 trees of 10k elements implicit), scaled by compartments; the explicit "
+                            "step takes several steps per launch, each of whose rows it reads once"
                             if per_el else None}
     roof_passes = None
     if passes is not None:

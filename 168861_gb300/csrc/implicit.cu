@@ -69,7 +69,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxPiece = 256;                 // longest segment piece one sweep handles
 constexpr int kMaxDots = kMaxRestart + 1;
 constexpr int kSumChunks = 8;                  // row chunks of an instance's sums at most (rows_reduce)
-constexpr int kTileBytes = 44 * 1024;          // shared memory of the preconditioners
+constexpr int kTileBytes = 44 * 1024;          // staging of the segment preconditioner
 constexpr int kLevels = 128;                   // level offsets kept in shared memory
 constexpr int kBlockWalkBytes = 24 * 1024;     // shared memory of a block's walk
 constexpr int kWalkBytes = 190 * 1024;         // shared memory of the one-tree launch's walk
@@ -1831,10 +1831,13 @@ int Engine::implicit_plan(size_t &bytes) {
     // pieces.  Otherwise the row passes and the windows are each split evenly: the rows over
     // as many CTAs as leave each kRowsPerCta (FP64: an SM evaluates one HH row in about 60
     // cycles of its FP64 pipe, so small trees gain from every SM), the windows over the same
-    // CTAs as far as they go.
+    // CTAs as far as they go.  With the tree preconditioner one CTA per SM: a second repeats the
+    // walk and lengthens the syncs (100k compartments, per step: mixed 130 -> 113 us, FP64 186 ->
+    // 156; the depth-10 binary tree 119 and 212 either way), and it keeps other streams' trees
+    // off the GPU (64 served requests: 7.8 -> 6.6 s).
     const int64_t rows_per_cta = segs ? 4 * kThreads : (mixed ? 256 : 64);
     const int64_t want = (N + rows_per_cta - 1) / rows_per_cta;
-    int G = (int)std::min<int64_t>((int64_t)dev_sms * std::min(per_sm, 2), std::max<int64_t>(1, want));
+    int G = (int)std::min<int64_t>((int64_t)dev_sms * (tree ? 1 : std::min(per_sm, 2)), std::max<int64_t>(1, want));
     G = std::max(1, std::min(G, 4096));
     S.cta_row.assign(G + 1, (int)N);
     S.cta_tile.assign(G + 1, 0);

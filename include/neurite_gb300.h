@@ -118,8 +118,9 @@ typedef struct nrt_options {
   int32_t max_iter;              /* Krylov iterations per step; 0 -> num_elem */
   int32_t device;                /* CUDA device ordinal; -1 -> current device */
   int32_t use_graphs;            /* capture nrt_run time loops in CUDA graphs (default 1) */
-  int32_t schedule;              /* implicit: 0 = auto (one tree -> cooperative whole-GPU
-                                    launch), 1 = always block per instance */
+  int32_t schedule;              /* implicit: 0 = auto (by number and size of the trees: the
+                                    whole GPU, a cluster or a block per instance),
+                                    1 = always block per instance */
   int32_t tiled;                 /* mixed explicit: 1 (default) = element arrays staged into
                                     shared memory by bulk copies, tile by tile; 0 = one
                                     thread per element loading its own (same results) */

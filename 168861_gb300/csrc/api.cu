@@ -653,9 +653,9 @@ int Engine::block_advance(int64_t left) {
 
 void Engine::drop_graphs() {
   for (int q = 0; q < 2; q++) {
-    if (graph_exec[q]) cudaGraphExecDestroy(graph_exec[q]);
-    graph_exec[q] = nullptr;
     for (int g = 0; g < 2; g++) {
+      if (graph_exec[q][g]) cudaGraphExecDestroy(graph_exec[q][g]);
+      graph_exec[q][g] = nullptr;
       if (block_exec[q][g]) cudaGraphExecDestroy(block_exec[q][g]);
       block_exec[q][g] = nullptr;
     }
@@ -842,7 +842,8 @@ int Engine::advance(int64_t steps) {
   if (use_blocks(left)) return block_advance(left);
   const bool graphs = opt.use_graphs != 0 && opt.mode == NRT_EXPLICIT && host.fusable;
   if (graphs && left >= kChunk) {
-    if (!graph_exec[cur]) {
+    cudaGraphExec_t &exec = graph_exec[cur][gcur];
+    if (!exec) {
       cudaGraph_t g;
       NRT_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
       int rc = NRT_OK;
@@ -884,14 +885,14 @@ int Engine::advance(int64_t steps) {
       if (rc != NRT_OK) return rc;
       NRT_CUDA(e);
       size_t nodes = 0;  // every node of the captured chunk is a kernel of this library
-      if (cudaGraphGetNodes(g, nullptr, &nodes) == cudaSuccess) graph_nodes[cur] = (int64_t)nodes;
-      e = cudaGraphInstantiate(&graph_exec[cur], g, 0);
+      if (cudaGraphGetNodes(g, nullptr, &nodes) == cudaSuccess) graph_nodes[cur][gcur] = (int64_t)nodes;
+      e = cudaGraphInstantiate(&exec, g, 0);
       cudaGraphDestroy(g);
       NRT_CUDA(e);
     }
     while (left >= kChunk) {
-      NRT_CUDA(cudaGraphLaunch(graph_exec[cur], stream));
-      count_launches(graph_nodes[cur]);
+      NRT_CUDA(cudaGraphLaunch(exec, stream));
+      count_launches(graph_nodes[cur][gcur]);
       steps_done += kChunk;  // kChunk is even: cur is unchanged
       left -= kChunk;
       terminals_dirty = true;

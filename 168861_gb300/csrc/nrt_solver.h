@@ -36,8 +36,8 @@ struct Engine {
   int64_t nonconv_seen = 0;   // implicit: non-converged steps at the last look (nonconverged_total)
   bool terminals_dirty = false;
   bool general_next = false;  // explicit: the next step runs in the general form
-  cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};  // one per starting buffer parity
-  int64_t graph_nodes[2] = {0, 0};                       // kernels per replay of each
+  cudaGraphExec_t graph_exec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // by cur, gcur
+  int64_t graph_nodes[2][2] = {{0, 0}, {0, 0}};                       // kernels per replay of each
   std::vector<hvec<float>> hostf;  // staging for FP32 uploads
   ImplicitState *im = nullptr;
   RecState *rec = nullptr;                // recording at probes, or null

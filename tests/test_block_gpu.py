@@ -66,7 +66,7 @@ def run(pkg, specs, probs, calls, strain, precision, **opts):
 @pytest.mark.parametrize("name,strain", [("axon", False), ("myelin", False), ("myelin", True),
                                          ("twigs", False), ("tree", False), ("batch", False),
                                          ("batch", True)])
-@pytest.mark.parametrize("calls", [(3, 200), (64, 65, 130), (257,)])
+@pytest.mark.parametrize("calls", [(3, 200), (64, 65, 130), (257,), (64, 200, 64, 133, 64, 64)])
 def test_blocks_equal_single_steps(gpu, pkg, model, name, strain, calls):
     specs = trees(model, name)
     probs = problems(pkg, specs)

@@ -813,7 +813,11 @@ bool Engine::use_blocks(int64_t left) const {
 int Engine::advance(int64_t steps) {
   if (opt.mode == NRT_IMPLICIT_BE) return implicit_advance(*this, steps);
   int64_t left = steps;
-  if (left > 2) TRY(block_init());
+  // The plan of the several-step launches takes as long as they save in about 100 steps (0.35 ms on a
+  // small tree at 3 us a step, 9 ms on 1024 trees at 0.14 ms): it is built when the handle has
+  // been asked for more.
+  constexpr int64_t kPlanSteps = 128;
+  if (left > 2 && !block_tried && (asked_steps += left) >= kPlanSteps) TRY(block_init());
   while (left > 0 && needs_general()) {  // exact first step
     if (strain) TRY(launch_strain_update(*this, 0, stream));
     TRY(step(0, -1));

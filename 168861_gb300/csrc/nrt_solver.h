@@ -46,6 +46,7 @@ struct Engine {
   // several explicit steps per launch (block.cu), or bv.ntiles == 0
   BlockView bv{};
   bool block_tried = false;               // block_init has run
+  int64_t asked_steps = 0;                // steps asked for before it, in calls of several
   std::vector<BlockTile> btile;           // host copy of the tiles
   void *block_mem = nullptr, *probe_mem = nullptr;
   void *gate2[2] = {nullptr, nullptr};    // the two gate buffers; the pack's is gate2[gcur]

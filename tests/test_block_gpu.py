@@ -94,3 +94,23 @@ def compare(pkg, specs, probs, calls, strain, precision):
     np.testing.assert_array_equal(ra.num_spikes, rb.num_spikes)
     for x, y in zip(ra.values + ra.spikes, rb.values + rb.spikes):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("name", ["axon", "tree", "batch"])
+def test_plan_built_later(gpu, pkg, model, name, precision):
+    """Without recording the plan is built when calls have asked for 128 steps: runs that begin
+    with one launch per step and go on with several end as those that keep to one."""
+    specs = trees(model, name)
+    probs = problems(pkg, specs)
+    out = []
+    for opts in ({}, {"tiled": False}):
+        b = pkg.Batch(probs, precision=precision, **opts)
+        b.set_runs([(1, 1000, 0.0, 40 * p.dT) for p in probs])
+        for n in (40, 64, 20, 64, 3, 200, 64):
+            b.advance(n)
+        out.append([b.get_state(q) for q in range(len(specs))])
+        b.close()
+    for x, y in zip(*out):
+        for part in ("V", "V_other", "m", "h", "n"):
+            np.testing.assert_array_equal(getattr(x, part), getattr(y, part), err_msg=part)

@@ -1181,7 +1181,7 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
     tree_maps(c);
     group_sync<kMode>();
   }
-  if (tree) tree_factor(c, c.w.Wb, fused ? (const double *)c.w.Z : (const double *)nullptr);
+  if (tree) tree_factor(c, c.w.Wb, fused);
   const int budget = iv.max_iter > 0 ? iv.max_iter : (iv.max_iter < 0 ? 0 : (int)inst_n);
   const double inner_rel = iv.inner_rel;
   int iters = 0, n_res = 0, n_app = 0, n_xup = 0, n_basis = 0, n_rich = 0;
@@ -1238,16 +1238,15 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
         group_sync<kMode>();  // every window's elimination visible to the walk
         if (walks(c, iv)) refine_walk(c, pb);
         if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
-        const double *from = x0_pending ? (const double *)c.w.Z : Vout;
         const int e = max(-126, min(126, ilogb(res)));
         const float scale = pow2_of<float>(-e);
         // The first cycle's residual is eliminated at once: it is rarely the last.
         double acc[1];
         if (cycle == 0) {
           pb ^= 1;
-          acc[0] = (double)refine_update<kMode, true>(c, from, Vout, scale, pb);
+          acc[0] = (double)refine_update<kMode, true>(c, Vout, scale, pb);
         } else {
-          acc[0] = (double)refine_update<kMode, false>(c, from, Vout, scale, pb);
+          acc[0] = (double)refine_update<kMode, false>(c, Vout, scale, pb);
         }
         eliminated = cycle == 0;
         group_reduce<kMode>(acc, 1, S, iv.partials, parity);  // V and W_0 complete

@@ -51,7 +51,6 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
   Shared S = carve(dyn_smem(), iv.m);
   const int64_t N = pv.ntot;
   float *gate = pv.gatef;
-  double *x0 = (double *)c.w.Z;
   const bool dense = pv.hh_dense != 0;
   const int lane = threadIdx.x & 31;
   float bacc = 0;
@@ -159,7 +158,7 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
       res = fma(gdn, xp, res);
       if (dl) res = fma(gl, xl, res);
       if (f & R_IDENT) b = res = 0.0;
-      x0[row] = (f & R_IDENT) ? o : x;
+      x0_store(c.w.Z, iv.ld, row, (f & R_IDENT) ? o : x);
       iv.diag[row] = d;
       iv.rhs[row] = b;
       ((float *)iv.cdiag)[row] = d2f(cj);
@@ -253,12 +252,12 @@ __device__ __noinline__ void refine_walk(const Ctx<float, kMode> &c, int pb) {
   });
 }
 
-// x += z by substitution (x from Xin, to Vout), then the FP64
-// residual b - A x; returns the thread's part of ||scale r||^2 in FP32 (see ph_residual).
-// kElim: eliminates r into buffer pb of the pieces' values; else stores it (W_0).
+// x += z by substitution, then the FP64 residual b - A x; returns the thread's part of
+// ||scale r||^2 in FP32 (see ph_residual).  kElim, the step's first cycle: x starts from the
+// initial guess, and r is eliminated into buffer pb of the pieces' values; else x is updated in
+// Vout and r stored (W_0).
 template <int kMode, bool kElim>
-__device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const double *Xin, double *Vout,
-                                            float scale, int pb) {
+__device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, double *Vout, float scale, int pb) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<float> k = walk_of(c, iv, S);
@@ -277,7 +276,8 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, const do
       ld_rows((const float *)iv.te + rb, ee);
       ld_rows((const float *)iv.tinv + rb, inv);
       ld_rows((const float *)iv.tbeta + rb, be);
-      ld_rows(Xin + rb, x);
+      if (kElim) x0_rows(c.w.Z, iv.ld, rb, x);
+      else ld_rows(Vout + rb, x);
     }
     r.ids(c, iv);
     // substitution

@@ -116,6 +116,34 @@ struct WinRows {
   }
 };
 
+// The initial guess x0 of a step, as refine_assemble leaves it for the passes that would form it
+// again: a row's low word in Z_0, its high word in Z_1 (there are m + 1 >= 2 columns), at the
+// row's own place.  Z is one workspace of all trees, a column ld rows apart, and trees run side by
+// side: as an array of doubles x0 would lie on other trees' rows of Z_0 and Z_1, which one of them
+// may be using for its GMRES basis.
+template <typename T>
+__device__ __forceinline__ void x0_store(T *Z, int64_t ld, int64_t row, double x) {
+  static_assert(sizeof(T) == 4, "a word each");
+  ((int *)(void *)Z)[row] = __double2loint(x);
+  ((int *)(void *)Z)[ld + row] = __double2hiint(x);
+}
+template <typename T>
+__device__ __forceinline__ double x0_load(const T *Z, int64_t ld, int64_t row) {
+  if constexpr (sizeof(T) == 4) {
+    const int *z = (const int *)(const void *)Z;
+    return __hiloint2double(z[ld + row], z[row]);
+  } else {
+    return 0.0;  // FP64 steps keep no initial guess
+  }
+}
+__device__ __forceinline__ void x0_rows(const float *Z, int64_t ld, int64_t rb, double (&x)[kRW]) {
+  const int4 lo = *(const int4 *)(const void *)(Z + rb), hi = *(const int4 *)(const void *)(Z + ld + rb);
+  x[0] = __hiloint2double(hi.x, lo.x);
+  x[1] = __hiloint2double(hi.y, lo.y);
+  x[2] = __hiloint2double(hi.z, lo.z);
+  x[3] = __hiloint2double(hi.w, lo.w);
+}
+
 // ---- scans over the CTA's threads (every thread takes part)
 
 // Value entering this thread's part of kN affine recurrences y <- A + M y that share M, in
@@ -572,10 +600,10 @@ __device__ __noinline__ void tree_maps(const Ctx<T, kMode> &c) {
 
 // Pivots from the children's conductances: inv, e, beta of every row, and per piece the
 // product B of its e and bL.  The rows of v, the first right-hand side, are eliminated in the
-// same pass (tree_eliminate, into buffer 0 of the pieces' values).  x0 (may be null): the potential
-// of which each piece's first and last row is exported too, for the refinement's updates.
+// same pass (tree_eliminate, into buffer 0 of the pieces' values).  ends: the initial guess of each
+// piece's first and last row is exported too, for the refinement's updates.
 template <typename T, int kMode>
-__device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, const double *x0) {
+__device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, bool ends) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<T> k = walk_of(c, iv, S);
@@ -658,7 +686,7 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
         ps[3] = ee[u];
         pa[0] = cua;  // A
         pa[2] = inv[u] * al[u];
-        if (x0) pxb[2 * (int64_t)r.pid[u]] = x0[r.rb + u];
+        if (ends) pxb[2 * (int64_t)r.pid[u]] = x0_load(c.w.Z, iv.ld, r.rb + u);
       }
     }
 #pragma unroll
@@ -678,7 +706,7 @@ __device__ __noinline__ void tree_pivots(const Ctx<T, kMode> &c, const T *v, con
       if (r.is(u, P_LAST)) {
         pstat[4 * (int64_t)r.pid[u] + 1] = y[0];  // bL
         pval[4 * (int64_t)r.pid[u] + 1] = y[1];   // aL
-        if (x0) pxb[2 * (int64_t)r.pid[u] + 1] = x0[r.rb + u];
+        if (ends) pxb[2 * (int64_t)r.pid[u] + 1] = x0_load(c.w.Z, iv.ld, r.rb + u);
       }
     }
     if (r.ok) {
@@ -710,11 +738,11 @@ __device__ __noinline__ void walk_factor(const Ctx<T, kMode> &c) {
 // The factorisation once every piece's matrix is known (tree_maps, or the windowed assembly)
 // and visible to the walk.
 template <typename T, int kMode>
-__device__ __noinline__ void tree_factor(const Ctx<T, kMode> &c, const T *v, const double *x0) {
+__device__ __noinline__ void tree_factor(const Ctx<T, kMode> &c, const T *v, bool ends) {
   const ImView &iv = *c.iv;
   if (walks(c, iv)) walk_factor(c);
   if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
-  tree_pivots(c, v, x0);
+  tree_pivots(c, v, ends);
   __syncthreads();  // its scans' scratch is free for the next reduction
 }
 

@@ -459,7 +459,10 @@ __device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, i
 // rows or more: four warps keep an SM's FP64 pipe busy, and shorter ones, one after the other,
 // only add their latency (1000 cables of 60 compartments in FP64, 32 steps: 20.0 ms with 8 chunks
 // each, 6.4 with one).  The warps leave their sums of every chunk and meet once after the last
-// (400 trees of 3000: 27.0 -> 25.9 ms).
+// (400 trees of 3000: 27.0 -> 25.9 ms).  Where an instance never has more than a CTA (every
+// preconditioner but the tree's, and BiCGSTAB) the rows are one chunk: a GMRES cycle of many
+// Arnoldi steps reduces up to kG products per pass, and eight short passes took up to three times
+// one long one (Jacobi, FP64, 400 trees of 3000, 8 steps: 287 -> 116 ms; mixed, 24 of 3000: 72 -> 32).
 template <typename T, int kMode, typename F>
 __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Shared &S,
                                             double *partials, int &parity, int off, F f) {
@@ -1426,7 +1429,7 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
     const bool tree = iv.precond == NRT_PRECOND_TREE;
     if (threadIdx.x == 0) {
       c.n = n;
-      c.chunks = min(kSumChunks, (n + 127) / 128);
+      c.chunks = tree && iv.krylov == NRT_GMRES ? min(kSumChunks, (n + 127) / 128) : 1;
       c.v0 = c.chunks * c.rank / gsize;
       c.v1 = c.chunks * (c.rank + 1) / gsize;
       c.wrow0 = iv.inst_row[inst];

@@ -44,7 +44,7 @@
 //    into contiguous per-CTA ranges; grid-wide syncs separate the phases.
 //  * kBlock (batches): a persistent block-per-instance scheduler; each CTA takes the next
 //    instance (largest first) from an atomic queue and runs all of its steps with
-//    __syncthreads only;
+//    __syncthreads only.  kBlock4 is the same with registers for four CTAs on an SM;
 //  * kCluster (batches too small to fill the GPU, and small single trees): a cluster of up to
 //    eight CTAs per instance, with the cluster's barrier between the phases.
 #include <cooperative_groups.h>
@@ -213,9 +213,10 @@ __device__ Shared carve(double *base, int m) {
 
 // ---------------------------------------------------------------- groups
 //
-// The CTAs that step one instance: the CTA itself (kBlock), the whole cooperative launch
+// The CTAs that step one instance: the CTA itself (kBlock, kBlock4), the whole cooperative launch
 // (kGrid), or a thread-block cluster (kCluster).
-enum : int { kBlock = 0, kGrid = 1, kCluster = 2 };
+enum : int { kBlock = 0, kGrid = 1, kCluster = 2, kBlock4 = 3 };
+__host__ __device__ constexpr bool one_cta(int mode) { return mode == kBlock || mode == kBlock4; }
 
 __device__ __forceinline__ int cluster_rank() {
   int r;
@@ -311,7 +312,7 @@ template <int kMode, typename T, int kN>
 __device__ __forceinline__ void group_reduce(const T (&acc)[kN], int k, Shared &S,
                                              double *partials, int &parity, int off = 0) {
   block_reduce(acc, k, S.warp, S.red + off);
-  if (kMode != kBlock) group_finish<kMode>(k, S.red + off, partials, parity);
+  if (!one_cta(kMode)) group_finish<kMode>(k, S.red + off, partials, parity);
 }
 
 // ---------------------------------------------------------------- row kernels
@@ -441,12 +442,6 @@ struct Ctx {
   const int *lev;   // the instance's level offsets (in shared memory, when they fit)
 };
 
-// A sync of the group where one CTA's rows reach another's (nothing to do in one CTA).
-template <int kMode>
-__device__ __forceinline__ void level_sync() {
-  if (kMode != kBlock) group_sync<kMode>();
-}
-
 // The initial guess of a step: V^n extrapolated from V^{n-1} (which Vout holds until the
 // first solution update writes it).
 __device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, int64_t j) {
@@ -477,9 +472,18 @@ __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Share
     parity ^= 1;
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // A chunk of at most 128 rows is one row each for half of the CTA's threads, so the halves take
+  // a chunk in turn, the upper one from half a CTA before it (600 cables of 1000 in FP64: 12.3 ->
+  // 10.7 ms).  turn: this warp's half, 2 where all warps take every chunk.
+  const int turn = c.chunks > 1 && c.n <= kThreads / 2 * c.chunks ? w / (kWarps / 2) : 2;
   for (int v = c.v0; v < c.v1; v++) {  // no barrier between the chunks
-    auto acc = f(c.wrow0 + (int64_t)c.n * v / c.chunks, c.wrow0 + (int64_t)c.n * (v + 1) / c.chunks);
     double *to = S.wpart + ((v - c.v0) * kWarps + w) * kG;
+    if (turn != 2 && ((v - c.v0) & 1) != turn) {
+      if (lane < k) to[lane] = 0.0;
+      continue;
+    }
+    auto acc = f(c.wrow0 + (int64_t)c.n * v / c.chunks - (turn == 1 ? kThreads / 2 : 0),
+                 c.wrow0 + (int64_t)c.n * (v + 1) / c.chunks);
 #pragma unroll
     for (int i = 0; i < (int)(sizeof(acc.v) / sizeof(acc.v[0])); i++) {
       if (i < k) {
@@ -1240,7 +1244,7 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
         if (!eliminated) tree_eliminate(c, c.w.Wb, pb, Vout);
         group_sync<kMode>();  // every window's elimination visible to the walk
         if (walks(c, iv)) refine_walk(c, pb);
-        if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
+        if (!one_cta(kMode) && c.np > iv.walk_cap) group_sync<kMode>();
         const int e = max(-126, min(126, ilogb(res)));
         const float scale = pow2_of<float>(-e);
         // The first cycle's residual is eliminated at once: it is rarely the last.
@@ -1374,13 +1378,13 @@ __device__ __noinline__ void ph_record(const RecView *rp, int inst, int64_t i, c
 // Resident CTAs per SM that the registers allow.  FP32: 3 (80 registers; the 2048-tree batch
 // took 51.1 ms per 8 steps at 4, whose 64 registers spill in the fused passes, 41.7 at 3 and
 // 48.9 at 2).  FP64: 2 (128 registers): its FP64 pipe is full with 16 warps.
-template <typename T>
+template <typename T, int kMode>
 constexpr int ctas_per_sm() {
-  return sizeof(T) == 4 ? 3 : 2;
+  return kMode == kBlock4 ? 4 : sizeof(T) == 4 ? 3 : 2;
 }
 
 template <typename T, int kMode>
-__global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(const PackView *pvp, const ImView *ivp,
+__global__ void __launch_bounds__(kThreads, ctas_per_sm<T, kMode>()) implicit_steps(const PackView *pvp, const ImView *ivp,
                                                            int nsteps, int force, double *V0,
                                                            double *V1, int cur,
                                                            const RecView *rec) {
@@ -1415,7 +1419,7 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T>()) implicit_steps(con
   int q = kMode == kCluster ? (int)blockIdx.x / gsize : 0;
   for (;;) {
     int inst = 0;
-    if (kMode == kBlock) {
+    if (one_cta(kMode)) {
       if (threadIdx.x == 0) S.flag[1] = atomicAdd(iv.queue, 1);
       __syncthreads();
       q = S.flag[1];
@@ -1521,10 +1525,12 @@ static const void *implicit_kernel(bool mixed, int group) {
   if (mixed)
     return group == kGrid ? (const void *)implicit_steps<float, kGrid>
            : group == kCluster ? (const void *)implicit_steps<float, kCluster>
-                               : (const void *)implicit_steps<float, kBlock>;
+           : group == kBlock4 ? (const void *)implicit_steps<float, kBlock4>
+                              : (const void *)implicit_steps<float, kBlock>;
   return group == kGrid ? (const void *)implicit_steps<double, kGrid>
          : group == kCluster ? (const void *)implicit_steps<double, kCluster>
-                             : (const void *)implicit_steps<double, kBlock>;
+         : group == kBlock4 ? (const void *)implicit_steps<double, kBlock4>
+                            : (const void *)implicit_steps<double, kBlock>;
 }
 
 static size_t smem_bytes(int m, size_t tile) {
@@ -1675,6 +1681,37 @@ static void make_tiles(const hvec<int2> &pieces, int pa, int pb, int tile_rows,
   }
 }
 
+// Whether a batch of one CTA per tree runs kBlock4 (the same results: a tree's arithmetic and its
+// order are the same in both).
+//
+// With 64 registers instead of 80 (mixed) or 128 (FP64) a pass takes 5 to 50 % longer, and trees of
+// different sizes gain from few CTAs that are fast (1000 trees of 1e3 to 3e4: mixed 9.6 ms, 12.0 with
+// four; FP64 30.2 and 36.2).  Four are faster where the number of trees decides:
+//  - trees that are too small to occupy a CTA's warps, more than the usual CTAs take at once (32
+//    steps of 1000 cables of 60: FP64 6.3 ms, 3.9 with four; mixed 2.7, 2.4; of 300: 11.4, 10.0 and
+//    3.2, 2.8);
+//  - more trees of about one size than the usual CTAs take at once, when four CTAs need no more
+//    rounds' time.  A round of k CTAs per SM lasts as long as k trees on an SM even where it is not
+//    full (the trees of the last one meet on few SMs), except that a launch of fewer trees than
+//    places spreads them evenly: 400 cables of 3000 in FP64 are two rounds of two, 28.9 ms, or three
+//    at once, 21.0; 600 of 1000 mixed two rounds of three, 3.6, or four at once, 2.6; but 620 of
+//    1500 mixed two rounds of three, 2.6, or of four, 2.9.
+static bool four_per_sm(const HostPack &host, const nrt_options &opt, int sms) {
+  const int usual = opt.precision == NRT_MIXED ? ctas_per_sm<float, kBlock>() : ctas_per_sm<double, kBlock>();
+  if (opt.tile_ctas_per_sm > 0) return opt.tile_ctas_per_sm > usual;
+  const int64_t ni = host.ninst;
+  int64_t largest = 0, sum = 0;
+  for (int64_t i = 0; i < ni; i++) {
+    largest = std::max<int64_t>(largest, host.num_elem[i]);
+    sum += host.num_elem[i];
+  }
+  if (ni <= usual * (int64_t)sms) return false;
+  auto trees_per_sm = [&](int64_t k) {
+    return ni <= k * sms ? (ni + sms - 1) / sms : (ni + k * sms - 1) / (k * sms) * k;
+  };
+  return largest <= 512 || (4 * largest * ni <= 5 * sum && trees_per_sm(4) <= trees_per_sm(usual));
+}
+
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Row structure, launch shape and preconditioner schedule; the exact device bytes the
@@ -1754,7 +1791,11 @@ int Engine::implicit_plan(size_t &bytes) {
   const bool mixed = opt.precision == NRT_MIXED;
   const size_t tb = mixed ? 4 : 8;
   const int64_t ld = (N + kRW - 1) & ~(int64_t)(kRW - 1);
-  S.tile_rows = (int)(kTileBytes / (4 * tb));
+  int64_t max_n = 0;
+  for (int32_t i = 0; i < ni; i++) max_n = std::max<int64_t>(max_n, host.num_elem[i]);
+  // rows staged at a time: no more than a tree has, so that small trees' CTAs fit an SM
+  S.tile_rows = (int)std::min<int64_t>(kTileBytes / (4 * tb), (max_n + 31) & ~(int64_t)31);
+  S.tile_rows = std::max(S.tile_rows, kMaxPiece);
   int dev_sms = 0;
   NRT_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
   S.grid_mode = ni == 1 && opt.schedule == 0;
@@ -1763,8 +1804,6 @@ int Engine::implicit_plan(size_t &bytes) {
   // idle as long as there are fewer instances than SMs, and a small single tree spends most of a
   // cooperative launch's step in its grid-wide syncs (1.5 to 2 us each; a cluster's barrier
   // takes about 0.4).
-  int64_t max_n = 0;
-  for (int32_t i = 0; i < ni; i++) max_n = std::max<int64_t>(max_n, host.num_elem[i]);
   S.cluster = 0;
   if (tree && opt.krylov == NRT_GMRES && opt.schedule == 0 && opt.tile_ctas_per_sm == 0) {
     // No more CTAs than gain by it, since their barriers cost more than a CTA's: FP64 one per
@@ -1795,7 +1834,8 @@ int Engine::implicit_plan(size_t &bytes) {
     }
     build_tree_plan(host, S.rowf.data(), ld, S.win, S.tree);
   }
-  const int group = S.cluster ? kCluster : S.grid_mode ? kGrid : kBlock;
+  const int group = S.cluster ? kCluster : S.grid_mode ? kGrid
+                    : four_per_sm(host, opt, dev_sms) ? kBlock4 : kBlock;
   const void *kern = implicit_kernel(mixed, group);
   S.kern = kern;
   // shared memory: the segment preconditioner's staging, or the tree walk's numbers of
@@ -1804,9 +1844,9 @@ int Engine::implicit_plan(size_t &bytes) {
   // kWalkBytes; larger walks run in device memory.  A block stages the maps and links too where
   // they fit as well (1000 trees of 300 compartments, mixed, 32 steps: 6.03 -> 5.34 ms).
   size_t tile = 0;
-  if (segs) tile = kTileBytes;
+  if (segs) tile = (size_t)S.tile_rows * 4 * tb;
   if (tree) {
-    const bool grp = group != kBlock;
+    const bool grp = !one_cta(group);
     const size_t cap = S.grid_mode ? kWalkBytes : S.cluster ? kClusterWalkBytes : kBlockWalkBytes;
     S.iv.walk_cap = (int)std::min<size_t>(std::min<size_t>(cap / walk_bytes(tb, grp), kNoPiece - 1),
                                           (size_t)S.tree.max_pieces);

@@ -225,7 +225,7 @@ __device__ __noinline__ void refine_walk(const Ctx<float, kMode> &c, int pb) {
       if (q == kNoPiece) return;
       put(q, RefineX{ps[q], pa[q], px[q]}, k.yin[q], k.zpar[q], k.val[q], k.link[q].w != 0);
     };
-    if (kMode == kBlock) {
+    if (one_cta(kMode)) {
       for (int q = threadIdx.x; q < c.np; q += kThreads) one(q);
       __syncthreads();
       return;

@@ -314,7 +314,7 @@ __device__ __forceinline__ Mob<T> mob_shfl_down(const Mob<T> &m, int off) {
 // ---- the walk over the pieces (one CTA)
 
 // The numbers of the walk, one per piece of the instance (ids in level order, deepest first).
-// A CTA alone (kBlock) with many pieces keeps the first four in shared memory (or in device memory
+// A CTA alone with many pieces keeps the first four in shared memory (or in device memory
 // when there are too many) and loads each level's maps and links one level ahead.  In a group
 // every CTA walks all pieces redundantly, with the maps and links staged in shared memory as well: the
 // levels of a bushy tree hold a thousand pieces, and a walk that loads them level by level took
@@ -360,7 +360,7 @@ __device__ __forceinline__ Walk<T> walk_of(const Ctx<T, kMode> &c, const ImView 
 // when the walk's numbers fit its shared memory, else the group's first.
 template <typename T, int kMode>
 __device__ __forceinline__ bool walks(const Ctx<T, kMode> &c, const ImView &iv) {
-  return kMode == kBlock || c.np <= iv.walk_cap || c.rank == 0;
+  return one_cta(kMode) || c.np <= iv.walk_cap || c.rank == 0;
 }
 // Whether the maps and links of this walk are staged: in a group all that fit, in a block those
 // of few pieces (one warp's windows cut a long cable into a chain of them, and a level that waits
@@ -741,7 +741,7 @@ template <typename T, int kMode>
 __device__ __noinline__ void tree_factor(const Ctx<T, kMode> &c, const T *v, bool ends) {
   const ImView &iv = *c.iv;
   if (walks(c, iv)) walk_factor(c);
-  if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
+  if (!one_cta(kMode) && c.np > iv.walk_cap) group_sync<kMode>();
   tree_pivots(c, v, ends);
   __syncthreads();  // its scans' scratch is free for the next reduction
 }
@@ -908,7 +908,7 @@ __device__ __noinline__ void tree_apply(const Ctx<T, kMode> &c, const T *v, T *z
   if (!eliminated) tree_eliminate(c, v, 0, (const double *)nullptr);
   group_sync<kMode>();
   if (walks(c, iv)) walk_solve(c);
-  if (kMode != kBlock && c.np > iv.walk_cap) group_sync<kMode>();
+  if (!one_cta(kMode) && c.np > iv.walk_cap) group_sync<kMode>();
   tree_substitute(c, z);
   __syncthreads();  // the walk's numbers are read before the next walk writes them
 }

@@ -9,9 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("opts", [dict(precond="segment"), dict(precond="jacobi", max_iter=4000),
-                                  dict(krylov="bicgstab", precond="segment"),
                                   dict(krylov="bicgstab", precond="tree")],
-                         ids=["segment", "jacobi", "bicgstab-segment", "bicgstab-tree"])
+                         ids=["segment", "jacobi", "bicgstab-tree"])
 def test_batch_of_sizes(gpu, pkg, orc, model, opts):
     specs = [model.random_tree(seed=31 + q, n_target=n, dt=2.5e-5, tspan=1e-3)
              for q, n in enumerate((60, 255, 300, 1025, 2100))]

@@ -439,6 +439,8 @@ struct Ctx {
   int ip0, np, l0, l1;
   int rank;         // this CTA in its group
   int n, chunks, v0, v1;  // rows of the instance; their chunks, this CTA's of them (rows_reduce)
+  int wchunks, wv0, wv1;  // chunks of whole windows, this CTA's of them (refine.cuh)
+  int wend_of[kSumChunks];  // past the last window of each of this CTA's chunks
   const int *lev;   // the instance's level offsets (in shared memory, when they fit)
 };
 
@@ -446,6 +448,35 @@ struct Ctx {
 // first solution update writes it).
 __device__ __forceinline__ double x0_of(const double *Vin, const double *Vout, int64_t j) {
   return 2.0 * Vin[j] - Vout[j];
+}
+
+// Where a CTA puts the sums of its chunks, kMaxDots apart.
+template <int kMode>
+__device__ __forceinline__ double *chunk_sums(Shared &S, double *partials, int &parity) {
+  if (kMode != kCluster) return S.part;
+  parity ^= 1;
+  return group_partials<kMode>(partials, parity ^ 1);
+}
+
+// The totals of k sums over the instance's chunks, in the order of the chunks, to S.red[off ..], once
+// every CTA has put its chunks' (a grid's CTA one, its own).
+template <int kMode>
+__device__ __forceinline__ void total_chunks(int k, int chunks, const double *sum, Shared &S,
+                                             double *partials, int &parity, int off) {
+  if (kMode == kGrid) {
+    __syncthreads();
+    if (threadIdx.x < k) S.red[off + threadIdx.x] = sum[threadIdx.x];
+    __syncthreads();
+    group_finish<kMode>(k, S.red + off, partials, parity);
+    return;
+  }
+  group_sync<kMode>();
+  if (threadIdx.x < k) {
+    double s = 0;
+    for (int v = 0; v < chunks; v++) s += sum[v * kMaxDots + threadIdx.x];
+    S.red[off + threadIdx.x] = s;
+  }
+  __syncthreads();
 }
 
 // Sums k (<= kG) accumulators of a row pass f(first row, end) over the instance into S.red[off .. off + k).  In
@@ -465,11 +496,6 @@ __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Share
     auto acc = f(c.r0, c.r1);
     group_reduce<kMode>(acc.v, k, S, partials, parity, off);
     return;
-  }
-  double *sum = S.part;
-  if (kMode == kCluster) {
-    sum = group_partials<kMode>(partials, parity);
-    parity ^= 1;
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // A chunk of at most 128 rows is one row each for half of the CTA's threads, so the halves take
@@ -495,6 +521,7 @@ __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Share
   }
   __syncthreads();
   // the warps' sums of a chunk: eight lanes each
+  double *sum = chunk_sums<kMode>(S, partials, parity);
   const int count = (c.v1 - c.v0) * k;
   for (int q0 = 4 * w; q0 < count; q0 += 4 * kWarps) {
     const int q = q0 + (lane >> 3), v = q / k, i = q % k;
@@ -502,13 +529,7 @@ __device__ __forceinline__ void rows_reduce(const Ctx<T, kMode> &c, int k, Share
     for (int o = 4; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o, 8);
     if (q < count && (lane & 7) == 0) sum[(c.v0 + v) * kMaxDots + i] = x;
   }
-  group_sync<kMode>();
-  if (threadIdx.x < k) {
-    double s = 0;
-    for (int v = 0; v < c.chunks; v++) s += sum[v * kMaxDots + threadIdx.x];
-    S.red[off + threadIdx.x] = s;
-  }
-  __syncthreads();
+  total_chunks<kMode>(k, c.chunks, sum, S, partials, parity, off);
 }
 
 template <typename X, int kN>
@@ -1170,11 +1191,11 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
   };
   if (fused) {
     if constexpr (sizeof(T) == 4) {
-      const double2 br = iv.scheme == NRT_CRANK_NICOLSON
-                             ? refine_assemble<kMode, true>(c, Vin, Vout, active ? 1 : 0, inst)
-                             : refine_assemble<kMode, false>(c, Vin, Vout, active ? 1 : 0, inst);
-      const double acc[2] = {br.x, br.y};
-      group_reduce<kMode>(acc, 2, S, iv.partials, parity);  // also publishes W_0, the matrices
+      if (iv.scheme == NRT_CRANK_NICOLSON)
+        refine_assemble<kMode, true>(c, Vin, Vout, active ? 1 : 0, inst);
+      else
+        refine_assemble<kMode, false>(c, Vin, Vout, active ? 1 : 0, inst);
+      sum_windows<kMode, 2>(c, S, iv.partials, parity);  // also publishes W_0, the matrices
     }
   } else {
     rows_reduce(c, 2, S, iv.partials, parity, 0, assemble);  // also publishes W_0 and c
@@ -1248,15 +1269,14 @@ __device__ __forceinline__ void implicit_one_step(const Ctx<T, kMode> &c, Shared
         const int e = max(-126, min(126, ilogb(res)));
         const float scale = pow2_of<float>(-e);
         // The first cycle's residual is eliminated at once: it is rarely the last.
-        double acc[1];
         if (cycle == 0) {
           pb ^= 1;
-          acc[0] = (double)refine_update<kMode, true>(c, Vout, scale, pb);
+          refine_update<kMode, true>(c, Vout, scale, pb);
         } else {
-          acc[0] = (double)refine_update<kMode, false>(c, Vout, scale, pb);
+          refine_update<kMode, false>(c, Vout, scale, pb);
         }
         eliminated = cycle == 0;
-        group_reduce<kMode>(acc, 1, S, iv.partials, parity);  // V and W_0 complete
+        sum_windows<kMode, 1>(c, S, iv.partials, parity);  // V and W_0 complete
         prev_res = res;
         res = sqrt(S.red[0]) * pow2_of<double>(e);
         w0_valid = cycle != 0;
@@ -1444,6 +1464,11 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T, kMode>()) implicit_st
       c.iw1 = tree ? iv.inst_win[inst + 1] : 0;
       c.w0 = c.iw0 + (c.iw1 - c.iw0) * c.rank / gsize;
       c.w1 = c.iw0 + (c.iw1 - c.iw0) * (c.rank + 1) / gsize;
+      // gsize divides kSumChunks, so a CTA's windows are whole chunks
+      c.wchunks = min(kSumChunks, c.iw1 - c.iw0);
+      c.wv0 = c.wchunks * c.rank / gsize;
+      c.wv1 = c.wchunks * (c.rank + 1) / gsize;
+      for (int v = c.wv0; v < c.wv1; v++) c.wend_of[v - c.wv0] = c.iw0 + (c.iw1 - c.iw0) * (v + 1) / c.wchunks;
       c.ip0 = tree ? iv.inst_piece[inst] : 0;
       c.np = tree ? iv.inst_piece[inst + 1] - c.ip0 : 0;
       c.l0 = tree ? iv.inst_lev[inst] : 0;
@@ -1456,6 +1481,9 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm<T, kMode>()) implicit_st
         if (tree) {
           c.w0 = iv.cta_win[blockIdx.x];
           c.w1 = iv.cta_win[blockIdx.x + 1];
+          c.wchunks = c.wv1 = 1;
+          c.wv0 = 0;
+          c.wend_of[0] = c.w1;
         }
       } else {
         c.t0 = iv.inst_tile[inst];

@@ -21,18 +21,61 @@
 namespace nrt {
 
 // x of the row before this thread's first and after its last, in the window.  ends: 2 * kWarps
-// doubles; one CTA barrier unless solo.
+// doubles; one CTA barrier.
 __device__ __forceinline__ void window_ends(const double (&x)[kRW], double *ends, double &xm,
-                                            double &xp, bool solo) {
+                                            double &xp) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   xm = __shfl_up_sync(0xffffffffu, x[kRW - 1], 1);
   xp = __shfl_down_sync(0xffffffffu, x[0], 1);
-  if (solo) return;  // a piece never reaches over a window's ends
   if (lane == 31) ends[w] = x[kRW - 1];
   if (lane == 0) ends[kWarps + w] = x[0];
   __syncthreads();
   if (lane == 0 && w > 0) xm = ends[w - 1];
   if (lane == 31 && w + 1 < kWarps) xp = ends[kWarps + w + 1];
+}
+
+// The sums of a pass (||b||^2, ||r||^2) are taken by chunks of whole windows, up to kSumChunks of
+// them, whose edges depend on the tree alone: as with rows_reduce, the result does not depend on how
+// many CTAs share the tree, and so not on the trees beside it.  After a chunk a warp leaves kG numbers
+// in S.wpart (of two sums four each) and starts afresh, and after the pass a warp sums each chunk's.
+// Against one sum per CTA, whose bits changed with the cluster's size, clusters take the same time and
+// batches of one CTA per tree 2 to 5 % more (8 steps of 1000 trees of 1e3 to 3e4: 9.5 -> 9.8 ms, 320
+// of them 7.8 -> 8.2, the 2048 trees of 1e3 to 1e5 36.3 -> 37.1).  Forms measured and not taken: the
+// passes called once per chunk (37.5 for the last), every chunk summed up where it ends (37.6), every
+// thread's parts in shared memory (37.2 with 24 KB of it, 1000 trees 10.4).
+template <int kN>
+__device__ __forceinline__ void leave_chunk(const Shared &S, int chunk, double a, double b) {
+  static_assert(kG == 8 && kWarps == 8, "a warp's places in S.wpart");
+  const int lane = threadIdx.x & 31;
+  double *to = S.wpart + (chunk * kWarps + (threadIdx.x >> 5)) * kG;
+#pragma unroll
+  for (int o = 16; o >= (kN == 1 ? 8 : 4); o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    if (kN == 2) b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (lane < kG / kN) {
+    to[lane] = a;
+    if (kN == 2) to[lane + kG / 2] = b;
+  }
+}
+
+// kN sums to S.red[0 ..].
+template <int kMode, int kN>
+__device__ __forceinline__ void sum_windows(const Ctx<float, kMode> &c, Shared &S, double *partials,
+                                            int &parity) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __syncthreads();
+  double *sum = chunk_sums<kMode>(S, partials, parity);
+  for (int v = w; v < c.wv1 - c.wv0; v += kWarps) {
+    const double *from = S.wpart + v * kWarps * kG + lane;
+    double x = 0;
+    if (kMode != kGrid || c.w0 < c.w1) x = from[0] + from[32];  // lane & 7: the place of a warp
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (kN == 1 || o != 4) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0 || (kN == 2 && lane == 4)) sum[(c.wv0 + v) * kMaxDots + (lane >> 2)] = x;
+  }
+  total_chunks<kMode>(kN, c.wchunks, sum, S, partials, parity, 0);
 }
 
 // kCn: Crank-Nicolson.  The rows' part takes one row per thread, a warp 32 neighbours: with the
@@ -44,8 +87,8 @@ __device__ __forceinline__ void window_ends(const double (&x)[kRW], double *ends
 // operation), so rare rows share one x0 with the warp's ends, and x0 goes to Z for the passes that
 // would form it again (the pieces' ends, the first update): 3.13 -> 3.00 ms, 38.2 -> 37.8 ms.
 template <int kMode, bool kCn>
-__device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, const double *Vin,
-                                                const double *Vout, int active, int inst) {
+__device__ __noinline__ void refine_assemble(const Ctx<float, kMode> &c, const double *Vin,
+                                             const double *Vout, int active, int inst) {
   const PackView &pv = *c.pv;
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
@@ -55,14 +98,12 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
   const int lane = threadIdx.x & 31;
   float bacc = 0;
   double racc = 0;
-  int par = 0;
-  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
-    float *sc = (float *)S.warp + par * 5 * kWarps;
-    par ^= 1;
+  int chunk = 0;
+  for (int w = c.w0; w < c.w1; w++) {
     const int64_t r0 = c.wrow0 + (int64_t)(w - c.iw0) * iv.win;
     const int nr = (int)min((int64_t)iv.win, c.wend - r0);
 #pragma unroll 1
-    for (int l = window_thread(iv); l - lane < nr; l += iv.solo ? 32 : kThreads) {
+    for (int l = threadIdx.x; l - lane < nr; l += kThreads) {
       const int64_t row = min(r0 + l, N - 1);
       const bool ok = l < nr;
       const double v = Vin[row], o = Vout[row], cm = iv.cmdt[row], g = iv.g64[row];
@@ -167,8 +208,7 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
       bacc += bf * bf;
       racc += res * res;
     }
-    if (iv.solo) __syncwarp();  // the window's rows are there
-    else __syncthreads();
+    __syncthreads();  // the window's rows are there
     WinRows<float, kMode> r(c, iv, w);
     float cc[kRW] = {}, gf[kRW] = {};
     if (r.ok) {
@@ -177,10 +217,14 @@ __device__ __noinline__ double2 refine_assemble(const Ctx<float, kMode> &c, cons
     }
     r.ids(c, iv);
     window_maps(r, cc, gf, (Mob<float> *)iv.pmob + c.ip0,
-                (float *)iv.tent + 4 * thread_slot(iv, w), sc);
+                (float *)iv.tent + 4 * thread_slot(iv, w), (float *)S.warp);
+    if (w + 1 == c.wend_of[chunk]) {
+      leave_chunk<2>(S, chunk, f2d(bacc), racc);
+      bacc = 0;
+      racc = 0;
+      chunk++;
+    }
   }
-  __syncthreads();  // its scans' scratch is free for the next reduction
-  return make_double2((double)bacc, racc);
 }
 
 struct RefineX {
@@ -252,12 +296,12 @@ __device__ __noinline__ void refine_walk(const Ctx<float, kMode> &c, int pb) {
   });
 }
 
-// x += z by substitution, then the FP64 residual b - A x; returns the thread's part of
-// ||scale r||^2 in FP32 (see ph_residual).  kElim, the step's first cycle: x starts from the
+// x += z by substitution, then the FP64 residual b - A x; leaves the warps' parts of
+// ||scale r||^2, of FP32 sums per thread (see ph_residual).  kElim, the step's first cycle: x starts from the
 // initial guess, and r is eliminated into buffer pb of the pieces' values; else x is updated in
 // Vout and r stored (W_0).
 template <int kMode, bool kElim>
-__device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, double *Vout, float scale, int pb) {
+__device__ __noinline__ void refine_update(const Ctx<float, kMode> &c, double *Vout, float scale, int pb) {
   const ImView &iv = *c.iv;
   Shared S = carve(dyn_smem(), iv.m);
   const Walk<float> k = walk_of(c, iv, S);
@@ -266,7 +310,8 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, double *
   float *pval = (float *)iv.pval + 4 * ((int64_t)c.ip0 + (int64_t)pb * iv.npieces);
   double *pxb = (double *)iv.pxb + 2 * ((int64_t)c.ip0 + (int64_t)pb * iv.npieces);
   float acc = 0;
-  for (int w = first_window(c, iv); w < c.w1; w += window_stride(iv)) {
+  int chunk = 0;
+  for (int w = c.w0; w < c.w1; w++) {
     WinRows<float, kMode> r(c, iv, w);
     const int64_t rb = r.rb;
     float al[kRW] = {}, ee[kRW] = {}, inv[kRW] = {}, be[kRW] = {};
@@ -295,7 +340,7 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, double *
         M *= ee[u];
       }
     }
-    affine_enter<float, 1, false>(A, M, scz, y, r.idle, r.solo);
+    affine_enter<float, 1, false>(A, M, scz, y, r.idle, false);
     float cur = y[0];
 #pragma unroll
     for (int u = 0; u < kRW; u++) {
@@ -308,7 +353,7 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, double *
     }
     if (r.ok) st_rows(Vout + rb, x);
     double xm, xp;
-    window_ends(x, ends, xm, xp, r.solo);
+    window_ends(x, ends, xm, xp);
     // residual
     double rh[kRW] = {}, dg[kRW] = {}, g[kRW] = {}, gnext = 0;
     if (r.ok) {
@@ -355,9 +400,12 @@ __device__ __noinline__ float refine_update(const Ctx<float, kMode> &c, double *
     } else if (r.ok) {
       st_rows(c.w.Wb + rb, al);
     }
+    if (w + 1 == c.wend_of[chunk]) {
+      leave_chunk<1>(S, chunk, f2d(acc), 0.0);
+      acc = 0;
+      chunk++;
+    }
   }
-  __syncthreads();  // its scans' scratch is free for the next reduction
-  return acc;
 }
 
 }  // namespace nrt

@@ -48,3 +48,32 @@ def test_trees_that_reach_gmres_next_to_trees_that_do_not(gpu, pkg, model, shape
         if shape:  # one CTA per tree, as alone
             np.testing.assert_array_equal(V[q], alone[k][0][0])
             assert pc["basis"][q] == alone[k][1]["basis"][0]
+
+
+def test_a_tree_does_not_depend_on_its_company(gpu, pkg, model):
+    """The number of trees and the largest of them decide whether a tree has one CTA or a cluster of
+    2, 4 or 8, and how many CTAs an SM holds: the potential and the residual's norm that ends a step
+    are the same bits in all of them (windows and chunks of windows depend on the tree alone)."""
+    base = [model.random_tree(seed=80 + q, n_target=n, dt=2.5e-5, tspan=1e-3)
+            for q, n in enumerate((900, 1500, 2600, 9000, 30000))]
+    probs = [pkg.ProblemArrays.from_spec(sp, pkg.derive(sp)) for sp in base]
+    opts = dict(mode=1, precision="mixed", restart=20, tol=1e-10, tol_mode="rel")
+
+    def go(which, **shape):
+        b = pkg.Batch([probs[q] for q in which], **opts, **shape)
+        b.set_runs([(1, 1 + STEPS, base[q].init_time, base[q].end_input) for q in which])
+        b.advance(STEPS)
+        V, st = b.snapshot_all(), b.instance_stats()
+        b.close()
+        assert (st["nonconverged"] == 0).all()
+        return V, st["last_residual"]
+
+    ref, res = go(range(5), tile_ctas_per_sm=3)  # a CTA each
+    small = [0, 1, 2]
+    for which, shape in (([0, 1], {}), ([0, 2, 1], {}), (list(range(5)), {}), (list(range(5)) * 10, {}),
+                         (small * 30, {}), (small * 60, {}), (small * 170, {}),
+                         (list(range(5)), {"tile_ctas_per_sm": 4}), (list(range(5)), {"schedule": 1})):
+        V, r = go(which, **shape)
+        for k, q in enumerate(which):
+            np.testing.assert_array_equal(V[k], ref[q], err_msg=f"{len(which)} trees {shape}")
+            assert r[k] == res[q], (len(which), shape, k)

@@ -5,10 +5,12 @@
 
 #include <algorithm>
 #include <atomic>
+#include <exception>
 #include <memory>
-#include <utility>
 #include <string>
+#include <system_error>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "guard.h"
@@ -83,24 +85,36 @@ inline void set_window(InstDev &in) {
 }
 
 // Runs f(i) for every i in [0, n) on the host's cores, handing out indices one at a time
-// (instances differ in size by orders of magnitude).
+// (instances differ in size by orders of magnitude).  The first exception of a thread ends the loop
+// and is thrown again here, in the caller's thread.
 template <class F>
 void parallel_for(int64_t n, F f) {
   unsigned nt = std::thread::hardware_concurrency();
   nt = std::max(1u, std::min(nt, 64u));
   nt = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)nt, n));
   std::atomic<int64_t> next(0);
+  std::atomic<bool> failed(false);
+  std::exception_ptr error;
   auto work = [&]() {
-    for (;;) {
-      const int64_t i = next.fetch_add(1);
-      if (i >= n) break;
-      f(i);
+    try {
+      for (;;) {
+        const int64_t i = next.fetch_add(1);
+        if (i >= n || failed) break;
+        f(i);
+      }
+    } catch (...) {
+      if (!failed.exchange(true)) error = std::current_exception();
     }
   };
   std::vector<std::thread> th;
-  for (unsigned t = 1; t < nt; t++) th.emplace_back(work);
+  th.reserve(nt);
+  try {
+    for (unsigned t = 1; t < nt; t++) th.emplace_back(work);
+  } catch (const std::system_error &) {  // no more threads: with those there are
+  }
   work();
   for (std::thread &t : th) t.join();
+  if (error) std::rethrow_exception(error);
 }
 
 // f(a, b) over [0, n) in chunks of about 1M.

@@ -499,16 +499,12 @@ int Engine::init(const nrt_problem *probs, int32_t count, const nrt_options *o) 
   return NRT_OK;
 }
 
-// The plan of several explicit steps per launch, its device copy and the second gate buffer:
-// made when a time loop, a recording or a strain first needs it (the drop-in's update() and
-// calculate() never do).
-// Without the memory for them (or with a tree that does not tile) the time loop takes one
-// launch per step, as it does when the options name a shape of the per-step kernels other
-// than the staged tiles.
+// The plan of several explicit steps per launch, its device copy and the second gate buffer: made
+// by the time loop once the steps asked for are worth it.  Without the memory for them (or with a
+// tree that does not tile) the time loop takes one launch per step, as it does when the options name
+// a shape of the per-step kernels other than the staged tiles.
 int Engine::block_init() {
-  if (block_tried || opt.mode != NRT_EXPLICIT) return NRT_OK;
   block_tried = true;
-  if (!host.fusable || opt.tiled == 0 || opt.step_threads > 0 || opt.step_launch != 0) return NRT_OK;
   BlockPlan plan;
   const bool mixed = opt.precision == NRT_MIXED;
   const size_t gate_bytes = (mixed ? 12 : 24) * (size_t)host.ntot;
@@ -540,12 +536,15 @@ int Engine::block_init() {
   bv.lanes = plan.lanes;
   bv.ntiles = (int)plan.tile.size();
   btile.swap(plan.tile);
-  return NRT_OK;
+  TRY(block_probes());
+  return block_strain();
 }
 
-// The probes of each tile (src: the element each recording slot reads).
-int Engine::block_probes(const std::vector<int64_t> *src) {
+// The probes of each tile.  Without the memory for them the time loop keeps to one launch per step
+// while this recording lasts.
+int Engine::block_probes() {
   if (bv.ntiles == 0) return NRT_OK;
+  const std::vector<int64_t> *src = record_sources();
   NRT_CUDA(cudaStreamSynchronize(stream));
   if (probe_mem) cudaFree(probe_mem);
   probe_mem = nullptr;
@@ -571,7 +570,12 @@ int Engine::block_probes(const std::vector<int64_t> *src) {
       bv.max_probes = std::max(bv.max_probes, t.p1 - t.p0);
       list.push_back(make_int2((int)((*src)[at[q].second] - t.s), at[q].second));
     }
-    NRT_CUDA(cudaMalloc(&probe_mem, sizeof(int2) * list.size()));
+    if (cudaMalloc(&probe_mem, sizeof(int2) * list.size()) != cudaSuccess) {
+      cudaGetLastError();
+      probe_mem = nullptr;
+      bv.max_probes = kTooManyProbes;
+      return NRT_OK;
+    }
     NRT_CUDA(cudaMemcpyAsync(probe_mem, list.data(), sizeof(int2) * list.size(),
                              cudaMemcpyHostToDevice, stream));
     bv.probe = (const int2 *)probe_mem;
@@ -794,15 +798,18 @@ bool Engine::chunk_kernel() const {
   return !strain || strain_tabled(*this);
 }
 
-// Whether `left` steps run several per launch.  Not the shortest calls (the last step is a
-// launch of its own anyway), and in mixed precision not up to two chunks of a pack of fewer than kBlockMinElems
-// elements: there the documented form, a launch per step, stays (callers can count on the launch
-// counter, and the whole call saves less than half a millisecond).
-bool Engine::use_blocks(int64_t left) const {
+// Whether a call of `left` steps takes several per launch when there is a plan.  Not the shortest
+// calls (the last step is a launch of its own anyway), and in mixed precision not up to two chunks of
+// a pack of fewer than kBlockMinElems elements: such calls keep a launch per step, which is what the
+// launch counter reports for them (128 steps of a 3000-compartment tree 0.5 ms, 0.2 with a plan).
+bool Engine::block_call(int64_t left) const {
   constexpr int64_t kBlockMinElems = 8192;
+  if (opt.mode != NRT_EXPLICIT || !host.fusable || opt.tiled == 0 || opt.step_threads > 0 ||
+      opt.step_launch != 0)
+    return false;
   // (a tile's probes hold 8 bytes per step each in shared memory)
   const bool mixed = opt.precision == NRT_MIXED;
-  return left > 2 && bv.ntiles > 0 && (!strain || (mixed && strain_tabled(*this))) &&
+  return left > 2 && (!strain || (mixed && strain_tabled(*this))) &&
          8 * (int64_t)bv.max_probes * bv.depth <= 24 * 1024 &&
          (!mixed || host.ntot >= kBlockMinElems || left > 2 * kChunk);
 }
@@ -813,11 +820,11 @@ bool Engine::use_blocks(int64_t left) const {
 int Engine::advance(int64_t steps) {
   if (opt.mode == NRT_IMPLICIT_BE) return implicit_advance(*this, steps);
   int64_t left = steps;
-  // The plan of the several-step launches takes as long as they save in about 100 steps (0.35 ms on a
-  // small tree at 3 us a step, 9 ms on 1024 trees at 0.14 ms): it is built when the handle has
-  // been asked for more.
-  constexpr int64_t kPlanSteps = 128;
-  if (left > 2 && !block_tried && (asked_steps += left) >= kPlanSteps) TRY(block_init());
+  // the plan of the several-step launches, once the calls that would use it have asked for enough
+  if (!block_tried && block_call(left)) {
+    asked_steps += left;
+    if (block_plan_pays(host, pv, opt.precision == NRT_MIXED, asked_steps)) TRY(block_init());
+  }
   while (left > 0 && needs_general()) {  // exact first step
     if (strain) TRY(launch_strain_update(*this, 0, stream));
     TRY(step(0, -1));

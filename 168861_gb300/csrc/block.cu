@@ -476,42 +476,55 @@ static void block_shape(const PackView &pv, int &depth, int &cap) {
 }
 
 static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan &plan);
+static bool sample_plan(const HostPack &host, int depth, int cap, double &local);
 
 // Estimated microseconds per step of a plan, and of the per-step kernels: a launch boundary and
 // the elements' share (measured on 5.4 and 22 million compartments: 9 to 11 ps per local
 // element, 14.5 ps per element one step at a time; small packs 4.6 us per launch).
-static double block_cost(const BlockPlan &P) {
+static double block_cost(int depth, double local) { return 4.0 / depth + 1e-5 * local; }
+static double local_elements(const BlockPlan &P) {
   double local = 0;
   for (const BlockTile &t : P.tile) local += t.cnt + t.nh;
-  return 4.0 / P.depth + 1e-5 * local;
+  return local;
 }
 
 // FP64 shapes, by estimated microseconds per step: a launch boundary of 3 us, 1.3 us per round of
 // 16 eight-lane elements on an SM and 3.8 us per round of 128 one-thread ones (39 and 115
 // operations of 64 cycles), against the per-step kernels' 3.3 us and the same rounds without
 // halos.  Above a million elements the launch boundary is nothing to the rounds.
+struct F64Shape {
+  int lanes, depth, cap;
+};
+constexpr F64Shape kF64Shapes[] = {{8, 4, 16}, {8, 4, 32}, {1, 8, 128}, {1, 4, 128}, {1, 4, 256}, {1, 2, 256}};
+constexpr int64_t kF64MaxElems = 1000000;
+
+static double f64_rounds(int64_t local, int lanes, int64_t sms) {
+  const double per = lanes == 8 ? 16.0 : 128.0, x = (double)local / (double)sms / per;
+  return (lanes == 8 ? 1.3 : 3.8) * (x < 4 ? std::max(1.0, std::ceil(x - 0.05)) : x);
+}
+static double f64_single_cost(int64_t N, const PackView &pv) {
+  const int64_t sms = pv.sms > 0 ? pv.sms : 1;
+  return 3.3 + std::min(f64_rounds(N, 1, sms), N <= 8192 ? f64_rounds(N, 8, sms) : 1e30);
+}
+static double f64_cost(const F64Shape &s, int64_t tiles, const PackView &pv) {
+  const int64_t sms = pv.sms > 0 ? pv.sms : 1;
+  // whole tiles go to an SM, so the fullest SM holds ceil(tiles / SMs) of them
+  return 3.0 / s.depth + f64_rounds((tiles + sms - 1) / sms * s.cap * sms, s.lanes, sms);
+}
+
 static bool choose_f64(const HostPack &host, const PackView &pv, BlockPlan &plan) {
-  const int64_t N = host.ntot, sms = pv.sms > 0 ? pv.sms : 1;
-  if (N > 1000000) return false;
-  auto rounds = [&](int64_t local, int lanes) {
-    const double per = lanes == 8 ? 16.0 : 128.0, x = (double)local / (double)sms / per;
-    return (lanes == 8 ? 1.3 : 3.8) * (x < 4 ? std::max(1.0, std::ceil(x - 0.05)) : x);
-  };
-  double best = 3.3 + std::min(rounds(N, 1), N <= 8192 ? rounds(N, 8) : 1e30);
+  const int64_t N = host.ntot;
+  if (N > kF64MaxElems) return false;
+  double best = f64_single_cost(N, pv);
   bool found = false;
-  const struct { int lanes, depth, cap; } shapes[] = {{8, 4, 16}, {8, 4, 32}, {1, 8, 128}, {1, 4, 128}, {1, 4, 256}, {1, 2, 256}};
-  for (const auto &s : shapes) {
+  for (const F64Shape &s : kF64Shapes) {
     const int own = s.cap - 2 * s.depth;  // at best: a cable
-    const int64_t tiles = (N + own - 1) / own;
-    auto cost = [&](int64_t n_tiles) {
-      // whole tiles go to an SM, so the fullest SM holds ceil(tiles / SMs) of them
-      return 3.0 / s.depth + rounds((n_tiles + sms - 1) / sms * s.cap * sms, s.lanes);
-    };
-    if (cost(tiles) >= best) continue;
+    if (f64_cost(s, (N + own - 1) / own, pv) >= best) continue;
     BlockPlan P;
     if (!build_block_plan(host, s.depth, s.cap, P)) continue;
-    if (cost((int64_t)P.tile.size()) >= best) continue;
-    best = cost((int64_t)P.tile.size());
+    const double cost = f64_cost(s, (int64_t)P.tile.size(), pv);
+    if (cost >= best) continue;
+    best = cost;
     P.lanes = s.lanes;
     plan = std::move(P);
     found = true;
@@ -524,17 +537,17 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
   int depth = 0, cap = 0;
   block_shape(pv, depth, cap);
   const int largest = pv.hh_dense ? 512 : 256;
-  double best = 4.6 + 1.45e-5 * (double)host.ntot;
-  bool found = false;
+  const double single = 4.6 + 1.45e-5 * (double)host.ntot;
+  struct Shape {
+    double cost;
+    int depth, cap;
+  };
+  std::vector<Shape> shapes;
   for (int d = depth, c = cap; d >= 2;) {
-    BlockPlan P;
-    const bool ok = build_block_plan(host, d, c, P);
-    const double cost = ok ? block_cost(P) : 0.0;
-    if (ok && cost < best) {
-      best = cost;
-      plan = std::move(P);
-      found = true;
-    }
+    double local = 0;
+    const bool ok = sample_plan(host, d, c, local);
+    const double cost = block_cost(d, local);
+    if (ok && cost < single) shapes.push_back(Shape{cost, d, c});
     // good as it is: the halos are below a third
     if (ok && cost < 4.0 / d + 1.33e-5 * (double)host.ntot) break;
     if (c < largest)
@@ -542,20 +555,56 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
     else
       d /= 2;
   }
-  return found;
+  std::stable_sort(shapes.begin(), shapes.end(), [](const Shape &a, const Shape &b) { return a.cost < b.cost; });
+  for (const Shape &x : shapes) {  // nearly always the first
+    BlockPlan P;
+    if (!build_block_plan(host, x.depth, x.cap, P) || block_cost(x.depth, local_elements(P)) >= single) continue;
+    plan = std::move(P);
+    return true;
+  }
+  return false;
 }
 
-// Tiles of at most `cap` local elements for `depth` steps per launch; false when some tile
-// would hold fewer than a quarter of its elements itself (a dense tangle of branches).
-static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan &plan) {
-  plan.depth = depth;
-  plan.cap = cap;
-  // elements tiled by one host thread at a time
-  const int64_t N = host.ntot,
-                chunk = std::min<int64_t>(1 << 16, std::max<int64_t>(1 << 14, N / 64));
-  const int64_t nc = (N + chunk - 1) / chunk;
-  std::vector<BlockPlan> part(nc);
-  std::vector<char> ok(nc, 1);
+// Whether `steps` steps are worth a plan: what they would save, against the plan's making.  Both are
+// estimates from what was measured (16 host cores, a first call on a fresh handle):
+//  - making: 0.1 ms (allocation, upload, the second gate buffer) and per host thread 0.6 us for each
+//    terminal (the elements around a branch are searched again for every tile) and 5 ns for each
+//    element: 0.12 ms for a 10,000-element tree, 0.6 ms for 24 bushy trees (102,815 elements, 4,400
+//    terminals), 9 ms for 1024 trees (22 million);
+//  - saved per step, mixed: 4.0 us per launch or 14.5 ps per element, whichever is more, becomes 2 us
+//    per depth and 8 ps per local element (102,815 elements 4.5 -> 1.2 us, a million 14.5 -> 7.9);
+//    FP64: half of what choose_f64's estimates say (a 1 cm axon 3.7 -> 2.7 us, 10,000 elements 6.8 ->
+//    5.4).
+// With 128 steps for every pack, the 24 trees' first call of 128 steps took 1.28 ms instead of 0.82.
+bool block_plan_pays(const HostPack &host, const PackView &pv, bool mixed, int64_t steps) {
+  const double N = (double)host.ntot;
+  const double chunks = std::ceil(N / (1 << 14)), cores = std::max(1u, std::thread::hardware_concurrency());
+  const double making =
+      100.0 + (0.6 * (double)host.terms.size() + 0.005 * N) / std::min(std::min(cores, 64.0), chunks);
+  double saved;
+  if (mixed) {
+    int depth = 0, cap = 0;
+    block_shape(pv, depth, cap);
+    saved = std::max(4.0, 1.45e-5 * N) - (2.0 / depth + 8e-6 * 1.15 * N);
+  } else {
+    double best = f64_single_cost(host.ntot, pv);
+    const double single = best;
+    for (const F64Shape &s : kF64Shapes) {
+      const int64_t own = s.cap - 2 * s.depth;
+      best = std::min(best, f64_cost(s, (host.ntot + own - 1) / own, pv));
+    }
+    saved = host.ntot > kF64MaxElems ? 0.0 : 0.5 * (single - best);
+  }
+  return saved > 0 && (double)steps * saved >= making;
+}
+
+// The plan of elements [c0, c1) (local entries h0, x0 count from P's own lists); false when some
+// tile would hold fewer than a quarter of its elements itself (a dense tangle of branches).
+static bool tile_range(const HostPack &host, int depth, int cap, int64_t c0, int64_t c1, BlockPlan &P) {
+  struct H {
+    int64_t g;
+    int dist;
+  };
   // what element j's step reads besides its own state, -1 where it reads nothing
   auto deps = [&](int64_t j, int64_t (&d)[3]) {
     const Topo &t = host.topo[j];
@@ -568,105 +617,139 @@ static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan
     if (!(t.flags & F_DR_TERM)) d[1] = t.dr;
     if ((t.flags & F_BRANCH) && !(t.flags & F_DL_TERM)) d[2] = t.dl;
   };
-  parallel_for(nc, [&](int64_t c) {
-    BlockPlan &P = part[c];
-    const int64_t end = std::min(N, (c + 1) * chunk);
-    struct H {
-      int64_t g;
-      int dist;
+  // the elements with a neighbour that is not j - 1 or j + 1: with the two ends of a tile the only
+  // ones whose step can read outside it
+  std::vector<int64_t> far;
+  for (int64_t j = c0; j < c1; j++)
+    if (host.topo[j].flags & F_XTOPO) far.push_back(j);
+  std::vector<H> halo;
+  std::vector<int64_t> key(4096, -1);  // open-addressing map: element -> local index
+  std::vector<int> val(4096);
+  std::vector<size_t> used;
+  auto slot = [&](int64_t g) {
+    size_t h = (size_t)(g * 0x9E3779B97F4A7C15ull >> 40) & 4095;
+    while (key[h] >= 0 && key[h] != g) h = (h + 1) & 4095;
+    return h;
+  };
+  int64_t s = c0;
+  size_t f0 = 0;                   // the first of `far` at or after s
+  int64_t want = cap - 2 * depth;  // then what the last tile held and a little more
+  while (s < c1) {
+    int64_t cnt = std::min(want, c1 - s);
+    int64_t d[3];
+    // f(j) for the tile's elements that may read outside it, in ascending order
+    auto each = [&](auto f) {
+      size_t q = f0;
+      if (q == far.size() || far[q] != s) f(s);
+      for (; q < far.size() && far[q] < s + cnt; q++) f(far[q]);
+      if (cnt > 1 && (q == f0 || far[q - 1] != s + cnt - 1)) f(s + cnt - 1);
     };
-    std::vector<H> halo;
-    std::vector<int64_t> key;  // open-addressing map: element -> local index
-    std::vector<int> val;
-    std::vector<size_t> used;
-    key.assign(4096, -1);
-    val.resize(4096);
-    auto slot = [&](int64_t g) {
-      size_t h = (size_t)(g * 0x9E3779B97F4A7C15ull >> 40) & 4095;
-      while (key[h] >= 0 && key[h] != g) h = (h + 1) & 4095;
-      return h;
-    };
-    int64_t s = c * chunk;
-    int64_t want = cap - 2 * depth;  // then what the last tile held and a little more
-    while (s < end) {
-      int64_t cnt = std::min(want, end - s);
-      int64_t d[3];
-      bool fits = false;
-      while (!fits) {
-        for (size_t q : used) key[q] = -1;
-        used.clear();
-        halo.clear();
-        bool full = false;
-        auto add = [&](int64_t g, int dist) {
-          if (g < 0 || (g >= s && g < s + cnt)) return;
-          const size_t h = slot(g);
-          if (key[h] == g) return;
-          if (cnt + (int64_t)halo.size() >= cap) {
-            full = true;
-            return;
-          }
-          key[h] = g;
-          used.push_back(h);
-          val[h] = (int)(cnt + (int64_t)halo.size());
-          halo.push_back(H{g, dist});
-        };
-        for (int64_t j = s; j < s + cnt && !full; j++) {
-          if (!(host.topo[j].flags & F_XTOPO) && j != s && j != s + cnt - 1) continue;
-          deps(j, d);
-          for (int64_t g : d) add(g, 1);
-        }
-        for (size_t q = 0; q < halo.size() && !full; q++) {
-          if (halo[q].dist >= depth) break;  // sorted by distance
-          deps(halo[q].g, d);
-          for (int64_t g : d) add(g, halo[q].dist + 1);
-        }
-        fits = !full;
-        if (!fits) {
-          cnt -= std::max<int64_t>(depth, cnt / 16);
-          if (cnt < std::max(1, cap / 4)) {
-            ok[c] = 0;
-            return;
-          }
-        }
-      }
-      auto local = [&](int64_t g, int self) -> int {
-        if (g < 0) return self;
-        if (g >= s && g < s + cnt) return (int)(g - s);
+    for (bool fits = false; !fits;) {
+      for (size_t q : used) key[q] = -1;
+      used.clear();
+      halo.clear();
+      bool full = false;
+      auto add = [&](int64_t g, int dist) {
+        if (g < 0 || (g >= s && g < s + cnt)) return;
         const size_t h = slot(g);
-        return key[h] == g ? val[h] : self;
-      };
-      BlockTile t{};
-      t.s = (int32_t)s;
-      t.cnt = (int32_t)cnt;
-      t.nh = (int32_t)halo.size();
-      t.h0 = (int32_t)P.halo.size();
-      t.x0 = (int32_t)P.spec.size();
-      for (int64_t j = s; j < s + cnt; j++) {
-        if (!(host.topo[j].flags & F_XTOPO) && j != s && j != s + cnt - 1) continue;
-        const int l = (int)(j - s);
-        deps(j, d);
-        P.spec.push_back(make_ushort4((unsigned short)l, (unsigned short)local(d[0], l),
-                                      (unsigned short)local(d[1], l), (unsigned short)local(d[2], l)));
-      }
-      t.nx = (int32_t)P.spec.size() - t.x0;
-      for (size_t q = 0; q < halo.size(); q++) {
-        const int l = (int)(cnt + (int64_t)q);
-        int nbr[3] = {l, l, l};
-        if (halo[q].dist < depth) {
-          deps(halo[q].g, d);
-          for (int u = 0; u < 3; u++) nbr[u] = local(d[u], l);
+        if (key[h] == g) return;
+        if (cnt + (int64_t)halo.size() >= cap) {
+          full = true;
+          return;
         }
-        P.halo.push_back(make_int4((int)halo[q].g, nbr[0] | (nbr[1] << 16),
-                                   nbr[2] | (halo[q].dist << 16), 0));
+        key[h] = g;
+        used.push_back(h);
+        val[h] = (int)(cnt + (int64_t)halo.size());
+        halo.push_back(H{g, dist});
+      };
+      each([&](int64_t j) {
+        if (full) return;
+        deps(j, d);
+        for (int64_t g : d) add(g, 1);
+      });
+      for (size_t q = 0; q < halo.size() && !full; q++) {
+        if (halo[q].dist >= depth) break;  // sorted by distance
+        deps(halo[q].g, d);
+        for (int64_t g : d) add(g, halo[q].dist + 1);
       }
-      P.tile.push_back(t);
-      s += cnt;
-      want = std::min<int64_t>(cap - 2 * depth, cnt + std::max(depth, cap / 32));
+      fits = !full;
+      if (!fits) {
+        cnt -= std::max<int64_t>(depth, cnt / 16);
+        if (cnt < std::max(1, cap / 4)) return false;
+      }
     }
+    auto local = [&](int64_t g, int self) -> int {
+      if (g < 0) return self;
+      if (g >= s && g < s + cnt) return (int)(g - s);
+      const size_t h = slot(g);
+      return key[h] == g ? val[h] : self;
+    };
+    BlockTile t{};
+    t.s = (int32_t)s;
+    t.cnt = (int32_t)cnt;
+    t.nh = (int32_t)halo.size();
+    t.h0 = (int32_t)P.halo.size();
+    t.x0 = (int32_t)P.spec.size();
+    each([&](int64_t j) {
+      const int l = (int)(j - s);
+      deps(j, d);
+      P.spec.push_back(make_ushort4((unsigned short)l, (unsigned short)local(d[0], l),
+                                    (unsigned short)local(d[1], l), (unsigned short)local(d[2], l)));
+    });
+    t.nx = (int32_t)P.spec.size() - t.x0;
+    for (size_t q = 0; q < halo.size(); q++) {
+      const int l = (int)(cnt + (int64_t)q);
+      int nbr[3] = {l, l, l};
+      if (halo[q].dist < depth) {
+        deps(halo[q].g, d);
+        for (int u = 0; u < 3; u++) nbr[u] = local(d[u], l);
+      }
+      P.halo.push_back(make_int4((int)halo[q].g, nbr[0] | (nbr[1] << 16), nbr[2] | (halo[q].dist << 16), 0));
+    }
+    P.tile.push_back(t);
+    s += cnt;
+    while (f0 < far.size() && far[f0] < s) f0++;
+    want = std::min<int64_t>(cap - 2 * depth, cnt + std::max(depth, cap / 32));
+  }
+  return true;
+}
+
+// The local elements (owned and halo) that a plan would have, from tiles of up to four stretches of
+// the pack; false when one of them does not tile.  A whole plan that is then not taken costs as much
+// as the one that is: of 24 bushy trees (100,000 elements) 0.6 ms each.
+static bool sample_plan(const HostPack &host, int depth, int cap, double &local) {
+  const int64_t N = host.ntot, span = 4096, n = std::min<int64_t>(4, (N + span - 1) / span);
+  double sum[4] = {0, 0, 0, 0}, seen[4] = {0, 0, 0, 0};
+  std::atomic<bool> tangle(false);
+  parallel_for(n, [&](int64_t q) {
+    const int64_t a = n * span >= N ? q * span : (N - span) * q / (n - 1), b = std::min(N, a + span);
+    BlockPlan P;
+    if (tangle) return;
+    if (!tile_range(host, depth, cap, a, b, P)) tangle = true;
+    sum[q] = local_elements(P);
+    seen[q] = (double)(b - a);
   });
+  if (tangle) return false;
+  local = (sum[0] + sum[1] + sum[2] + sum[3]) * (double)N / (seen[0] + seen[1] + seen[2] + seen[3]);
+  return true;
+}
+
+// Tiles of at most `cap` local elements for `depth` steps per launch; false where tile_range says
+// so.  Ranges of elements are tiled by one host thread each.
+static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan &plan) {
+  plan.depth = depth;
+  plan.cap = cap;
+  const int64_t N = host.ntot, chunk = std::min<int64_t>(1 << 16, std::max<int64_t>(1 << 14, N / 64));
+  const int64_t nc = (N + chunk - 1) / chunk;
+  std::vector<BlockPlan> part(nc);
+  std::atomic<bool> tangle(false);
+  parallel_for(nc, [&](int64_t c) {
+    if (tangle) return;
+    if (!tile_range(host, depth, cap, c * chunk, std::min(N, (c + 1) * chunk), part[c])) tangle = true;
+  });
+  if (tangle) return false;
   size_t nt = 0, nh = 0, nx = 0;
   for (int64_t c = 0; c < nc; c++) {
-    if (!ok[c]) return false;
     nt += part[c].tile.size();
     nh += part[c].halo.size();
     nx += part[c].spec.size();

@@ -41,6 +41,9 @@ struct BlockPlan {
 // The plan expected to be fastest; false when one launch per step is.
 bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, BlockPlan &plan);
 
+// Whether `steps` steps save more than making a plan takes.
+bool block_plan_pays(const HostPack &host, const PackView &pv, bool mixed, int64_t steps);
+
 struct StrainView;
 // nk (<= depth) steps from loop index base + k0: V and its FP32 shadow from Vin to Vout / Fout,
 // gates from gin to gout.  r.nprobe > 0: the tiles' probes record after every step.  s.n > 0:

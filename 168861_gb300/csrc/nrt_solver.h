@@ -7,6 +7,7 @@
 namespace nrt {
 
 constexpr int kChunk = 64;        // steps per captured graph (even: buffer parity returns)
+constexpr int kTooManyProbes = 1 << 20;  // in one explicit tile: more than its shared memory holds
 constexpr int kMaxRestart = 32;   // GMRES restart limit (dot accumulators live in registers)
 
 struct Arena {
@@ -46,7 +47,7 @@ struct Engine {
   // several explicit steps per launch (block.cu), or bv.ntiles == 0
   BlockView bv{};
   bool block_tried = false;               // block_init has run
-  int64_t asked_steps = 0;                // steps asked for before it, in calls of several
+  int64_t asked_steps = 0;                // steps asked for before it, in calls that would use it
   std::vector<BlockTile> btile;           // host copy of the tiles
   void *block_mem = nullptr, *probe_mem = nullptr;
   void *gate2[2] = {nullptr, nullptr};    // the two gate buffers; the pack's is gate2[gcur]
@@ -60,9 +61,13 @@ struct Engine {
   int advance(int64_t steps);
   bool chunk_kernel() const;  // explicit time loops run a chunk of steps per launch
   int block_init();
-  int block_probes(const std::vector<int64_t> *src);  // null: no recording
+  int block_probes();                // the recording's probes by tile (none without one)
+  int block_strain();                // the strained elements' classes
   int block_steps(int k0, int nk);   // launches for nk steps from loop index base + k0
-  bool use_blocks(int64_t left) const;
+  bool block_call(int64_t left) const;  // a call of `left` steps would use the plan
+  bool use_blocks(int64_t left) const {
+    return bv.ntiles > 0 && block_call(left) && (!strain || bv.scls);
+  }
   int block_advance(int64_t left);
   void drop_graphs();                // the time loop's captured graphs are stale
   int fixup();
@@ -82,6 +87,7 @@ struct Engine {
                   double *spike_times);
   const RecView *record_view() const;  // device copy for the implicit kernel, or null
   const RecView &rec_view_host() const;  // host copy (device pointers) for kernel arguments
+  const std::vector<int64_t> *record_sources() const;  // element read per slot, or null
   int upload_and_init(RecState *R, const std::vector<int64_t> &src,
                       const std::vector<int64_t> &raw, const std::vector<int32_t> &sinst,
                       const std::vector<int32_t> &p0);

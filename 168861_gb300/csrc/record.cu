@@ -50,6 +50,7 @@ struct RecState {
   int64_t *d_raw = nullptr;    // each probe's own element (initial values)
   std::vector<int32_t> order;  // sorted slot -> configuration index
   std::vector<int32_t> inst;   // instance per sorted slot
+  std::vector<int64_t> src;    // element read per sorted slot
   ~RecState() {
     if (mem) cudaFree(mem);
   }
@@ -64,6 +65,7 @@ int launch_record_step(const RecView &r, const InstDev *inst, int k, const doubl
 
 const RecView *Engine::record_view() const { return rec ? rec->d_view : nullptr; }
 const RecView &Engine::rec_view_host() const { return rec->view; }
+const std::vector<int64_t> *Engine::record_sources() const { return rec ? &rec->src : nullptr; }
 
 void Engine::record_release() {
   delete rec;
@@ -100,8 +102,7 @@ int Engine::record_config(const nrt_record_config *c) {
   drop_graphs();
   record_release();
   {
-    int rc = P > 0 ? block_init() : NRT_OK;
-    if (rc == NRT_OK) rc = block_probes(nullptr);
+    const int rc = block_probes();
     if (rc) return rc;
   }
   if (P == 0) return NRT_OK;
@@ -173,14 +174,17 @@ int Engine::record_config(const nrt_record_config *c) {
   v.spk = (double *)take(8 * (size_t)P * (size_t)std::max<int64_t>(ms, 1));
   // installed only once complete: a failed call leaves no recording behind
   int rc = upload_and_init(R, src, raw, sinst, p0);
-  if (rc == NRT_OK) rc = block_probes(&src);
+  R->src.swap(src);
+  if (rc == NRT_OK) {
+    rec = R;
+    rc = block_probes();
+    if (rc) rec = nullptr;
+  }
   if (rc) {
     cudaStreamSynchronize(stream);
     delete R;
-    return rc;
   }
-  rec = R;
-  return NRT_OK;
+  return rc;
 }
 
 int Engine::upload_and_init(RecState *R, const std::vector<int64_t> &src,

@@ -24,8 +24,13 @@ namespace nrt {
 struct StrainState {
   void *mem = nullptr;
   StrainView view{};
+  // host copies for the tiles of several steps per launch, and each element's class there
+  std::vector<int64_t> elem;
+  std::vector<int32_t> cls;
+  void *scls = nullptr;
   ~StrainState() {
     if (mem) cudaFree(mem);
+    if (scls) cudaFree(scls);
   }
 };
 
@@ -200,10 +205,6 @@ int Engine::strain_config(const nrt_strain_config *c) {
   drop_graphs();  // the time loop gains (or loses) launches
   strain_release();
   if (n == 0) return NRT_OK;
-  {
-    const int rc = block_init();
-    if (rc) return rc;
-  }
   std::unique_ptr<StrainState> S(new (std::nothrow) StrainState());
   if (!S) {
     set_error("host allocation");
@@ -309,12 +310,9 @@ int Engine::strain_config(const nrt_strain_config *c) {
   const bool alt = tabled && mixed;
   auto rnd = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t fold_bytes = alt ? 4 * rnd(4 * (size_t)N) + rnd(48 * (size_t)pv.hp_ld) : 0;
-  // several steps per launch: each element's class (block.cu)
-  const bool classes = tabled && bv.ntiles > 0;
   const size_t bytes = 8 * (size_t)n * 2 + 4 * (size_t)n + 4 * (size_t)ncls * 2 +
                        8 * c_spec.size() +
-                       (tabled ? tab_entries * (8 * kStrainOut + 4) : 0) + fold_bytes + 256 * 8 +
-                       (classes ? rnd(4 * (size_t)N) : 0);
+                       (tabled ? tab_entries * (8 * kStrainOut + 4) : 0) + fold_bytes + 256 * 8;
   if (cudaMalloc(&S->mem, bytes) != cudaSuccess) {
     cudaGetLastError();
     set_error("device allocation for the strain");
@@ -338,13 +336,6 @@ int Engine::strain_config(const nrt_strain_config *c) {
   v.alt_wdxf = alt ? (float *)take(4 * (size_t)N) : nullptr;
   v.alt_kdxf = alt ? (float *)take(4 * (size_t)N) : nullptr;
   v.alt_hpq = alt ? (float4 *)take(48 * (size_t)pv.hp_ld) : nullptr;
-  int32_t *d_scls = classes ? (int32_t *)take(4 * (size_t)N) : nullptr;
-  hvec<int32_t> scls(classes ? N : 0);
-  if (classes) {
-    std::fill(scls.begin(), scls.end(), 0);
-    for (int32_t r = 0; r < n; r++) scls[s_elem[r]] = s_cls[r] + 1;
-    NRT_CUDA(cudaMemcpyAsync(d_scls, scls.data(), 4 * (size_t)N, cudaMemcpyHostToDevice, stream));
-  }
   NRT_CUDA(cudaMemcpyAsync(d_elem, s_elem.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, stream));
   NRT_CUDA(cudaMemcpyAsync(d_col, s_col.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, stream));
   NRT_CUDA(cudaMemcpyAsync(d_cls, s_cls.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, stream));
@@ -378,9 +369,31 @@ int Engine::strain_config(const nrt_strain_config *c) {
     NRT_CUDA(cudaMemcpyAsync(v.alt_hpq, pv.hpq, 48 * (size_t)pv.hp_ld, d2d, stream));
   }
   NRT_CUDA(cudaStreamSynchronize(stream));
-  bv.scls = d_scls;
-  bv.rows = 4 * (size_t)bv.depth * ncls * kStrainOut <= 8 * 1024;
+  S->elem.swap(s_elem);
+  S->cls.swap(s_cls);
   strain = S.release();
+  const int rc = block_strain();
+  if (rc) strain_release();
+  return rc;
+}
+
+// Several steps per launch (block.cu): each element's class + 1, 0 where it is not strained.  Without
+// the memory for them the time loop keeps to one launch per step while this strain lasts.
+int Engine::block_strain() {
+  if (bv.ntiles == 0 || !strain_tabled(*this) || opt.precision != NRT_MIXED) return NRT_OK;
+  StrainState &S = *strain;
+  const size_t bytes = 4 * (size_t)host.ntot;
+  if (!S.scls && cudaMalloc(&S.scls, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    S.scls = nullptr;
+    return NRT_OK;
+  }
+  std::vector<int32_t> scls(host.ntot, 0);
+  for (size_t r = 0; r < S.elem.size(); r++) scls[S.elem[r]] = S.cls[r] + 1;
+  NRT_CUDA(cudaMemcpyAsync(S.scls, scls.data(), bytes, cudaMemcpyHostToDevice, stream));
+  NRT_CUDA(cudaStreamSynchronize(stream));
+  bv.scls = (const int32_t *)S.scls;
+  bv.rows = 4 * (size_t)bv.depth * S.view.ncls * kStrainOut <= 8 * 1024;
   return NRT_OK;
 }
 

@@ -476,16 +476,14 @@ static void block_shape(const PackView &pv, int &depth, int &cap) {
 }
 
 static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan &plan);
-static bool sample_plan(const HostPack &host, int depth, int cap, double &local);
 
 // Estimated microseconds per step of a plan, and of the per-step kernels: a launch boundary and
 // the elements' share (measured on 5.4 and 22 million compartments: 9 to 11 ps per local
 // element, 14.5 ps per element one step at a time; small packs 4.6 us per launch).
-static double block_cost(int depth, double local) { return 4.0 / depth + 1e-5 * local; }
-static double local_elements(const BlockPlan &P) {
+static double block_cost(const BlockPlan &P) {
   double local = 0;
   for (const BlockTile &t : P.tile) local += t.cnt + t.nh;
-  return local;
+  return 4.0 / P.depth + 1e-5 * local;
 }
 
 // FP64 shapes, by estimated microseconds per step: a launch boundary of 3 us, 1.3 us per round of
@@ -537,17 +535,17 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
   int depth = 0, cap = 0;
   block_shape(pv, depth, cap);
   const int largest = pv.hh_dense ? 512 : 256;
-  const double single = 4.6 + 1.45e-5 * (double)host.ntot;
-  struct Shape {
-    double cost;
-    int depth, cap;
-  };
-  std::vector<Shape> shapes;
+  double best = 4.6 + 1.45e-5 * (double)host.ntot;
+  bool found = false;
   for (int d = depth, c = cap; d >= 2;) {
-    double local = 0;
-    const bool ok = sample_plan(host, d, c, local);
-    const double cost = block_cost(d, local);
-    if (ok && cost < single) shapes.push_back(Shape{cost, d, c});
+    BlockPlan P;
+    const bool ok = build_block_plan(host, d, c, P);
+    const double cost = ok ? block_cost(P) : 0.0;
+    if (ok && cost < best) {
+      best = cost;
+      plan = std::move(P);
+      found = true;
+    }
     // good as it is: the halos are below a third
     if (ok && cost < 4.0 / d + 1.33e-5 * (double)host.ntot) break;
     if (c < largest)
@@ -555,22 +553,16 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
     else
       d /= 2;
   }
-  std::stable_sort(shapes.begin(), shapes.end(), [](const Shape &a, const Shape &b) { return a.cost < b.cost; });
-  for (const Shape &x : shapes) {  // nearly always the first
-    BlockPlan P;
-    if (!build_block_plan(host, x.depth, x.cap, P) || block_cost(x.depth, local_elements(P)) >= single) continue;
-    plan = std::move(P);
-    return true;
-  }
-  return false;
+  return found;
 }
 
 // Whether `steps` steps are worth a plan: what they would save, against the plan's making.  Both are
 // estimates from what was measured (16 host cores, a first call on a fresh handle):
-//  - making: 0.1 ms (allocation, upload, the second gate buffer) and per host thread 0.6 us for each
-//    terminal (the elements around a branch are searched again for every tile) and 5 ns for each
-//    element: 0.12 ms for a 10,000-element tree, 0.6 ms for 24 bushy trees (102,815 elements, 4,400
-//    terminals), 9 ms for 1024 trees (22 million);
+//  - making: 60 us (allocation, upload, the second gate buffer), 20 us per host thread, and per
+//    thread 0.45 us for each terminal (the elements around a branch are searched again for every
+//    tile) and 5 ns for each element: 0.15 ms for a 10,000-element tree, 0.6 ms for 24 bushy trees
+//    (102,815 elements, 4,400 terminals), 0.5 ms for a myelinated axon of 199,202, 12 ms for 1024
+//    trees (22 million);
 //  - saved per step, mixed: 4.0 us per launch or 14.5 ps per element, whichever is more, becomes 2 us
 //    per depth and 8 ps per local element (102,815 elements 4.5 -> 1.2 us, a million 14.5 -> 7.9);
 //    FP64: half of what choose_f64's estimates say (a 1 cm axon 3.7 -> 2.7 us, 10,000 elements 6.8 ->
@@ -578,9 +570,8 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
 // With 128 steps for every pack, the 24 trees' first call of 128 steps took 1.28 ms instead of 0.82.
 bool block_plan_pays(const HostPack &host, const PackView &pv, bool mixed, int64_t steps) {
   const double N = (double)host.ntot;
-  const double chunks = std::ceil(N / (1 << 14)), cores = std::max(1u, std::thread::hardware_concurrency());
-  const double making =
-      100.0 + (0.6 * (double)host.terms.size() + 0.005 * N) / std::min(std::min(cores, 64.0), chunks);
+  const double threads = std::min(std::ceil(N / (1 << 14)), (double)host_threads());
+  const double making = 60.0 + 20.0 * threads + (0.45 * (double)host.terms.size() + 0.005 * N) / threads;
   double saved;
   if (mixed) {
     int depth = 0, cap = 0;
@@ -711,26 +702,6 @@ static bool tile_range(const HostPack &host, int depth, int cap, int64_t c0, int
     while (f0 < far.size() && far[f0] < s) f0++;
     want = std::min<int64_t>(cap - 2 * depth, cnt + std::max(depth, cap / 32));
   }
-  return true;
-}
-
-// The local elements (owned and halo) that a plan would have, from tiles of up to four stretches of
-// the pack; false when one of them does not tile.  A whole plan that is then not taken costs as much
-// as the one that is: of 24 bushy trees (100,000 elements) 0.6 ms each.
-static bool sample_plan(const HostPack &host, int depth, int cap, double &local) {
-  const int64_t N = host.ntot, span = 4096, n = std::min<int64_t>(4, (N + span - 1) / span);
-  double sum[4] = {0, 0, 0, 0}, seen[4] = {0, 0, 0, 0};
-  std::atomic<bool> tangle(false);
-  parallel_for(n, [&](int64_t q) {
-    const int64_t a = n * span >= N ? q * span : (N - span) * q / (n - 1), b = std::min(N, a + span);
-    BlockPlan P;
-    if (tangle) return;
-    if (!tile_range(host, depth, cap, a, b, P)) tangle = true;
-    sum[q] = local_elements(P);
-    seen[q] = (double)(b - a);
-  });
-  if (tangle) return false;
-  local = (sum[0] + sum[1] + sum[2] + sum[3]) * (double)N / (seen[0] + seen[1] + seen[2] + seen[3]);
   return true;
 }
 

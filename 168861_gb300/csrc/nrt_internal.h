@@ -84,14 +84,18 @@ inline void set_window(InstDev &in) {
   in.ioff = i1;
 }
 
+// Host threads of a parallel loop at most (asking the system takes 15 us).
+inline unsigned host_threads() {
+  static const unsigned n = std::min(std::max(1u, std::thread::hardware_concurrency()), 64u);
+  return n;
+}
+
 // Runs f(i) for every i in [0, n) on the host's cores, handing out indices one at a time
 // (instances differ in size by orders of magnitude).  The first exception of a thread ends the loop
 // and is thrown again here, in the caller's thread.
 template <class F>
 void parallel_for(int64_t n, F f) {
-  unsigned nt = std::thread::hardware_concurrency();
-  nt = std::max(1u, std::min(nt, 64u));
-  nt = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)nt, n));
+  const unsigned nt = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)host_threads(), n));
   std::atomic<int64_t> next(0);
   std::atomic<bool> failed(false);
   std::exception_ptr error;

@@ -516,6 +516,7 @@ int Engine::block_init() {
     block_mem = nullptr;
     return NRT_OK;
   }
+  block_bytes = bt + bh + bx + bg;
   char *m = (char *)block_mem;
   NRT_CUDA(cudaMemcpyAsync(m, plan.tile.data(), sizeof(BlockTile) * plan.tile.size(),
                            cudaMemcpyHostToDevice, stream));
@@ -548,6 +549,7 @@ int Engine::block_probes() {
   NRT_CUDA(cudaStreamSynchronize(stream));
   if (probe_mem) cudaFree(probe_mem);
   probe_mem = nullptr;
+  probe_bytes = 0;
   bv.probe = nullptr;
   bv.max_probes = 0;
   for (BlockTile &t : btile) t.p0 = t.p1 = 0;
@@ -576,6 +578,7 @@ int Engine::block_probes() {
       bv.max_probes = kTooManyProbes;
       return NRT_OK;
     }
+    probe_bytes = sizeof(int2) * list.size();
     NRT_CUDA(cudaMemcpyAsync(probe_mem, list.data(), sizeof(int2) * list.size(),
                              cudaMemcpyHostToDevice, stream));
     bv.probe = (const int2 *)probe_mem;

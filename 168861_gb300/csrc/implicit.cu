@@ -2297,7 +2297,7 @@ void Engine::implicit_release() {
 int Engine::get_stats(nrt_stats *st) {
   memset(st, 0, sizeof(*st));
   st->steps = steps_done;
-  st->device_bytes = (int64_t)arena.cap;
+  st->device_bytes = (int64_t)device_bytes();
   if (opt.mode == NRT_IMPLICIT_BE && im) {
     std::vector<InstStat> s(host.ninst);
     NRT_CUDA(cudaMemcpyAsync(s.data(), im->iv.stats, sizeof(InstStat) * host.ninst,

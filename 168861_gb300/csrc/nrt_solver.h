@@ -50,11 +50,13 @@ struct Engine {
   int64_t asked_steps = 0;                // steps asked for before it, in calls that would use it
   std::vector<BlockTile> btile;           // host copy of the tiles
   void *block_mem = nullptr, *probe_mem = nullptr;
+  size_t block_bytes = 0, probe_bytes = 0;  // their sizes
   void *gate2[2] = {nullptr, nullptr};    // the two gate buffers; the pack's is gate2[gcur]
   int gcur = 0;
   cudaGraphExec_t block_exec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // by cur, gcur
   int64_t block_nodes = 0;                // kernels per replay
   std::vector<void *> extra_mem;          // device tables that replaced the arena's (freed last)
+  size_t extra_bytes = 0;
 
   int init(const nrt_problem *probs, int32_t count, const nrt_options *o);
   int step(int k, int force);
@@ -92,9 +94,15 @@ struct Engine {
                       const std::vector<int64_t> &raw, const std::vector<int32_t> &sinst,
                       const std::vector<int32_t> &p0);
   void record_release();
+  size_t record_bytes() const;
   // strain.cu
   int strain_config(const nrt_strain_config *c);
   void strain_release();
+  size_t strain_bytes() const;
+  // all device memory of this handle
+  size_t device_bytes() const {
+    return arena.cap + block_bytes + probe_bytes + extra_bytes + record_bytes() + strain_bytes();
+  }
   ~Engine();
 };
 

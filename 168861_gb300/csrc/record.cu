@@ -45,6 +45,7 @@ size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
 
 struct RecState {
   void *mem = nullptr;
+  size_t bytes = 0;
   RecView view{};
   RecView *d_view = nullptr;
   int64_t *d_raw = nullptr;    // each probe's own element (initial values)
@@ -65,6 +66,7 @@ int launch_record_step(const RecView &r, const InstDev *inst, int k, const doubl
 
 const RecView *Engine::record_view() const { return rec ? rec->d_view : nullptr; }
 const RecView &Engine::rec_view_host() const { return rec->view; }
+size_t Engine::record_bytes() const { return rec ? rec->bytes : 0; }
 const std::vector<int64_t> *Engine::record_sources() const { return rec ? &rec->src : nullptr; }
 
 void Engine::record_release() {
@@ -145,6 +147,7 @@ int Engine::record_config(const nrt_record_config *c) {
     set_error("device allocation for the recording (" + std::to_string(bytes) + " bytes)");
     return NRT_ENOMEM;
   }
+  R->bytes = bytes;
   char *m = (char *)R->mem;
   auto take = [&](size_t b) {
     char *r = m;

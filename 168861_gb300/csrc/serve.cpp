@@ -121,14 +121,22 @@ struct MicroBatch {
 constexpr double kTickMs = 10.0;   // target device time of one tick per resident batch
 constexpr int32_t kWideRows = 20000;  // implicit requests this large step on the whole GPU
 
-// Device footprint of one tree in a batch (the arena sizes of the engine, rounded up).
+// Device footprint of one tree in a batch (the arena sizes of the engine, rounded up, and what an
+// explicit handle allocates for its several-step plan: the second gate buffer and the tiles).
 size_t estimate_bytes(const nrt_problem &p, const nrt_options &o) {
   const double N = (double)p.num_elem;
   const bool mixed = o.precision == NRT_MIXED;
   const double tb = mixed ? 4 : 8;
   double per = 16 + 16 + 16 + (mixed ? (7 * 4 + 12 + 44) : (5 * 8 + 24 + 88));
-  if (o.mode == NRT_IMPLICIT_BE) per += 48 + 8 + 8 + 2 * tb * (o.restart + 1) + 3 * tb + 16;
-  return (size_t)(N * per * 1.15) + (1 << 20);
+  double pieces = 0;
+  if (o.mode == NRT_IMPLICIT_BE) {
+    per += 48 + 8 + 8 + 2 * tb * (o.restart + 1) + 3 * tb + 16;
+    // the tree preconditioner's tables by piece: two for every branch point, one per window
+    if (o.precond == NRT_PRECOND_TREE) pieces = (76 + 19 * tb) * (2.0 * p.num_term + N / 128 + 2);
+  } else {
+    per += (mixed ? 12 : 24) + 8;
+  }
+  return (size_t)((N * per + pieces) * 1.15) + (1 << 20);
 }
 
 }  // namespace

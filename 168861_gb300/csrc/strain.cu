@@ -23,6 +23,7 @@ namespace nrt {
 
 struct StrainState {
   void *mem = nullptr;
+  size_t bytes = 0;
   StrainView view{};
   // host copies for the tiles of several steps per launch, and each element's class there
   std::vector<int64_t> elem;
@@ -164,6 +165,10 @@ int launch_strain_apply(const Engine &e, int k, cudaStream_t st) {
   return NRT_OK;
 }
 
+size_t Engine::strain_bytes() const {
+  return strain ? strain->bytes + (strain->scls ? 4 * (size_t)host.ntot : 0) : 0;
+}
+
 void Engine::strain_release() {
   delete strain;
   strain = nullptr;
@@ -244,6 +249,7 @@ int Engine::strain_config(const nrt_strain_config *c) {
     }
     extra_mem.push_back(d_tab);  // the pack reads these from now on: freed with the engine
     extra_mem.push_back(d_cls);
+    extra_bytes += tab_bytes + 4 * (size_t)N;
     std::vector<float> q32;
     if (mixed) {
       q32.assign((size_t)12 * L1, 0.0f);
@@ -318,6 +324,7 @@ int Engine::strain_config(const nrt_strain_config *c) {
     set_error("device allocation for the strain");
     return NRT_ENOMEM;
   }
+  S->bytes = bytes;
   char *m = (char *)S->mem;
   auto take = [&](size_t b) {
     char *r = m;

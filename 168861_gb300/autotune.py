@@ -1,28 +1,29 @@
 """Launch-shape autotuner for batches of trees (`Batch(..., autotune=True)`).
 
-The explicit steps have launch shapes that do not change their results (each element's
-arithmetic is the same whatever the grid):
-- the mixed step: staged tiles (`tiled`) with 1 .. 4 persistent CTAs per SM
-  (`tile_ctas_per_sm`), or one thread per element (`tiled=0`) with 64 .. 256 threads per
-  block (`step_threads`);
-- the FP64 step: 32 .. 256 threads per block.
+The steps have launch shapes that do not change their results:
+- mixed explicit: several steps per launch on tiles, and for what remains staged tiles (`tiled`)
+  with 1 .. 4 persistent CTAs per SM (`tile_ctas_per_sm`); or one launch per step with one thread
+  per element (`tiled=0`) and 64 .. 256 threads per block (`step_threads`);
+- FP64 explicit: 32 .. 256 threads per block in the steps that have a launch of their own;
+- implicit batches: how many CTAs an SM holds (`tile_ctas_per_sm`, 2 .. 4), which decides between
+  a cluster and a CTA per tree and between the block kernel's two register budgets.
 
-Which one is fastest depends on the tree sizes, the share of HH compartments and the
-device, so `tune` times every candidate on the workload itself, in a batch of its own, so
-the caller's state is never touched. The explicit steps tile the elements, and a sample
-stands for the workload: every k-th tree (the workload's mix of sizes), about
-`sample_elements` compartments. The implicit kernel gives each tree to one CTA, and its best
-CTA count depends on the whole population: on a quarter of the 4096-tree batch, 2 CTAs per
-SM ran fastest (the largest trees, which set a sample's time, share their SMs less), while on
-the whole batch 4 per SM beat 2 by a third (throughput over all trees). So the implicit
-kernel is timed on the whole workload, over fewer steps. It keeps the fastest. Results are cached in a JSON file
-per device, mode, precision and workload size, so a workload is tuned once per machine.
+No shape leaves out what the automatic choice (no overrides) would do: clusters and several steps
+per launch stay on, so the fastest candidate is at least as fast as an untuned batch, up to noise.
 
-The implicit block-per-instance kernel (batches) has one shape-only knob: how many of its
-persistent CTAs run per SM (`tile_ctas_per_sm`, 1 .. 4; its register budget allows 4). Each
-instance is one CTA's from start to end, so the trees come out bit for bit the same. Its other
-tunable, the GMRES restart length, changes the iteration count but leaves the answer within
-the solve tolerance; it is searched (with every CTA count) only when `restarts` is given.
+Which one is fastest depends on the tree sizes, the share of HH compartments and the device, so
+`tune` times every candidate on the workload itself, in a batch of its own, so the caller's state is
+never touched, and keeps the fastest.  The explicit steps tile the elements, and a sample stands for
+the workload: every k-th tree (the workload's mix of sizes), about `sample_elements` compartments.
+They are timed over calls of 256 steps after one such call untimed: the plan of several steps per
+launch is made once a handle has been asked for enough steps, and small mixed packs use it in calls
+of more than 128.  An implicit batch's best CTA count depends on the whole population (on a sample
+the largest trees, which set its time, share their SMs less), so it is timed on the whole workload,
+over fewer steps.  Results are cached in a JSON file per device, mode, precision and workload size,
+so a workload is tuned once per machine.
+
+The GMRES restart length changes the iteration count but leaves the answer within the solve
+tolerance; it is searched (with every CTA count) only when `restarts` is given.
 """
 from __future__ import annotations
 
@@ -100,19 +101,23 @@ def device_name(device: int = -1) -> str:
 def time_candidate(problems, mode: int, precision: str, overrides: dict, steps: int,
                    warmup: int, repeats: int = 2, runs=None, **opts) -> float:
     """Seconds per step of a batch of `problems` built with `overrides`: the best of
-    `repeats` timings of `steps` steps after `warmup` steps, with the device idle on both
-    sides of each timing.  runs: each tree's (i_begin, i_end, init_time, end_input), whose
+    `repeats` timings of `steps` steps after `warmup` steps (explicit: and `steps` more, so
+    that what a first call makes is there), with the device idle on both sides of each
+    timing.  runs: each tree's (i_begin, i_end, init_time, end_input), whose
     stimulus windows the timed steps use (the loop ranges are lengthened to cover them);
     None: no stimulus."""
     from .solver import Batch
     b = Batch(problems, mode, precision=precision, **{**opts, **overrides})
     try:
-        total = warmup + repeats * steps
+        first = steps if mode == _lib.NRT_EXPLICIT else 0
+        total = warmup + first + repeats * steps
         if runs is None:
             b.set_runs([(1, 1 + total, 0.0, -1.0)] * len(problems))
         else:
             b.set_runs([(a, max(e, a + total), t0, t1) for a, e, t0, t1 in runs])
         b.advance(warmup)
+        if first:
+            b.advance(first)
         b.synchronize()
         best = math.inf
         for _ in range(repeats):
@@ -155,7 +160,7 @@ def tune(problems, mode: int = _lib.NRT_EXPLICIT, precision: str = "fp64", *,
 
     timer(problems, mode, precision, overrides) -> seconds per step replaces the device
     timing (tests use it); device_key replaces the device's name in the cache key.
-    steps: timed steps per repeat (0: 64 explicit, 16 implicit); sample_elements: the sample's
+    steps: timed steps per repeat (0: 256 explicit, 16 implicit); sample_elements: the sample's
     size (0: 4e6 compartments explicit, the whole workload implicit); min_trees: the sample's
     fewest trees.  runs: the trees' loop ranges and stimulus windows (as Batch.set_runs), so
     the timed steps see the workload's stimulus (None: none).  `opts` are the caller's other
@@ -171,7 +176,7 @@ def tune(problems, mode: int = _lib.NRT_EXPLICIT, precision: str = "fp64", *,
     if len(cands) == 1:
         return {"options": dict(cands[0]), "key": key, "times": [None], "candidates": cands}
     explicit = mode == _lib.NRT_EXPLICIT
-    steps = steps or (64 if explicit else 16)
+    steps = steps or (256 if explicit else 16)
     sample_elements = sample_elements or (4e6 if explicit else math.inf)
     idx = sample_indices(problems, sample_elements, min_trees)
     part = [problems[i] for i in idx]

@@ -500,9 +500,8 @@ int Engine::init(const nrt_problem *probs, int32_t count, const nrt_options *o) 
 }
 
 // The plan of several explicit steps per launch, its device copy and the second gate buffer: made
-// by the time loop once the steps asked for are worth it.  Without the memory for them (or with a
-// tree that does not tile) the time loop takes one launch per step, as it does when the options name
-// a shape of the per-step kernels other than the staged tiles.
+// by the time loop once the steps asked for are worth it.  Without the memory for them, with a
+// tree that does not tile and with the option `tiled` off the time loop takes one launch per step.
 int Engine::block_init() {
   block_tried = true;
   BlockPlan plan;
@@ -807,9 +806,7 @@ bool Engine::chunk_kernel() const {
 // launch counter reports for them (128 steps of a 3000-compartment tree 0.5 ms, 0.2 with a plan).
 bool Engine::block_call(int64_t left) const {
   constexpr int64_t kBlockMinElems = 8192;
-  if (opt.mode != NRT_EXPLICIT || !host.fusable || opt.tiled == 0 || opt.step_threads > 0 ||
-      opt.step_launch != 0)
-    return false;
+  if (opt.mode != NRT_EXPLICIT || !host.fusable || opt.tiled == 0 || opt.step_launch != 0) return false;
   // (a tile's probes hold 8 bytes per step each in shared memory)
   const bool mixed = opt.precision == NRT_MIXED;
   return left > 2 && (!strain || (mixed && strain_tabled(*this))) &&

@@ -1833,14 +1833,16 @@ int Engine::implicit_plan(size_t &bytes) {
   // cooperative launch's step in its grid-wide syncs (1.5 to 2 us each; a cluster's barrier
   // takes about 0.4).
   S.cluster = 0;
-  if (tree && opt.krylov == NRT_GMRES && opt.schedule == 0 && opt.tile_ctas_per_sm == 0) {
+  if (tree && opt.krylov == NRT_GMRES && opt.schedule == 0) {
     // No more CTAs than gain by it, since their barriers cost more than a CTA's: FP64 one per
     // chunk of 128 rows, mixed batches one per window, and a mixed single tree of one window stays
     // with one CTA (32 steps: of 300 compartments 1.76 ms on 4 CTAs, 1.31 on one; of 1000 1.78 on
     // 8, 1.65 on one; of 2000 1.75 on 8, 2.02 on 2; 48 of 300 2.21 ms on 8 CTAs each, 1.33 on one).
     const int64_t part = mixed && (ni > 1 || max_n <= kMaxWin) ? kMaxWin : 128;
     const int64_t parts = (max_n + part - 1) / part;
-    const int64_t room = ni > 1 ? (int64_t)dev_sms * (mixed ? 3 : 2) / ni : max_n <= kClusterRows ? 8 : 0;
+    int64_t per = mixed ? ctas_per_sm<float, kCluster>() : ctas_per_sm<double, kCluster>();
+    if (opt.tile_ctas_per_sm > 0) per = std::min<int64_t>(per, opt.tile_ctas_per_sm);
+    const int64_t room = ni > 1 ? dev_sms * per / ni : max_n <= kClusterRows ? 8 : 0;
     for (int cs = 2; cs <= 8 && cs <= room && cs < 2 * parts; cs *= 2) S.cluster = cs;
     if (room && parts == 1) S.grid_mode = false;
   }
@@ -1947,8 +1949,8 @@ int Engine::implicit_plan(size_t &bytes) {
     for (int32_t i = 0; i < ni; i++) S.order[i] = i;
     std::stable_sort(S.order.begin(), S.order.end(),
                      [&](int a, int b) { return host.num_elem[a] > host.num_elem[b]; });
-    // persistent CTAs: as many per SM as fit, or at most tile_ctas_per_sm (a tuned shape;
-    // each instance is one CTA's from start to end, so results do not depend on it)
+    // persistent CTAs: as many per SM as fit, or at most tile_ctas_per_sm (a tuned shape; results do
+    // not depend on it)
     if (opt.tile_ctas_per_sm > 0) per_sm = std::min(per_sm, opt.tile_ctas_per_sm);
     S.grid_blocks = std::max(1, std::min<int>(dev_sms * std::max(per_sm, 1), ni));
     if (S.cluster) S.grid_blocks = ni * S.cluster;

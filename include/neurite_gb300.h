@@ -121,19 +121,22 @@ typedef struct nrt_options {
   int32_t schedule;              /* implicit: 0 = auto (by number and size of the trees: the
                                     whole GPU, a cluster or a block per instance),
                                     1 = always block per instance */
-  int32_t tiled;                 /* mixed explicit: 1 (default) = element arrays staged into
-                                    shared memory by bulk copies, tile by tile; 0 = one
-                                    thread per element loading its own (same results) */
+  int32_t tiled;                 /* explicit: 1 (default) = time loops may take several steps
+                                    per launch on tiles of elements (see step_launch), and the
+                                    mixed per-step kernel stages element arrays into shared
+                                    memory by bulk copies, tile by tile; 0 = one launch per
+                                    step, one thread per element loading its own (same
+                                    results) */
   int32_t scheme;                /* implicit: NRT_BACKWARD_EULER (default, the reference's)
                                     or NRT_CRANK_NICOLSON */
-  int32_t tile_ctas_per_sm;      /* persistent CTAs per SM, 1 .. as many as fit (0 = as many
-                                    as fit, the default): of the mixed explicit tiled step,
-                                    and of the implicit block-per-instance kernel (batches) */
-  int32_t step_threads;          /* explicit, one thread per element: threads per block, a
-                                    multiple of 32 up to 256 (0 = chosen from the tree size;
-                                    FP64 packs of up to 8192 elements then take eight lanes
-                                    per element).  Launch shapes only: results do not depend
-                                    on them */
+  int32_t tile_ctas_per_sm;      /* CTAs per SM at most, 1 .. as many as fit (0 = chosen, the
+                                    default): of the mixed explicit tiled step, and of
+                                    implicit batches (a block or a cluster per instance) */
+  int32_t step_threads;          /* explicit per-step kernels, one thread per element:
+                                    threads per block, a multiple of 32 up to 256 (0 = chosen
+                                    from the tree size; FP64 packs of up to 8192 elements then
+                                    take eight lanes per element).  Launch shapes only:
+                                    results do not depend on them */
   double inner_tol;              /* implicit, mixed precision: each FP64 refinement cycle's
                                     inner FP32 Krylov solve stops once its residual estimate
                                     is below inner_tol times the cycle's starting residual
@@ -142,12 +145,12 @@ typedef struct nrt_options {
   int32_t step_launch;           /* explicit time loops (nrt_run, nrt_batch_advance, the
                                     server): 0 = automatic (default): one launch per step, or
                                     several steps per launch on tiles with halos (2 to 16,
-                                    where tiled is set and step_threads is not), chained and replayed from a captured graph; 1 = up to
-                                    64 steps per
-                                    cooperative launch with a grid barrier between steps (on a
-                                    GB300 a barrier across both dies costs about what a chained
-                                    launch does, so this is not faster there).  Launch shapes
-                                    only: results do not depend on it */
+                                    where tiled is set), chained and replayed from a captured
+                                    graph; 1 = up to 64 steps per cooperative launch with a
+                                    grid barrier between steps (on a GB300 a barrier across
+                                    both dies costs about what a chained launch does, so this
+                                    is not faster there).  Launch shapes only: results do not
+                                    depend on it */
   int32_t refinement;            /* implicit, mixed precision, GMRES with the tree
                                     preconditioner: 0 = auto: each FP64 refinement cycle is
                                     one preconditioned Richardson step, x += M^-1 r (M, the

@@ -68,11 +68,12 @@ def test_a_tree_does_not_depend_on_its_company(gpu, pkg, model):
         assert (st["nonconverged"] == 0).all()
         return V, st["last_residual"]
 
-    ref, res = go(range(5), tile_ctas_per_sm=3)  # a CTA each
+    ref, res = go(range(5), schedule=1)  # a CTA each
     small = [0, 1, 2]
     for which, shape in (([0, 1], {}), ([0, 2, 1], {}), (list(range(5)), {}), (list(range(5)) * 10, {}),
                          (small * 30, {}), (small * 60, {}), (small * 170, {}),
-                         (list(range(5)), {"tile_ctas_per_sm": 4}), (list(range(5)), {"schedule": 1})):
+                         (list(range(5)), {"tile_ctas_per_sm": 4}), (small * 30, {"tile_ctas_per_sm": 2}),
+                         (list(range(5)) * 10, {"schedule": 1})):
         V, r = go(which, **shape)
         for k, q in enumerate(which):
             np.testing.assert_array_equal(V[k], ref[q], err_msg=f"{len(which)} trees {shape}")

@@ -1062,7 +1062,7 @@ int nrt_snapshot(nrt_solver *s, double *potential) {
     NRT_CUDA(cudaMemcpyAsync(potential, e.V[e.cur], sizeof(double) * e.host.num_elem[0],
                              cudaMemcpyDeviceToHost, e.stream));
     NRT_CUDA(cudaStreamSynchronize(e.stream));
-    return nrt::implicit_check(e);
+    return nrt::device_check(e);
   });
 }
 
@@ -1102,7 +1102,7 @@ int nrt_synchronize(nrt_solver *s) {
     if (!s) return nrt::fail(NRT_EINVAL, "null solver");
     NRT_CUDA(cudaSetDevice(s->eng.device));
     NRT_CUDA(cudaStreamSynchronize(s->eng.stream));
-    return nrt::implicit_check(s->eng);
+    return nrt::device_check(s->eng);
   });
 }
 
@@ -1238,7 +1238,7 @@ int nrt_batch_synchronize(nrt_batch *b) {
     if (!b) return nrt::fail(NRT_EINVAL, "null batch");
     NRT_CUDA(cudaSetDevice(b->eng.device));
     NRT_CUDA(cudaStreamSynchronize(b->eng.stream));
-    return nrt::implicit_check(b->eng);
+    return nrt::device_check(b->eng);
   });
 }
 
@@ -1254,7 +1254,7 @@ int nrt_batch_snapshot(nrt_batch *b, int32_t instance, double *potential) {
     NRT_CUDA(cudaMemcpyAsync(potential, e.V[e.cur] + o, sizeof(double) * e.host.num_elem[instance],
                              cudaMemcpyDeviceToHost, e.stream));
     NRT_CUDA(cudaStreamSynchronize(e.stream));
-    return nrt::implicit_check(e);
+    return nrt::device_check(e);
   });
 }
 
@@ -1273,7 +1273,7 @@ int nrt_batch_snapshot_all(nrt_batch *b, double *potential) {
     }
     NRT_CUDA(cudaMemcpyAsync(potential, src, sizeof(double) * n, cudaMemcpyDeviceToHost, e.stream));
     NRT_CUDA(cudaStreamSynchronize(e.stream));
-    return nrt::implicit_check(e);
+    return nrt::device_check(e);
   });
 }
 
@@ -1329,7 +1329,7 @@ int nrt_get_state(nrt_solver *s, double *V, double *V_other, double *m, double *
     if (!s) return nrt::fail(NRT_EINVAL, "null solver");
     NRT_CUDA(cudaSetDevice(s->eng.device));
     int rc = s->eng.get_state(0, V, V_other, m, h, n);
-    return rc ? rc : nrt::implicit_check(s->eng);
+    return rc ? rc : nrt::device_check(s->eng);
   });
 }
 
@@ -1349,7 +1349,7 @@ int nrt_batch_get_state(nrt_batch *b, int32_t instance, double *V, double *V_oth
     if (instance < 0 || instance >= b->eng.pv.ninst) return nrt::fail(NRT_EINVAL, "instance out of range");
     NRT_CUDA(cudaSetDevice(b->eng.device));
     int rc = b->eng.get_state(instance, V, V_other, m, h, n);
-    return rc ? rc : nrt::implicit_check(b->eng);
+    return rc ? rc : nrt::device_check(b->eng);
   });
 }
 
@@ -1407,7 +1407,7 @@ int nrt_record_read(nrt_solver *s, int64_t *num_samples, double *times, double *
     if (!s) return nrt::fail(NRT_EINVAL, "null solver");
     NRT_CUDA(cudaSetDevice(s->eng.device));
     int rc = s->eng.record_read(num_samples, times, values, num_spikes, spike_times);
-    return rc ? rc : nrt::implicit_check(s->eng);
+    return rc ? rc : nrt::device_check(s->eng);
   });
 }
 
@@ -1417,7 +1417,7 @@ int nrt_batch_record_read(nrt_batch *b, int64_t *num_samples, double *times, dou
     if (!b) return nrt::fail(NRT_EINVAL, "null batch");
     NRT_CUDA(cudaSetDevice(b->eng.device));
     int rc = b->eng.record_read(num_samples, times, values, num_spikes, spike_times);
-    return rc ? rc : nrt::implicit_check(b->eng);
+    return rc ? rc : nrt::device_check(b->eng);
   });
 }
 

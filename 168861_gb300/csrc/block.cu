@@ -112,7 +112,11 @@ __global__ void __launch_bounds__(kDense ? 512 : 256, kDense ? 2 : 6)
   const BlockTile t = bv.tile[blockIdx.x];
   const int l = threadIdx.x;
   const int64_t N = p.ntot;
-  // ---- what the time loop never changes: before the wait for the previous launch
+  // ---- what the time loop never changes: before the wait for the previous launch.  Topology, tiles
+  // and parameters are written when a handle, a recording or a strain is set up, with the stream
+  // idle.  The rows of strained elements (cdtf, gaxf, wdxf, kdxf and their columns of hpq) are
+  // rewritten by strain_apply in the same chain: their values read here are not used, row_take(0)
+  // and the re-read of gp and gd replace them after the wait.
   int dist = 1 << 20;
   int64_t j = -1;
   if (l < t.cnt) {
@@ -294,7 +298,8 @@ __global__ void __launch_bounds__(256, 2)
   const int l = threadIdx.x / kLanes, q = threadIdx.x % kLanes;
   const int64_t N = p.ntot;
   exp64_prefetch();
-  // ---- what the time loop never changes: before the wait for the previous launch
+  // ---- what the time loop never changes: before the wait for the previous launch (topology and
+  // conductances; FP64 packs with a strain, which rewrites conductances, do not come here)
   int dist = 1 << 20;
   int64_t j = -1;
   if (l < t.cnt) {

@@ -105,8 +105,6 @@ struct InstStat {
   int64_t residuals, applies, xupdates, basis, rich;
 };
 
-constexpr size_t kErrBytes = 16;  // the error word's place before the statistics
-
 struct ImView {
   int64_t ntot;
   int m;             // GMRES restart (BiCGSTAB: sizes the shared work vectors only)
@@ -139,7 +137,6 @@ struct ImView {
   int *queue;                     // batch: next index into order
   double *partials;               // kGrid: 2 x gridDim x kMaxDots
   InstStat *stats;
-  int *err;                       // set when a bounded wait gives up (device fault report)
   int64_t ld;                     // row-vector stride: ntot rounded up to kRW rows
   const int *inst_n;              // rows of each instance (inst_row holds where they start)
   const int64_t *inst_out;        // where each instance's rows go without the padding
@@ -1979,7 +1976,7 @@ int Engine::implicit_plan(size_t &bytes) {
     b += al256(4 * S.inst_tile.size()) + al256(4 * S.order.size());
   b += 2 * al256(8 * S.inst_row.size()) + al256(4 * S.inst_n.size());
   b += al256(4) + al256(sizeof(double) * 2 * 4096 * kMaxDots);
-  b += al256(kErrBytes + sizeof(InstStat) * ni) + al256(sizeof(PackView)) + al256(sizeof(ImView));
+  b += al256(sizeof(InstStat) * ni) + al256(sizeof(PackView)) + al256(sizeof(ImView));
   if (tree) {
     const TreePlan &T = S.tree;
     const size_t npc = std::max<size_t>(1, T.pmap.size());
@@ -2084,15 +2081,8 @@ int Engine::implicit_init() {
   TRYI(up(arena, pl, out.data(), out.size(), st)); iv.inst_out = pl;
   TRYI(up(arena, iv.queue, (const int *)nullptr, 1, st));
   TRYI(up(arena, iv.partials, (const double *)nullptr, (size_t)2 * 4096 * kMaxDots, st));
-  // the error word and the statistics lie side by side: one copy reads both
-  char *es = (char *)arena.take(kErrBytes + sizeof(InstStat) * ni);
-  if (!es) {
-    set_error("arena exhausted (statistics)");
-    return NRT_ENOMEM;
-  }
-  NRT_CUDA(cudaMemsetAsync(es, 0, kErrBytes + sizeof(InstStat) * ni, st));
-  iv.err = (int *)es;
-  iv.stats = (InstStat *)(es + kErrBytes);
+  TRYI(up(arena, iv.stats, (const InstStat *)nullptr, ni, st));
+  NRT_CUDA(cudaMemsetAsync(iv.stats, 0, sizeof(InstStat) * ni, st));
   if (tree) {
     const TreePlan &T = S.tree;
     const size_t npc = std::max<size_t>(1, T.pmap.size());
@@ -2225,17 +2215,15 @@ int pass_counts(Engine &e, int64_t *residuals, int64_t *applies, int64_t *xupdat
   return NRT_OK;
 }
 
-// NRT_EDEVICE when a kernel's bounded wait gave up (an error word is set); synchronises.
-int implicit_check(Engine &e) {
-  int err[2] = {0, 0};
-  if (e.im)
-    NRT_CUDA(cudaMemcpyAsync(&err[0], e.im->iv.err, sizeof(int), cudaMemcpyDeviceToHost, e.stream));
-  if (e.pv.err)
-    NRT_CUDA(cudaMemcpyAsync(&err[1], e.pv.err, sizeof(int), cudaMemcpyDeviceToHost, e.stream));
+// NRT_EDEVICE when a bounded wait of an explicit kernel gave up (the pack's error word is set; the
+// implicit kernels wait for nothing but their own CTAs); synchronises.
+int device_check(Engine &e) {
+  int err = 0;
+  if (e.pv.err && e.opt.mode == NRT_EXPLICIT)
+    NRT_CUDA(cudaMemcpyAsync(&err, e.pv.err, sizeof(int), cudaMemcpyDeviceToHost, e.stream));
   NRT_CUDA(cudaStreamSynchronize(e.stream));
-  if (err[0] || err[1]) {
-    set_error(err[0] ? "implicit kernel: a bounded wait for its tile copies expired"
-                     : "explicit step: a bounded wait for its tile copies expired");
+  if (err) {
+    set_error("explicit step: a bounded wait for its tile copies expired");
     return NRT_EDEVICE;
   }
   return NRT_OK;
@@ -2267,26 +2255,16 @@ int implicit_compact(Engine &e, const double *&src, int64_t &n) {
   return NRT_OK;
 }
 
-// Sum of non-converged steps over all instances (-1 on a device error); waits for the stream.
+// Sum of non-converged steps over all instances (-1 on a CUDA error); waits for the stream.
 int64_t nonconverged_total(Engine &e) {
   if (!e.im) return 0;
-  const size_t bytes = kErrBytes + sizeof(InstStat) * e.host.ninst;
-  std::vector<int64_t> buf(bytes / 8);  // InstStat is made of 8-byte fields and pairs of 4
-  if (cudaMemcpyAsync(buf.data(), e.im->iv.err, bytes, cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
+  std::vector<InstStat> s(e.host.ninst);
+  if (cudaMemcpyAsync(s.data(), e.im->iv.stats, sizeof(InstStat) * s.size(), cudaMemcpyDeviceToHost,
+                      e.stream) != cudaSuccess ||
       cudaStreamSynchronize(e.stream) != cudaSuccess)
     return -1;
-  int err;
-  memcpy(&err, buf.data(), sizeof(err));
-  if (err) {
-    set_error("implicit kernel: a bounded wait expired");
-    return -1;
-  }
   int64_t t = 0;
-  for (int32_t i = 0; i < e.host.ninst; i++) {
-    InstStat x;
-    memcpy(&x, (const char *)buf.data() + kErrBytes + sizeof(InstStat) * i, sizeof(x));
-    t += x.nonconv;
-  }
+  for (const InstStat &x : s) t += x.nonconv;
   e.nonconv_seen = t;
   return t;
 }

@@ -8,8 +8,11 @@
 // start at once when it ends, instead of after a full launch round trip.
 //
 // Rules that keep this correct:
-//  - every kernel launched with launch_chained() calls chain_acquire() before its first
-//    access to global memory;
+//  - every kernel launched with launch_chained() calls chain_acquire(), and before it reads
+//    only data that no kernel still running writes, or whose value it does not use.  Of the
+//    launches before it only the immediate predecessor can still run (that one released after
+//    its own chain_acquire(), so all earlier ones have completed).  The kernels that read
+//    before the wait say beside the loads why theirs meet this;
 //  - chain_release() only lets the successor be scheduled: the successor still waits for
 //    this grid's completion in its own chain_acquire().  Because the successor is
 //    scheduled only after every CTA of this grid has been scheduled and released, its CTAs

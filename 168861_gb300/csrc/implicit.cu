@@ -2235,7 +2235,7 @@ __global__ void compact_rows(const double *__restrict__ V, double *__restrict__ 
   const int i = blockIdx.x;
   const double *src = V + from[i];
   double *dst = out + to[i];
-  for (int j = threadIdx.x; j < n[i]; j += blockDim.x) dst[j] = src[j];
+  for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < n[i]; j += gridDim.y * blockDim.x) dst[j] = src[j];
 }
 
 // The Krylov workspace, dead between steps, takes the packed copy: Wb holds m + 1 >= 2 rows
@@ -2248,7 +2248,11 @@ int implicit_compact(Engine &e, const double *&src, int64_t &n) {
   if (total == e.host.ntot) return NRT_OK;  // no padding
   ImplicitState &S = *e.im;
   double *out = (double *)S.iv.Wb;
-  compact_rows<<<ni, 256, 0, e.stream>>>(src, out, S.iv.inst_row, S.iv.inst_n, S.iv.inst_out);
+  // as many CTAs per instance as leave each a few rows per thread (two trees of 100,000: the whole
+  // call 111 us with one CTA each, 25 so)
+  const int largest = *std::max_element(e.host.num_elem.begin(), e.host.num_elem.end());
+  const dim3 grid(ni, std::max(1, std::min(64, largest / 2048)));
+  compact_rows<<<grid, 256, 0, e.stream>>>(src, out, S.iv.inst_row, S.iv.inst_n, S.iv.inst_out);
   count_launch_on(e.stream);
   NRT_CUDA(cudaGetLastError());
   src = out;

@@ -563,11 +563,12 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
 
 // Whether `steps` steps are worth a plan: what they would save, against the plan's making.  Both are
 // estimates from what was measured (16 host cores, a first call on a fresh handle):
-//  - making: 60 us (allocation, upload, the second gate buffer), 20 us per host thread, and per
-//    thread 0.45 us for each terminal (the elements around a branch are searched again for every
+//  - making: 60 us (allocation, upload, the second gate buffer), 20 us per host thread, and over
+//    the threads (16 of them at most: a container's share of the cores can be less than the system
+//    says) 0.45 us for each terminal (the elements around a branch are searched again for every
 //    tile) and 5 ns for each element: 0.15 ms for a 10,000-element tree, 0.6 ms for 24 bushy trees
-//    (102,815 elements, 4,400 terminals), 0.5 ms for a myelinated axon of 199,202, 12 ms for 1024
-//    trees (22 million);
+//    (102,815 elements, 4,400 terminals), 0.5 ms for a myelinated axon of 199,202, 1.9 ms for a
+//    million elements, 13 ms for 1024 trees (22 million);
 //  - saved per step, mixed: 4.0 us per launch or 14.5 ps per element, whichever is more, becomes 2 us
 //    per depth and 8 ps per local element (102,815 elements 4.5 -> 1.2 us, a million 14.5 -> 7.9);
 //    FP64: half of what choose_f64's estimates say (a 1 cm axon 3.7 -> 2.7 us, 10,000 elements 6.8 ->
@@ -576,7 +577,8 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
 bool block_plan_pays(const HostPack &host, const PackView &pv, bool mixed, int64_t steps) {
   const double N = (double)host.ntot;
   const double threads = std::min(std::ceil(N / (1 << 14)), (double)host_threads());
-  const double making = 60.0 + 20.0 * threads + (0.45 * (double)host.terms.size() + 0.005 * N) / threads;
+  const double making =
+      60.0 + 20.0 * threads + (0.45 * (double)host.terms.size() + 0.005 * N) / std::min(threads, 16.0);
   double saved;
   if (mixed) {
     int depth = 0, cap = 0;

@@ -1709,9 +1709,9 @@ static void make_tiles(const hvec<int2> &pieces, int pa, int pb, int tile_rows,
 // Whether a batch of one CTA per tree runs kBlock4 (the same results: a tree's arithmetic and its
 // order are the same in both).
 //
-// With 64 registers instead of 80 (mixed) or 128 (FP64) a pass takes 5 to 50 % longer, and trees of
-// different sizes gain from few CTAs that are fast (1000 trees of 1e3 to 3e4: mixed 9.6 ms, 12.0 with
-// four; FP64 30.2 and 36.2).  Four are faster where the number of trees decides:
+// With 64 registers instead of 80 (mixed) or 128 (FP64) a CTA's passes take longer, and a batch lasts
+// as long as its largest tree's CTA does (1000 trees of 1e3 to 3e4: mixed 9.6 ms, 12.0 with four;
+// 2048 of 1e3 to 1e5 34.9 and 39.6).  Four are as fast or faster where the number of trees decides:
 //  - trees that are too small to occupy a CTA's warps, more than the usual CTAs take at once (32
 //    steps of 1000 cables of 60: FP64 6.3 ms, 3.9 with four; mixed 2.7, 2.4; of 300: 11.4, 10.0 and
 //    3.2, 2.8);
@@ -1720,7 +1720,10 @@ static void make_tiles(const hvec<int2> &pieces, int pa, int pb, int tile_rows,
 //    full (the trees of the last one meet on few SMs), except that a launch of fewer trees than
 //    places spreads them evenly: 400 cables of 3000 in FP64 are two rounds of two, 28.9 ms, or three
 //    at once, 21.0; 600 of 1000 mixed two rounds of three, 3.6, or four at once, 2.6; but 620 of
-//    1500 mixed two rounds of three, 2.6, or of four, 2.9.
+//    1500 mixed two rounds of three, 2.6, or of four, 2.9;
+//  - so many trees that the largest, on a quarter of an SM, is done in three quarters of the time
+//    that all take: 4096 trees of 1e3 to 1e5 mixed 69.5 ms, 68.9 with four, cables 65.0 and 62.7;
+//    3000 cables of 100 to 1000 mixed 2.51 and 2.35; 1500 of 1000 to 3000 in FP64 13.4 and 12.6.
 static bool four_per_sm(const HostPack &host, const nrt_options &opt, int sms) {
   const int usual = opt.precision == NRT_MIXED ? ctas_per_sm<float, kBlock>() : ctas_per_sm<double, kBlock>();
   if (opt.tile_ctas_per_sm > 0) return opt.tile_ctas_per_sm > usual;
@@ -1734,7 +1737,8 @@ static bool four_per_sm(const HostPack &host, const nrt_options &opt, int sms) {
   auto trees_per_sm = [&](int64_t k) {
     return ni <= k * sms ? (ni + sms - 1) / sms : (ni + k * sms - 1) / (k * sms) * k;
   };
-  return largest <= 512 || (4 * largest * ni <= 5 * sum && trees_per_sm(4) <= trees_per_sm(usual));
+  return largest <= 512 || (4 * largest * ni <= 5 * sum && trees_per_sm(4) <= trees_per_sm(usual)) ||
+         16 * largest * sms <= 3 * sum;
 }
 
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }

@@ -356,7 +356,9 @@ def run_ours(args, rank: int, world: int, dist, wl: str, extras: bool = True, st
     precision = "fp64" if wl.endswith("fp64") else "mixed"
     implicit = wl.startswith("batch-implicit")
     K = steps or args.steps or (40 if implicit else 2048)
-    W = max(3, args.warmup)
+    # explicit: long enough for what a handle makes once its calls have asked for enough steps (the
+    # plan of several steps per launch); the end-to-end leg pays for it in its timed region
+    W = max(3 if implicit else 512, args.warmup)
 
     t_build = time.time()
     strained = None

@@ -1394,7 +1394,8 @@ __device__ __noinline__ void ph_record(const RecView *rp, int inst, int64_t i, c
 
 // Resident CTAs per SM that the registers allow.  FP32: 3 (80 registers; the 2048-tree batch
 // took 51.1 ms per 8 steps at 4, whose 64 registers spill in the fused passes, 41.7 at 3 and
-// 48.9 at 2).  FP64: 2 (128 registers): its FP64 pipe is full with 16 warps.
+// 48.9 at 2).  FP64: 2 (128 registers): its FP64 pipe is full with 16 warps.  kBlock4: 4, for the
+// batches that four_per_sm names.
 template <typename T, int kMode>
 constexpr int ctas_per_sm() {
   return kMode == kBlock4 ? 4 : sizeof(T) == 4 ? 3 : 2;
@@ -1851,8 +1852,8 @@ int Engine::implicit_plan(size_t &bytes) {
   if (tree) {
     // Rows per window: 1024, a CTA's.  In an FP64 batch 128, a warp's: its passes lose their
     // barriers, a cluster's CTAs share a tree evenly, and the longer chains of pieces cost less
-    // (48 trees of 10k, 8 steps: 2.50 -> 2.31 ms; 1000 of 300: 5.83 -> 5.18).  The mixed step
-    // does not gain: with its warps apart in its longer code 2048 trees of 10k took 43.0 ms
+    // (48 trees of 1e3 to 1e4, 8 steps: 2.50 -> 2.31 ms; 1000 of 300: 5.83 -> 5.18).  The mixed step
+    // does not gain: with its warps apart in its longer code 2048 trees of 1e3 to 1e5 took 43.0 ms
     // instead of 37.8.  In a single tree fewer than 1024 (down to 128) where its CTAs
     // would otherwise not all have a window: a window's FP64 arithmetic is bound by its SM's
     // FP64 pipe, so a small tree's windows go to as many SMs as it has CTAs.  (The windows set

@@ -81,7 +81,7 @@ __device__ __forceinline__ void sum_windows(const Ctx<float, kMode> &c, Shared &
 // kCn: Crank-Nicolson.  The rows' part takes one row per thread, a warp 32 neighbours: with the
 // four rows per thread that the matrices' scan wants, its loads used half of each sector and its
 // numbers did not fit the registers (22 accesses of local memory per row and step, most of them
-// L2 round trips).  10k compartments x 2048: 39.2 -> 38.2 ms for 8 steps; one tree of 30k, whose
+// L2 round trips).  2048 trees of 1e3 to 1e5: 39.2 -> 38.2 ms for 8 steps; one tree of 30k, whose
 // windows are smaller than a CTA's threads times four: 3.35 -> 3.13 ms for 32.
 // What is left is bound by the FP64 pipe's latency and rate (16 cycles of an SM per warp's
 // operation), so rare rows share one x0 with the warp's ends, and x0 goes to Z for the passes that

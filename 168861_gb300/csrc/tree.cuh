@@ -248,7 +248,7 @@ __device__ __forceinline__ T max_of(T a, T b) {
 
 // Scales the numbers by one power of two so that the largest lies in [1, 2) (FP32: [1, 4)).  In
 // FP64 on the exponents, in integers: a comparison or a product of doubles takes an SM's FP64 pipe
-// 16 cycles, and of a matrix product's 15 such operations 7 were its scaling (48 trees of 10k in
+// 16 cycles, and of a matrix product's 15 such operations 7 were its scaling (48 trees of 1e3 to 1e4 in
 // FP64, 8 steps: 2.31 -> 2.17 ms).  What would leave
 // the range is 0, as far below the largest as 2^-1022; a largest number that is no positive normal
 // one (0, infinite, NaN, or a negative entry among them) takes the general way.

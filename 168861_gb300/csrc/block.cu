@@ -481,6 +481,7 @@ static void block_shape(const PackView &pv, int &depth, int &cap) {
 }
 
 static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan &plan);
+static unsigned plan_threads(int64_t N);
 
 // Estimated microseconds per step of a plan, and of the per-step kernels: a launch boundary and
 // the elements' share (measured on 5.4 and 22 million compartments: 9 to 11 ps per local
@@ -563,27 +564,27 @@ bool choose_block_plan(const HostPack &host, const PackView &pv, bool mixed, Blo
 
 // Whether `steps` steps are worth a plan: what they would save, against the plan's making.  Both are
 // estimates from what was measured (16 host cores, a first call on a fresh handle):
-//  - making: 60 us (allocation, upload, the second gate buffer), 20 us per host thread, and over
-//    the threads (16 of them at most: a container's share of the cores can be less than the system
-//    says) 0.45 us for each terminal (the elements around a branch are searched again for every
-//    tile) and 5 ns for each element: 0.15 ms for a 10,000-element tree, 0.6 ms for 24 bushy trees
-//    (102,815 elements, 4,400 terminals), 0.5 ms for a myelinated axon of 199,202, 1.9 ms for a
-//    million elements, 13 ms for 1024 trees (22 million);
-//  - saved per step, mixed: 4.0 us per launch or 14.5 ps per element, whichever is more, becomes 2 us
-//    per depth and 8 ps per local element (102,815 elements 4.5 -> 1.2 us, a million 14.5 -> 7.9);
+//  - making: 60 us, up to 150 for allocations and copies, 55 us per further host thread, and over the
+//    threads (16 of them at most: a container's share of the cores can be less than the system says)
+//    0.25 us for each terminal (the elements around a branch are searched again for every tile) and
+//    3.5 ns for each element; and 0.2 ns per element for the upload: 0.12 ms for a 10,000-element tree,
+//    0.7 ms for 24 bushy trees (102,815 elements, 4,400 terminals), 0.6 ms for a myelinated axon of
+//    199,202, 1.5 ms for a million elements, 13 ms for 1024 trees (22 million);
+//  - saved per step, mixed: 4.3 us per launch, or 2.5 and 14.5 ps per element if that is more, becomes
+//    2 us per depth and 6.8 ps per local element (102,815 elements 4.5 -> 1.2 us, a million 18.3 -> 7.9);
 //    FP64: half of what choose_f64's estimates say (a 1 cm axon 3.7 -> 2.7 us, 10,000 elements 6.8 ->
 //    5.4).
 // With 128 steps for every pack, the 24 trees' first call of 128 steps took 1.28 ms instead of 0.82.
 bool block_plan_pays(const HostPack &host, const PackView &pv, bool mixed, int64_t steps) {
   const double N = (double)host.ntot;
-  const double threads = std::min(std::ceil(N / (1 << 14)), (double)host_threads());
-  const double making =
-      60.0 + 20.0 * threads + (0.45 * (double)host.terms.size() + 0.005 * N) / std::min(threads, 16.0);
+  const double threads = plan_threads(host.ntot);
+  const double making = 60.0 + std::min(150.0, 0.0015 * N) + 55.0 * (threads - 1) + 0.0002 * N +
+                        (0.25 * (double)host.terms.size() + 0.0035 * N) / std::min(threads, 16.0);
   double saved;
   if (mixed) {
     int depth = 0, cap = 0;
     block_shape(pv, depth, cap);
-    saved = std::max(4.0, 1.45e-5 * N) - (2.0 / depth + 8e-6 * 1.15 * N);
+    saved = std::max(4.3, 2.5 + 1.45e-5 * N) - (2.0 / depth + 6.8e-6 * 1.15 * N);
   } else {
     double best = f64_single_cost(host.ntot, pv);
     const double single = best;
@@ -594,6 +595,14 @@ bool block_plan_pays(const HostPack &host, const PackView &pv, bool mixed, int64
     saved = host.ntot > kF64MaxElems ? 0.0 : 0.5 * (single - best);
   }
   return saved > 0 && (double)steps * saved >= making;
+}
+
+// Host threads of a plan.  A thread's start and its first allocations take about 55 us in a process
+// of many libraries, so small packs take four (a myelinated axon of 199,202 elements: 0.68 ms on
+// one, 0.42 on four, 0.83 to 1.4 on thirteen; 24 bushy trees 1.2, 0.6 and 0.8).
+static unsigned plan_threads(int64_t N) {
+  const int64_t chunks = (N + (1 << 14) - 1) / (1 << 14);
+  return (unsigned)std::min<int64_t>({chunks, std::max<int64_t>(4, N >> 17), (int64_t)host_threads()});
 }
 
 // The plan of elements [c0, c1) (local entries h0, x0 count from P's own lists); false when some
@@ -724,7 +733,7 @@ static bool build_block_plan(const HostPack &host, int depth, int cap, BlockPlan
   parallel_for(nc, [&](int64_t c) {
     if (tangle) return;
     if (!tile_range(host, depth, cap, c * chunk, std::min(N, (c + 1) * chunk), part[c])) tangle = true;
-  });
+  }, plan_threads(N));
   if (tangle) return false;
   size_t nt = 0, nh = 0, nx = 0;
   for (int64_t c = 0; c < nc; c++) {

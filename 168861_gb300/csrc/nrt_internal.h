@@ -91,11 +91,11 @@ inline unsigned host_threads() {
 }
 
 // Runs f(i) for every i in [0, n) on the host's cores, handing out indices one at a time
-// (instances differ in size by orders of magnitude).  The first exception of a thread ends the loop
-// and is thrown again here, in the caller's thread.
+// (instances differ in size by orders of magnitude), at most `threads` of them.  The first exception
+// of a thread ends the loop and is thrown again here, in the caller's thread.
 template <class F>
-void parallel_for(int64_t n, F f) {
-  const unsigned nt = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)host_threads(), n));
+void parallel_for(int64_t n, F f, unsigned threads = host_threads()) {
+  const unsigned nt = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)threads, n));
   std::atomic<int64_t> next(0);
   std::atomic<bool> failed(false);
   std::exception_ptr error;
